@@ -238,7 +238,7 @@ class Engine {
   void RankerTrain();
   void RankerFinishIteration();
   void LaunchPrepare(const BlockPlan& bp);
-  bool RowSumsOn(const BlockPlan& bp) const;
+  bool RowSumsOn() const;
   void PlanOnDevice();
   void SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nbig, long long max_mat, long long max_slots);
   void PrepareIterationBuffers();
@@ -325,11 +325,9 @@ class Engine {
   DevBuf<int> d_real_;
   std::vector<long long> h_cand_off_, h_sel_off_, h_mat_off_;
   std::vector<BlockPlan> plans_;  // this iteration's blocks
-  // per-row sums of a one-block iteration's block-start state (exact gain
-  // from the shared neighbours only)
-  DevBuf<long long> d_rc_before_, d_rc_light_;
-  DevBuf<int4> d_rc_heavy_;
-  DevBuf<int> d_rc_nheavy_;
+  // sums of a block's start state that the exact gains are made from: per row,
+  // and per candidate slot
+  DevBuf<unsigned char> d_rc_, d_info_;
   bool plan_on_device_ = false;
   int accum_grid_ = 152 * 4;  // resident CTAs of the dynamically scheduled kernels
   int score_grid_ = 152 * 4;   // one-block iteration: Merge plans it on the device

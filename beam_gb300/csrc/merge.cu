@@ -190,44 +190,188 @@ __device__ void WarpExactGain(const QuotientView& Q, int a, int b, long long* ga
   }
 }
 
-// Per-row sums of the block-start state, for WarpExactGainShared:
-//   before[r] = sum over the row of BlockCost(size_r, size_x, c_rx),
-//   light[r]  = sum of c_rx over the row's light entries,
-// where an entry is light when 1 + (size_r + 1) * size_x >= 2 c_rx: its
-// after-merge term min(c, 1 + s * size_x - c) is c for every merged size
-// s >= size_r + 1. The positions of the heavy entries are kept when there
-// are at most kHeavyMax of them; a row with more is scored by the full merge.
-constexpr int kHeavyMax = 4;
-
-struct RowConsts {
-  const long long* before;
-  const long long* light;
-  const int4* heavy;   // positions of the heavy entries, -1 unused
-  const int* nheavy;   // heavy entries of the row
+// The exact gain from sums. The gain
+// of a pair is a sum over the union of its two rows. The prepare kernels read
+// every member row with its target sizes anyway, and visit every target that
+// two members share, so they leave behind all that the gain needs: sums per
+// row (RowSums) and the shared targets' part per candidate (PairInfo). The
+// scoring pass then reads no row at all.
+//
+// With s = size_a + size_b and f_s(c) = min(c, 1 + s * size_x - c):
+//   before = before[a] + before[b] - BC(s_b, s_a, e_ab) + BC_int(a) + BC_int(b)
+//   after  = F_a(s) + F_b(s) - BC(s, s_b, e_ab) - BC(s, s_a, e_ab) + shared
+//            + BC_int(s, i_a + i_b + e_ab),
+//   F_r(s) = sum over row r of f_s(c),
+//   shared = sum over shared x of [f_s(c_ax + c_bx) - f_s(c_ax) - f_s(c_bx)]:
+// the integers of QuotientGraph::ExactMergeGainPersistentImpl, regrouped.
+//
+// F_r(s) without the row: an entry is light when 1 + (size_r + 1) * size_x >=
+// 2c, so f_s(c) = c for every merged size; of the others (heavy) each is
+// dense, f_s(c) = 1 + s * size_x - c, up to its own size limit
+// (2c - 2) / size_x, and c beyond. smin / smax are the least and the largest of
+// those limits: for s <= smin all heavy entries are dense, for s > smax none.
+// Sizes in between (rows with several heavy entries of different limits) read
+// the row.
+constexpr int kHeavyFew = 4;
+struct __align__(64) RowSums {
+  long long before;    // sum of BC(size_r, size_x, c)
+  long long light;     // sum of c over the light entries
+  long long heavy_sx;  // over the heavy entries: sum of size_x
+  long long heavy_c;   //                         sum of c
+  int smin, smax;      //                         least / largest size limit
+  long long internal;  // internal edges of the supernode
+  int size, len;
+  int nheavy;          // heavy entries
+  int sbad;            // a size below this holds fewer edges than some entry counts (0: none does)
 };
+static_assert(sizeof(RowSums) == 64, "two sectors per row");
 
-// Row sums are written by the prepare kernels, which read every member row
-// of the block's groups with the target sizes anyway.
 __device__ __forceinline__ bool HeavyEntry(long long size_r, long long size_x, long long c) {
   return 1 + (size_r + 1) * size_x < 2 * c;
 }
 
-// Warp-uniform call per 32-entry step of a row: records the positions of the
-// step's heavy entries after the nh found so far.
-__device__ __forceinline__ void RecordHeavy(int4* slot, int& nh, bool heavy, int k) {
-  const int lane = threadIdx.x & 31;
-  const unsigned hm = __ballot_sync(0xffffffffu, heavy);
-  if (heavy) {
-    const int rank = nh + __popc(hm & ((1u << lane) - 1u));
-    if (rank < kHeavyMax) reinterpret_cast<int*>(slot)[rank] = k;
-  }
-  nh += __popc(hm);
+__device__ __forceinline__ int HeavyLimit(long long size_x, long long c) {
+  const long long l = (2 * c - 2) / size_x;
+  return l > 0x7fffffffll ? 0x7fffffff : static_cast<int>(l);
 }
 
-// Skewed pairs (the long row at least kProbeMinLong entries and kProbeRatio
-// times the short one) look the short row up in the long one.
-constexpr int kProbeMinLong = 256;
-constexpr int kProbeRatio = 8;
+// Least size whose block with a target of size_x holds cnt edges. An entry
+// beyond its own block's capacity is always heavy.
+__device__ __forceinline__ int HeavyNeed(long long size_x, long long cnt) {
+  const long long n = (cnt + size_x - 1) / size_x;
+  return n > 0x7fffffffll ? 0x7fffffff : static_cast<int>(n);
+}
+
+// The heavy part of a row's sums; one lane's share, then the warp's.
+struct HeavyAcc {
+  long long sx = 0, c = 0;
+  int smin = 0x7fffffff, smax = 0, n = 0, sbad = 0;
+  __device__ __forceinline__ void Add(long long size_x, long long cnt) {
+    const int l = HeavyLimit(size_x, cnt);
+    const int need = HeavyNeed(size_x, cnt);
+    sbad = need > sbad ? need : sbad;
+    sx += size_x;
+    c += cnt;
+    smin = l < smin ? l : smin;
+    smax = l > smax ? l : smax;
+    ++n;
+  }
+  __device__ __forceinline__ void Merge(const HeavyAcc& o) {
+    sx += o.sx;
+    c += o.c;
+    smin = o.smin < smin ? o.smin : smin;
+    smax = o.smax > smax ? o.smax : smax;
+    sbad = o.sbad > sbad ? o.sbad : sbad;
+    n += o.n;
+  }
+  __device__ __forceinline__ void WarpReduce() {
+    n = WarpSumInt(n);
+    if (n == 0) return;
+    sx = WarpSum(sx);
+    c = WarpSum(c);
+    smin = __reduce_min_sync(0xffffffffu, smin);
+    smax = __reduce_max_sync(0xffffffffu, smax);
+    sbad = __reduce_max_sync(0xffffffffu, sbad);
+  }
+};
+
+__device__ __forceinline__ void StoreRowSums(RowSums* out, long long before, long long light, const HeavyAcc& h,
+                                             long long internal, int size, int len) {
+  RowSums r;
+  r.before = before;
+  r.light = light;
+  r.heavy_sx = h.sx;
+  r.heavy_c = h.c;
+  r.smin = h.smin;
+  r.smax = h.smax;
+  r.internal = internal;
+  r.size = size;
+  r.len = len;
+  r.nheavy = h.n;
+  r.sbad = h.sbad;
+  *out = r;
+}
+
+__device__ __forceinline__ bool RowAfterKnown(const RowSums& r, long long s) {
+  return r.nheavy == 0 || s <= r.smin || s > r.smax;
+}
+
+// F_r(s) from the sums; false: the row has to be read (WarpRowAfter); *out is its light part then.
+__device__ __forceinline__ bool RowAfter(const RowSums& r, long long s, long long* out) {
+  *out = r.light;
+  if (r.nheavy == 0) return true;
+  if (s <= r.smin) {
+    *out += r.nheavy + s * r.heavy_sx - r.heavy_c;
+    return true;
+  }
+  if (s > r.smax) {
+    *out += r.heavy_c;
+    return true;
+  }
+  return false;
+}
+
+// Sum of f_s(c) over row r, by a warp.
+__device__ long long WarpRowAfter(const QuotientView& Q, int r, long long s) {
+  const int lane = threadIdx.x & 31;
+  const Entry* row = Q.ent + Q.off[r];
+  const int len = Q.len[r];
+  long long sum = 0;
+  for (int k = lane; k < len; k += 32) {
+    const Entry e = row[k];
+    const long long c = EntCnt(e);
+    const long long alt = 1 + s * Q.size[EntNb(e)] - c;
+    sum += c < alt ? c : alt;
+  }
+  return WarpSum(sum);
+}
+
+// The shared part of a candidate pair.
+struct __align__(16) PairInfo {
+  long long shared;  // sum over the shared targets (see above)
+  unsigned ovl;      // shared targets (low 30 bits) and the flags below
+  unsigned eab;      // edges between the two
+};
+constexpr unsigned kPairBad = 1u << 31;   // a shared target's count exceeds its block capacity
+constexpr unsigned kPairAsym = 1u << 30;  // the two rows disagree about e(a, b)
+
+// The pair tables of a big group (g x g words, row-major). Word (i, j), i < j:
+// the EA proxy in the low kProxyBits, the number of shared targets above it,
+// bit 62 set when row i lists j, bit 63 when row j lists i. Word (j, i): the
+// shared part plus the proxy's own (shared = that word - proxy of the targets),
+// zero unless a target of the pair is dense in one of the rows; a target whose
+// count exceeds the merged block adds kCorrBad instead. A proxy is at most the
+// two rows' counts plus the direct edges, below 2^34 (edges < 2^32); shared
+// targets are counted only with row sums, on graphs of fewer than 2^30 arcs:
+// two rows share fewer than 2^28 targets there.
+constexpr int kProxyBits = 34;
+constexpr unsigned long long kProxyMask = (1ull << kProxyBits) - 1;
+constexpr unsigned long long kOvlOne = 1ull << kProxyBits;
+constexpr unsigned long long kOvlMask = (1ull << (62 - kProxyBits)) - 1;
+constexpr unsigned long long kRowILists = 1ull << 62;
+constexpr unsigned long long kRowJLists = 1ull << 63;
+constexpr long long kCorrBad = 1ll << 36;
+constexpr long long kFusedMaxArcs = 1ll << 30;
+
+// One target of size st shared by members of sizes sa and sb with counts ca
+// and cb: the EA proxy's term max(0, old - new) (src/sweg.cpp:1598-1727) and
+// corr = f(ca + cb) - f(ca) - f(cb) + that term.
+struct SharedTerm {
+  long long delta, corr;
+};
+
+__device__ __forceinline__ SharedTerm TermOf(long long sa, long long sb, long long st, long long ca, long long cb,
+                                             bool* bad) {
+  auto mn = [](long long x, long long y) { return x < y ? x : y; };
+  const long long cap_a = sa * st, cap_b = sb * st, cap = cap_a + cap_b, c = ca + cb;
+  const long long ga = mn(ca, 1 + cap_a - ca), gb = mn(cb, 1 + cap_b - cb), f = mn(c, 1 + cap - c);
+  const long long d = ga + gb - f;
+  SharedTerm t;
+  t.delta = d > 0 ? d : 0;
+  t.corr = f - mn(ca, 1 + cap - ca) - mn(cb, 1 + cap - cb) + t.delta;
+  *bad = c > cap;
+  return t;
+}
 
 // The last index i of [lo, hi) with a[i] <= x, for a non-decreasing array
 // with a[lo] <= x, found by the whole warp (warp-uniform arguments): each
@@ -245,190 +389,6 @@ __device__ __forceinline__ int WarpLastLE(const long long* __restrict__ a, int l
     if (k < 32) hi = p_hi;
   }
   return lo;
-}
-
-// First position of a sorted row whose neighbour is >= x.
-__device__ __forceinline__ int RowLowerBound(const Entry* row, int len, int x) {
-  int lo = 0, hi = len;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (EntNb(row[mid]) < x) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
-// ExactMergeGainPersistentImpl from the row sums: with s = size_a + size_b,
-//   before = before[a] + before[b] - BC(s_b, s_a, e_ab) + BC_int(a) + BC_int(b)
-//   after  = F_a(s) + F_b(s) - BC(s, s_b, e_ab) - BC(s, s_a, e_ab)
-//            + sum over shared x of [BC(s, s_x, c_ax + c_bx) - BC(s, s_x, c_ax) - BC(s, s_x, c_bx)]
-//            + BC_int(s, i_a + i_b + e_ab),
-// F_r(s) = light[r] + the heavy entries' exact terms. Only the shared
-// neighbours need sizes and cost terms; the tiled merge that finds them is
-// the one of WarpExactGain. The same integers as the full merge, term by
-// term regrouped.
-// The scalars of one row that the row-sum gain reads: staged in shared memory
-// by the scoring warp for a whole fetch of pairs at once (independent loads,
-// one latency for all of them), then read by every lane as broadcasts.
-struct RowMeta {
-  long long off, internal, before, light;
-  int4 heavy;
-  int len, size, nheavy;
-  int rep;  // the row's supernode
-};
-
-__device__ __forceinline__ void LoadRowMeta(const QuotientView& Q, const RowConsts& RC, int r, RowMeta* m) {
-  RowMeta v;
-  v.off = Q.off[r];
-  v.internal = Q.internal[r];
-  v.before = RC.before[r];
-  v.light = RC.light[r];
-  v.heavy = RC.heavy[r];
-  v.len = Q.len[r];
-  v.size = Q.size[r];
-  v.nheavy = RC.nheavy[r];
-  v.rep = r;
-  *m = v;
-}
-
-__device__ void WarpExactGainShared(const QuotientView& Q, int a, int b, const RowMeta& A, const RowMeta& B,
-                                    long long* gain_out, long long* before_out, GainWork* work, DevError* err) {
-  constexpr unsigned kFull = 0xffffffffu;
-  constexpr Entry kPadEntry = static_cast<Entry>(0x7fffffffull) << 32;
-  const int ha = A.nheavy;
-  const int hb = B.nheavy;
-  if (ha > kHeavyMax || hb > kHeavyMax) {
-    WarpExactGain(Q, a, b, gain_out, before_out, work, err);
-    return;
-  }
-  const int lane = threadIdx.x & 31;
-  const long long sa = A.size;
-  const long long sb = B.size;
-  const long long sw = sa + sb;
-  const Entry* ra = Q.ent + A.off;
-  const Entry* rb = Q.ent + B.off;
-  const int la = A.len;
-  const int lb = B.len;
-  long long shared = 0, eab_a = 0, eab_b = 0;
-  int ovl = 0, bad = 0;
-  const bool a_long = la >= lb;
-  const int ll = a_long ? la : lb;
-  const int ls = a_long ? lb : la;
-  const bool probe = ll >= kProbeMinLong && ll >= kProbeRatio * ls;
-  if (probe) {
-    // skewed pair: each entry of the short row is looked up in the long row
-    // by binary search instead of streaming the long row
-    const Entry* rl = a_long ? ra : rb;
-    const Entry* rs = a_long ? rb : ra;
-    const int long_rep = a_long ? a : b;
-    const int short_rep = a_long ? b : a;
-    long long e_long = 0, e_short = 0;  // e(a, b) as read from the long / the short row
-    for (int k0 = 0; k0 < ls; k0 += 32) {
-      const int k = k0 + lane;
-      if (k < ls) {
-        const Entry e = rs[k];
-        const int x = EntNb(e);
-        const long long cs = EntCnt(e);
-        if (x == long_rep) {
-          e_short = cs;
-        } else {
-          const int at = RowLowerBound(rl, ll, x);
-          if (at < ll && EntNb(rl[at]) == x) {
-            const long long cl = EntCnt(rl[at]);
-            const long long ca = a_long ? cl : cs;
-            const long long cb = a_long ? cs : cl;
-            const long long sx = Q.size[x];
-            shared += BlockCost(sw, sx, ca + cb, false, bad) - BlockCost(sw, sx, ca, false, bad) -
-                      BlockCost(sw, sx, cb, false, bad);
-            ++ovl;
-          }
-        }
-      }
-    }
-    if (lane == 0) {
-      const int at = RowLowerBound(rl, ll, short_rep);
-      if (at < ll && EntNb(rl[at]) == short_rep) e_long = EntCnt(rl[at]);
-    }
-    eab_a = a_long ? e_long : e_short;
-    eab_b = a_long ? e_short : e_long;
-  }
-  // otherwise the tiled merge of the two rows
-  int pa = probe ? la : 0;
-  int pb = probe ? lb : 0;
-  while (pa < la || pb < lb) {
-    const bool va = pa + lane < la;
-    const bool vb = pb + lane < lb;
-    const Entry ea_e = va ? ra[pa + lane] : kPadEntry;
-    const Entry eb_e = vb ? rb[pb + lane] : kPadEntry;
-    const int xa = EntNb(ea_e);
-    const int xb = EntNb(eb_e);
-    const int last_a = __shfl_sync(kFull, xa, 31);
-    const int last_b = __shfl_sync(kFull, xb, 31);
-    const int lim = last_a < last_b ? last_a : last_b;
-    int pos_b = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-      const int probe_b = __shfl_sync(kFull, xb, pos_b + step - 1);
-      if (probe_b < xa) pos_b += step;
-    }
-    const Entry cand_b = __shfl_sync(kFull, eb_e, pos_b);
-    const bool fin_a = va && xa <= lim;
-    const bool fin_b = vb && xb <= lim;
-    if (fin_a) {
-      if (xa == b) {
-        eab_a = EntCnt(ea_e);
-      } else if (EntNb(cand_b) == xa) {
-        const long long ca = EntCnt(ea_e);
-        const long long cb = EntCnt(cand_b);
-        const long long sx = Q.size[xa];
-        shared += BlockCost(sw, sx, ca + cb, false, bad) - BlockCost(sw, sx, ca, false, bad) -
-                  BlockCost(sw, sx, cb, false, bad);
-        ++ovl;
-      }
-    }
-    if (fin_b && xb == a) eab_b = EntCnt(eb_e);
-    pa += __popc(__ballot_sync(kFull, fin_a));
-    pb += __popc(__ballot_sync(kFull, fin_b));
-  }
-  // heavy entries: lanes 0..3 of row a, lanes 4..7 of row b
-  long long heavy_a = 0, heavy_b = 0;
-  if (lane < 2 * kHeavyMax) {
-    const bool on_a = lane < kHeavyMax;
-    const int h = on_a ? lane : lane - kHeavyMax;
-    if (h < (on_a ? ha : hb)) {
-      const int4 hp = on_a ? A.heavy : B.heavy;
-      const int pos = h == 0 ? hp.x : h == 1 ? hp.y : h == 2 ? hp.z : hp.w;
-      const Entry e = (on_a ? ra : rb)[pos];
-      const long long term = BlockCost(sw, Q.size[EntNb(e)], EntCnt(e), false, bad);
-      (on_a ? heavy_a : heavy_b) = term;
-    }
-  }
-  // one 64-bit sum; e(a,b) is read by one lane per row (counts < 2^32)
-  shared = WarpSum(shared + heavy_a + heavy_b);
-  eab_a = __reduce_max_sync(kFull, static_cast<unsigned>(eab_a));
-  eab_b = __reduce_max_sync(kFull, static_cast<unsigned>(eab_b));
-  ovl = static_cast<int>(__reduce_add_sync(kFull, static_cast<unsigned>(ovl)));
-  bad = __any_sync(kFull, bad);
-  if (eab_a != eab_b) {
-    if (lane == 0) RaiseError(err, kErrAsymmetric, a, b, 0);
-  }
-  const long long ia = A.internal;
-  const long long ib = B.internal;
-  const long long before = A.before + B.before - BlockCost(sb, sa, eab_b, false, bad) +
-                           BlockCost(sa, sa, ia, true, bad) + BlockCost(sb, sb, ib, true, bad);
-  const long long after = A.light + B.light - BlockCost(sw, sb, eab_a, false, bad) -
-                          BlockCost(sw, sa, eab_b, false, bad) + shared +
-                          BlockCost(sw, sw, ia + ib + eab_a, true, bad);
-  if (bad && lane == 0) RaiseError(err, kErrBlockCost, a, b, 0);
-  *gain_out = before - after;
-  *before_out = before;
-  if (work) {
-    work->raw_a += la;
-    work->raw_b += lb;
-    work->uni += (la - (eab_a > 0 ? 1 : 0)) + (lb - (eab_b > 0 ? 1 : 0)) - ovl;
-    work->ovl += ovl;
-    // 8 B per row entry, 4 B per shared-neighbour size gather, 36 B of row sums
-    work->bytes += 8ll * (la + lb) + 4ll * ovl + 36;
-  }
 }
 
 // ------------------------------------------------------------ prepare
@@ -502,11 +462,9 @@ struct PrepareParams {
   const long long* mat_off;
   unsigned char* mat;
   int mat_zeroed;  // the pair tables were cleared by one memset of the block
-  // row sums for the scoring pass (rc_before == nullptr: not needed)
-  long long* rc_before;
-  long long* rc_light;
-  int4* rc_heavy;
-  int* rc_nheavy;
+  // row sums and pair sums for the scoring pass (nullptr: not needed)
+  RowSums* rc;
+  PairInfo* info;
   unsigned char* scratch;
   unsigned long long scratch_cap;
   BlockCtl* ctl;
@@ -515,7 +473,7 @@ struct PrepareParams {
   DevError* err;
 };
 
-// Per big group: proxy int64[g*g] | kept flag u8[g*g] | old cost int64[g];
+// Per big group: pair words u64[g*g] | kept flag u8[g*g] | old cost int64[g];
 // the flag table starts at FlagOffset and the old costs at OldCostOffset
 // (rounded up to 8-byte alignment).
 __host__ __device__ __forceinline__ long long FlagOffset(long long gg) { return 8 * gg; }
@@ -574,6 +532,40 @@ __device__ __forceinline__ bool RatioAtLeast(long long gain, long long before, d
 
 __device__ __forceinline__ unsigned BucketHash(int t, unsigned mask) {
   return (static_cast<unsigned>(t) * 0x9E3779B1u) >> 7 & mask;
+}
+
+// Adds a shared target (size st; counts ca, cb in the rows of members i, j) to
+// the pair's words: one atomic, and a second one where a dense entry is part
+// of it. counted: the shared part of the gain is wanted too.
+__device__ __forceinline__ void AddShared(unsigned long long* pmat, int g, int i, int j, long long si, long long sj,
+                                          long long st, long long ca, long long cb, bool counted) {
+  bool bad;
+  const SharedTerm t = TermOf(si, sj, st, ca, cb, &bad);
+  const long long lo = i < j ? i : j;
+  const long long hi = i < j ? j : i;
+  const unsigned long long add = static_cast<unsigned long long>(t.delta) + (counted ? kOvlOne : 0ull);
+  if (add != 0) atomicAdd(&pmat[lo * g + hi], add);
+  if (counted && (t.corr != 0 || bad)) {
+    atomicAdd(&pmat[hi * g + lo], static_cast<unsigned long long>(bad ? kCorrBad : t.corr));
+  }
+}
+
+// Member i's row lists member j with c edges: counted once, from the lower
+// index; the other side leaves its mark.
+__device__ __forceinline__ void AddDirect(unsigned long long* pmat, int g, int i, int j, long long c) {
+  if (i < j) {
+    atomicAdd(&pmat[static_cast<long long>(i) * g + j], static_cast<unsigned long long>(c) | kRowILists);
+  } else {
+    atomicAdd(&pmat[static_cast<long long>(j) * g + i], kRowJLists);
+  }
+}
+
+__device__ __forceinline__ unsigned long long PairWord(const unsigned long long* pmat, int g, int i, int j) {
+  return i < j ? pmat[static_cast<long long>(i) * g + j] : pmat[static_cast<long long>(j) * g + i];
+}
+
+__device__ __forceinline__ long long ProxyOf(unsigned long long word) {
+  return static_cast<long long>(word & kProxyMask);
 }
 
 struct PrepSmem {
@@ -658,7 +650,7 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareKernel(PrepareParams P) {
   if (tid == 0) S.eoff[g] = E;
   const long long gg = static_cast<long long>(g) * g;
   unsigned char* mat = P.mat + P.mat_off[ri];
-  long long* pmat = reinterpret_cast<long long*>(mat);
+  unsigned long long* pmat = reinterpret_cast<unsigned long long*>(mat);
   unsigned char* fmat = mat + FlagOffset(gg);
   if (slots > 0) {
     // deferred group: row offsets and member scalars in block scratch, pair
@@ -689,13 +681,8 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareKernel(PrepareParams P) {
       const long long si = S.sz[i];
       const long long internal = Q.internal[S.q[i]];
       old_out[i] = internal > 0 ? EncodeCostForPair(S.q[i], si, S.q[i], si, 2 * internal) : 0;
-      if (P.rc_before) {
-        // the fill pass adds the row sums
-        P.rc_before[S.q[i]] = 0;
-        P.rc_light[S.q[i]] = 0;
-        P.rc_nheavy[S.q[i]] = 0;
-        P.rc_heavy[S.q[i]] = make_int4(-1, -1, -1, -1);
-      }
+      // the fill pass adds the row's entries
+      if (P.rc) StoreRowSums(&P.rc[S.q[i]], 0, 0, HeavyAcc(), internal, S.sz[i], S.len[i]);
     }
     if (tid == 0) V.eoff[g] = E;
     if (!P.mat_zeroed) {
@@ -745,39 +732,28 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareKernel(PrepareParams P) {
     const int len = S.len[i];
     const int eo = S.eoff[i];
     long long old = 0, light = 0;
-    int nh = 0;
-    if (P.rc_before && lane == 0) P.rc_heavy[rep] = make_int4(-1, -1, -1, -1);
-    __syncwarp();
-    for (int k0 = 0; k0 < len; k0 += 32) {
-      const int k = k0 + lane;
-      bool heavy = false;
-      if (k < len) {
-        const Entry e = row[k];
-        const int t = EntNb(e);
-        const long long c = EntCnt(e);
-        const long long st = Q.size[t];
-        old += EncodeCostForPair(rep, si, t, st, c);
-        heavy = HeavyEntry(si, st, c);
-        if (!heavy) light += c;
-        et[eo + k] = t;
-        ei[eo + k] = i;
-        ee[eo + k] = static_cast<unsigned>(c);
-        enx[eo + k] = atomicExch(&heads[BucketHash(t, hmask)], eo + k);
-        // direct in-group edge: row i holds j and row j holds i with the same
-        // count, so each half of the table gets it once
-        if (P.group_of[t] == gid) pmat[static_cast<long long>(i) * g + P.idx_in_group[t]] = c;
-      }
-      if (P.rc_before) RecordHeavy(P.rc_heavy + rep, nh, heavy, k);
+    HeavyAcc heavy;
+    for (int k = lane; k < len; k += 32) {
+      const Entry e = row[k];
+      const int t = EntNb(e);
+      const long long c = EntCnt(e);
+      const long long st = Q.size[t];
+      old += EncodeCostForPair(rep, si, t, st, c);
+      if (HeavyEntry(si, st, c)) heavy.Add(st, c); else light += c;
+      et[eo + k] = t;
+      ei[eo + k] = i;
+      ee[eo + k] = static_cast<unsigned>(c);
+      enx[eo + k] = atomicExch(&heads[BucketHash(t, hmask)], eo + k);
+      if (P.group_of[t] == gid) AddDirect(pmat, g, i, P.idx_in_group[t], c);
     }
     old = WarpSum(old);
-    if (P.rc_before) light = WarpSum(light);
+    if (P.rc) {
+      light = WarpSum(light);
+      heavy.WarpReduce();
+    }
     if (lane == 0) {
-      if (P.rc_before) {
-        P.rc_before[rep] = old;
-        P.rc_light[rep] = light;
-        P.rc_nheavy[rep] = nh;
-      }
       const long long internal = Q.internal[rep];
+      if (P.rc) StoreRowSums(&P.rc[rep], old, light, heavy, internal, S.sz[i], len);
       if (internal > 0) old += EncodeCostForPair(rep, si, rep, si, 2 * internal);
       S.old[i] = old;
     }
@@ -794,25 +770,8 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareKernel(PrepareParams P) {
       if (et[k] != t) continue;
       if (st < 0) st = Q.size[t];
       const int j = ei[k];
-      const int a = i < j ? i : j;
-      const int b = i < j ? j : i;
-      const long long ea = a == i ? c : static_cast<long long>(ee[k]);
-      const long long eb = a == i ? static_cast<long long>(ee[k]) : c;
-      const long long sa = S.sz[a];
-      const long long sb = S.sz[b];
-      const int qa = S.q[a];
-      const int qb = S.q[b];
       ++examined;
-      const long long oldc = EncodeCostForPair(qa, sa, t, st, ea) + EncodeCostForPair(qb, sb, t, st, eb);
-      const long long newc = EncodeCostForPair(qa, sa + sb, t, st, ea + eb);
-      const long long delta = oldc - newc;
-      if (delta > 0) {
-        // both halves, so every member's partners are one contiguous row
-        atomicAdd(reinterpret_cast<unsigned long long*>(&pmat[static_cast<long long>(a) * g + b]),
-                  static_cast<unsigned long long>(delta));
-        atomicAdd(reinterpret_cast<unsigned long long*>(&pmat[static_cast<long long>(b) * g + a]),
-                  static_cast<unsigned long long>(delta));
-      }
+      AddShared(pmat, g, i, j, S.sz[i], S.sz[j], st, c, static_cast<long long>(ee[k]), P.rc != nullptr);
     }
   }
   examined = WarpSum(static_cast<long long>(examined));
@@ -870,6 +829,7 @@ __global__ void __launch_bounds__(kFillThreads) PrepareFillKernel(PrepareParams 
       long long run = -1;  // (group, member) of this lane's entry, -1 none
       long long cost = 0, light = 0;
       int rep = -1;
+      HeavyAcc heavy;
       if (s < P.nslots) {
         const int k0 = k;
         while (k + 1 < P.nlist && P.soff[P.list0 + k + 1] - P.slot0 <= s) ++k;
@@ -896,20 +856,14 @@ __global__ void __launch_bounds__(kFillThreads) PrepareFillKernel(PrepareParams 
           const long long c = EntCnt(e);
           const long long st = Q.size[t];
           cost = EncodeCostForPair(rep, V.msz[i], t, st, c);
-          if (P.rc_before) {
-            if (HeavyEntry(V.msz[i], st, c)) {
-              const int rank = atomicAdd(&P.rc_nheavy[rep], 1);
-              if (rank < kHeavyMax) reinterpret_cast<int*>(&P.rc_heavy[rep])[rank] = static_cast<int>(idx - e0);
-            } else {
-              light = c;
-            }
+          if (P.rc) {
+            if (HeavyEntry(V.msz[i], st, c)) heavy.Add(st, c); else light = c;
           }
           const long long slot = P.soff[P.list0 + k] - P.slot0 + idx;
           P.skey[slot] = (static_cast<unsigned long long>(k) << P.tbits) | static_cast<unsigned>(t);
           P.sval[slot] = static_cast<unsigned long long>(i) << 32 | static_cast<unsigned long long>(c);
           if (P.group_of[t] == gid) {
-            long long* pmat = reinterpret_cast<long long*>(P.mat + P.mat_off[ri]);
-            pmat[static_cast<long long>(i) * g + P.idx_in_group[t]] = c;
+            AddDirect(reinterpret_cast<unsigned long long*>(P.mat + P.mat_off[ri]), g, i, P.idx_in_group[t], c);
           }
           run = (static_cast<long long>(k) << 11) | i;
         }
@@ -931,9 +885,32 @@ __global__ void __launch_bounds__(kFillThreads) PrepareFillKernel(PrepareParams 
         unsigned long long* old_out =
             reinterpret_cast<unsigned long long*>(P.mat + P.mat_off[ri] + OldCostOffset(static_cast<long long>(g) * g));
         if (cost != 0) atomicAdd(&old_out[i], static_cast<unsigned long long>(cost));
-        if (P.rc_before) {
-          if (cost != 0) atomicAdd(reinterpret_cast<unsigned long long*>(&P.rc_before[rep]), static_cast<unsigned long long>(cost));
-          if (light != 0) atomicAdd(reinterpret_cast<unsigned long long*>(&P.rc_light[rep]), static_cast<unsigned long long>(light));
+        if (P.rc) {
+          if (cost != 0) atomicAdd(reinterpret_cast<unsigned long long*>(&P.rc[rep].before), static_cast<unsigned long long>(cost));
+          if (light != 0) atomicAdd(reinterpret_cast<unsigned long long*>(&P.rc[rep].light), static_cast<unsigned long long>(light));
+        }
+      }
+      // heavy entries: the run's lanes by segmented scans too, where there are any
+      if (__any_sync(0xffffffffu, heavy.n != 0)) {
+        for (int o = 1; o < 32; o <<= 1) {
+          const long long vr = __shfl_up_sync(0xffffffffu, run, o);
+          HeavyAcc v;
+          v.sx = __shfl_up_sync(0xffffffffu, heavy.sx, o);
+          v.c = __shfl_up_sync(0xffffffffu, heavy.c, o);
+          v.smin = __shfl_up_sync(0xffffffffu, heavy.smin, o);
+          v.smax = __shfl_up_sync(0xffffffffu, heavy.smax, o);
+          v.sbad = __shfl_up_sync(0xffffffffu, heavy.sbad, o);
+          v.n = __shfl_up_sync(0xffffffffu, heavy.n, o);
+          if (lane >= o && vr == run) heavy.Merge(v);
+        }
+        if (run >= 0 && (lane == 31 || next_run != run) && heavy.n != 0) {
+          RowSums* r = &P.rc[rep];
+          atomicAdd(reinterpret_cast<unsigned long long*>(&r->heavy_sx), static_cast<unsigned long long>(heavy.sx));
+          atomicAdd(reinterpret_cast<unsigned long long*>(&r->heavy_c), static_cast<unsigned long long>(heavy.c));
+          atomicMin(&r->smin, heavy.smin);
+          atomicMax(&r->smax, heavy.smax);
+          atomicMax(&r->sbad, heavy.sbad);
+          atomicAdd(&r->nheavy, heavy.n);
         }
       }
     }
@@ -946,12 +923,11 @@ __global__ void __launch_bounds__(kFillThreads) PrepareFillKernel(PrepareParams 
 // run; each lane pairs its entry with the earlier entries of its run: those
 // in its own chunk by shuffles, and, for the run that reaches back past the
 // chunk's start, those of the earlier chunks, 32 at a time. Every member pair
-// sharing a target is visited once and adds proxy += max(0, old - new) to
-// both halves of the pair table.
+// sharing a target is visited once and added to the pair's words (AddShared).
 struct RunEntry {
   unsigned long long key;
-  long long c, s;  // edge count to the target, member size
-  int i, q;        // member index, member supernode
+  long long c;  // edge count to the target
+  int i, s;     // member index, member size
 };
 
 __device__ __forceinline__ RunEntry LoadRunEntry(const PrepareParams& P, long long p, const DeferredView& V) {
@@ -960,7 +936,6 @@ __device__ __forceinline__ RunEntry LoadRunEntry(const PrepareParams& P, long lo
   r.i = static_cast<int>(v >> 32);
   r.c = static_cast<long long>(v & 0xffffffffu);
   r.s = V.msz[r.i];
-  r.q = V.mq[r.i];
   return r;
 }
 
@@ -970,22 +945,7 @@ __device__ __forceinline__ RunEntry ShflRunEntry(const RunEntry& r, int src) {
   o.c = __shfl_sync(0xffffffffu, r.c, src);
   o.s = __shfl_sync(0xffffffffu, r.s, src);
   o.i = __shfl_sync(0xffffffffu, r.i, src);
-  o.q = __shfl_sync(0xffffffffu, r.q, src);
   return o;
-}
-
-__device__ __forceinline__ void AccumPair(const RunEntry& a, const RunEntry& b, int t, long long st, int g,
-                                          long long* pmat, unsigned long long& examined) {
-  ++examined;
-  const long long oldc = EncodeCostForPair(a.q, a.s, t, st, a.c) + EncodeCostForPair(b.q, b.s, t, st, b.c);
-  const long long newc = EncodeCostForPair(a.q, a.s + b.s, t, st, a.c + b.c);
-  const long long delta = oldc - newc;
-  if (delta > 0) {
-    atomicAdd(reinterpret_cast<unsigned long long*>(&pmat[static_cast<long long>(a.i) * g + b.i]),
-              static_cast<unsigned long long>(delta));
-    atomicAdd(reinterpret_cast<unsigned long long*>(&pmat[static_cast<long long>(b.i) * g + a.i]),
-              static_cast<unsigned long long>(delta));
-  }
 }
 
 // kAccumSplit warps share a chunk: warp y pairs the chunk with the earlier
@@ -1003,6 +963,7 @@ constexpr int kAccumFetch = 8;
 __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PrepareParams P) {
   const int lane = threadIdx.x & 31;
   unsigned long long examined = 0;
+  const bool counted = P.rc != nullptr;
   const long long nchunks = (P.nslots + 31) >> 5;
   const long long ngroups8 = (nchunks + kAccumFetch - 1) / kAccumFetch;
   const long long nfetch = ngroups8 * kAccumSplit;
@@ -1030,23 +991,22 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
     const long long p = p0 + lane;
     RunEntry me;
     me.key = p < P.nslots ? P.skey_sorted[p] : kSlotPad;
-    me.c = me.s = 0;
-    me.i = me.q = 0;
+    me.c = 0;
+    me.s = me.i = 0;
     const bool valid = me.key != kSlotPad && static_cast<int>(me.key >> P.tbits) < P.nlist;
-    int t = 0, g = 0;
+    int g = 0;
     long long st = 0;
-    long long* pmat = nullptr;
+    unsigned long long* pmat = nullptr;
     if (valid) {
       const int bl = static_cast<int>(me.key >> P.tbits);
-      t = static_cast<int>(me.key & ((1ull << P.tbits) - 1ull));
+      const int t = static_cast<int>(me.key & ((1ull << P.tbits) - 1ull));
       const int ri = P.list[P.list0 + bl];
       g = P.glen[P.real[ri]];
-      pmat = reinterpret_cast<long long*>(P.mat + P.mat_off[ri]);
+      pmat = reinterpret_cast<unsigned long long*>(P.mat + P.mat_off[ri]);
       const RunEntry r = LoadRunEntry(P, p, Deferred(P.desc[P.list0 + bl].base, g));
       me.c = r.c;
       me.s = r.s;
       me.i = r.i;
-      me.q = r.q;
       st = P.Q.size[t];
     }
     // pairs inside the chunk: each lane visits the earlier lanes holding its
@@ -1060,7 +1020,8 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
         const int src = earlier != 0u ? __ffs(earlier) - 1 : lane;
         const RunEntry o = ShflRunEntry(me, src);
         if (earlier != 0u) {
-          AccumPair(me, o, t, st, g, pmat, examined);
+          ++examined;
+          AddShared(pmat, g, me.i, o.i, me.s, o.s, st, me.c, o.c, counted);
           earlier &= earlier - 1u;
         }
       }
@@ -1078,12 +1039,15 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
       if (P.skey_sorted[c0 + 31] != first) break;
       RunEntry o;
       o.key = P.skey_sorted[c0 + lane];
-      o.c = o.s = 0;
-      o.i = o.q = 0;
+      o.c = 0;
+      o.s = o.i = 0;
       if (o.key == first) o = [&] { RunEntry r = LoadRunEntry(P, c0 + lane, FV); r.key = first; return r; }();
       for (int src = 0; src < 32; ++src) {
         const RunEntry b = ShflRunEntry(o, src);
-        if (mine && b.key == first) AccumPair(me, b, t, st, g, pmat, examined);
+        if (mine && b.key == first) {
+          ++examined;
+          AddShared(pmat, g, me.i, b.i, me.s, b.s, st, me.c, b.c, counted);
+        }
       }
       // the run continues below this chunk iff its first slot is in the run
       if (c0 < 32ll * kAccumSplit || __shfl_sync(0xffffffffu, o.key, 0) != first) break;
@@ -1096,8 +1060,8 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
 // Top-k partners of member i of a big group whose partners fill NT slots of
 // 32 (the fp32 prescreen branch of PrepareMembersKernel).
 template <int NT>
-__device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int top_k, int cnt, const long long* prow,
-                                            const long long* old, long long old_i, const int* q, int* cj,
+__device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int top_k, int cnt,
+                                            const unsigned long long* pmat, const long long* old, long long old_i, const int* q, int* cj,
                                             unsigned char* fmat) {
   auto ratio_of = [&](int j, long long pg) {
     long long denom = old_i + old[j];
@@ -1117,7 +1081,7 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     const int j = lane + 32 * t;
     float v = 0.0f;  // not a candidate
     if (j < g && j != i) {
-      const long long pg = prow[j];
+      const long long pg = ProxyOf(PairWord(pmat, g, i, j));
       if (pg > 0) {
         long long denom = old_i + old[j];
         if (denom < 1) denom = 1;
@@ -1177,7 +1141,7 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     mine.j = -1;
     if (have) {
       const int j = cj[lane];
-      const long long pg = prow[j];
+      const long long pg = ProxyOf(PairWord(pmat, g, i, j));
       const int qj = q[j];
       mine.j = j;
       mine.rb = ratio_of(j, pg);
@@ -1208,7 +1172,7 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     for (int t = 0; t < NT; ++t) {
       const int j = lane + 32 * t;
       if (rf[t] <= 0.0f || rf[t] < cut) continue;
-      const long long pg = prow[j];
+      const long long pg = ProxyOf(PairWord(pmat, g, i, j));
       RankKey k;
       k.j = j;
       k.rb = ratio_of(j, pg);
@@ -1275,14 +1239,13 @@ __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
   const int* q = P.order + P.gstart[gid];
   const long long gg = static_cast<long long>(g) * g;
   unsigned char* mat = P.mat + P.mat_off[ri];
-  const long long* pmat = reinterpret_cast<const long long*>(mat);
+  const unsigned long long* pmat = reinterpret_cast<const unsigned long long*>(mat);
   unsigned char* fmat = mat + FlagOffset(gg);
   const long long* old = reinterpret_cast<const long long*>(mat + OldCostOffset(gg));
   // per member: candidates with positive proxy, ratio, top-k (the ratio is
   // recomputed where it is needed instead of being stored)
   int top_k = P.top_k < g - 1 ? P.top_k : g - 1;
   if (top_k < 1) top_k = 1;
-  const long long* prow = pmat + static_cast<long long>(i) * g;
   const long long old_i = old[i];
   auto ratio_of = [&](int j, long long pg) {
     long long denom = old_i + old[j];
@@ -1293,13 +1256,13 @@ __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
   int cnt = 0;
   for (int base = 0; base < g; base += 32) {
     const int j = base + lane;
-    const bool pred = j < g && j != i && prow[j] > 0;
+    const bool pred = j < g && j != i && ProxyOf(PairWord(pmat, g, i, j)) > 0;
     cnt += __popc(__ballot_sync(0xffffffffu, pred));
   }
   const int qi = q[i];
   if (cnt <= top_k) {
     for (int j = lane; j < g; j += 32) {
-      if (j == i || prow[j] <= 0) continue;
+      if (j == i || ProxyOf(PairWord(pmat, g, i, j)) <= 0) continue;
       const int a = i < j ? i : j;
       const int b = i < j ? j : i;
       fmat[static_cast<long long>(a) * g + b] = 1;
@@ -1308,15 +1271,15 @@ __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
     int* cj = cand_j[threadIdx.x >> 5];
     const int nt = (g + 31) >> 5;
     if (nt <= 1) {
-      MembersTopK<1>(lane, g, i, qi, top_k, cnt, prow, old, old_i, q, cj, fmat);
+      MembersTopK<1>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
     } else if (nt <= 2) {
-      MembersTopK<2>(lane, g, i, qi, top_k, cnt, prow, old, old_i, q, cj, fmat);
+      MembersTopK<2>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
     } else if (nt <= 4) {
-      MembersTopK<4>(lane, g, i, qi, top_k, cnt, prow, old, old_i, q, cj, fmat);
+      MembersTopK<4>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
     } else if (nt <= 8) {
-      MembersTopK<8>(lane, g, i, qi, top_k, cnt, prow, old, old_i, q, cj, fmat);
+      MembersTopK<8>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
     } else {
-      MembersTopK<kMaxGroup / 32>(lane, g, i, qi, top_k, cnt, prow, old, old_i, q, cj, fmat);
+      MembersTopK<kMaxGroup / 32>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
     }
   } else {
     RankKey prev;
@@ -1326,7 +1289,7 @@ __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
       bool have = false;
       for (int j = lane; j < g; j += 32) {
         if (j == i) continue;
-        const long long pg = prow[j];
+        const long long pg = ProxyOf(PairWord(pmat, g, i, j));
         if (pg <= 0) continue;
         RankKey k;
         k.j = j;
@@ -1378,6 +1341,24 @@ __device__ __forceinline__ unsigned long long RowFlagBits(const unsigned long lo
   return fw[w] & m;
 }
 
+// The shared part of pair (a, b) from its two words.
+__device__ __forceinline__ PairInfo PairInfoOf(const QuotientView& Q, int a, int b, unsigned long long word,
+                                               long long corr) {
+  PairInfo p;
+  p.ovl = static_cast<unsigned>((word >> kProxyBits) & kOvlMask);
+  p.eab = 0;
+  if (word & (kRowILists | kRowJLists)) {
+    const long long ea = RowLookup(Q.ent + Q.off[a], Q.len[a], b);
+    const long long eb = RowLookup(Q.ent + Q.off[b], Q.len[b], a);
+    if (ea != eb) p.ovl |= kPairAsym;
+    p.eab = static_cast<unsigned>(ea);
+  }
+  if (corr >= kCorrBad / 2 || corr <= -kCorrBad / 2) p.ovl |= kPairBad;
+  // the proxy holds the direct edges as listed by row a
+  p.shared = corr - (ProxyOf(word) - static_cast<long long>(p.eab));
+  return p;
+}
+
 // Output pass of the big groups: the union of kept pairs in (a_idx, b_idx)
 // order, one CTA per group.
 __global__ void __launch_bounds__(kPrepThreads) PrepareOutputKernel(PrepareParams P) {
@@ -1394,7 +1375,7 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareOutputKernel(PrepareParam
   const int g = P.glen[gid];
   const long long gg = static_cast<long long>(g) * g;
   const unsigned char* fmat = P.mat + P.mat_off[ri] + FlagOffset(gg);
-  const long long* pmat = reinterpret_cast<const long long*>(P.mat + P.mat_off[ri]);
+  const unsigned long long* pmat = reinterpret_cast<const unsigned long long*>(P.mat + P.mat_off[ri]);
   const long long* old = reinterpret_cast<const long long*>(P.mat + P.mat_off[ri] + OldCostOffset(gg));
   const int* q = P.order + P.gstart[gid];
   // union of kept pairs in (a_idx, b_idx) order. The flags of row a,
@@ -1447,8 +1428,13 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareOutputKernel(PrepareParam
         const int b = static_cast<int>(w * 8 + k - row0);
         out[at] = make_int2(a, b);
         P.cand_rep[P.cand_off[ri] + at] = make_int2(q[a], q[b]);
+        const unsigned long long word = pmat[static_cast<long long>(a) * g + b];
+        if (P.info) {
+          P.info[P.cand_off[ri] + at] =
+              PairInfoOf(P.Q, q[a], q[b], word, static_cast<long long>(pmat[static_cast<long long>(b) * g + a]));
+        }
         if (P.cand_feat) {
-          const long long pg = pmat[static_cast<long long>(a) * g + b];
+          const long long pg = ProxyOf(word);
           long long denom = old[a] + old[b];
           if (denom < 1) denom = 1;
           // a ranker feature, not a decision: single precision is enough
@@ -1468,32 +1454,37 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareOutputKernel(PrepareParam
 
 // ------------------------------------------------------------ prepare, small groups
 
-// Groups of at most kSmallGroup members (99% of the real groups on R-MAT
-// workloads): one warp per group, no block-wide barrier. The group's rows and
-// their target sizes are staged in shared memory in one coalesced pass when
-// they fit; the EA-proxy sum over targets shared by two members then equals,
-// per member pair, the sum over the intersection of their two sorted rows (a
-// row never holds its own rep, so the reference's own-rep exclusion is
-// implied), which one lane computes per pair with a two-pointer merge while
-// the other lanes do the other pairs. Groups whose rows do not fit are handled
-// warp-cooperatively from global memory. Output and counters equal those of
-// PrepareKernel.
+// Groups of at most kSmallGroup members whose rows hold at most kSmallStage
+// entries (99% of the real groups on R-MAT workloads): one warp per group, no
+// block-wide barrier. The group's rows and their target sizes are staged in
+// shared memory in one coalesced pass; the EA-proxy sum over targets shared by
+// two members then equals, per member pair, the sum over the intersection of
+// their two sorted rows (a row never holds its own rep, so the reference's
+// own-rep exclusion is implied), which one lane computes per pair with a
+// two-pointer merge while the other lanes do the other pairs. Output and
+// counters equal those of PrepareKernel.
 constexpr int kSmallGroup = 32;
 constexpr int kSmallWarps = 4;
 constexpr int kSmallPairs = kSmallGroup * (kSmallGroup - 1) / 2;
 constexpr int kSmallStage = 256;  // staged row entries per group
+// Pair sums are kept in 32 bits where the group's counts sum to less than
+// this (every term is at most 4 counts); other groups merge a pair's rows
+// again whenever they need its sums.
+constexpr long long kSmallNarrow = 1ll << 28;
+constexpr unsigned kSmallBad = 1u << 15;  // flag of SmallWarpSmem::ovl
 
 struct SmallWarpSmem {
-  long long p[kSmallPairs];  // upper triangle, TriIndex(a, b)
   long long old[kSmallGroup];
+  long long off[kSmallGroup];
   Entry ent[kSmallStage];
+  unsigned p[kSmallPairs];  // upper triangle, TriIndex(a, b)
+  int corr[kSmallPairs];
+  unsigned short ovl[kSmallPairs];
   int tsz[kSmallStage];
   int q[kSmallGroup];
   int sz[kSmallGroup];
-  int len[kSmallGroup];
   int start[kSmallGroup + 1];
   unsigned fmask[kSmallGroup];
-  long long off[kSmallGroup];
 };
 
 struct SmallSmem {
@@ -1501,6 +1492,49 @@ struct SmallSmem {
 };
 
 __device__ __forceinline__ int TriIndex(int a, int b, int g) { return a * (2 * g - a - 1) / 2 + (b - a - 1); }
+
+// Members a < b of a staged group by one lane.
+struct SmallPair {
+  long long proxy;  // EA proxy, direct edges included
+  long long corr;   // as in the pair tables
+  int ovl;
+  bool bad;
+};
+
+__device__ __forceinline__ SmallPair SmallMerge(const SmallWarpSmem& S, int a, int b) {
+  const int qb = S.q[b];
+  const long long sa = S.sz[a], sb = S.sz[b];
+  int ia = S.start[a], ib = S.start[b];
+  const int ea_end = S.start[a + 1], eb_end = S.start[b + 1];
+  SmallPair r{0, 0, 0, false};
+  while (ia < ea_end && ib < eb_end) {
+    const Entry ea = S.ent[ia], eb = S.ent[ib];
+    const int ta = EntNb(ea), tb = EntNb(eb);
+    if (ta < tb) {
+      if (ta == qb) r.proxy += EntCnt(ea);
+      ++ia;
+    } else if (tb < ta) {
+      ++ib;
+    } else {
+      bool bad;
+      const SharedTerm t = TermOf(sa, sb, S.tsz[ia], EntCnt(ea), EntCnt(eb), &bad);
+      r.proxy += t.delta;
+      r.corr += t.corr;
+      r.bad |= bad;
+      ++r.ovl;
+      ++ia;
+      ++ib;
+    }
+  }
+  for (; ia < ea_end; ++ia) {
+    if (EntNb(S.ent[ia]) == qb) r.proxy += EntCnt(S.ent[ia]);
+  }
+  return r;
+}
+
+__device__ __forceinline__ long long StagedLookup(const SmallWarpSmem& S, int a, int key) {
+  return RowLookup(S.ent + S.start[a], S.start[a + 1] - S.start[a], key);
+}
 
 __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PrepareParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1513,16 +1547,13 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
   const int g = P.glen[gid];
   const QuotientView& Q = P.Q;
   const int* order = P.order + P.gstart[gid];
-  long long off = 0;
   int len = 0;
   if (lane < g) {
     const int rep = order[lane];
     S.q[lane] = rep;
     S.sz[lane] = Q.size[rep];
     len = Q.len[rep];
-    off = Q.off[rep];
-    S.len[lane] = len;
-    S.off[lane] = off;
+    S.off[lane] = Q.off[rep];
     S.fmask[lane] = 0;
   }
   // row starts in the staging buffer
@@ -1535,174 +1566,70 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
   if (lane < g) S.start[lane] = incl - len;
   if (lane == 0) S.start[g] = E;
   const int npairs = g * (g - 1) / 2;
-  for (int k = lane; k < npairs; k += 32) S.p[k] = 0;
-  const bool staged = E <= kSmallStage;
-  __syncwarp();
-  if (staged) {
-    // one flat pass over the group's entries (independent loads), then the
-    // target sizes
-#pragma unroll 4
-    for (int k = lane; k < E; k += 32) {
-      int lo = 0, hi = g;  // row of entry k: last i with start[i] <= k
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (S.start[mid] <= k) lo = mid; else hi = mid;
-      }
-      S.ent[k] = Q.ent[S.off[lo] + (k - S.start[lo])];
+  if (E > kSmallStage) {  // not by the plan: row entries counted at Divide time only shrink
+    if (lane == 0) {
+      RaiseError(P.err, kErrSlots, gid, E, 0);
+      P.cand_cnt[ri] = 0;
     }
-    __syncwarp();
-#pragma unroll 4
-    for (int k = lane; k < E; k += 32) S.tsz[k] = Q.size[EntNb(S.ent[k])];
+    return;
   }
+  __syncwarp();
+  // one flat pass over the group's entries (independent loads), then the
+  // target sizes
+  long long counts = 0;
+#pragma unroll 4
+  for (int k = lane; k < E; k += 32) {
+    int lo = 0, hi = g;  // row of entry k: last i with start[i] <= k
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (S.start[mid] <= k) lo = mid; else hi = mid;
+    }
+    const Entry e = Q.ent[S.off[lo] + (k - S.start[lo])];
+    S.ent[k] = e;
+    counts += EntCnt(e);
+  }
+  __syncwarp();
+#pragma unroll 4
+  for (int k = lane; k < E; k += 32) S.tsz[k] = Q.size[EntNb(S.ent[k])];
+  const bool wide = WarpSum(counts) >= kSmallNarrow;
   __syncwarp();
   unsigned long long examined = 0;
-  if (staged) {
-    // approximate old cost: one lane per member
-    if (lane < g) {
-      const int rep = S.q[lane];
-      const long long si = S.sz[lane];
-      long long old = 0, light = 0;
-      int nh = 0;
-      int4 hp = make_int4(-1, -1, -1, -1);
-      for (int k = S.start[lane]; k < S.start[lane + 1]; ++k) {
-        const long long c = EntCnt(S.ent[k]);
-        const long long st = S.tsz[k];
-        old += EncodeCostForPair(rep, si, EntNb(S.ent[k]), st, c);
-        if (HeavyEntry(si, st, c)) {
-          const int pos = k - S.start[lane];
-          if (nh == 0) hp.x = pos; else if (nh == 1) hp.y = pos; else if (nh == 2) hp.z = pos; else if (nh == 3) hp.w = pos;
-          ++nh;
-        } else {
-          light += c;
-        }
-      }
-      if (P.rc_before) {
-        P.rc_before[rep] = old;
-        P.rc_light[rep] = light;
-        P.rc_heavy[rep] = hp;
-        P.rc_nheavy[rep] = nh;
-      }
-      const long long internal = Q.internal[rep];
-      if (internal > 0) old += EncodeCostForPair(rep, si, rep, si, 2 * internal);
-      S.old[lane] = old;
+  // approximate old cost: one lane per member
+  if (lane < g) {
+    const int rep = S.q[lane];
+    const long long si = S.sz[lane];
+    long long old = 0, light = 0;
+    HeavyAcc heavy;
+    for (int k = S.start[lane]; k < S.start[lane + 1]; ++k) {
+      const long long c = EntCnt(S.ent[k]);
+      const long long st = S.tsz[k];
+      old += EncodeCostForPair(rep, si, EntNb(S.ent[k]), st, c);
+      if (HeavyEntry(si, st, c)) heavy.Add(st, c); else light += c;
     }
-    // pair proxies: one lane per member pair
-    for (int pidx = lane; pidx < npairs; pidx += 32) {
-      int a = 0, rem = pidx;
-      while (rem >= g - 1 - a) {
-        rem -= g - 1 - a;
-        ++a;
-      }
-      const int b = a + 1 + rem;
-      const int qa = S.q[a], qb = S.q[b];
-      const long long sa = S.sz[a], sb = S.sz[b];
-      int ia = S.start[a];
-      const int ea_end = S.start[a + 1];
-      int ib = S.start[b];
-      const int eb_end = S.start[b + 1];
-      long long sum = 0, direct = 0;
-      while (ia < ea_end && ib < eb_end) {
-        const int ta = EntNb(S.ent[ia]);
-        const int tb = EntNb(S.ent[ib]);
-        if (ta < tb) {
-          if (ta == qb) direct = EntCnt(S.ent[ia]);
-          ++ia;
-        } else if (tb < ta) {
-          ++ib;
-        } else {
-          const long long ea = EntCnt(S.ent[ia]);
-          const long long eb = EntCnt(S.ent[ib]);
-          const long long st = S.tsz[ia];
-          const long long delta = EncodeCostForPair(qa, sa, ta, st, ea) + EncodeCostForPair(qb, sb, ta, st, eb) -
-                                  EncodeCostForPair(qa, sa + sb, ta, st, ea + eb);
-          if (delta > 0) sum += delta;
-          ++examined;
-          ++ia;
-          ++ib;
-        }
-      }
-      for (; ia < ea_end; ++ia) {
-        if (EntNb(S.ent[ia]) == qb) direct = EntCnt(S.ent[ia]);
-      }
-      S.p[pidx] = sum + direct;
+    const long long internal = Q.internal[rep];
+    if (P.rc) StoreRowSums(&P.rc[rep], old, light, heavy, internal, S.sz[lane], len);
+    if (internal > 0) old += EncodeCostForPair(rep, si, rep, si, 2 * internal);
+    S.old[lane] = old;
+  }
+  // pair sums: one lane per member pair
+  for (int pidx = lane; pidx < npairs; pidx += 32) {
+    int a = 0, rem = pidx;
+    while (rem >= g - 1 - a) {
+      rem -= g - 1 - a;
+      ++a;
     }
-  } else {
-    // rows too long to stage: warp-cooperative passes over global memory
-    for (int i = 0; i < g; ++i) {
-      const int rep = S.q[i];
-      const long long si = S.sz[i];
-      const long long oi = __shfl_sync(0xffffffffu, off, i);
-      const int li2 = S.len[i];
-      long long old = 0, light = 0;
-      int nh = 0;
-      if (P.rc_before && lane == 0) P.rc_heavy[rep] = make_int4(-1, -1, -1, -1);
-      __syncwarp();
-      for (int k0 = 0; k0 < li2; k0 += 32) {
-        const int k = k0 + lane;
-        bool heavy = false;
-        if (k < li2) {
-          const Entry e = Q.ent[oi + k];
-          const long long c = EntCnt(e);
-          const long long st = Q.size[EntNb(e)];
-          old += EncodeCostForPair(rep, si, EntNb(e), st, c);
-          heavy = HeavyEntry(si, st, c);
-          if (!heavy) light += c;
-        }
-        if (P.rc_before) RecordHeavy(P.rc_heavy + rep, nh, heavy, k);
-      }
-      old = WarpSum(old);
-      if (P.rc_before) light = WarpSum(light);
-      if (lane == 0) {
-        if (P.rc_before) {
-          P.rc_before[rep] = old;
-          P.rc_light[rep] = light;
-          P.rc_nheavy[rep] = nh;
-        }
-        const long long internal = Q.internal[rep];
-        if (internal > 0) old += EncodeCostForPair(rep, si, rep, si, 2 * internal);
-        S.old[i] = old;
-      }
-    }
-    for (int a = 0; a < g; ++a) {
-      const int qa = S.q[a];
-      const long long sa = S.sz[a];
-      const Entry* ra = Q.ent + __shfl_sync(0xffffffffu, off, a);
-      const int la = S.len[a];
-      for (int b = a + 1; b < g; ++b) {
-        const int qb = S.q[b];
-        const long long sb = S.sz[b];
-        const Entry* rb = Q.ent + __shfl_sync(0xffffffffu, off, b);
-        const int lb = S.len[b];
-        const bool a_short = la <= lb;
-        const Entry* rs = a_short ? ra : rb;
-        const Entry* rl = a_short ? rb : ra;
-        const int ls = a_short ? la : lb;
-        const int ll = a_short ? lb : la;
-        long long sum = 0;
-        int shared = 0;
-        for (int k = lane; k < ls; k += 32) {
-          const Entry e = rs[k];
-          const int t = EntNb(e);
-          const long long co = RowLookup(rl, ll, t);
-          if (co == 0) continue;
-          ++shared;
-          const long long ea = a_short ? EntCnt(e) : co;
-          const long long eb = a_short ? co : EntCnt(e);
-          const long long st = Q.size[t];
-          const long long delta = EncodeCostForPair(qa, sa, t, st, ea) + EncodeCostForPair(qb, sb, t, st, eb) -
-                                  EncodeCostForPair(qa, sa + sb, t, st, ea + eb);
-          if (delta > 0) sum += delta;
-        }
-        sum = WarpSum(sum);
-        const int sh = WarpSumInt(shared);
-        if (lane == 0) {
-          examined += static_cast<unsigned long long>(sh);
-          S.p[TriIndex(a, b, g)] = sum + RowLookup(ra, la, qb);
-        }
-      }
+    const SmallPair r = SmallMerge(S, a, a + 1 + rem);
+    examined += static_cast<unsigned long long>(r.ovl);
+    if (!wide) {
+      S.p[pidx] = static_cast<unsigned>(r.proxy);
+      S.corr[pidx] = static_cast<int>(r.corr);
+      S.ovl[pidx] = static_cast<unsigned short>(static_cast<unsigned>(r.ovl) | (r.bad ? kSmallBad : 0u));
     }
   }
   __syncwarp();
+  auto proxy_of = [&](int a, int b) {  // a < b
+    return wide ? SmallMerge(S, a, b).proxy : static_cast<long long>(S.p[TriIndex(a, b, g)]);
+  };
   // per member (one lane each): positive partners, ratio, top-k
   int top_k = P.top_k < g - 1 ? P.top_k : g - 1;
   if (top_k < 1) top_k = 1;
@@ -1710,7 +1637,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
     // every member has at most top_k partners: all positive ones are kept
     const int i = lane;
     for (int j = i + 1; j < g; ++j) {
-      if (S.p[TriIndex(i, j, g)] > 0) atomicOr(&S.fmask[i], 1u << j);
+      if (proxy_of(i, j) > 0) atomicOr(&S.fmask[i], 1u << j);
     }
   } else if (g - 1 > P.top_k) {
     // ranking, one member at a time by the whole warp, lane j holding
@@ -1722,7 +1649,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
     const int j = lane;
     for (int i = 0; i < g; ++i) {
       long long pg = 0;
-      if (j < g && j != i) pg = S.p[i < j ? TriIndex(i, j, g) : TriIndex(j, i, g)];
+      if (j < g && j != i) pg = i < j ? proxy_of(i, j) : proxy_of(j, i);
       const bool valid = pg > 0;
       const unsigned vm = __ballot_sync(0xffffffffu, valid);
       const int cnt = __popc(vm);
@@ -1768,15 +1695,37 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
   ex -= cnt;
   int2* out = P.cand + P.cand_off[ri];
   float2* feat = P.cand_feat ? P.cand_feat + P.cand_off[ri] : nullptr;
+  PairInfo* info = P.info ? P.info + P.cand_off[ri] : nullptr;
   unsigned bits = mine;
   while (bits) {
     const int b = __ffs(bits) - 1;
     bits &= bits - 1;
-    if (feat) {
-      const long long pg = S.p[TriIndex(lane, b, g)];
-      long long denom = S.old[lane] + S.old[b];
-      if (denom < 1) denom = 1;
-      feat[ex] = make_float2(static_cast<float>(pg), __fdividef(static_cast<float>(pg), static_cast<float>(denom)));
+    if (feat || info) {
+      SmallPair r;
+      if (wide) {
+        r = SmallMerge(S, lane, b);
+      } else {
+        const int t = TriIndex(lane, b, g);
+        r.proxy = S.p[t];
+        r.corr = S.corr[t];
+        r.ovl = S.ovl[t] & (kSmallBad - 1u);
+        r.bad = (S.ovl[t] & kSmallBad) != 0;
+      }
+      if (feat) {
+        long long denom = S.old[lane] + S.old[b];
+        if (denom < 1) denom = 1;
+        feat[ex] =
+            make_float2(static_cast<float>(r.proxy), __fdividef(static_cast<float>(r.proxy), static_cast<float>(denom)));
+      }
+      if (info) {
+        const long long ea = StagedLookup(S, lane, S.q[b]);
+        const long long eb = StagedLookup(S, b, S.q[lane]);
+        PairInfo pi;
+        pi.shared = r.corr - (r.proxy - ea);
+        pi.ovl = static_cast<unsigned>(r.ovl) | (r.bad ? kPairBad : 0u) | (ea != eb ? kPairAsym : 0u);
+        pi.eab = static_cast<unsigned>(ea);
+        info[ex] = pi;
+      }
     }
     P.cand_rep[P.cand_off[ri] + ex] = make_int2(S.q[lane], S.q[b]);
     out[ex++] = make_int2(lane, b);
@@ -1823,19 +1772,56 @@ struct ScoreParams {
   double threshold;
   ThresholdBits thr;  // threshold split for the integer test
   int use_threshold;
-  RowConsts rc;  // row sums of the block-start state (rc.before == nullptr: full merge)
+  const RowSums* rc;     // row sums of the block-start state (nullptr: full merge of the two rows)
+  const PairInfo* info;  // per candidate slot (with rc)
+  int strict;            // check every entry of both rows against its block's capacity (as the full merge does)
   unsigned long long* stats;
   DevError* err;
 };
 
-// m: the two rows' staged scalars (read only with row sums)
-__device__ __forceinline__ void ScoreGain(const ScoreParams& P, int a, int b, const RowMeta* m, long long* gain,
-                                          long long* before, GainWork* w) {
-  if (P.rc.before) {
-    WarpExactGainShared(P.Q, a, b, m[0], m[1], gain, before, w, P.err);
-  } else {
-    WarpExactGain(P.Q, a, b, gain, before, w, P.err);
-  }
+// The exact gain of candidate (a, b) from the row sums and the pair's shared
+// part, by one lane; false: a row's heavy entries are neither all dense nor
+// all light at this size, and have to be read.
+struct GainParts {
+  long long gain, before;
+  int uni, ovl;
+};
+
+__device__ __forceinline__ bool GainFromSums(const RowSums& A, const RowSums& B, const PairInfo& p, int a, int b,
+                                             int strict, DevError* err, GainParts* out) {
+  const long long sa = A.size, sb = B.size, s = sa + sb;
+  const long long eab = p.eab;
+  long long fa, fb;
+  const bool have_a = RowAfter(A, s, &fa);
+  const bool have_b = RowAfter(B, s, &fb);
+  // counts beyond their block's capacity: at the merged size, and at the
+  // row's own size where asked for or with more than a few heavy entries
+  int bad = (p.ovl & kPairBad) != 0 || s < A.sbad || s < B.sbad;
+  if (strict || A.nheavy > kHeavyFew || B.nheavy > kHeavyFew) bad |= sa < A.sbad || sb < B.sbad;
+  const long long before = A.before + B.before - BlockCost(sb, sa, eab, false, bad) +
+                           BlockCost(sa, sa, A.internal, true, bad) + BlockCost(sb, sb, B.internal, true, bad);
+  const long long after = fa + fb - BlockCost(s, sb, eab, false, bad) - BlockCost(s, sa, eab, false, bad) + p.shared +
+                          BlockCost(s, s, A.internal + B.internal + eab, true, bad);
+  if (p.ovl & kPairAsym) RaiseError(err, kErrAsymmetric, a, b, 0);
+  if (bad) RaiseError(err, kErrBlockCost, a, b, 0);
+  out->gain = before - after;  // without the F of a row that has to be read
+  out->before = before;
+  out->ovl = static_cast<int>(p.ovl & ((1u << 30) - 1u));
+  const int e = eab > 0 ? 1 : 0;
+  out->uni = (A.len - e) + (B.len - e) - out->ovl;
+  return have_a && have_b;
+}
+
+// The same, by a warp, for the pairs GainFromSums leaves.
+__device__ GainParts WarpGainReadingRows(const QuotientView& Q, const RowSums& A, const RowSums& B, const PairInfo& p,
+                                         int a, int b, int strict, DevError* err) {
+  const long long s = static_cast<long long>(A.size) + B.size;
+  GainParts g;
+  GainFromSums(A, B, p, a, b, strict, err, &g);
+  long long part;
+  if (!RowAfter(A, s, &part)) g.gain += part - WarpRowAfter(Q, a, s);
+  if (!RowAfter(B, s, &part)) g.gain += part - WarpRowAfter(Q, b, s);
+  return g;
 }
 
 __device__ __forceinline__ bool PassesFilter(long long gain, long long before, double threshold, ThresholdBits thr,
@@ -1858,44 +1844,46 @@ __device__ __forceinline__ void FlushScoreStats(unsigned long long* stats, const
   atomicAdd(&stats[kStScoreBytes], static_cast<unsigned long long>(w.bytes + 24 * pairs));
 }
 
-// One warp per candidate slot of the block (the concatenated per-group
-// candidate capacities); slots past a group's candidate count hold -1 and
-// are skipped.
-// Slots are fetched from the block's queue kScoreFetch at a time (pairs over
-// hub rows cost orders of magnitude more than the rest). Fetch c takes the
-// slots c, c + F, c + 2F, ... (F = the number of fetches): the candidates of
-// one member are consecutive slots, and a hub member's pairs must not all
-// land on one warp. The warp loads the fetch's pair ids and (with row sums)
-// the scalars of their rows together, one slot or row per lane, before it
-// scores the pairs one by one: one load latency per fetch instead of a chain
-// of them per pair.
-constexpr int kScoreFetch = 16;
-static_assert(2 * kScoreFetch == 32, "one staged row per lane");
+// Candidate slots of a block are the concatenated per-group capacities; slots
+// past a group's candidate count hold -1 and are skipped. A warp takes
+// kScoreFetch slots at a time from the block's queue; fetch f holds the slots
+// f, f + F, f + 2F, ... (F = the number of fetches): the candidates of one
+// member are consecutive slots, and a hub member's pairs, where they have to
+// read rows, must not all land on one warp.
+//
+// With row sums each lane scores its own pair from two 64-byte row records and
+// one 16-byte pair record, the pairs that still have to read a row follow one
+// by one by the whole warp. Before, every pair merged its two rows here
+// (8-byte entries, 32 of each per step), although the prepare kernels had
+// already visited every shared target: at R-MAT scale 23 that was 330 ms of a
+// 1,291 ms run; now the run takes 973 ms. Without row sums (graphs beyond kFusedMaxArcs) a warp merges
+// one pair's rows at a time, and fetches fewer of them.
+constexpr int kScoreFetch = 32;
+constexpr int kScoreFetchMerge = 8;
 
 __global__ void __launch_bounds__(kScoreThreads, 4) ScoreKernel(ScoreParams P) {
-  __shared__ RowMeta s_meta[kScoreThreads / 32][2 * kScoreFetch];
   constexpr unsigned kFull = 0xffffffffu;
   const long long s0 = P.cand_off[P.rg0];
   const long long s1 = P.cand_off[P.rg0 + P.nrg];
   const int lane = threadIdx.x & 31;
-  RowMeta* wm = s_meta[threadIdx.x >> 5];
   GainWork w = {0, 0, 0, 0, 0};
   long long pairs = 0, view_nnz = 0;
   unsigned long long pruned = 0;
   const float cutoff = P.phase == 2 ? *P.cutoff : 0.0f;
   unsigned long long* queue = &P.ctl->work_next[P.phase == 2 ? 2 : 1];
-  const long long nfetch = (s1 - s0 + kScoreFetch - 1) / kScoreFetch;
+  const int fetch = P.rc ? kScoreFetch : kScoreFetchMerge;
+  const long long nfetch = (s1 - s0 + fetch - 1) / fetch;
   for (;;) {
     long long f = 0;
     if (lane == 0) f = static_cast<long long>(atomicAdd(queue, 1ull));
     f = __shfl_sync(kFull, f, 0);
     if (f >= nfetch) break;
-    // lane j < kScoreFetch: slot j of the fetch, its pair, and what to do
-    // with it (0 nothing, 1 score, 2 pruned by the ranker)
-    const long long slot = s0 + f + static_cast<long long>(lane & (kScoreFetch - 1)) * nfetch;
+    // what to do with this lane's slot: 0 nothing, 1 score, 2 pruned by the
+    // ranker (scored aside by the audit)
+    const long long slot = s0 + f + static_cast<long long>(lane) * nfetch;
     int2 ab = make_int2(-1, -1);
     int todo = 0;
-    if (lane < kScoreFetch && slot < s1) {
+    if (lane < fetch && slot < s1) {
       ab = P.cand_rep[slot];
       if (ab.x >= 0) {
         todo = 1;
@@ -1909,69 +1897,83 @@ __global__ void __launch_bounds__(kScoreThreads, 4) ScoreKernel(ScoreParams P) {
         }
       }
     }
-    // lane l stages row (l & 1) of pair l >> 1: its supernode and, with row
-    // sums, its scalars
-    {
-      const int j = lane >> 1;
-      const int ja = __shfl_sync(kFull, ab.x, j);
-      const int jb = __shfl_sync(kFull, ab.y, j);
-      const int jt = __shfl_sync(kFull, todo, j);
-      const int r = (lane & 1) ? jb : ja;
-      if (P.rc.before && (jt == 1 || (jt == 2 && P.audit))) {
-        LoadRowMeta(P.Q, P.rc, r, &wm[lane]);
+    const bool score = todo == 1 || (todo == 2 && P.audit);
+    GainParts g = {0, 0, 0, 0};
+    RowSums A, B;
+    PairInfo p;
+    bool by_warp = score;
+    if (score && P.rc) {
+      A = P.rc[ab.x];
+      B = P.rc[ab.y];
+      p = P.info[slot];
+      by_warp = !GainFromSums(A, B, p, ab.x, ab.y, P.strict, P.err, &g);
+    }
+    for (unsigned rest = __ballot_sync(kFull, by_warp); rest != 0u; rest &= rest - 1u) {
+      const int j = __ffs(rest) - 1;
+      const int a = __shfl_sync(kFull, ab.x, j);
+      const int b = __shfl_sync(kFull, ab.y, j);
+      GainParts r;
+      if (P.rc) {
+        const long long sj = __shfl_sync(kFull, slot, j);
+        r = WarpGainReadingRows(P.Q, P.rc[a], P.rc[b], P.info[sj], a, b, P.strict, P.err);
       } else {
-        wm[lane].rep = r;
+        GainWork one = {0, 0, 0, 0, 0};
+        WarpExactGain(P.Q, a, b, &r.gain, &r.before, &one, P.err);
+        r.uni = static_cast<int>(one.uni);
+        r.ovl = static_cast<int>(one.ovl);
       }
+      if (lane == j) g = r;
     }
-    const unsigned prune = __ballot_sync(kFull, todo == 2);
-    unsigned live = __ballot_sync(kFull, todo != 0);
-    __syncwarp();
-    for (; live != 0u; live &= live - 1u) {
-      const int j = __ffs(live) - 1;
-      const RowMeta* m = wm + 2 * j;
-      const int a = m[0].rep;
-      const int b = m[1].rep;
-      const long long sj = s0 + f + static_cast<long long>(j) * nfetch;
-      long long gain = 0, before = 0;
-      if ((prune >> j) & 1u) {
-        // pruned by the ranker: not scored (the audit scores it aside)
-        if (P.audit) {
-          GainWork aw = {0, 0, 0, 0, 0};
-          ScoreGain(P, a, b, m, &gain, &before, &aw);
-          if (lane == 0 && PassesFilter(gain, before, P.threshold, P.thr, P.use_threshold)) {
-            atomicAdd(&P.stats[kStRkAuditPassing], 1ull);
-            atomicAdd(&P.stats[kStRkAuditLost], 1ull);
-          }
-        }
-        if (lane == 0) {
-          P.res[sj] = make_longlong2(0, -1);
-          ++pruned;
-        }
-        continue;
+    if (todo == 0) continue;
+    const bool passes = score && PassesFilter(g.gain, g.before, P.threshold, P.thr, P.use_threshold);
+    if (todo == 2) {
+      if (P.audit && passes) {
+        atomicAdd(&P.stats[kStRkAuditPassing], 1ull);
+        atomicAdd(&P.stats[kStRkAuditLost], 1ull);
       }
-      ScoreGain(P, a, b, m, &gain, &before, &w);
-      if (lane == 0) {
-        if (P.phase != 0 && PassesFilter(gain, before, P.threshold, P.thr, P.use_threshold)) {
-          if (P.audit) atomicAdd(&P.stats[kStRkAuditPassing], 1ull);
-          if (P.phase == 1) {
-            const unsigned at = atomicAdd(P.npos, 1u);
-            if (at < P.zcap) {
-              P.zpos[at] = P.zbuf[sj];
-              P.zgain[at] = gain;
-            }
-          }
-        }
-        P.res[sj] = make_longlong2(gain, before);
-        ++pairs;
-        if (P.rc.before) {
-          view_nnz += m[0].len + (m[0].internal > 0 ? 1 : 0) + m[1].len + (m[1].internal > 0 ? 1 : 0);
-        } else {
-          view_nnz += P.Q.len[a] + (P.Q.internal[a] > 0 ? 1 : 0) + P.Q.len[b] + (P.Q.internal[b] > 0 ? 1 : 0);
+      P.res[slot] = make_longlong2(0, -1);
+      ++pruned;
+      continue;
+    }
+    if (P.phase != 0 && passes) {
+      if (P.audit) atomicAdd(&P.stats[kStRkAuditPassing], 1ull);
+      if (P.phase == 1) {
+        const unsigned at = atomicAdd(P.npos, 1u);
+        if (at < P.zcap) {
+          P.zpos[at] = P.zbuf[slot];
+          P.zgain[at] = g.gain;
         }
       }
     }
-    __syncwarp();  // the next fetch restages this warp's rows
+    P.res[slot] = make_longlong2(g.gain, g.before);
+    ++pairs;
+    const int la = P.rc ? A.len : P.Q.len[ab.x];
+    const int lb = P.rc ? B.len : P.Q.len[ab.y];
+    const long long ia = P.rc ? A.internal : P.Q.internal[ab.x];
+    const long long ib = P.rc ? B.internal : P.Q.internal[ab.y];
+    view_nnz += la + (ia > 0 ? 1 : 0) + lb + (ib > 0 ? 1 : 0);
+    w.raw_a += la;
+    w.raw_b += lb;
+    w.uni += g.uni;
+    w.ovl += g.ovl;
+    // with row sums: two row records and a pair record; a pair that reads rows
+    // (or merges them) 8 B per entry and 4 B per size
+    w.bytes += P.rc ? 2ll * sizeof(RowSums) + sizeof(PairInfo) : 0ll;
+    if (by_warp) {
+      w.bytes += P.rc ? 12ll * ((RowAfterKnown(A, A.size + B.size) ? 0 : la) +
+                                (RowAfterKnown(B, A.size + B.size) ? 0 : lb))
+                      : 8ll * (la + lb) + 4ll * g.uni;
+    }
   }
+  __syncwarp();
+  pairs = WarpSum(pairs);
+  view_nnz = WarpSum(view_nnz);
+  w.raw_a = WarpSum(w.raw_a);
+  w.raw_b = WarpSum(w.raw_b);
+  w.uni = WarpSum(w.uni);
+  w.ovl = WarpSum(w.ovl);
+  w.bytes = WarpSum(w.bytes);
+  pruned = static_cast<unsigned long long>(WarpSum(static_cast<long long>(pruned)));
   if (lane == 0) {
     FlushScoreStats(P.stats, w, pairs, view_nnz);
     if (pruned) atomicAdd(&P.stats[kStRkPruned], pruned);
@@ -3581,6 +3583,7 @@ void Engine::SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nb
   d_cand_rep_.ensure(ncand + 1);
   CheckCuda(cudaMemsetAsync(d_cand_rep_.p, 0xff, sizeof(int2) * (ncand + 1), stream_), "memset cand reps");
   d_res_.ensure(ncand + 1);
+  d_info_.ensure(sizeof(PairInfo) * (ncand + 1));
   if (cfg_.ranker) {
     d_cand_feat_.ensure(ncand + 1);
     d_rk_keep_.ensure(ncand + 1);
@@ -3735,13 +3738,10 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify) {
 
 // EA-proxy candidates for the small-group list entries [s0, s1) (one warp
 // per group) and the big-group entries [b0, b1) (one CTA per group).
-// Row sums for the scoring pass: in a large block of a one-block iteration
-// (the prepare kernels write them while reading the member rows; scoring from
-// them pays in a large block).
-// Row sums are written by the block's own prepare kernels from its block-start
-// state and read by its scoring pass only, so every block of more than
-// kFewGroups groups uses them, one-block iterations or not.
-bool Engine::RowSumsOn(const BlockPlan& bp) const { return bp.rg1 - bp.rg0 > kFewGroups; }
+// Row sums and pair sums are written by the block's own prepare kernels from
+// its block-start state and read by its scoring pass only, so every block uses
+// them, on graphs whose shared targets fit their field of the pair words.
+bool Engine::RowSumsOn() const { return arcs_ < kFusedMaxArcs; }
 
 void Engine::LaunchPrepare(const BlockPlan& bp) {
   const int s0 = bp.s0, s1 = bp.s1, b0 = bp.b0, b1 = bp.b1;
@@ -3759,19 +3759,12 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
   PP.mat_off = d_mat_off_.p;
   PP.mat = d_mat_.p;
   PP.mat_zeroed = 0;
-  PP.rc_before = nullptr;
-  PP.rc_light = nullptr;
-  PP.rc_heavy = nullptr;
-  PP.rc_nheavy = nullptr;
-  if (RowSumsOn(bp)) {
-    d_rc_before_.ensure(static_cast<size_t>(n_));
-    d_rc_light_.ensure(static_cast<size_t>(n_));
-    d_rc_heavy_.ensure(static_cast<size_t>(n_));
-    d_rc_nheavy_.ensure(static_cast<size_t>(n_));
-    PP.rc_before = d_rc_before_.p;
-    PP.rc_light = d_rc_light_.p;
-    PP.rc_heavy = d_rc_heavy_.p;
-    PP.rc_nheavy = d_rc_nheavy_.p;
+  PP.rc = nullptr;
+  PP.info = nullptr;
+  if (RowSumsOn()) {
+    d_rc_.ensure(sizeof(RowSums) * static_cast<size_t>(n_));
+    PP.rc = reinterpret_cast<RowSums*>(d_rc_.p);
+    PP.info = reinterpret_cast<PairInfo*>(d_info_.p);
   }
   PP.scratch = d_scratch_.p;
   PP.scratch_cap = d_scratch_.n;
@@ -3877,13 +3870,17 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
   SP.npos = d_rk_npos_.p;
   SP.zcap = 0;
   SP.cutoff = d_rk_cut_.p;
-  SP.rc = RowConsts{nullptr, nullptr, nullptr, nullptr};
-  if (RowSumsOn(bp)) {
+  SP.rc = nullptr;
+  SP.info = nullptr;
+  if (RowSumsOn()) {
     // written by this block's prepare kernels
-    SP.rc = RowConsts{d_rc_before_.p, d_rc_light_.p, d_rc_heavy_.p, d_rc_nheavy_.p};
+    SP.rc = reinterpret_cast<const RowSums*>(d_rc_.p);
+    SP.info = reinterpret_cast<const PairInfo*>(d_info_.p);
   }
+  SP.strict = nrg <= kFewGroups ? 1 : 0;
+  const int fetch = SP.rc ? kScoreFetch : kScoreFetchMerge;
   const int sgrid = static_cast<int>(
-      std::min<long long>((slots + kScoreFetch * 8 - 1) / (kScoreFetch * 8), score_grid_));
+      std::min<long long>((slots + fetch * 8 - 1) / (fetch * 8), score_grid_));
   // learned ranker: trained after the logging iterations; afterwards the
   // exploration subset is scored first, then the rest above the cutoff
   const bool ranking = cfg_.ranker && rk_trained_ && iter > cfg_.ranker_train_iters;

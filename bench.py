@@ -508,7 +508,7 @@ def run_ours(args, dist: Dist) -> dict | None:
             "peak_source": peak_kind,
             "traffic": traffic,
             "algorithmic_bytes_per_launch": round(t["kernel_bytes"] / max(1, kernel_launches), 1),
-            "bytes_counted": "8 B per row entry read, 4 B per shared-neighbour size, 36 B of row sums and 24 B "
+            "bytes_counted": "two 64 B row records, a 16 B pair record and 24 B "
                              "per scored pair (the kernel's own reads)",
             "union_count": union_roofline(t, peak),
             "avg_launch_us": round(1000.0 * kernel_ms / max(1, kernel_launches), 3),
