@@ -137,6 +137,8 @@ struct BlockCtl {
   unsigned int short_cnt;   // claimed neighbour rows rewritten by one warp each
   unsigned int long_cnt;    // claimed neighbour rows rewritten by one CTA each
   unsigned int sel_total;   // selected pairs of the block (entries of the selection list)
+  unsigned int huge_cnt;    // claimed neighbour rows rewritten in two steps
+  unsigned int huge_units;  // their scan units
   unsigned int pad;
   // work queues of the dynamically scheduled kernels: the accumulate pass and
   // the two scoring passes (exploration / the rest, or the only one)
@@ -274,6 +276,8 @@ class Engine {
   DevBuf<int> d_label_, d_head_, d_next_, d_tail_, d_fwd_;
   DevBuf<int> d_stamp_, d_partner_, d_claim_, d_seq_;
   DevBuf<int> d_rows_short_, d_rows_long_;  // claimed neighbour rows of a block
+  DevBuf<unsigned char> d_rows_huge_;
+  DevBuf<int2> d_huge_units_;
   DevBuf<int> d_sel_list_;                   // selection slots of a block's selected pairs
   DevBuf<unsigned> d_rw_ticket_;             // last-CTA counter of the rewrite kernel
 

@@ -62,6 +62,14 @@ constexpr int kRowsThreads = 256;
 constexpr int kRowSmem = 2048;       // staged row entries in shared memory
 constexpr int kWarpRow = 32;         // neighbour rows rewritten by one warp in registers
 constexpr int kWarpRowMax = 256;     // neighbour rows rewritten by one warp through shared memory
+// Neighbour rows of more than kRowSmem entries are rewritten in two steps: the
+// renamed entries found by warps over kHugeUnit entries each, the row moved by
+// one CTA in chunks of kHugeChunk.
+constexpr int kHugeUnit = 1024;
+constexpr int kHugeThreads = 1024;
+constexpr int kHugePer = 8;
+constexpr int kHugeChunk = kHugeThreads * kHugePer;
+constexpr int kHugeGrid = 152;
 constexpr int kKeyIdxBits = 10;      // a_idx, b_idx < kMaxGroup
 constexpr long long kKeyGainMax = (1ll << (64 - 2 * kKeyIdxBits)) - 1;
 
@@ -2484,6 +2492,19 @@ __global__ void __launch_bounds__(kSelectSmallWarps * 32) SelectSmallKernel(Sele
 
 // ------------------------------------------------------------ commit
 
+// A claimed neighbour row of more than kRowSmem entries and its block scratch:
+// one mask bit per entry (renamed or not), the entries to insert (room for a
+// power of two of at least the row's length), a copy of the row where needed.
+struct HugeRow {
+  int x;
+  int len;
+  int nins;  // entries to insert
+  int pad;
+  unsigned* mask;
+  Entry* ins;
+  Entry* copy;
+};
+
 struct CommitParams {
   QuotientView Q;
   int rg0;
@@ -2511,8 +2532,10 @@ struct CommitParams {
   unsigned long long* stats;
   DevError* err;
   int* rows_short;  // claimed neighbour rows of at most kWarpRowMax entries (count: ctl->short_cnt)
-  int* rows_long;   // the other claimed neighbour rows (count: ctl->long_cnt)
-  unsigned* ticket; // last-CTA counter of the rewrite kernel, left at 0
+  int* rows_long;   // those of at most kRowSmem (count: ctl->long_cnt)
+  HugeRow* rows_huge;  // the other claimed neighbour rows (count: ctl->huge_cnt)
+  int2* huge_units;    // {index into rows_huge, first entry} of their scan units (count: ctl->huge_units)
+  unsigned* ticket; // last-CTA counter of the long-row rewrite kernel, left at 0
   const int* sel_list;  // selection slots of the block's selected pairs (count: ctl->sel_total)
   int warp_pairs;       // 1: pairs with at most kWarpRow row entries go to CommitShortKernel
 };
@@ -2690,6 +2713,38 @@ __device__ bool StageBuffers(const CommitParams& P, RowsSmem& R, int L, Entry** 
   return true;
 }
 
+// Row x holds an entry of a supernode removed in this block: listed once for
+// the rewrite, by its length.
+__device__ __forceinline__ void ClaimRow(const CommitParams& P, int x) {
+  if (atomicExch(&P.claim[x], P.block_stamp) == P.block_stamp) return;
+  const int len = P.Q.len[x];
+  if (len <= kWarpRowMax) {
+    P.rows_short[atomicAdd(&P.ctl->short_cnt, 1u)] = x;
+  } else if (len <= kRowSmem) {
+    P.rows_long[atomicAdd(&P.ctl->long_cnt, 1u)] = x;
+  } else {
+    int pow2 = 1;
+    while (pow2 < len) pow2 <<= 1;
+    const unsigned long long mask_bytes = ((static_cast<unsigned long long>(len) + 31) / 32 * 4 + 15) & ~15ull;
+    unsigned char* mem = reinterpret_cast<unsigned char*>(
+        ScratchAlloc(P.scratch, P.scratch_cap, P.ctl, mask_bytes + 8ull * pow2 + 8ull * len, P.err));
+    if (mem == nullptr) return;
+    HugeRow h;
+    h.x = x;
+    h.len = len;
+    h.nins = 0;
+    h.pad = 0;
+    h.mask = reinterpret_cast<unsigned*>(mem);
+    h.ins = reinterpret_cast<Entry*>(mem + mask_bytes);
+    h.copy = h.ins + pow2;
+    const unsigned at = atomicAdd(&P.ctl->huge_cnt, 1u);
+    P.rows_huge[at] = h;
+    const unsigned units = static_cast<unsigned>((len + kHugeUnit - 1) / kHugeUnit);
+    const unsigned u0 = atomicAdd(&P.ctl->huge_units, units);
+    for (unsigned u = 0; u < units; ++u) P.huge_units[u0 + u] = make_int2(static_cast<int>(at), static_cast<int>(u) * kHugeUnit);
+  }
+}
+
 // One CTA per selected pair of the block (persistent grid over the block's
 // selection slots). Per pair:
 //   Update_S bookkeeping: size, internal count, member list, forwarding, and
@@ -2731,13 +2786,7 @@ __global__ void __launch_bounds__(kRowsThreads) CommitKernel(CommitParams P) {
       const int sx = P.stamp[x];
       if (sx == remove_stamp && P.seq[x] < my_seq && RowLookup(rr, lr, P.partner[x]) != 0) ++folded;
       if ((sx >> 1) == P.block_stamp) continue;  // keep/remove rows are rebuilt by their own pair
-      if (atomicExch(&P.claim[x], P.block_stamp) != P.block_stamp) {
-        if (Q.len[x] <= kWarpRowMax) {
-          P.rows_short[atomicAdd(&P.ctl->short_cnt, 1u)] = x;
-        } else {
-          P.rows_long[atomicAdd(&P.ctl->long_cnt, 1u)] = x;
-        }
-      }
+      ClaimRow(P, x);
     }
     folded = WarpSumInt(folded);
     if ((tid & 31) == 0 && folded) atomicAdd(&folded_sum, folded);
@@ -2827,13 +2876,7 @@ __global__ void __launch_bounds__(256) CommitShortKernel(CommitParams P) {
       if (x != k) {
         const int sx = P.stamp[x];
         if (sx == remove_stamp && P.seq[x] < my_seq && RowLookup(rr, lr, P.partner[x]) != 0) folded = 1;
-        if ((sx >> 1) != P.block_stamp && atomicExch(&P.claim[x], P.block_stamp) != P.block_stamp) {
-          if (Q.len[x] <= kWarpRowMax) {
-            P.rows_short[atomicAdd(&P.ctl->short_cnt, 1u)] = x;
-          } else {
-            P.rows_long[atomicAdd(&P.ctl->long_cnt, 1u)] = x;
-          }
-        }
+        if ((sx >> 1) != P.block_stamp) ClaimRow(P, x);
       }
     }
     const int folded_sum = __popc(__ballot_sync(0xffffffffu, folded != 0));
@@ -3082,7 +3125,8 @@ __device__ void RewriteShortRows(const CommitParams& P, RowsSmem& R) {
   }
 }
 
-// Claimed neighbour rows longer than kWarpRow entries, one CTA per row.
+// Claimed neighbour rows of kWarpRowMax < L <= kRowSmem entries, one CTA per
+// row, staged in shared memory.
 __device__ void RewriteLongRows(const CommitParams& P, RowsSmem& R) {
   const QuotientView& Q = P.Q;
   const unsigned cnt = P.ctl->long_cnt;
@@ -3090,12 +3134,9 @@ __device__ void RewriteLongRows(const CommitParams& P, RowsSmem& R) {
     const int x = P.rows_long[idx];
     Entry* rowp = Q.ent + Q.off[x];
     const int lx = Q.len[x];
-    Entry *S2, *INS2;
-    int* D2;
-    if (!StageBuffers(P, R, lx, &S2, &D2, &INS2)) return;
-    for (int i = threadIdx.x; i < lx; i += kRowsThreads) S2[i] = rowp[i];
+    for (int i = threadIdx.x; i < lx; i += kRowsThreads) R.s[i] = rowp[i];
     __syncthreads();
-    const int nlx = RewriteRow(P, S2, lx, D2, INS2, -1, -1, rowp);
+    const int nlx = RewriteRow(P, R.s, lx, R.d, R.ins, -1, -1, rowp);
     if (threadIdx.x == 0) {
       Q.len[x] = nlx;
       atomicAdd(&P.stats[kStRowsRewritten], 1ull);
@@ -3106,25 +3147,232 @@ __device__ void RewriteLongRows(const CommitParams& P, RowsSmem& R) {
   }
 }
 
-// All claimed neighbour rows of a block: the long ones by whole CTAs first,
-// then the short ones by single warps.
+// First step of the longer rows, a warp per kHugeUnit entries: marks the
+// entries of supernodes removed in this block, adds each one's count to its
+// keep's entry in the row (ids stay in place, so the row stays searchable) or
+// lists it for insertion.
+__device__ void ScanHugeRows(const CommitParams& P) {
+  constexpr int kDeep = 8;
+  const QuotientView& Q = P.Q;
+  const int lane = threadIdx.x & 31;
+  const unsigned units = P.ctl->huge_units;
+  const int remove_stamp = 2 * P.block_stamp + 1;
+  const unsigned nw = (gridDim.x * blockDim.x) >> 5;
+  for (unsigned u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units; u += nw) {
+    const int2 unit = P.huge_units[u];
+    HugeRow* h = P.rows_huge + unit.x;
+    const int x = h->x, len = h->len;
+    unsigned* mask = h->mask;
+    Entry* row = Q.ent + Q.off[x];
+    const int end = unit.y + kHugeUnit < len ? unit.y + kHugeUnit : len;
+    for (int i0 = unit.y; i0 < end; i0 += 32 * kDeep) {
+      Entry e[kDeep];
+      int st[kDeep];
+#pragma unroll
+      for (int d = 0; d < kDeep; ++d) {
+        const int i = i0 + 32 * d + lane;
+        e[d] = i < end ? row[i] : 0;
+      }
+#pragma unroll
+      for (int d = 0; d < kDeep; ++d) {
+        const int i = i0 + 32 * d + lane;
+        st[d] = i < end ? P.stamp[EntNb(e[d])] : 0;
+      }
+#pragma unroll
+      for (int d = 0; d < kDeep; ++d) {
+        const bool renamed = st[d] == remove_stamp;
+        const unsigned m = __ballot_sync(0xffffffffu, renamed);
+        if (lane == 0 && i0 + 32 * d < end) mask[(i0 >> 5) + d] = m;
+        if (renamed) {
+          const int kp = P.partner[EntNb(e[d])];
+          const long long c = EntCnt(e[d]);
+          const int p = RowLowerBound(row, len, kp);
+          if (p < len && EntNb(row[p]) == kp) {
+            atomicAdd(&row[p], static_cast<unsigned long long>(c));
+          } else {
+            h->ins[atomicAdd(&h->nins, 1)] = MakeEnt(kp, c);
+          }
+        }
+      }
+    }
+  }
+}
+
+// All claimed neighbour rows of a block: the long ones by whole CTAs, then the
+// first step of the longest, then the short ones by single warps.
 __global__ void __launch_bounds__(kRowsThreads) RewriteRowsKernel(CommitParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RowsSmem& R = *reinterpret_cast<RowsSmem*>(smem_raw);
-  __shared__ bool last;
+  ScanHugeRows(P);
   RewriteLongRows(P, R);
   __syncthreads();  // the shared buffers pass from the CTA's long rows to its warps
   RewriteShortRows(P, R);
-  // the last CTA to finish clears the block control words for the next
-  // block (every CTA has read them and made its scratch allocations by now)
-  __threadfence();
+}
+
+struct HugeSmem {
+  Entry ins[kHugeChunk];
+  int at[kHugeChunk];  // per inserted entry: first staying or renamed entry above it
+  unsigned word[kHugeChunk / 32];
+  int before[kHugeChunk / 32];  // renamed entries of the chunk before each mask word
+  int deleted;                  // renamed entries of the chunk
+};
+
+// Renamed entries before position p of the row: `base` of them before the
+// chunk, whose mask words are staged.
+__device__ __forceinline__ int RenamedBefore(const HugeSmem& H, int base, int p_in_chunk) {
+  const int w = p_in_chunk >> 5;
+  return base + H.before[w] + __popc(H.word[w] & ((1u << (p_in_chunk & 31)) - 1u));
+}
+
+// Stages a chunk's mask words and their running counts; all threads, with
+// barriers (words past the row read as zero).
+__device__ void StageMask(HugeSmem& H, const unsigned* mask, int base, int len) {
+  constexpr int kWords = kHugeChunk / 32;
+  const int words = (len + 31) / 32;
+  for (int w = threadIdx.x; w < kWords; w += kHugeThreads) {
+    H.word[w] = base / 32 + w < words ? mask[base / 32 + w] : 0u;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(P.ticket, 1u) == gridDim.x - 1;
+  if (threadIdx.x < 32) {
+    constexpr int kPer = kWords / 32;
+    int v[kPer], sum = 0;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      v[u] = __popc(H.word[threadIdx.x * kPer + u]);
+      sum += v[u];
+    }
+    int incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (static_cast<int>(threadIdx.x) >= o) incl += y;
+    }
+    int run = incl - sum;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      H.before[threadIdx.x * kPer + u] = run;
+      run += v[u];
+    }
+    if (threadIdx.x == 31) H.deleted = incl;
+  }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
+}
+
+// Second step of the longest rows, a CTA per row: without its renamed entries
+// and with the inserted ones, in place. An entry moves left by the renamed
+// entries before it and right by the inserted ones below it, at most
+// kHugeChunk of them: every chunk is in registers before the one before it is
+// written, so nothing unread is overwritten. (A row with more to insert
+// goes through a copy.) One CTA with everything
+// staged in global memory took 431 us for a row of 27,500 entries, most of it
+// in dependent loads; the split takes the loads of the scan off that chain.
+// The last CTA clears the block control words for the next block: all their
+// readers are done by then.
+__global__ void __launch_bounds__(kHugeThreads) RewriteHugeKernel(CommitParams P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  HugeSmem& H = *reinterpret_cast<HugeSmem*>(smem_raw);
+  __shared__ bool last;
+  const QuotientView& Q = P.Q;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const unsigned cnt = P.ctl->huge_cnt;
+  for (unsigned idx = blockIdx.x; idx < cnt; idx += gridDim.x) {
+    const HugeRow h = P.rows_huge[idx];
+    const int len = h.len, m = h.nins;
+    Entry* row = Q.ent + Q.off[h.x];
+    int pow2 = 1;
+    while (pow2 < m) pow2 <<= 1;
+    const bool in_place = m <= kHugeChunk;
+    Entry* ins = in_place ? H.ins : h.ins;
+    if (in_place) {
+      for (int j = tid; j < m; j += kHugeThreads) ins[j] = h.ins[j];
+    }
+    for (int j = m + tid; j < pow2; j += kHugeThreads) ins[j] = ~0ull;
+    __syncthreads();
+    if (m > 1) CtaBitonicSort(ins, pow2);
+    int deleted = 0;  // renamed entries before the chunk
+    if (in_place) {
+      for (int j = tid; j < m; j += kHugeThreads) H.at[j] = RowLowerBound(row, len, EntNb(ins[j]));
+      Entry cur[kHugePer], nxt[kHugePer];
+#pragma unroll
+      for (int d = 0; d < kHugePer; ++d) {
+        const int i = d * kHugeThreads + tid;
+        cur[d] = i < len ? row[i] : 0;
+      }
+      for (int base = 0; base < len; base += kHugeChunk) {
+#pragma unroll
+        for (int d = 0; d < kHugePer; ++d) {
+          const int i = base + kHugeChunk + d * kHugeThreads + tid;
+          nxt[d] = i < len ? row[i] : 0;
+        }
+        StageMask(H, h.mask, base, len);
+        // ends with a barrier: the next chunk is in registers everywhere
+#pragma unroll
+        for (int d = 0; d < kHugePer; ++d) {
+          const int in = d * kHugeThreads + tid;
+          const int i = base + in;
+          if (i < len && !((H.word[in >> 5] >> lane) & 1u)) {
+            int lo = 0, hi = m;  // inserted entries at or before this position
+            while (lo < hi) {
+              const int mid = (lo + hi) >> 1;
+              if (H.at[mid] <= i) lo = mid + 1; else hi = mid;
+            }
+            const int to = i - RenamedBefore(H, deleted, in) + lo;
+            if (to != i) row[to] = cur[d];
+          }
+        }
+        const bool last_chunk = base + kHugeChunk >= len;
+        for (int j = tid; j < m; j += kHugeThreads) {
+          const int p = H.at[j];
+          if (p < base || (p >= base + kHugeChunk && !last_chunk)) continue;
+          // p == len: past the last word of a full last chunk
+          const int before = p - base < kHugeChunk ? RenamedBefore(H, deleted, p - base) : deleted + H.deleted;
+          row[j + p - before] = ins[j];
+        }
+        deleted += H.deleted;
+        __syncthreads();  // the staged words are replaced
+#pragma unroll
+        for (int d = 0; d < kHugePer; ++d) cur[d] = nxt[d];
+      }
+    } else {
+      for (int i = tid; i < len; i += kHugeThreads) h.copy[i] = row[i];
+      __syncthreads();
+      for (int base = 0; base < len; base += kHugeChunk) {
+        StageMask(H, h.mask, base, len);
+        const bool last_chunk = base + kHugeChunk >= len;
+        for (int in = tid; in < kHugeChunk && base + in < len; in += kHugeThreads) {
+          if ((H.word[in >> 5] >> (in & 31)) & 1u) continue;
+          const Entry e = h.copy[base + in];
+          row[base + in - RenamedBefore(H, deleted, in) + RowLowerBound(ins, m, EntNb(e))] = e;
+        }
+        for (int j = tid; j < m; j += kHugeThreads) {
+          const int p = RowLowerBound(h.copy, len, EntNb(ins[j]));
+          if (p < base || (p >= base + kHugeChunk && !last_chunk)) continue;
+          const int before = p - base < kHugeChunk ? RenamedBefore(H, deleted, p - base) : deleted + H.deleted;
+          row[j + p - before] = ins[j];
+        }
+        deleted += H.deleted;
+        __syncthreads();
+      }
+    }
+    if (tid == 0) {
+      const int nl = len - deleted + m;
+      Q.len[h.x] = nl;
+      atomicAdd(&P.stats[kStRowsRewritten], 1ull);
+      atomicAdd(&P.stats[kStRowEntriesRewritten], static_cast<unsigned long long>(len));
+      atomicAdd(&P.stats[kStUpdateBytes], 8ull * (len + nl));
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(P.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last && tid == 0) {
     P.ctl->scratch_top = 0;
     P.ctl->short_cnt = 0;
     P.ctl->long_cnt = 0;
+    P.ctl->huge_cnt = 0;
+    P.ctl->huge_units = 0;
     P.ctl->sel_total = 0;
     P.ctl->work_next[0] = 0;
     P.ctl->work_next[1] = 0;
@@ -3162,6 +3410,8 @@ void Engine::ConfigureKernels() {
                                  static_cast<int>(sizeof(RowsSmem))), "commit smem attribute");
   CheckCuda(cudaFuncSetAttribute(RewriteRowsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(sizeof(RowsSmem))), "rewrite smem attribute");
+  CheckCuda(cudaFuncSetAttribute(RewriteHugeKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(sizeof(HugeSmem))), "long-row rewrite smem attribute");
   // the queue-fed kernels launch exactly the CTAs that fit on the GPU at once
   int sms = 0, per_sm = 0;
   CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg_.device), "SM count");
@@ -3710,6 +3960,11 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify) {
   C.err = d_err_.p;
   C.rows_short = d_rows_short_.p;
   C.rows_long = d_rows_long_.p;
+  // a row of more than kRowSmem entries holds that many of the arcs
+  d_rows_huge_.ensure(sizeof(HugeRow) * (static_cast<size_t>(arcs_) / kRowSmem + 1));
+  d_huge_units_.ensure(static_cast<size_t>(arcs_) / kHugeUnit + static_cast<size_t>(arcs_) / kRowSmem + 1);
+  C.rows_huge = reinterpret_cast<HugeRow*>(d_rows_huge_.p);
+  C.huge_units = d_huge_units_.p;
   C.ticket = d_rw_ticket_.p;
   C.sel_list = d_sel_list_.p;
   // warp-per-pair commit for short pairs, except in small blocks, where one
@@ -3733,6 +3988,8 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify) {
   CommitKernel<<<grid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
   ++launches_;
   RewriteRowsKernel<<<kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
+  ++launches_;
+  RewriteHugeKernel<<<kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_>>>(C);
   EndTimed(kTimeUpdate);
 }
 
@@ -3841,7 +4098,7 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
   const long long slots = bp.slots;
   const long long sel_slots = bp.sel_slots;
   // the block control words are zero: cleared by Merge before the first
-  // block and by the previous block's rewrite kernel
+  // block and by the previous block's last kernel
   LaunchPrepare(bp);
   ScoreParams SP;
   SP.Q = View();

@@ -1,0 +1,47 @@
+"""Neighbour rows longer than the rewrite kernels stage in shared memory
+(beam_gb300/csrc/merge.cu, ScanHugeRows and RewriteHugeKernel): a hub's row
+after an explicit batch of merges of its neighbours, against the row made from
+the merged ids. Lengths around the row limit and the chunk size; entries that
+fold into one already there, that move left, that move right, and more
+insertions than a chunk holds."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_graph(length, outside, low):
+    """Hub with `length` neighbours and as many nodes as `outside` not listed by
+    it (tied to one another), with ids below (low) or above the neighbours."""
+    a, b = (1, 1 + outside) if low else (1 + length, 1)
+    out, nbr = np.arange(a, a + outside), np.arange(b, b + length)
+    u = np.concatenate([np.zeros(length, np.int32), out[:-1]]).astype(np.int32)
+    v = np.concatenate([nbr, out[1:]]).astype(np.int32)
+    return u, v, out, nbr
+
+
+@pytest.mark.parametrize("length", [2048, 2049, 8191, 8192, 8193, 16384, 20011])
+@pytest.mark.parametrize("kind", ["fold", "left", "right", "mixed", "all_right"])
+def test_hub_row_after_merges(length, kind):
+    from beam_gb300 import Engine, Graph
+    rng = np.random.default_rng(length)
+    count = {"all_right": length, "fold": length // 2}.get(kind, min(length, 97))
+    u, v, out, nbr = hub_graph(length, max(2, count), kind in ("right", "all_right", "mixed"))
+    g = Graph.from_edges(u, v)
+    picked = rng.permutation(nbr)
+    if kind == "fold":      # both ends are listed by the hub
+        keep, rem = picked[:count], picked[count:2 * count]
+    else:                   # the kept end is not
+        keep, rem = rng.permutation(out)[:count], picked[:count]
+        if kind == "mixed":
+            keep, rem = np.concatenate([keep, picked[count:count + 40]]), np.concatenate([rem, picked[count + 40:count + 80]])
+    into = np.arange(g.n)
+    into[rem] = keep
+    with Engine(g) as e:
+        e.merge_pairs(keep, rem)
+        got_nb, got_cnt, _, _ = e.row(0)
+        ids, counts = np.unique(into[nbr], return_counts=True)
+        assert np.array_equal(got_nb, ids)
+        assert np.array_equal(got_cnt, counts)
+        e.validate_quotient()
