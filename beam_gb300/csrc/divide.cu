@@ -618,7 +618,8 @@ void Engine::Divide(int iter) {
   // one block of every group: Merge plans the iteration on the device from
   // d_glen_ / d_gent_, so nothing is read back here
   plan_on_device_ = static_cast<long long>(cfg_.group_batch_size) >= static_cast<long long>(segs);
-  if (!plan_on_device_) {
+  windowed_ = !plan_on_device_ && WindowsOn();
+  if (!plan_on_device_ && !windowed_) {
     h_glen_.resize(static_cast<size_t>(segs));
     h_gent_.resize(static_cast<size_t>(segs));
     if (segs > 0) {

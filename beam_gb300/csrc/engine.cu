@@ -273,6 +273,8 @@ void Engine::Reset() {
   CheckCuda(cudaMemsetAsync(d_err_.p, 0, sizeof(DevError), stream_), "memset err");
   CheckCuda(cudaMemsetAsync(d_ctl_.p, 0, sizeof(BlockCtl), stream_), "memset ctl");
   CheckCuda(cudaMemsetAsync(d_rw_ticket_.p, 0, sizeof(unsigned), stream_), "memset ticket");
+  d_wctl_.ensure(256);
+  CheckCuda(cudaMemsetAsync(d_wctl_.p, 0, 256, stream_), "memset window control");
   ++launches_;
   InitRowsKernel<<<152 * 16, 256, 0, stream_>>>(d_rowptr_.p, d_col_.p, n_, d_pool_[0].p, d_qoff_.p, d_qlen_.p,
                                                 d_qcap_.p, d_arc_src_.p, d_err_.p);

@@ -241,14 +241,17 @@ class Engine {
   void RankerFinishIteration();
   void LaunchPrepare(const BlockPlan& bp);
   bool RowSumsOn() const;
+  bool WindowsOn() const;
+  void RunWindows(double threshold);
   void PlanOnDevice();
-  void SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nbig, long long max_mat, long long max_slots);
+  void SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nbig, long long max_mat, long long max_slots,
+                            bool windows);
   void PrepareIterationBuffers();
   void BeginTimed(int which);
   void EndTimed(int which);
   void ConfigureKernels();
   QuotientView View();
-  void LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify);
+  void LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, const void* window);
 
   int n_;
   int64_t arcs_;
@@ -333,6 +336,12 @@ class Engine {
   // and per candidate slot
   DevBuf<unsigned char> d_rc_, d_info_;
   bool plan_on_device_ = false;
+  // windows of blocks (window.cuh)
+  bool windowed_ = false;
+  DevBuf<int> d_ri_of_, d_node_ri_, d_blk_end_, d_dirty_, d_win_list_;
+  DevBuf<long long> d_win_off_;
+  DevBuf<int> d_conflict_;
+  DevBuf<unsigned char> d_gs_, d_wctl_, d_units_;
   int accum_grid_ = 152 * 4;  // resident CTAs of the dynamically scheduled kernels
   int score_grid_ = 152 * 4;   // one-block iteration: Merge plans it on the device
   DevBuf<unsigned char> d_plan_tiles_;

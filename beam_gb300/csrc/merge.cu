@@ -72,6 +72,13 @@ constexpr int kHugeChunk = kHugeThreads * kHugePer;
 constexpr int kHugeGrid = 152;
 constexpr int kKeyIdxBits = 10;      // a_idx, b_idx < kMaxGroup
 constexpr long long kKeyGainMax = (1ll << (64 - 2 * kKeyIdxBits)) - 1;
+constexpr unsigned long long kKeyIdxMask = (1ull << kKeyIdxBits) - 1;
+
+// Selection key: ascending order is g0's (gain desc, a_idx asc, b_idx asc).
+__device__ __forceinline__ unsigned long long PackKey(long long gain, int a, int b) {
+  return (static_cast<unsigned long long>(kKeyGainMax - gain) << (2 * kKeyIdxBits)) |
+         (static_cast<unsigned long long>(a) << kKeyIdxBits) | static_cast<unsigned long long>(b);
+}
 
 __device__ __forceinline__ unsigned long long* ScratchAlloc(unsigned char* base, unsigned long long cap,
                                                            BlockCtl* ctl, unsigned long long bytes,
@@ -1067,10 +1074,10 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
 
 // Top-k partners of member i of a big group whose partners fill NT slots of
 // 32 (the fp32 prescreen branch of PrepareMembersKernel).
-template <int NT>
+template <int NT, typename KeepFn>
 __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int top_k, int cnt,
                                             const unsigned long long* pmat, const long long* old, long long old_i, const int* q, int* cj,
-                                            unsigned char* fmat) {
+                                            KeepFn keep) {
   auto ratio_of = [&](int j, long long pg) {
     long long denom = old_i + old[j];
     if (denom < 1) denom = 1;
@@ -1169,7 +1176,7 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     if (have && rank < top_k) {
       const int a = i < mine.j ? i : mine.j;
       const int b = i < mine.j ? mine.j : i;
-      fmat[static_cast<long long>(a) * g + b] = 1;
+      keep(a, b);
     }
   } else {
     // each lane keeps its best top_k candidates sorted, then the warp merges
@@ -1223,36 +1230,25 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
       if (lane == 0) {
         const int a = i < best.j ? i : best.j;
         const int b = i < best.j ? best.j : i;
-        fmat[static_cast<long long>(a) * g + b] = 1;
+        keep(a, b);
       }
     }
   }
 }
 
-// Member pass of the big groups: one warp per member of every group in the
-// launch's big-group list (moff = prefix of the member counts), so a large
-// group's members are ranked by the whole GPU instead of one CTA.
-__global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
-  __shared__ int cand_j[8][32];  // per warp: the candidates that survive the prescreen
+// Member i of a big group (members q, pair tables mat) by one warp: keep(a, b)
+// is called for the pair of each of its top_k partners, by some lane. cj: 32
+// words of the warp's own.
+template <typename KeepFn>
+__device__ __forceinline__ void RankMember(int g, int i, const int* q, const unsigned char* mat, int top_k_max, int* cj,
+                                           KeepFn keep) {
   const int lane = threadIdx.x & 31;
-  const long long wg = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long total = P.moff[P.list0 + P.nlist] - P.moff[P.list0];
-  if (wg >= total) return;
-  const long long target = P.moff[P.list0] + wg;
-  const int lo = WarpLastLE(P.moff, P.list0, P.list0 + P.nlist, target);  // last entry with moff <= target
-  const int ri = P.list[lo];
-  const int i = static_cast<int>(target - P.moff[lo]);
-  const int gid = P.real[ri];
-  const int g = P.glen[gid];
-  const int* q = P.order + P.gstart[gid];
   const long long gg = static_cast<long long>(g) * g;
-  unsigned char* mat = P.mat + P.mat_off[ri];
   const unsigned long long* pmat = reinterpret_cast<const unsigned long long*>(mat);
-  unsigned char* fmat = mat + FlagOffset(gg);
   const long long* old = reinterpret_cast<const long long*>(mat + OldCostOffset(gg));
-  // per member: candidates with positive proxy, ratio, top-k (the ratio is
-  // recomputed where it is needed instead of being stored)
-  int top_k = P.top_k < g - 1 ? P.top_k : g - 1;
+  // candidates with positive proxy, ratio, top-k (the ratio is recomputed where
+  // it is needed instead of being stored)
+  int top_k = top_k_max < g - 1 ? top_k_max : g - 1;
   if (top_k < 1) top_k = 1;
   const long long old_i = old[i];
   auto ratio_of = [&](int j, long long pg) {
@@ -1273,21 +1269,20 @@ __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
       if (j == i || ProxyOf(PairWord(pmat, g, i, j)) <= 0) continue;
       const int a = i < j ? i : j;
       const int b = i < j ? j : i;
-      fmat[static_cast<long long>(a) * g + b] = 1;
+      keep(a, b);
     }
   } else if (top_k <= kLaneTopK) {
-    int* cj = cand_j[threadIdx.x >> 5];
     const int nt = (g + 31) >> 5;
     if (nt <= 1) {
-      MembersTopK<1>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
+      MembersTopK<1>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
     } else if (nt <= 2) {
-      MembersTopK<2>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
+      MembersTopK<2>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
     } else if (nt <= 4) {
-      MembersTopK<4>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
+      MembersTopK<4>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
     } else if (nt <= 8) {
-      MembersTopK<8>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
+      MembersTopK<8>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
     } else {
-      MembersTopK<kMaxGroup / 32>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, fmat);
+      MembersTopK<kMaxGroup / 32>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
     }
   } else {
     RankKey prev;
@@ -1329,12 +1324,32 @@ __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
       if (lane == 0) {
         const int a = i < best.j ? i : best.j;
         const int b = i < best.j ? best.j : i;
-        fmat[static_cast<long long>(a) * g + b] = 1;
+        keep(a, b);
       }
       prev = best;
       have_prev = true;
     }
   }
+}
+
+// Member pass of the big groups: one warp per member of every group in the
+// launch's big-group list (moff = prefix of the member counts), so a large
+// group's members are ranked by the whole GPU instead of one CTA.
+__global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
+  __shared__ int cand_j[8][32];  // per warp: the candidates that survive the prescreen
+  const long long wg = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const long long total = P.moff[P.list0 + P.nlist] - P.moff[P.list0];
+  if (wg >= total) return;
+  const long long target = P.moff[P.list0] + wg;
+  const int lo = WarpLastLE(P.moff, P.list0, P.list0 + P.nlist, target);  // last entry with moff <= target
+  const int ri = P.list[lo];
+  const int i = static_cast<int>(target - P.moff[lo]);
+  const int gid = P.real[ri];
+  const int g = P.glen[gid];
+  const int* q = P.order + P.gstart[gid];
+  unsigned char* fmat = P.mat + P.mat_off[ri] + FlagOffset(static_cast<long long>(g) * g);
+  RankMember(g, i, q, P.mat + P.mat_off[ri], P.top_k, cand_j[threadIdx.x >> 5],
+             [&](int a, int b) { fmat[static_cast<long long>(a) * g + b] = 1; });
 }
 
 // Flag bytes (0 or 1) of table word w that lie in [beg, end), as a bit set
@@ -1468,31 +1483,46 @@ __global__ void __launch_bounds__(kPrepThreads) PrepareOutputKernel(PrepareParam
 // shared memory in one coalesced pass; the EA-proxy sum over targets shared by
 // two members then equals, per member pair, the sum over the intersection of
 // their two sorted rows (a row never holds its own rep, so the reference's
-// own-rep exclusion is implied), which one lane computes per pair with a
-// two-pointer merge while the other lanes do the other pairs. Output and
-// counters equal those of PrepareKernel.
+// own-rep exclusion is implied). One lane per staged entry looks its target up
+// in the rows of the later members and adds what it finds to the pair's sums in
+// shared memory: the lanes' work is even, where a lane per pair merging two
+// rows made the group wait for its longest row. Output and counters equal
+// those of PrepareKernel.
 constexpr int kSmallGroup = 32;
 constexpr int kSmallWarps = 4;
 constexpr int kSmallPairs = kSmallGroup * (kSmallGroup - 1) / 2;
 constexpr int kSmallStage = 256;  // staged row entries per group
-// Pair sums are kept in 32 bits where the group's counts sum to less than
-// this (every term is at most 4 counts); other groups merge a pair's rows
-// again whenever they need its sums.
+// Sums are kept in 32 bits where the group's counts sum to less than this
+// (every term is at most 4 counts); the other groups, and those with a count
+// beyond its block's capacity, merge a pair's rows again whenever they need
+// its sums.
 constexpr long long kSmallNarrow = 1ll << 28;
-constexpr unsigned kSmallBad = 1u << 15;  // flag of SmallWarpSmem::ovl
 
-struct SmallWarpSmem {
+struct SmallRowsSmem {
   long long old[kSmallGroup];
   long long off[kSmallGroup];
   Entry ent[kSmallStage];
-  unsigned p[kSmallPairs];  // upper triangle, TriIndex(a, b)
-  int corr[kSmallPairs];
-  unsigned short ovl[kSmallPairs];
+  HeavyAcc heavy[kSmallGroup];
   int tsz[kSmallStage];
+  unsigned light[kSmallGroup];
+  unsigned char row[kSmallStage];  // member of the entry
   int q[kSmallGroup];
   int sz[kSmallGroup];
   int start[kSmallGroup + 1];
   unsigned fmask[kSmallGroup];
+};
+
+// Pair sums, upper triangle by TriIndex(a, b): proxy << 32 | corr, and the
+// number of shared targets (at most kSmallStage / 2 of them: a byte each).
+template <int kPairs>
+struct SmallPairsSmem {
+  unsigned long long pc[kPairs];
+  unsigned ovl[(kPairs + 3) / 4];
+};
+
+struct SmallWarpSmem {
+  SmallRowsSmem rows;
+  SmallPairsSmem<kSmallPairs> pairs;
 };
 
 struct SmallSmem {
@@ -1500,6 +1530,25 @@ struct SmallSmem {
 };
 
 __device__ __forceinline__ int TriIndex(int a, int b, int g) { return a * (2 * g - a - 1) / 2 + (b - a - 1); }
+
+// The pair at a position of the upper triangle.
+__device__ __forceinline__ void TriPair(int pidx, int g, int* a, int* b) {
+  int x = 0, rem = pidx;
+  if (g > kSmallGroup) {
+    // a is near the root of a * (2g - a - 1) / 2 = pidx
+    const float d = (2.0f * g - 1.0f) * (2.0f * g - 1.0f) - 8.0f * static_cast<float>(pidx);
+    x = static_cast<int>((2.0f * g - 1.0f - sqrtf(d > 0.0f ? d : 0.0f)) * 0.5f);
+    x = x < 0 ? 0 : x > g - 2 ? g - 2 : x;
+    while (x > 0 && TriIndex(x, x + 1, g) > pidx) --x;
+    rem = pidx - TriIndex(x, x + 1, g);
+  }
+  while (rem >= g - 1 - x) {
+    rem -= g - 1 - x;
+    ++x;
+  }
+  *a = x;
+  *b = x + 1 + rem;
+}
 
 // Members a < b of a staged group by one lane.
 struct SmallPair {
@@ -1509,7 +1558,7 @@ struct SmallPair {
   bool bad;
 };
 
-__device__ __forceinline__ SmallPair SmallMerge(const SmallWarpSmem& S, int a, int b) {
+__device__ __forceinline__ SmallPair SmallMerge(const SmallRowsSmem& S, int a, int b) {
   const int qb = S.q[b];
   const long long sa = S.sz[a], sb = S.sz[b];
   int ia = S.start[a], ib = S.start[b];
@@ -1540,21 +1589,27 @@ __device__ __forceinline__ SmallPair SmallMerge(const SmallWarpSmem& S, int a, i
   return r;
 }
 
-__device__ __forceinline__ long long StagedLookup(const SmallWarpSmem& S, int a, int key) {
+__device__ __forceinline__ long long StagedLookup(const SmallRowsSmem& S, int a, int key) {
   return RowLookup(S.ent + S.start[a], S.start[a + 1] - S.start[a], key);
 }
 
-__global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PrepareParams P) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmallWarpSmem& S = reinterpret_cast<SmallSmem*>(smem_raw)->w[threadIdx.x >> 5];
+__device__ __forceinline__ PairInfo SmallPairInfo(const SmallRowsSmem& S, int a, int b, const SmallPair& r) {
+  const long long ea = StagedLookup(S, a, S.q[b]);
+  const long long eb = StagedLookup(S, b, S.q[a]);
+  PairInfo pi;
+  pi.shared = r.corr - (r.proxy - ea);
+  pi.ovl = static_cast<unsigned>(r.ovl) | (r.bad ? kPairBad : 0u) | (ea != eb ? kPairAsym : 0u);
+  pi.eab = static_cast<unsigned>(ea);
+  return pi;
+}
+
+// Stages a group's rows and their target sizes: one flat pass over the entries
+// (independent loads), then the sizes. Returns the entries, nothing staged when
+// they are more than kSmallStage (not by the plan: row entries counted at
+// Divide time only shrink); wide: the group's counts reach kSmallNarrow.
+__device__ __forceinline__ int StageSmallRows(const QuotientView& Q, const int* order, int g, SmallRowsSmem& S,
+                                              bool* wide) {
   const int lane = threadIdx.x & 31;
-  const int li = blockIdx.x * kSmallWarps + (threadIdx.x >> 5);
-  if (li >= P.nlist) return;
-  const int ri = P.list[P.list0 + li];
-  const int gid = P.real[ri];
-  const int g = P.glen[gid];
-  const QuotientView& Q = P.Q;
-  const int* order = P.order + P.gstart[gid];
   int len = 0;
   if (lane < g) {
     const int rep = order[lane];
@@ -1564,7 +1619,6 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
     S.off[lane] = Q.off[rep];
     S.fmask[lane] = 0;
   }
-  // row starts in the staging buffer
   int incl = len;
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -1573,17 +1627,9 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
   const int E = __shfl_sync(0xffffffffu, incl, 31);
   if (lane < g) S.start[lane] = incl - len;
   if (lane == 0) S.start[g] = E;
-  const int npairs = g * (g - 1) / 2;
-  if (E > kSmallStage) {  // not by the plan: row entries counted at Divide time only shrink
-    if (lane == 0) {
-      RaiseError(P.err, kErrSlots, gid, E, 0);
-      P.cand_cnt[ri] = 0;
-    }
-    return;
-  }
+  *wide = false;
+  if (E > kSmallStage) return E;
   __syncwarp();
-  // one flat pass over the group's entries (independent loads), then the
-  // target sizes
   long long counts = 0;
 #pragma unroll 4
   for (int k = lane; k < E; k += 32) {
@@ -1594,60 +1640,166 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
     }
     const Entry e = Q.ent[S.off[lo] + (k - S.start[lo])];
     S.ent[k] = e;
+    S.row[k] = static_cast<unsigned char>(lo);
     counts += EntCnt(e);
   }
   __syncwarp();
 #pragma unroll 4
   for (int k = lane; k < E; k += 32) S.tsz[k] = Q.size[EntNb(S.ent[k])];
-  const bool wide = WarpSum(counts) >= kSmallNarrow;
+  *wide = WarpSum(counts) >= kSmallNarrow;
   __syncwarp();
-  unsigned long long examined = 0;
-  // approximate old cost: one lane per member
+  return E;
+}
+
+// The staged group's row sums and pair sums, by a warp: S.old (with the
+// internal term), S.light and S.heavy per member, and the pair sums. Returns
+// the shared targets visited; *slow: the 32-bit sums do not hold, SmallMerge
+// gives the pairs'.
+template <int kPairs>
+__device__ __forceinline__ unsigned SmallSums(const QuotientView& Q, SmallRowsSmem& S, SmallPairsSmem<kPairs>& T, int g,
+                                              int E, bool wide, bool* slow) {
+  const int lane = threadIdx.x & 31;
+  const int npairs = g * (g - 1) / 2;
+  for (int k = lane; k < npairs; k += 32) T.pc[k] = 0;
+  for (int k = lane; k < (npairs + 3) / 4; k += 32) T.ovl[k] = 0;
+  unsigned examined = 0;
+  bool any_bad = false;
   if (lane < g) {
-    const int rep = S.q[lane];
-    const long long si = S.sz[lane];
-    long long old = 0, light = 0;
-    HeavyAcc heavy;
-    for (int k = S.start[lane]; k < S.start[lane + 1]; ++k) {
-      const long long c = EntCnt(S.ent[k]);
-      const long long st = S.tsz[k];
-      old += EncodeCostForPair(rep, si, EntNb(S.ent[k]), st, c);
-      if (HeavyEntry(si, st, c)) heavy.Add(st, c); else light += c;
-    }
-    const long long internal = Q.internal[rep];
-    if (P.rc) StoreRowSums(&P.rc[rep], old, light, heavy, internal, S.sz[lane], len);
-    if (internal > 0) old += EncodeCostForPair(rep, si, rep, si, 2 * internal);
-    S.old[lane] = old;
-  }
-  // pair sums: one lane per member pair
-  for (int pidx = lane; pidx < npairs; pidx += 32) {
-    int a = 0, rem = pidx;
-    while (rem >= g - 1 - a) {
-      rem -= g - 1 - a;
-      ++a;
-    }
-    const SmallPair r = SmallMerge(S, a, a + 1 + rem);
-    examined += static_cast<unsigned long long>(r.ovl);
-    if (!wide) {
-      S.p[pidx] = static_cast<unsigned>(r.proxy);
-      S.corr[pidx] = static_cast<int>(r.corr);
-      S.ovl[pidx] = static_cast<unsigned short>(static_cast<unsigned>(r.ovl) | (r.bad ? kSmallBad : 0u));
-    }
+    S.heavy[lane] = HeavyAcc();
+    S.old[lane] = 0;
+    S.light[lane] = 0;
   }
   __syncwarp();
-  auto proxy_of = [&](int a, int b) {  // a < b
-    return wide ? SmallMerge(S, a, b).proxy : static_cast<long long>(S.p[TriIndex(a, b, g)]);
-  };
-  // per member (one lane each): positive partners, ratio, top-k
-  int top_k = P.top_k < g - 1 ? P.top_k : g - 1;
+  if (!wide) {
+    for (int k0 = 0; k0 < E; k0 += 32) {
+      const int k = k0 + lane;
+      if (k >= E) continue;
+      const Entry e = S.ent[k];
+      const int t = EntNb(e), i = S.row[k];
+      const long long c = EntCnt(e), st = S.tsz[k], si = S.sz[i];
+      // row sums: below 2^28 in all, so the low words hold them
+      const long long alt = 1 + si * st - c;
+      const long long old = c < alt ? c : alt;
+      if (old >= 0) {
+        atomicAdd(reinterpret_cast<unsigned*>(&S.old[i]), static_cast<unsigned>(old));
+      } else {
+        atomicAdd(reinterpret_cast<unsigned long long*>(&S.old[i]), static_cast<unsigned long long>(old));
+      }
+      if (HeavyEntry(si, st, c)) {
+        HeavyAcc h;
+        h.Add(st, c);
+        HeavyAcc* a = &S.heavy[i];
+        atomicAdd(reinterpret_cast<unsigned long long*>(&a->sx), static_cast<unsigned long long>(h.sx));
+        atomicAdd(reinterpret_cast<unsigned long long*>(&a->c), static_cast<unsigned long long>(h.c));
+        atomicMin(&a->smin, h.smin);
+        atomicMax(&a->smax, h.smax);
+        atomicMax(&a->sbad, h.sbad);
+        atomicAdd(&a->n, 1);
+      } else {
+        atomicAdd(&S.light[i], static_cast<unsigned>(c));
+      }
+      for (int j = i + 1; j < g; ++j) {
+        const int b = TriIndex(i, j, g);
+        if (t == S.q[j]) {  // a row does not list itself: no search needed
+          atomicAdd(reinterpret_cast<unsigned*>(&T.pc[b]) + 1, static_cast<unsigned>(c));
+          continue;
+        }
+        int lo = S.start[j], hi = S.start[j + 1];
+        const int end = hi;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (EntNb(S.ent[mid]) < t) lo = mid + 1; else hi = mid;
+        }
+        if (lo == end || EntNb(S.ent[lo]) != t) continue;
+        bool bad;
+        const SharedTerm x = TermOf(si, S.sz[j], st, c, EntCnt(S.ent[lo]), &bad);
+        ++examined;
+        any_bad |= bad;
+        if (x.delta != 0) atomicAdd(reinterpret_cast<unsigned*>(&T.pc[b]) + 1, static_cast<unsigned>(x.delta));
+        if (x.corr != 0) atomicAdd(reinterpret_cast<int*>(&T.pc[b]), static_cast<int>(x.corr));
+        atomicAdd(&T.ovl[b >> 2], 1u << (8 * (b & 3)));
+      }
+    }
+  }
+  *slow = __any_sync(0xffffffffu, any_bad) || wide;
+  __syncwarp();
+  if (wide) {
+    // too large for 32 bits: a lane per member, a lane per pair
+    if (lane < g) {
+      long long old = 0;
+      for (int k = S.start[lane]; k < S.start[lane + 1]; ++k) {
+        const long long c = EntCnt(S.ent[k]), st = S.tsz[k];
+        old += EncodeCostForPair(S.q[lane], S.sz[lane], EntNb(S.ent[k]), st, c);
+        if (HeavyEntry(S.sz[lane], st, c)) S.heavy[lane].Add(st, c);
+      }
+      S.old[lane] = old;
+    }
+    for (int pidx = lane; pidx < npairs; pidx += 32) {
+      int a, b;
+      TriPair(pidx, g, &a, &b);
+      examined += static_cast<unsigned>(SmallMerge(S, a, b).ovl);
+    }
+  }
+  return examined;
+}
+
+// Member i's record and its old cost's internal term, by one lane.
+__device__ __forceinline__ void SmallFinishRow(const QuotientView& Q, SmallRowsSmem& S, int i, bool wide,
+                                               RowSums* out) {
+  const int rep = S.q[i];
+  const long long si = S.sz[i];
+  const long long internal = Q.internal[rep];
+  if (out) {
+    long long light = S.light[i];
+    if (wide) {
+      for (int k = S.start[i]; k < S.start[i + 1]; ++k) {
+        const long long c = EntCnt(S.ent[k]);
+        if (!HeavyEntry(si, S.tsz[k], c)) light += c;
+      }
+    }
+    StoreRowSums(out, S.old[i], light, S.heavy[i], internal, S.sz[i], S.start[i + 1] - S.start[i]);
+  }
+  if (internal > 0) S.old[i] += EncodeCostForPair(rep, si, rep, si, 2 * internal);
+}
+
+// Pair (a, b) at position t of the pair sums.
+template <int kPairs>
+__device__ __forceinline__ SmallPair SmallPairAt(const SmallRowsSmem& S, const SmallPairsSmem<kPairs>& T, int t, int a,
+                                                 int b, bool slow) {
+  if (slow) return SmallMerge(S, a, b);
+  SmallPair r;
+  r.proxy = static_cast<long long>(T.pc[t] >> 32);
+  r.corr = static_cast<int>(T.pc[t] & 0xffffffffull);
+  r.ovl = (T.ovl[t >> 2] >> (8 * (t & 3))) & 0xff;
+  r.bad = false;
+  return r;
+}
+
+// Sum of f_s(c) over staged row i, by one lane.
+__device__ __forceinline__ long long StagedRowAfter(const SmallRowsSmem& S, int i, long long s) {
+  long long sum = 0;
+  for (int k = S.start[i]; k < S.start[i + 1]; ++k) {
+    const long long c = EntCnt(S.ent[k]);
+    const long long alt = 1 + s * S.tsz[k] - c;
+    sum += c < alt ? c : alt;
+  }
+  return sum;
+}
+
+// Marks every member's top_k partners in fmask (bit b of word a, a < b), by a
+// warp; proxy_of(a, b), a < b.
+template <typename ProxyFn>
+__device__ __forceinline__ void SmallTopK(SmallRowsSmem& S, int g, int top_k_max, ProxyFn proxy_of) {
+  const int lane = threadIdx.x & 31;
+  int top_k = top_k_max < g - 1 ? top_k_max : g - 1;
   if (top_k < 1) top_k = 1;
-  if (lane < g && g - 1 <= P.top_k) {
+  if (lane < g && g - 1 <= top_k_max) {
     // every member has at most top_k partners: all positive ones are kept
     const int i = lane;
     for (int j = i + 1; j < g; ++j) {
       if (proxy_of(i, j) > 0) atomicOr(&S.fmask[i], 1u << j);
     }
-  } else if (g - 1 > P.top_k) {
+  } else if (g - 1 > top_k_max) {
     // ranking, one member at a time by the whole warp, lane j holding
     // partner j: a partner's rank is the number of partners better than it
     // under ranked_better (ratio desc, proxy gain desc, rep_lo asc, rep_hi
@@ -1691,6 +1843,34 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
     }
   }
   __syncwarp();
+}
+
+__global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PrepareParams P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SmallWarpSmem& W = reinterpret_cast<SmallSmem*>(smem_raw)->w[threadIdx.x >> 5];
+  SmallRowsSmem& S = W.rows;
+  const int lane = threadIdx.x & 31;
+  const int li = blockIdx.x * kSmallWarps + (threadIdx.x >> 5);
+  if (li >= P.nlist) return;
+  const int ri = P.list[P.list0 + li];
+  const int gid = P.real[ri];
+  const int g = P.glen[gid];
+  bool wide;
+  const int E = StageSmallRows(P.Q, P.order + P.gstart[gid], g, S, &wide);
+  if (E > kSmallStage) {
+    if (lane == 0) {
+      RaiseError(P.err, kErrSlots, gid, E, 0);
+      P.cand_cnt[ri] = 0;
+    }
+    return;
+  }
+  bool slow;
+  unsigned examined = SmallSums(P.Q, S, W.pairs, g, E, wide, &slow);
+  if (lane < g) SmallFinishRow(P.Q, S, lane, wide, P.rc ? &P.rc[S.q[lane]] : nullptr);
+  __syncwarp();
+  SmallTopK(S, g, P.top_k, [&](int a, int b) {
+    return slow ? SmallMerge(S, a, b).proxy : static_cast<long long>(W.pairs.pc[TriIndex(a, b, g)] >> 32);
+  });
   // union of kept pairs in (a_idx, b_idx) order
   const unsigned mine = lane < g ? S.fmask[lane] : 0u;
   const int cnt = __popc(mine);
@@ -1709,43 +1889,26 @@ __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PreparePa
     const int b = __ffs(bits) - 1;
     bits &= bits - 1;
     if (feat || info) {
-      SmallPair r;
-      if (wide) {
-        r = SmallMerge(S, lane, b);
-      } else {
-        const int t = TriIndex(lane, b, g);
-        r.proxy = S.p[t];
-        r.corr = S.corr[t];
-        r.ovl = S.ovl[t] & (kSmallBad - 1u);
-        r.bad = (S.ovl[t] & kSmallBad) != 0;
-      }
+      const SmallPair r = SmallPairAt(S, W.pairs, TriIndex(lane, b, g), lane, b, slow);
       if (feat) {
         long long denom = S.old[lane] + S.old[b];
         if (denom < 1) denom = 1;
         feat[ex] =
             make_float2(static_cast<float>(r.proxy), __fdividef(static_cast<float>(r.proxy), static_cast<float>(denom)));
       }
-      if (info) {
-        const long long ea = StagedLookup(S, lane, S.q[b]);
-        const long long eb = StagedLookup(S, b, S.q[lane]);
-        PairInfo pi;
-        pi.shared = r.corr - (r.proxy - ea);
-        pi.ovl = static_cast<unsigned>(r.ovl) | (r.bad ? kPairBad : 0u) | (ea != eb ? kPairAsym : 0u);
-        pi.eab = static_cast<unsigned>(ea);
-        info[ex] = pi;
-      }
+      if (info) info[ex] = SmallPairInfo(S, lane, b, r);
     }
     P.cand_rep[P.cand_off[ri] + ex] = make_int2(S.q[lane], S.q[b]);
     out[ex++] = make_int2(lane, b);
   }
-  examined = static_cast<unsigned long long>(WarpSum(static_cast<long long>(examined)));
+  examined = __reduce_add_sync(0xffffffffu, examined);
   if (lane == 0) {
     P.cand_cnt[ri] = total;
     atomicAdd(&P.stats[kStGroupCount], 1ull);
     atomicMax(&P.stats[kStGroupMaxSize], static_cast<unsigned long long>(g));
     atomicAdd(&P.stats[kStRawPairCount], static_cast<unsigned long long>(g) * (g - 1) / 2);
     atomicAdd(&P.stats[kStCandAfterPrune], static_cast<unsigned long long>(total));
-    atomicAdd(&P.stats[kStProxyExamined], examined);
+    atomicAdd(&P.stats[kStProxyExamined], static_cast<unsigned long long>(examined));
     atomicAdd(&P.stats[kStPrepareBytes], 12ull * static_cast<unsigned long long>(E));
   }
 }
@@ -1793,10 +1956,11 @@ struct ScoreParams {
 struct GainParts {
   long long gain, before;
   int uni, ovl;
+  int err;  // ErrCode of an invalid pair
 };
 
-__device__ __forceinline__ bool GainFromSums(const RowSums& A, const RowSums& B, const PairInfo& p, int a, int b,
-                                             int strict, DevError* err, GainParts* out) {
+__device__ __forceinline__ bool GainFromSums(const RowSums& A, const RowSums& B, const PairInfo& p, int strict,
+                                             GainParts* out) {
   const long long sa = A.size, sb = B.size, s = sa + sb;
   const long long eab = p.eab;
   long long fa, fb;
@@ -1810,8 +1974,7 @@ __device__ __forceinline__ bool GainFromSums(const RowSums& A, const RowSums& B,
                            BlockCost(sa, sa, A.internal, true, bad) + BlockCost(sb, sb, B.internal, true, bad);
   const long long after = fa + fb - BlockCost(s, sb, eab, false, bad) - BlockCost(s, sa, eab, false, bad) + p.shared +
                           BlockCost(s, s, A.internal + B.internal + eab, true, bad);
-  if (p.ovl & kPairAsym) RaiseError(err, kErrAsymmetric, a, b, 0);
-  if (bad) RaiseError(err, kErrBlockCost, a, b, 0);
+  out->err = (p.ovl & kPairAsym) ? kErrAsymmetric : bad ? kErrBlockCost : kErrNone;
   out->gain = before - after;  // without the F of a row that has to be read
   out->before = before;
   out->ovl = static_cast<int>(p.ovl & ((1u << 30) - 1u));
@@ -1822,10 +1985,10 @@ __device__ __forceinline__ bool GainFromSums(const RowSums& A, const RowSums& B,
 
 // The same, by a warp, for the pairs GainFromSums leaves.
 __device__ GainParts WarpGainReadingRows(const QuotientView& Q, const RowSums& A, const RowSums& B, const PairInfo& p,
-                                         int a, int b, int strict, DevError* err) {
+                                         int a, int b, int strict) {
   const long long s = static_cast<long long>(A.size) + B.size;
   GainParts g;
-  GainFromSums(A, B, p, a, b, strict, err, &g);
+  GainFromSums(A, B, p, strict, &g);
   long long part;
   if (!RowAfter(A, s, &part)) g.gain += part - WarpRowAfter(Q, a, s);
   if (!RowAfter(B, s, &part)) g.gain += part - WarpRowAfter(Q, b, s);
@@ -1906,7 +2069,7 @@ __global__ void __launch_bounds__(kScoreThreads, 4) ScoreKernel(ScoreParams P) {
       }
     }
     const bool score = todo == 1 || (todo == 2 && P.audit);
-    GainParts g = {0, 0, 0, 0};
+    GainParts g = {0, 0, 0, 0, 0};
     RowSums A, B;
     PairInfo p;
     bool by_warp = score;
@@ -1914,16 +2077,17 @@ __global__ void __launch_bounds__(kScoreThreads, 4) ScoreKernel(ScoreParams P) {
       A = P.rc[ab.x];
       B = P.rc[ab.y];
       p = P.info[slot];
-      by_warp = !GainFromSums(A, B, p, ab.x, ab.y, P.strict, P.err, &g);
+      by_warp = !GainFromSums(A, B, p, P.strict, &g);
+      if (g.err) RaiseError(P.err, g.err, ab.x, ab.y, 0);
     }
     for (unsigned rest = __ballot_sync(kFull, by_warp); rest != 0u; rest &= rest - 1u) {
       const int j = __ffs(rest) - 1;
       const int a = __shfl_sync(kFull, ab.x, j);
       const int b = __shfl_sync(kFull, ab.y, j);
-      GainParts r;
+      GainParts r = {0, 0, 0, 0, 0};
       if (P.rc) {
         const long long sj = __shfl_sync(kFull, slot, j);
-        r = WarpGainReadingRows(P.Q, P.rc[a], P.rc[b], P.info[sj], a, b, P.strict, P.err);
+        r = WarpGainReadingRows(P.Q, P.rc[a], P.rc[b], P.info[sj], a, b, P.strict);
       } else {
         GainWork one = {0, 0, 0, 0, 0};
         WarpExactGain(P.Q, a, b, &r.gain, &r.before, &one, P.err);
@@ -2205,13 +2369,75 @@ __global__ void __launch_bounds__(kThreads) SelectKernel(SelectParams P) {
 constexpr int kMatchThreads = 512;
 constexpr int kMatchSmemKeys = 8192;
 
+struct MatchSmem {
+  unsigned long long best[kMaxGroup];
+  unsigned long long chosen[kMaxGroup / 2];
+  unsigned char matched[kMaxGroup];
+  int nchosen, live_any;
+};
+
+// The greedy choice among m keys of a group of g members by a CTA of
+// kMatchThreads (kin, kout: two buffers of m keys, the first holds them);
+// chosen[] gets the selected keys in ascending order, their number is
+// returned. Ends with a barrier.
+__device__ int MatchKeys(MatchSmem& M, unsigned long long* kin, unsigned long long* kout, int m, int g) {
+  const int tid = threadIdx.x;
+  if (tid == 0) M.nchosen = 0;
+  for (int i = tid; i < g; i += kMatchThreads) M.matched[i] = 0;
+  // rounds of locally dominant keys (each round selects at least the
+  // smallest live key, so at most g/2 rounds); the keys still live after a
+  // round move to the other buffer (the matching depends on the key values
+  // only, not on their order)
+  int nlive = m;
+  for (int round = 0; round <= kMaxGroup / 2 && nlive > 0; ++round) {
+    for (int i = tid; i < g; i += kMatchThreads) M.best[i] = ~0ull;
+    if (tid == 0) M.live_any = 0;
+    __syncthreads();
+    for (int k = tid; k < nlive; k += kMatchThreads) {
+      const unsigned long long key = kin[k];
+      atomicMin(&M.best[(key >> kKeyIdxBits) & kKeyIdxMask], key);
+      atomicMin(&M.best[key & kKeyIdxMask], key);
+    }
+    __syncthreads();
+    for (int k = tid; k < nlive; k += kMatchThreads) {
+      const unsigned long long key = kin[k];
+      const int a = static_cast<int>((key >> kKeyIdxBits) & kKeyIdxMask);
+      const int b = static_cast<int>(key & kKeyIdxMask);
+      if (M.best[a] == key && M.best[b] == key) {
+        M.matched[a] = 1;
+        M.matched[b] = 1;
+        M.chosen[atomicAdd(&M.nchosen, 1)] = key;
+      }
+    }
+    __syncthreads();
+    for (int k = tid; k < nlive; k += kMatchThreads) {
+      const unsigned long long key = kin[k];
+      if (!M.matched[(key >> kKeyIdxBits) & kKeyIdxMask] && !M.matched[key & kKeyIdxMask]) {
+        kout[atomicAdd(&M.live_any, 1)] = key;
+      }
+    }
+    __syncthreads();
+    nlive = M.live_any;
+    unsigned long long* t = kin;
+    kin = kout;
+    kout = t;
+    __syncthreads();  // every thread has read live_any before the next round resets it
+  }
+  __syncthreads();
+  const int ns = M.nchosen;
+  int pow2 = 1;
+  while (pow2 < ns) pow2 <<= 1;
+  for (int i = ns + tid; i < pow2; i += kMatchThreads) M.chosen[i] = ~0ull;
+  __syncthreads();
+  if (ns > 1) CtaBitonicSort(M.chosen, pow2);
+  return ns;
+}
+
 __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned long long* skeys = reinterpret_cast<unsigned long long*>(smem_raw);
-  __shared__ unsigned long long best[kMaxGroup];
-  __shared__ unsigned long long chosen[kMaxGroup / 2];
-  __shared__ unsigned char matched[kMaxGroup];
-  __shared__ int nkeys, nchosen, live_any;
+  __shared__ MatchSmem M;
+  __shared__ int nkeys;
   __shared__ unsigned long long* gkeys;
   __shared__ unsigned long long rej_thr;
   const int tid = threadIdx.x;
@@ -2224,14 +2450,12 @@ __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) 
   }
   if (tid == 0) {
     nkeys = 0;
-    nchosen = 0;
     rej_thr = 0;
     // two key buffers of cnt entries: the live keys are compacted from one
     // into the other every round
     gkeys = 2 * cnt <= kMatchSmemKeys ? skeys
                                       : ScratchAlloc(P.scratch, P.scratch_cap, P.ctl, 16ull * cnt, P.err);
   }
-  for (int i = tid; i < g; i += kMatchThreads) matched[i] = 0;
   __syncthreads();
   unsigned long long* keys = gkeys;
   if (keys == nullptr) {
@@ -2255,70 +2479,21 @@ __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) 
     }
     if (gain > kKeyGainMax) RaiseError(P.err, kErrKeyRange, gid, c, 0);
     const int2 ab = P.cand[base + c];
-    keys[atomicAdd(&nkeys, 1)] = (static_cast<unsigned long long>(kKeyGainMax - gain) << (2 * kKeyIdxBits)) |
-                                 (static_cast<unsigned long long>(ab.x) << kKeyIdxBits) |
-                                 static_cast<unsigned long long>(ab.y);
+    keys[atomicAdd(&nkeys, 1)] = PackKey(gain, ab.x, ab.y);
   }
   if (my_rej) atomicAdd(&rej_thr, my_rej);
   __syncthreads();
   const int m = nkeys;
-  const unsigned long long idx_mask = (1ull << kKeyIdxBits) - 1;
-  // rounds of locally dominant keys (each round selects at least the
-  // smallest live key, so at most g/2 rounds); the keys still live after a
-  // round move to the other buffer (the matching depends on the key values
-  // only, not on their order)
-  unsigned long long* kin = keys;
-  unsigned long long* kout = keys + cnt;
-  int nlive = m;
-  for (int round = 0; round <= kMaxGroup / 2 && nlive > 0; ++round) {
-    for (int i = tid; i < g; i += kMatchThreads) best[i] = ~0ull;
-    if (tid == 0) live_any = 0;
-    __syncthreads();
-    for (int k = tid; k < nlive; k += kMatchThreads) {
-      const unsigned long long key = kin[k];
-      atomicMin(&best[(key >> kKeyIdxBits) & idx_mask], key);
-      atomicMin(&best[key & idx_mask], key);
-    }
-    __syncthreads();
-    for (int k = tid; k < nlive; k += kMatchThreads) {
-      const unsigned long long key = kin[k];
-      const int a = static_cast<int>((key >> kKeyIdxBits) & idx_mask);
-      const int b = static_cast<int>(key & idx_mask);
-      if (best[a] == key && best[b] == key) {
-        matched[a] = 1;
-        matched[b] = 1;
-        chosen[atomicAdd(&nchosen, 1)] = key;
-      }
-    }
-    __syncthreads();
-    for (int k = tid; k < nlive; k += kMatchThreads) {
-      const unsigned long long key = kin[k];
-      if (!matched[(key >> kKeyIdxBits) & idx_mask] && !matched[key & idx_mask]) {
-        kout[atomicAdd(&live_any, 1)] = key;
-      }
-    }
-    __syncthreads();
-    nlive = live_any;
-    unsigned long long* t = kin;
-    kin = kout;
-    kout = t;
-    __syncthreads();  // every thread has read live_any before the next round resets it
-  }
   // the selected keys in greedy (ascending key) order
-  const int ns = nchosen;
-  int pow2 = 1;
-  while (pow2 < ns) pow2 <<= 1;
-  for (int i = ns + tid; i < pow2; i += kMatchThreads) chosen[i] = ~0ull;
-  __syncthreads();
-  if (ns > 1) CtaBitonicSort(chosen, pow2);
+  const int ns = MatchKeys(M, keys, keys + cnt, m, g);
   const int* q = P.order + P.gstart[gid];
   const long long so = P.sel_off[ri];
   long long my_total = 0;
   unsigned long long my_work = 0;
   for (int i = tid; i < ns; i += kMatchThreads) {
-    const unsigned long long key = chosen[i];
-    const int a = static_cast<int>((key >> kKeyIdxBits) & idx_mask);
-    const int b = static_cast<int>(key & idx_mask);
+    const unsigned long long key = M.chosen[i];
+    const int a = static_cast<int>((key >> kKeyIdxBits) & kKeyIdxMask);
+    const int b = static_cast<int>(key & kKeyIdxMask);
     const long long gain = kKeyGainMax - static_cast<long long>(key >> (2 * kKeyIdxBits));
     const int keep = q[a];
     const int rem = q[b];
@@ -2337,19 +2512,19 @@ __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) 
   // chosen[] is no longer needed: reuse best[] for the two sums
   __syncthreads();
   if (tid == 0) {
-    best[0] = 0;
-    best[1] = 0;
+    M.best[0] = 0;
+    M.best[1] = 0;
   }
   __syncthreads();
   my_total = WarpSum(my_total);
   my_work = static_cast<unsigned long long>(WarpSum(static_cast<long long>(my_work)));
   if ((tid & 31) == 0) {
-    if (my_total) atomicAdd(&best[0], static_cast<unsigned long long>(my_total));
-    if (my_work) atomicAdd(&best[1], my_work);
+    if (my_total) atomicAdd(&M.best[0], static_cast<unsigned long long>(my_total));
+    if (my_work) atomicAdd(&M.best[1], my_work);
   }
   __syncthreads();
   if (tid == 0) {
-    const unsigned long long total = best[0];
+    const unsigned long long total = M.best[0];
     P.sel_cnt[ri] = ns;
     atomicAdd(&P.stats[kStRejThreshold], rej_thr);
     atomicAdd(&P.stats[kStPositive], static_cast<unsigned long long>(m));
@@ -2358,7 +2533,7 @@ __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) 
     atomicAdd(&P.stats[kStSelected], static_cast<unsigned long long>(ns));
     atomicAdd(&P.stats[kStLocalGain], total);
     atomicAdd(&P.stats[kStValidationCalls], static_cast<unsigned long long>(ns));
-    atomicAdd(&P.stats[kStValidationWork], best[1]);
+    atomicAdd(&P.stats[kStValidationWork], M.best[1]);
     atomicAdd(&P.stats[kStIsolatedGain], total);
   }
 }
@@ -2490,6 +2665,8 @@ __global__ void __launch_bounds__(kSelectSmallWarps * 32) SelectSmallKernel(Sele
   }
 }
 
+#include "window.cuh"
+
 // ------------------------------------------------------------ commit
 
 // A claimed neighbour row of more than kRowSmem entries and its block scratch:
@@ -2538,6 +2715,8 @@ struct CommitParams {
   unsigned* ticket; // last-CTA counter of the long-row rewrite kernel, left at 0
   const int* sel_list;  // selection slots of the block's selected pairs (count: ctl->sel_total)
   int warp_pairs;       // 1: pairs with at most kWarpRow row entries go to CommitShortKernel
+  int windowed;         // 1: the batch of a window of blocks (W): the groups it touches are listed
+  WindowParams W;
 };
 
 // Optional re-validation (--verify-cuda-gain): recomputes the exact gain of
@@ -2745,6 +2924,15 @@ __device__ __forceinline__ void ClaimRow(const CommitParams& P, int x) {
   }
 }
 
+// A neighbour x of a merged pair: its group has to be evaluated again if it has
+// been already ([p, e): evaluated, not committed).
+__device__ __forceinline__ void MarkTouched(const CommitParams& P, int x, int p, int e) {
+  const int ri = P.W.node_ri[x];
+  if (ri < p || ri >= e) return;
+  if (atomicExch(&P.W.dirty[ri], P.block_stamp) == P.block_stamp) return;
+  P.W.list_dirty[atomicAdd(&P.W.ctl->ndirty, 1)] = ri;
+}
+
 // One CTA per selected pair of the block (persistent grid over the block's
 // selection slots). Per pair:
 //   Update_S bookkeeping: size, internal count, member list, forwarding, and
@@ -2765,6 +2953,8 @@ __global__ void __launch_bounds__(kRowsThreads) CommitKernel(CommitParams P) {
   const int tid = threadIdx.x;
   const int remove_stamp = 2 * P.block_stamp + 1;
   const unsigned total = P.ctl->sel_total;
+  const int win_p = P.windowed ? P.W.ctl->p : 0;
+  const int win_e = P.windowed ? P.W.ctl->e : 0;
   for (unsigned idx = blockIdx.x; idx < total; idx += gridDim.x) {
     const long long slot = P.sel_list[idx];
     const int k = P.sel_keep[slot];
@@ -2783,6 +2973,7 @@ __global__ void __launch_bounds__(kRowsThreads) CommitKernel(CommitParams P) {
     for (int i = tid; i < lr; i += kRowsThreads) {
       const int x = EntNb(rr[i]);
       if (x == k) continue;
+      if (P.windowed) MarkTouched(P, x, win_p, win_e);
       const int sx = P.stamp[x];
       if (sx == remove_stamp && P.seq[x] < my_seq && RowLookup(rr, lr, P.partner[x]) != 0) ++folded;
       if ((sx >> 1) == P.block_stamp) continue;  // keep/remove rows are rebuilt by their own pair
@@ -2798,6 +2989,7 @@ __global__ void __launch_bounds__(kRowsThreads) CommitKernel(CommitParams P) {
     if (!StageBuffers(P, R, L, &S, &D, &INS)) return;
     for (int i = tid; i < lk; i += kRowsThreads) {
       const Entry e = rk[i];
+      if (P.windowed && EntNb(e) != r) MarkTouched(P, EntNb(e), win_p, win_e);
       S[i + RowLowerBound(rr, lr, EntNb(e))] = e;
     }
     for (int j = tid; j < lr; j += kRowsThreads) {
@@ -3274,7 +3466,6 @@ __global__ void __launch_bounds__(kHugeThreads) RewriteHugeKernel(CommitParams P
   const QuotientView& Q = P.Q;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
-  const int warp = tid >> 5;
   const unsigned cnt = P.ctl->huge_cnt;
   for (unsigned idx = blockIdx.x; idx < cnt; idx += gridDim.x) {
     const HugeRow h = P.rows_huge[idx];
@@ -3364,6 +3555,7 @@ __global__ void __launch_bounds__(kHugeThreads) RewriteHugeKernel(CommitParams P
     }
     __syncthreads();
   }
+  __threadfence();
   __syncthreads();
   if (tid == 0) last = atomicAdd(P.ticket, 1u) == gridDim.x - 1;
   __syncthreads();
@@ -3379,6 +3571,7 @@ __global__ void __launch_bounds__(kHugeThreads) RewriteHugeKernel(CommitParams P
     P.ctl->work_next[2] = 0;
     *P.ticket = 0u;
   }
+  if (last && P.windowed) BuildLists(P.W);
 }
 
 __global__ void ScatterGroupKernel(const int* __restrict__ q, const int* __restrict__ idx, int g,
@@ -3412,6 +3605,10 @@ void Engine::ConfigureKernels() {
                                  static_cast<int>(sizeof(RowsSmem))), "rewrite smem attribute");
   CheckCuda(cudaFuncSetAttribute(RewriteHugeKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(sizeof(HugeSmem))), "long-row rewrite smem attribute");
+  CheckCuda(cudaFuncSetAttribute(WindowEvalKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(sizeof(EvalSmem))), "window evaluation smem attribute");
+  CheckCuda(cudaFuncSetAttribute(WindowSelectKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 8 * kMatchSmemKeys), "window selection smem attribute");
   // the queue-fed kernels launch exactly the CTAs that fit on the GPU at once
   int sms = 0, per_sm = 0;
   CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg_.device), "SM count");
@@ -3481,14 +3678,14 @@ __device__ __forceinline__ PlanSums PlanZero() {
 }
 
 // one group's contribution: the same rules as the host plan
-__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k) {
+__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, int small_max) {
   PlanSums f = PlanZero();
   if (g < 2) return f;
   const long long gl = g;
   f.real = 1;
   f.cand = gl * (gl - 1) / 2 < gl * k ? gl * (gl - 1) / 2 : gl * k;
   f.sel = gl / 2;
-  if (g <= kSmallGroup && e <= static_cast<unsigned>(kSmallStage)) {
+  if (g <= small_max && e <= static_cast<unsigned>(kSmallStage)) {
     f.small[SmallClass(g)] = 1;
   } else {
     f.big = 1;
@@ -3511,6 +3708,7 @@ struct PlanParams {
   const unsigned* gent;
   long long G;
   long long top_k;
+  int small_max;  // members of a group that one warp handles
   PlanSums* tile_sums;
   PlanSums* tile_off;
   int tiles;
@@ -3526,6 +3724,7 @@ struct PlanParams {
   int* sel_small;
   int* sel_mid;
   int* sel_big;
+  int* ri_of;  // per Divide group: its position, -1 for a group of one (nullptr: not needed)
 };
 
 __global__ void __launch_bounds__(kPlanThreads) PlanTileKernel(PlanParams P) {
@@ -3537,7 +3736,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanTileKernel(PlanParams P) {
   for (int j = 0; j < kPlanItems; ++j) {
     const long long gi = base + j;
     if (gi >= P.G) break;
-    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k);
+    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k, P.small_max);
     acc = PlanSumOp()(acc, f);
     max_e = f.soff > max_e ? f.soff : max_e;
   }
@@ -3606,13 +3805,14 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
     const long long gi = base + j;
     g[j] = gi < P.G ? P.glen[gi] : 0;
     e[j] = gi < P.G ? P.gent[gi] : 0u;
-    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k));
+    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k, P.small_max));
   }
   PlanSums off;
   Scan(tmp).ExclusiveScan(acc, off, P.tile_off[blockIdx.x], PlanSumOp());
 #pragma unroll
   for (int j = 0; j < kPlanItems; ++j) {
-    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k);
+    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k, P.small_max);
+    if (P.ri_of && base + j < P.G) P.ri_of[base + j] = f.real ? off.real : -1;
     if (f.real) {
       const int ri = off.real;
       P.real[ri] = static_cast<int>(base + j);
@@ -3782,7 +3982,7 @@ void Engine::PrepareIterationBuffers() {
                               cudaMemcpyHostToDevice, stream_), "h2d mat_off");
   }
   SizeIterationBuffers(R, static_cast<size_t>(h_cand_off_[R]), static_cast<size_t>(h_sel_off_[R]), h_big_.size(),
-                       max_mat, max_slots);
+                       max_mat, max_slots, false);
   plans_.clear();
   for (size_t b = 0; b + 1 < h_block_rg_.size(); ++b) {
     BlockPlan bp;
@@ -3813,7 +4013,14 @@ void Engine::PrepareIterationBuffers() {
 
 // Buffers whose sizes follow from the plan's totals (either planner).
 void Engine::SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nbig, long long max_mat,
-                                  long long max_slots) {
+                                  long long max_slots, bool windows) {
+  d_sel_cnt_.ensure(R + 1);
+  d_res_.ensure(ncand + 1);
+  d_sel_keep_.ensure(nsel + 1);
+  d_sel_rem_.ensure(nsel + 1);
+  d_sel_gain_.ensure(nsel + 1);
+  d_mat_.ensure(static_cast<size_t>(max_mat) + 256);
+  if (windows) return;  // neither candidate lists nor sort slots
   d_bigdesc_.ensure(sizeof(BigDesc) * (nbig + 1));
   max_slots = std::max(max_slots, 1ll);
   for (int k = 0; k < 2; ++k) {
@@ -3828,11 +4035,9 @@ void Engine::SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nb
     d_cub_tmp_.ensure(bytes);
   }
   d_cand_cnt_.ensure(R + 1);
-  d_sel_cnt_.ensure(R + 1);
   d_cand_.ensure(ncand + 1);
   d_cand_rep_.ensure(ncand + 1);
   CheckCuda(cudaMemsetAsync(d_cand_rep_.p, 0xff, sizeof(int2) * (ncand + 1), stream_), "memset cand reps");
-  d_res_.ensure(ncand + 1);
   d_info_.ensure(sizeof(PairInfo) * (ncand + 1));
   if (cfg_.ranker) {
     d_cand_feat_.ensure(ncand + 1);
@@ -3844,10 +4049,6 @@ void Engine::SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nb
     }
   }
   rk_iter_slots_ = static_cast<long long>(ncand);
-  d_sel_keep_.ensure(nsel + 1);
-  d_sel_rem_.ensure(nsel + 1);
-  d_sel_gain_.ensure(nsel + 1);
-  d_mat_.ensure(static_cast<size_t>(max_mat) + 256);
 }
 
 // The plan of a one-block iteration, made on the device from the Divide
@@ -3867,6 +4068,7 @@ void Engine::PlanOnDevice() {
   P.gent = d_gent_.p;
   P.G = G;
   P.top_k = cfg_.top_k > 0 ? cfg_.top_k : 1;
+  P.small_max = windowed_ ? kEvalSmall : kSmallGroup;
   P.tile_sums = reinterpret_cast<PlanSums*>(d_plan_tiles_.p);
   P.tile_off = P.tile_sums + tiles;
   P.tiles = tiles;
@@ -3882,6 +4084,11 @@ void Engine::PlanOnDevice() {
   P.sel_small = d_sel_small_.p;
   P.sel_mid = d_sel_mid_.p;
   P.sel_big = d_sel_big_.p;
+  P.ri_of = nullptr;
+  if (windowed_) {
+    d_ri_of_.ensure(cap);
+    P.ri_of = d_ri_of_.p;
+  }
   if (tiles > 0) {
     ++launches_;
     PlanTileKernel<<<tiles, kPlanThreads, 0, stream_>>>(P);
@@ -3892,7 +4099,7 @@ void Engine::PlanOnDevice() {
     ++launches_;
     PlanScatterKernel<<<tiles, kPlanThreads, 0, stream_>>>(P);
   }
-  long long* hs = h_pin_.p + 16;
+  long long* hs = h_pin_.p + 16;  // read back: totals and pool top
   CheckCuda(cudaMemcpyAsync(hs, d_plan_scalars_.p, sizeof(long long) * kPlanScalars, cudaMemcpyDeviceToHost,
                             stream_), "d2h plan");
   CheckCuda(cudaMemcpyAsync(hs + kPlanScalars, d_pool_top_.p, sizeof(long long), cudaMemcpyDeviceToHost, stream_),
@@ -3904,7 +4111,7 @@ void Engine::PlanOnDevice() {
   EnsurePoolRoom(static_cast<unsigned long long>(v[kPlanScalars]));
   const size_t R = static_cast<size_t>(v[kPlanR]);
   SizeIterationBuffers(R, static_cast<size_t>(v[kPlanCand]), static_cast<size_t>(v[kPlanSel]),
-                       static_cast<size_t>(v[kPlanBig]), v[kPlanMat], v[kPlanSlots]);
+                       static_cast<size_t>(v[kPlanBig]), v[kPlanMat], v[kPlanSlots], windowed_);
   BlockPlan bp;
   bp.rg1 = static_cast<int>(R);
   bp.slots = v[kPlanCand];
@@ -3932,8 +4139,21 @@ QuotientView Engine::View() {
   return Q;
 }
 
-void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify) {
+namespace {
+// The parts of the commit that a window sets.
+void CommitDefaults(CommitParams* C) {
+  C->windowed = 0;
+  C->W = WindowParams{};
+}
+}  // namespace
+
+void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, const void* window) {
   CommitParams C;
+  CommitDefaults(&C);
+  if (window) {
+    C.windowed = 1;
+    C.W = *static_cast<const WindowParams*>(window);
+  }
   C.Q = View();
   C.rg0 = rg0;
   C.nrg = nrg;
@@ -3969,7 +4189,7 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify) {
   C.sel_list = d_sel_list_.p;
   // warp-per-pair commit for short pairs, except in small blocks, where one
   // launch is cheaper than a second one
-  C.warp_pairs = nrg > kFewGroups ? 1 : 0;
+  C.warp_pairs = nrg > kFewGroups && !window ? 1 : 0;
   if (verify) {
     const int vb = static_cast<int>(std::min<int64_t>((max_pairs + 7) / 8 + 1, 152 * 8));
     ++launches_;
@@ -4197,7 +4417,7 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
     LP.nlist = nrg;
     ++launches_;
     SelectMatchKernel<<<nrg, kMatchThreads, 8 * kMatchSmemKeys, stream_>>>(LP);
-    LaunchCommit(rg0, nrg, sel_slots, cfg_.verify_cuda_gain);
+    LaunchCommit(rg0, nrg, sel_slots, cfg_.verify_cuda_gain, nullptr);
     return;
   }
   if (ss1 > ss0) {
@@ -4223,7 +4443,116 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
     ++launches_;
     SelectMatchKernel<<<sb1 - sb0, kMatchThreads, 8 * kMatchSmemKeys, stream_>>>(LP);
   }
-  LaunchCommit(rg0, nrg, sel_slots, cfg_.verify_cuda_gain);
+  LaunchCommit(rg0, nrg, sel_slots, cfg_.verify_cuda_gain, nullptr);
+}
+
+bool Engine::WindowsOn() const {
+  // the ranker calibrates itself on whole blocks
+  return cfg_.group_batch_size <= kWindowMaxBatch && !cfg_.ranker && RowSumsOn();
+}
+
+// An iteration's blocks through windows (window.cuh).
+void Engine::RunWindows(double threshold) {
+  const int R = plans_[0].rg1;
+  if (R == 0) return;
+  const size_t ur = static_cast<size_t>(R);
+  d_node_ri_.ensure(static_cast<size_t>(n_));
+  d_blk_end_.ensure(ur + 1);
+  d_dirty_.ensure(ur + 1);
+  d_gs_.ensure(sizeof(GroupStats) * (ur + 1));
+  d_win_list_.ensure(3 * static_cast<size_t>(kWindowList));
+  d_win_off_.ensure(2 * static_cast<size_t>(kWindowList) + 2);
+  d_conflict_.ensure(ur + 1);
+  d_units_.ensure(sizeof(LongUnit) * kLongUnits);
+  d_rc_.ensure(sizeof(RowSums) * static_cast<size_t>(n_));
+  WindowParams W{};
+  W.Q = View();
+  W.order = d_order_.p;
+  W.gstart = d_gstart_.p;
+  W.glen = d_glen_.p;
+  W.gent = d_gent_.p;
+  W.group_of = d_group_of_.p;
+  W.real = d_real_.p;
+  W.node_ri = d_node_ri_.p;
+  W.blk_end = d_blk_end_.p;
+  W.ctl = reinterpret_cast<WindowCtl*>(d_wctl_.p);
+  W.gs = reinterpret_cast<GroupStats*>(d_gs_.p);
+  W.conflict = d_conflict_.p;
+  W.units = reinterpret_cast<LongUnit*>(d_units_.p);
+  W.dirty = d_dirty_.p;
+  W.list_dirty = d_win_list_.p;
+  W.list_small = d_win_list_.p + kWindowList;
+  W.list_big = d_win_list_.p + 2 * kWindowList;
+  W.moff = d_win_off_.p;
+  W.poff = d_win_off_.p + kWindowList + 1;
+  W.mat_off = d_mat_off_.p;
+  W.mat = d_mat_.p;
+  W.cand_off = d_cand_off_.p;
+  W.keys = reinterpret_cast<unsigned long long*>(d_res_.p);
+  W.rc = reinterpret_cast<RowSums*>(d_rc_.p);
+  W.sel_off = d_sel_off_.p;
+  W.sel_keep = d_sel_keep_.p;
+  W.sel_rem = d_sel_rem_.p;
+  W.sel_gain = d_sel_gain_.p;
+  W.sel_cnt = d_sel_cnt_.p;
+  W.stamp = d_stamp_.p;
+  W.partner = d_partner_.p;
+  W.seq = d_seq_.p;
+  W.sel_list = d_sel_list_.p;
+  W.bctl = d_ctl_.p;
+  W.top_k = cfg_.top_k;
+  W.threshold = threshold;
+  W.thr = SplitThreshold(threshold);
+  W.use_threshold = cfg_.ea_use_threshold ? 1 : 0;
+  W.stats = d_stats_.p;
+  W.err = d_err_.p;
+  // the frontier and the rounds done, written by the device after each round
+  int* seen = reinterpret_cast<int*>(h_pin_.p + 48);
+  __atomic_store_n(&seen[0], 0, __ATOMIC_RELEASE);
+  __atomic_store_n(&seen[1], 0, __ATOMIC_RELEASE);
+  W.host_f = seen;
+  CheckCuda(cudaMemsetAsync(&W.ctl->blocks, 0, sizeof(long long), stream_), "memset blocks");
+  const int count = static_cast<int>(n_active_);
+  ++launches_;
+  WindowSetupKernel<<<(std::max(count, R) + 255) / 256, 256, 0, stream_>>>(
+      W.order, W.group_of, d_ri_of_.p, count, W.real, R, cfg_.group_batch_size, d_node_ri_.p, d_blk_end_.p, W.dirty,
+      W.ctl);
+  ++launches_;
+  WindowBeginKernel<<<1, kHugeThreads, 0, stream_>>>(W, R);
+  // the host keeps a few rounds queued behind the one running; a round past
+  // the end finds nothing to do
+  long long queued = 0;
+  for (long long idle = 0;;) {
+    const int done = __atomic_load_n(&seen[1], __ATOMIC_ACQUIRE) - 1;  // the first lists count as one
+    if (__atomic_load_n(&seen[0], __ATOMIC_ACQUIRE) >= R) break;
+    if (queued - done >= kWindowAhead) {
+      if (++idle % 4096 == 0) {
+        const cudaError_t st = cudaStreamQuery(stream_);
+        if (st != cudaErrorNotReady) CheckCuda(st, "window rounds");
+      }
+      continue;
+    }
+    // every round commits at least one block
+    if (queued > R + kWindowAhead) throw std::runtime_error("merge windows made no progress");
+    ++queued;
+    ++block_stamp_;
+    W.block_stamp = block_stamp_;
+    BeginTimed(kTimePrepare);
+    WindowEvalKernel<<<kEvalGrid, kEvalWarps * 32, sizeof(EvalSmem), stream_>>>(W);
+    WindowLongKernel<<<kLongGrid, kLongThreads, 0, stream_>>>(W);
+    EndTimed(kTimePrepare);
+    BeginTimed(kTimeScore);
+    WindowScoreKernel<<<kBigGrid, 256, 0, stream_>>>(W);
+    WindowSelectKernel<<<kBigGrid, kMatchThreads, 8 * kMatchSmemKeys, stream_>>>(W);
+    EndTimed(kTimeScore);
+    WindowMarkKernel<<<kMarkGrid, kMarkThreads, 0, stream_>>>(W);
+    launches_ += 5;
+    LaunchCommit(0, R, kBigGrid, cfg_.verify_cuda_gain, &W);
+  }
+  CheckCuda(cudaMemcpyAsync(h_pin_.p + 9, &W.ctl->blocks, sizeof(long long), cudaMemcpyDeviceToHost, stream_),
+            "d2h blocks");
+  CheckCuda(cudaStreamSynchronize(stream_), "windows sync");
+  hstats_.blocks += static_cast<uint64_t>(h_pin_.p[9]);
 }
 
 void Engine::Merge(int iter, int total_iterations) {
@@ -4231,15 +4560,19 @@ void Engine::Merge(int iter, int total_iterations) {
   if (n_groups_ < 0) throw std::runtime_error("Merge requires a preceding Divide");
   // ComputeMergeThreshold, reciprocal policy (src/sweg.cpp:400-406)
   const double threshold = 1.0 / static_cast<double>(iter + 1);
-  if (plan_on_device_) {
+  if (plan_on_device_ || windowed_) {
     PlanOnDevice();
   } else {
     EnsurePoolRoom();
     PrepareIterationBuffers();
   }
   CheckCuda(cudaMemsetAsync(d_ctl_.p, 0, sizeof(BlockCtl), stream_), "memset ctl");
-  for (const BlockPlan& bp : plans_) {
-    if (bp.rg1 > bp.rg0) RunBlock(bp, threshold, iter, total_iterations);
+  if (windowed_) {
+    RunWindows(threshold);
+  } else {
+    for (const BlockPlan& bp : plans_) {
+      if (bp.rg1 > bp.rg0) RunBlock(bp, threshold, iter, total_iterations);
+    }
   }
   ++launches_;
   RelabelKernel<<<(n_ + 255) / 256, 256, 0, stream_>>>(d_label_.p, d_fwd_.p, n_);
@@ -4400,7 +4733,7 @@ void Engine::MergePairs(const int32_t* keep, const int32_t* remove, int64_t coun
   ++launches_;
   MarkKernel<<<(cnt + 255) / 256, 256, 0, stream_>>>(d_sel_keep_.p, d_sel_rem_.p, cnt, d_stamp_.p, d_partner_.p,
                                                     d_seq_.p, block_stamp_, d_sel_list_.p, d_ctl_.p);
-  LaunchCommit(0, 1, count, false);
+  LaunchCommit(0, 1, count, false, nullptr);
   ++launches_;
   RelabelKernel<<<(n_ + 255) / 256, 256, 0, stream_>>>(d_label_.p, d_fwd_.p, n_);
   n_groups_ = -1;
