@@ -90,10 +90,10 @@ void FinishEncoding(int32_t n, int64_t arcs, const int32_t* head, const int32_t*
   if (out) {
     std::memset(out, 0, sizeof(*out));
     out->supernodes = enc.supernodes;
-    out->p = static_cast<int64_t>(enc.P.size());
-    out->cp = static_cast<int64_t>(enc.Cp.size());
-    out->cm = static_cast<int64_t>(enc.Cm.size());
-    for (const unsigned long long key : enc.P) out->superedges_loop += (key >> 32) == (key & 0xffffffffu);
+    out->p = enc.p;
+    out->cp = enc.cp;
+    out->cm = enc.cm;
+    out->superedges_loop = enc.p_loops;
     out->superedges_nonloop = out->p - out->superedges_loop;
     out->encoding_cost_standard = out->p + out->cp + out->cm;
     out->encoding_cost_mags_x2 = 2 * out->encoding_cost_standard;
@@ -190,6 +190,10 @@ int beam_encode(int32_t n, int64_t arcs, const int64_t* row_ptr, const int32_t* 
     for (const EdgePair& e : P) enc.P.push_back(PairKey(e));
     for (const EdgePair& e : Cp) enc.Cp.push_back(PairKey(e));
     for (const EdgePair& e : Cm) enc.Cm.push_back(PairKey(e));
+    enc.p = static_cast<int64_t>(P.size());
+    enc.cp = static_cast<int64_t>(Cp.size());
+    enc.cm = static_cast<int64_t>(Cm.size());
+    for (const EdgePair& e : P) enc.p_loops += e.a == e.b;
     beam::FinishEncoding(n, row_ptr[n], head, next, enc, out_dir, out);
     return 0;
   } catch (const std::exception& e) {

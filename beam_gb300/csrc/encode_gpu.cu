@@ -9,8 +9,10 @@
 //   decision           per block: corrections only (Cp: all its edges) when
 //                      edges <= 1 + capacity - edges, else a superedge (P) and
 //                      the block's missing member pairs (Cm)
-//   Cm                 per dense block, every member pair is looked up among
-//                      the block's sorted edges
+//   Cm                 per dense block with missing pairs, every member pair is
+//                      looked up among the block's sorted edges
+// The lengths of the lists alone (EncodeCounts) need no list: the quotient
+// rows hold every block's edge count.
 // P comes out sorted; Cp and Cm are radix-sorted by (u, v). The host writes
 // G.txt / P.txt / Cp.txt / Cm.txt with the same formatting as beam_encode.
 #include <cub/device/device_radix_sort.cuh>
@@ -140,21 +142,48 @@ __global__ void EmitSparseKernel(EmitParams E, long long positions) {
   }
 }
 
-__global__ void EmitDenseKernel(EmitParams E) {
+// A share of a dense block's member pairs.
+struct DenseUnit {
+  long long t0;  // first pair
+  int r;         // block
+  int pad;
+};
+constexpr int kDenseUnit = 1024;
+
+// A thread per block: the superedges, and the units of the blocks that miss
+// pairs (a complete block has none). A CTA per block in turn spent 20 ms on the
+// 15 million blocks of an R-MAT-20 summary, nearly all of them sparse.
+__global__ void DenseUnitsKernel(EmitParams E, DenseUnit* units, unsigned long long* nunits) {
   const int nruns = *E.nruns;
-  for (int r = blockIdx.x; r < nruns; r += gridDim.x) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nruns; r += gridDim.x * blockDim.x) {
     if (E.uniq[r] == kNone) continue;
     if (E.p_off[r + 1] == E.p_off[r]) continue;  // sparse block
+    E.P[E.p_off[r]] = E.uniq[r];
+    if (E.cm_off[r + 1] == E.cm_off[r]) continue;
+    const long long pairs = static_cast<long long>(E.ssize[E.uniq[r] >> 32]) * E.ssize[E.uniq[r] & 0xffffffffu];
+    const long long n = (pairs + kDenseUnit - 1) / kDenseUnit;
+    const unsigned long long at = atomicAdd(nunits, static_cast<unsigned long long>(n));
+    for (long long k = 0; k < n; ++k) units[at + k] = DenseUnit{k * kDenseUnit, r, 0};
+  }
+}
+
+// A warp per unit: the pairs without an edge.
+__global__ void EmitMissingKernel(EmitParams E, const DenseUnit* units, const unsigned long long* nunits) {
+  const int lane = threadIdx.x & 31;
+  const long long total = static_cast<long long>(*nunits);
+  const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  for (long long w = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < total; w += nw) {
+    const int r = units[w].r;
     const int A = static_cast<int>(E.uniq[r] >> 32);
     const int B = static_cast<int>(E.uniq[r] & 0xffffffffu);
-    if (threadIdx.x == 0) E.P[E.p_off[r]] = E.uniq[r];
     const long long sa = E.ssize[A], sb = E.ssize[B];
     const int* ma = E.members + E.moff[A];
     const int* mb = E.members + E.moff[B];
     const long long lo0 = E.run_off[r];
     const long long hi0 = lo0 + E.cnt[r];
     const long long cm_base = E.cm_off[r];
-    for (long long t = threadIdx.x; t < sa * sb; t += blockDim.x) {
+    const long long t1 = units[w].t0 + kDenseUnit < sa * sb ? units[w].t0 + kDenseUnit : sa * sb;
+    for (long long t = units[w].t0 + lane; t < t1; t += 32) {
       const int u = ma[t / sb];
       const int v = mb[t % sb];
       if (A == B && u >= v) continue;
@@ -179,7 +208,95 @@ __global__ void EmitDenseKernel(EmitParams E) {
   }
 }
 
+// Lengths of the lists from the quotient rows: every block once, from its
+// smaller id, and the blocks inside. out: supernodes, p, loops among p, cp, cm.
+struct EncodeSums {
+  long long v[5] = {0, 0, 0, 0, 0};
+  __device__ __forceinline__ void Block(long long cap, long long e, bool loop) {
+    if (e <= 1 + cap - e) {
+      v[3] += e;
+    } else {
+      v[1] += 1;
+      v[2] += loop ? 1 : 0;
+      v[4] += cap - e;
+    }
+  }
+  __device__ __forceinline__ void Row(const QuotientView& Q, int r, long long sr, int first, int stride) {
+    const Entry* row = Q.ent + Q.off[r];
+    const int len = Q.len[r];
+#pragma unroll 4
+    for (int k = first; k < len; k += stride) {
+      const Entry e = row[k];
+      if (EntNb(e) > r) Block(sr * Q.size[EntNb(e)], EntCnt(e), false);
+    }
+  }
+  __device__ __forceinline__ void Flush(unsigned long long* out) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const long long x = WarpSum(v[k]);
+      if ((threadIdx.x & 31) == 0 && x != 0) atomicAdd(&out[k], static_cast<unsigned long long>(x));
+    }
+  }
+};
+constexpr int kCountsLong = 1024;  // rows beyond this are a CTA's work (a hub's row, a warp's, was the pass's tail)
+
+// A warp per supernode; the long rows are listed.
+__global__ void EncodeCountsKernel(QuotientView Q, int n, unsigned long long* out, int* list, unsigned* nlist) {
+  const int lane = threadIdx.x & 31;
+  const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  EncodeSums sums;
+  for (long long r = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < n; r += nw) {
+    const long long sr = Q.size[r];
+    if (sr <= 0) continue;
+    if (lane == 0) {
+      ++sums.v[0];
+      if (Q.internal[r] > 0) sums.Block(sr * (sr - 1) / 2, Q.internal[r], true);
+    }
+    if (Q.len[r] > kCountsLong) {
+      if (lane == 0) list[atomicAdd(nlist, 1u)] = static_cast<int>(r);
+      continue;
+    }
+    sums.Row(Q, static_cast<int>(r), sr, lane, 32);
+  }
+  sums.Flush(out);
+}
+
+__global__ void __launch_bounds__(1024) EncodeLongRowsKernel(QuotientView Q, unsigned long long* out, const int* list,
+                                                             const unsigned* nlist) {
+  EncodeSums sums;
+  for (unsigned i = blockIdx.x; i < *nlist; i += gridDim.x) {
+    const int r = list[i];
+    sums.Row(Q, r, Q.size[r], threadIdx.x, 1024);
+  }
+  sums.Flush(out);
+}
+
 }  // namespace
+
+void Engine::EncodeCounts(EncodeOutput* out) {
+  AllocScope alloc(stream_);
+  d_pc_scalars_.ensure(8);
+  CheckCuda(cudaMemsetAsync(d_pc_scalars_.p, 0, 8 * sizeof(unsigned long long), stream_), "memset counts");
+  ++launches_;
+  // a long row holds that many of the arcs
+  DevBuf<int> list;
+  list.ensure(static_cast<size_t>(arcs_) / kCountsLong + 1);
+  unsigned* nlist = reinterpret_cast<unsigned*>(d_pc_scalars_.p + 5);
+  EncodeCountsKernel<<<static_cast<int>(std::min<long long>((static_cast<long long>(n_) + 7) / 8, 152 * 16)), 256, 0,
+                       stream_>>>(View(), n_, d_pc_scalars_.p, list.p, nlist);
+  ++launches_;
+  EncodeLongRowsKernel<<<152 * 2, 1024, 0, stream_>>>(View(), d_pc_scalars_.p, list.p, nlist);
+  CheckCuda(cudaMemcpyAsync(h_pin_.p, d_pc_scalars_.p, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_),
+            "d2h counts");
+  CheckCuda(cudaStreamSynchronize(stream_), "encode sync");
+  CheckError();
+  out->supernodes = h_pin_.p[0];
+  out->p = h_pin_.p[1];
+  out->p_loops = h_pin_.p[2];
+  out->cp = h_pin_.p[3];
+  out->cm = h_pin_.p[4];
+  if (out->cm < 0) throw std::invalid_argument("edge count exceeds block capacity");
+}
 
 void Engine::Encode(EncodeOutput* out) {
   AllocScope alloc(stream_);
@@ -195,11 +312,11 @@ void Engine::Encode(EncodeOutput* out) {
     d_cub_tmp_.ensure(bytes);
     CheckCuda(cub::DeviceRadixSort::SortPairs(d_cub_tmp_.p, bytes, kin, kout, vin, vout, items, 0, 64, s), "sort");
   };
-  auto sort_keys = [&](const unsigned long long* kin, unsigned long long* kout, long long items) {
+  auto sort_keys = [&](const unsigned long long* kin, unsigned long long* kout, long long items, int bit0 = 0) {
     size_t bytes = 0;
-    CheckCuda(cub::DeviceRadixSort::SortKeys(nullptr, bytes, kin, kout, items, 0, 64, s), "sort size");
+    CheckCuda(cub::DeviceRadixSort::SortKeys(nullptr, bytes, kin, kout, items, bit0, 64, s), "sort size");
     d_cub_tmp_.ensure(bytes);
-    CheckCuda(cub::DeviceRadixSort::SortKeys(d_cub_tmp_.p, bytes, kin, kout, items, 0, 64, s), "sort");
+    CheckCuda(cub::DeviceRadixSort::SortKeys(d_cub_tmp_.p, bytes, kin, kout, items, bit0, 64, s), "sort");
   };
   auto scan_ll = [&](const long long* in, long long* outp, long long items) {
     size_t bytes = 0;
@@ -242,7 +359,7 @@ void Engine::Encode(EncodeOutput* out) {
   members.ensure(un);
   ++launches_;
   NodeSidKernel<<<(n + T - 1) / T, T, 0, s>>>(d_label_.p, sid_of_rep.p, d_qsize_.p, n, nts.p, mkey.p, ssize.p);
-  sort_keys(mkey.p, mkey2.p, n);
+  sort_keys(mkey.p, mkey2.p, n, 32);  // stable: the nodes come in ascending order
   // member offsets: exclusive scan of the supernode sizes; members in
   // (supernode, node) order: the low halves of the sorted keys
   moff.ensure(static_cast<size_t>(S) + 1);
@@ -330,10 +447,21 @@ void Engine::Encode(EncodeOutput* out) {
   ++launches_;
   EmitSparseKernel<<<blocks(arcs), T, 0, s>>>(E, arcs);
   ++launches_;
-  EmitDenseKernel<<<152 * 8, T, 0, s>>>(E);
+  // the member pairs of a block are below 7 times its edges where it is dense
+  DevBuf<DenseUnit> units;
+  DevBuf<unsigned long long> nunits;
+  units.ensure(static_cast<size_t>(np) + static_cast<size_t>(arcs) * 4 / kDenseUnit + 1);
+  nunits.ensure(1);
+  CheckCuda(cudaMemsetAsync(nunits.p, 0, sizeof(unsigned long long), s), "memset");
+  DenseUnitsKernel<<<blocks(nruns), T, 0, s>>>(E, units.p, nunits.p);
+  ++launches_;
+  EmitMissingKernel<<<152 * 8, T, 0, s>>>(E, units.p, nunits.p);
   if (ncp > 0) sort_keys(Cp.p, Cp2.p, ncp);
   if (ncm > 0) sort_keys(Cm.p, Cm2.p, ncm);
   out->supernodes = S;
+  out->p = np;
+  out->cp = ncp;
+  out->cm = ncm;
   out->P.resize(static_cast<size_t>(np));
   out->Cp.resize(static_cast<size_t>(ncp));
   out->Cm.resize(static_cast<size_t>(ncm));
@@ -351,6 +479,7 @@ void Engine::Encode(EncodeOutput* out) {
   }
   CheckCuda(cudaStreamSynchronize(s), "encode sync");
   CheckError();
+  for (const unsigned long long key : out->P) out->p_loops += (key >> 32) == (key & 0xffffffffu);
 }
 
 }  // namespace beam

@@ -14,11 +14,12 @@ namespace beam {
 
 struct EncodeOutput {
   int64_t supernodes = 0;
-  std::vector<unsigned long long> P, Cp, Cm;  // (a << 32 | b), sorted by (a, b)
+  int64_t p = 0, p_loops = 0, cp = 0, cm = 0;  // list lengths, and the loops among P
+  std::vector<unsigned long long> P, Cp, Cm;   // (a << 32 | b), sorted by (a, b); filled for the files only
 };
 
-// Fills `out` from the encoding and writes the four files when out_dir is not
-// NULL; throws std::runtime_error on I/O errors.
+// Fills `out` from the encoding's counts and writes the four files when out_dir
+// is not NULL; throws std::runtime_error on I/O errors.
 void FinishEncoding(int32_t n, int64_t arcs, const int32_t* head, const int32_t* next, const EncodeOutput& enc,
                     const char* out_dir, beam_encoding* out);
 

@@ -738,10 +738,16 @@ int beam_engine_ranker_info(beam_engine* e, beam_ranker_info* out) {
 int beam_engine_encode(beam_engine* e, const char* out_dir, beam_encoding* out) {
   return Guard([&] {
     const int n = e->impl->n();
-    std::vector<int32_t> labels(static_cast<size_t>(n)), head(static_cast<size_t>(n)), next(static_cast<size_t>(n));
-    e->impl->Partition(labels.data(), head.data(), next.data());
+    std::vector<int32_t> head, next;  // read for the files only
     beam::EncodeOutput enc;
-    e->impl->Encode(&enc);
+    if (out_dir) {
+      head.resize(static_cast<size_t>(n));
+      next.resize(static_cast<size_t>(n));
+      e->impl->Partition(nullptr, head.data(), next.data());
+      e->impl->Encode(&enc);
+    } else {
+      e->impl->EncodeCounts(&enc);
+    }
     beam::FinishEncoding(n, e->impl->arcs(), head.data(), next.data(), enc, out_dir, out);
   });
 }

@@ -200,8 +200,10 @@ class Engine {
   int64_t ExactPartitionCost();
   // QuotientGraph::ValidateAgainstOriginalGraph: throws on the first mismatch.
   void ValidateQuotient();
-  // Sweg::Encode of the current partition: P (supernode ids), Cp and Cm.
+  // Sweg::Encode of the current partition: P (supernode ids), Cp and Cm; or
+  // their lengths alone.
   void Encode(EncodeOutput* out);
+  void EncodeCounts(EncodeOutput* out);
   const HostStats& host_stats() const { return hstats_; }
   const RankerInfo& ranker_info() const { return rk_info_; }
   int64_t active_count() const { return n_active_; }
@@ -230,6 +232,7 @@ class Engine {
   void EnsurePoolRoom();
   void EnsurePoolRoom(unsigned long long top);
   void CompactPool();
+  int PairCounts();
   void RunBlock(const BlockPlan& bp, double threshold, int iter, int total_iterations);
   void RankerReset();
   void RankerEnsure();

@@ -1,8 +1,9 @@
 // CostOracle::ExactPartitionCost (src/cost_oracle.cpp:112-124) on the device:
 // the encoding cost of the current partition, recomputed from the resident
 // input graph rather than from the quotient graph. Every undirected edge
-// {u, v} becomes the key (min(label u, label v), max(...)); a radix sort and
-// a run-length encode give the edge count of every supernode pair, and each
+// {u, v} becomes the key (min(label u, label v), max(...)), packed into as many
+// bits as the node count needs; a radix sort of these bits and a run-length
+// encode give the edge count of every supernode pair, and each
 // pair contributes BlockCost(size_a, size_b, count, a == b). The reference
 // builds the same counts in a hash map; the sum is the same integer.
 //
@@ -19,36 +20,73 @@
 namespace beam {
 namespace {
 
-constexpr unsigned long long kNoKey = ~0ull;
+// The keys of the edges, in any order: every CTA packs the arcs with u < v of
+// its share. Half the arcs and, at 2^20 nodes, five of eight digits: the sort
+// moves a third of what it did with a 64-bit key per arc.
+constexpr int kKeyTile = 2048;
 
-__global__ void PairKeysKernel(const int* __restrict__ arc_src, const int* __restrict__ col,
-                               const int* __restrict__ label, long long arcs,
-                               unsigned long long* __restrict__ keys) {
-  for (long long k = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; k < arcs;
-       k += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int u = arc_src[k];
-    const int v = col[k];
-    if (u >= v) {
-      keys[k] = kNoKey;  // each undirected edge once (u < v)
-      continue;
+__global__ void __launch_bounds__(256) PairKeysKernel(const int* __restrict__ arc_src, const int* __restrict__ col,
+                                                      const int* __restrict__ label, long long arcs, int bits,
+                                                      unsigned long long* __restrict__ keys,
+                                                      unsigned long long* __restrict__ count) {
+  constexpr int kPer = kKeyTile / 256;
+  __shared__ unsigned warp_n[8];
+  __shared__ unsigned long long base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long t0 = static_cast<long long>(blockIdx.x) * kKeyTile; t0 < arcs;
+       t0 += static_cast<long long>(gridDim.x) * kKeyTile) {
+    unsigned long long key[kPer];
+    unsigned have = 0, mine = 0;
+#pragma unroll
+    for (int d = 0; d < kPer; ++d) {
+      const long long k = t0 + d * 256 + threadIdx.x;
+      key[d] = 0;
+      if (k >= arcs) continue;
+      const int u = arc_src[k];
+      const int v = col[k];
+      if (u >= v) continue;  // each undirected edge once (u < v)
+      const unsigned long long a = static_cast<unsigned>(label[u]);
+      const unsigned long long b = static_cast<unsigned>(label[v]);
+      key[d] = a < b ? a << bits | b : b << bits | a;
+      have |= 1u << d;
+      ++mine;
     }
-    const unsigned a = static_cast<unsigned>(label[u]);
-    const unsigned b = static_cast<unsigned>(label[v]);
-    keys[k] = a < b ? (static_cast<unsigned long long>(a) << 32 | b) : (static_cast<unsigned long long>(b) << 32 | a);
+    unsigned incl = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_n[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned total = 0;
+      for (int w = 0; w < 8; ++w) {
+        const unsigned x = warp_n[w];
+        warp_n[w] = total;
+        total += x;
+      }
+      base = atomicAdd(count, static_cast<unsigned long long>(total));
+    }
+    __syncthreads();
+    unsigned long long at = base + warp_n[warp] + (incl - mine);
+#pragma unroll
+    for (int d = 0; d < kPer; ++d) {
+      if ((have >> d) & 1u) keys[at++] = key[d];
+    }
+    __syncthreads();  // the shared words are rewritten by the next tile
   }
 }
 
 __global__ void PairCostKernel(const unsigned long long* __restrict__ uniq, const int* __restrict__ counts,
-                               const int* __restrict__ nruns_p, const int* __restrict__ size,
+                               const int* __restrict__ nruns_p, int bits, const int* __restrict__ size,
                                unsigned long long* __restrict__ total, DevError* err) {
   const int nruns = *nruns_p;
   long long acc = 0;
   int bad = 0;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nruns; r += gridDim.x * blockDim.x) {
     const unsigned long long key = uniq[r];
-    if (key == kNoKey) continue;
-    const int a = static_cast<int>(key >> 32);
-    const int b = static_cast<int>(key & 0xffffffffu);
+    const int a = static_cast<int>(key >> bits);
+    const int b = static_cast<int>(key & ((1ull << bits) - 1));
     acc += BlockCost(size[a], size[b], counts[r], a == b, bad);
   }
   if (bad) RaiseError(err, kErrBlockCost, 0, 0, 0);
@@ -63,14 +101,13 @@ __global__ void PairCostKernel(const unsigned long long* __restrict__ uniq, cons
 // as the rebuild has distinct neighbours. Mismatches are recorded as the
 // smallest representative they concern.
 __global__ void ValidatePairsKernel(const unsigned long long* __restrict__ uniq, const int* __restrict__ counts,
-                                    const int* __restrict__ nruns_p, QuotientView Q, int* __restrict__ nbr_cnt,
+                                    const int* __restrict__ nruns_p, int bits, QuotientView Q, int* __restrict__ nbr_cnt,
                                     int* __restrict__ int_seen, int* __restrict__ bad_rep) {
   const int nruns = *nruns_p;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nruns; r += gridDim.x * blockDim.x) {
     const unsigned long long key = uniq[r];
-    if (key == kNoKey) continue;
-    const int a = static_cast<int>(key >> 32);
-    const int b = static_cast<int>(key & 0xffffffffu);
+    const int a = static_cast<int>(key >> bits);
+    const int b = static_cast<int>(key & ((1ull << bits) - 1));
     const long long c = counts[r];
     if (a == b) {
       int_seen[a] = 1;
@@ -127,6 +164,36 @@ __global__ void SizesMatchKernel(const int* __restrict__ size_cnt, int n, const 
 
 }  // namespace
 
+// Sorts the edges' supernode-pair keys and counts them: the pairs in
+// d_pc_keys_[0], their edges in d_pc_counts_, their number in the int at
+// d_pc_scalars_ + 1. Returns the bits of a supernode id in a key.
+int Engine::PairCounts() {
+  const long long arcs = arcs_;
+  cudaStream_t s = stream_;
+  int bits = 1;
+  while ((1ll << bits) < n_) ++bits;
+  int* nruns = reinterpret_cast<int*>(d_pc_scalars_.p + 1);
+  const int grid = static_cast<int>(std::min<long long>((arcs + kKeyTile - 1) / kKeyTile, 152 * 8));
+  ++launches_;
+  PairKeysKernel<<<grid, 256, 0, s>>>(d_arc_src_.p, d_col_.p, d_label_.p, arcs, bits, d_pc_keys_[0].p,
+                                      d_pc_scalars_.p + 3);
+  CheckCuda(cudaMemcpyAsync(h_pin_.p, d_pc_scalars_.p + 3, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
+            "d2h edge count");
+  CheckCuda(cudaStreamSynchronize(s), "sync");
+  const long long edges = h_pin_.p[0];
+  size_t sort_bytes = 0, rle_bytes = 0;
+  CheckCuda(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, d_pc_keys_[0].p, d_pc_keys_[1].p, edges, 0, 2 * bits,
+                                           s), "cub sort size");
+  CheckCuda(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, d_pc_keys_[1].p, d_pc_keys_[0].p, d_pc_counts_.p,
+                                               nruns, edges, s), "cub rle size");
+  d_cub_tmp_.ensure(std::max(sort_bytes, rle_bytes));
+  CheckCuda(cub::DeviceRadixSort::SortKeys(d_cub_tmp_.p, sort_bytes, d_pc_keys_[0].p, d_pc_keys_[1].p, edges, 0,
+                                           2 * bits, s), "cub sort");
+  CheckCuda(cub::DeviceRunLengthEncode::Encode(d_cub_tmp_.p, rle_bytes, d_pc_keys_[1].p, d_pc_keys_[0].p,
+                                               d_pc_counts_.p, nruns, edges, s), "cub rle");
+  return bits;
+}
+
 void Engine::ValidateQuotient() {
   AllocScope alloc(stream_);
   const long long arcs = arcs_;
@@ -135,7 +202,7 @@ void Engine::ValidateQuotient() {
   d_pc_keys_[0].ensure(static_cast<size_t>(arcs) + 1);
   d_pc_keys_[1].ensure(static_cast<size_t>(arcs) + 1);
   d_pc_counts_.ensure(static_cast<size_t>(arcs) + 1);
-  d_pc_scalars_.ensure(4);
+  d_pc_scalars_.ensure(8);
   DevBuf<int> cnt;  // neighbour counts | internal seen | label sizes | 2 bad markers
   cnt.ensure(3 * un + 2);
   int* nbr_cnt = cnt.p;
@@ -148,23 +215,12 @@ void Engine::ValidateQuotient() {
   const int grid = static_cast<int>(std::min<long long>((std::max<long long>(arcs, n_) + 255) / 256, 152 * 16));
   int* nruns = reinterpret_cast<int*>(d_pc_scalars_.p + 1);
   if (arcs > 0) {
+    const int bits = PairCounts();
     ++launches_;
-    PairKeysKernel<<<grid, 256, 0, s>>>(d_arc_src_.p, d_col_.p, d_label_.p, arcs, d_pc_keys_[0].p);
-    size_t sort_bytes = 0, rle_bytes = 0;
-    CheckCuda(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, d_pc_keys_[0].p, d_pc_keys_[1].p, arcs, 0, 64, s),
-              "cub sort size");
-    CheckCuda(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, d_pc_keys_[1].p, d_pc_keys_[0].p,
-                                                 d_pc_counts_.p, nruns, arcs, s), "cub rle size");
-    d_cub_tmp_.ensure(std::max(sort_bytes, rle_bytes));
-    CheckCuda(cub::DeviceRadixSort::SortKeys(d_cub_tmp_.p, sort_bytes, d_pc_keys_[0].p, d_pc_keys_[1].p, arcs, 0,
-                                             64, s), "cub sort");
-    CheckCuda(cub::DeviceRunLengthEncode::Encode(d_cub_tmp_.p, rle_bytes, d_pc_keys_[1].p, d_pc_keys_[0].p,
-                                                 d_pc_counts_.p, nruns, arcs, s), "cub rle");
-    ++launches_;
-    ValidatePairsKernel<<<grid, 256, 0, s>>>(d_pc_keys_[0].p, d_pc_counts_.p, nruns, View(), nbr_cnt, int_seen,
+    ValidatePairsKernel<<<grid, 256, 0, s>>>(d_pc_keys_[0].p, d_pc_counts_.p, nruns, bits, View(), nbr_cnt, int_seen,
                                              bad + 1);
     ++launches_;
-    PairCostKernel<<<grid, 256, 0, s>>>(d_pc_keys_[0].p, d_pc_counts_.p, nruns, d_qsize_.p, d_pc_scalars_.p,
+    PairCostKernel<<<grid, 256, 0, s>>>(d_pc_keys_[0].p, d_pc_counts_.p, nruns, bits, d_qsize_.p, d_pc_scalars_.p,
                                         d_err_.p);
   }
   ++launches_;
@@ -192,25 +248,14 @@ int64_t Engine::ExactPartitionCost() {
   d_pc_keys_[0].ensure(static_cast<size_t>(arcs) + 1);
   d_pc_keys_[1].ensure(static_cast<size_t>(arcs) + 1);
   d_pc_counts_.ensure(static_cast<size_t>(arcs) + 1);
-  d_pc_scalars_.ensure(4);
+  d_pc_scalars_.ensure(8);
   CheckCuda(cudaMemsetAsync(d_pc_scalars_.p, 0, 4 * sizeof(unsigned long long), s), "memset cost");
   const int grid = static_cast<int>(std::min<long long>((arcs + 255) / 256, 152 * 16));
   if (arcs > 0) {
-    ++launches_;
-    PairKeysKernel<<<grid, 256, 0, s>>>(d_arc_src_.p, d_col_.p, d_label_.p, arcs, d_pc_keys_[0].p);
-    size_t sort_bytes = 0, rle_bytes = 0;
     int* nruns = reinterpret_cast<int*>(d_pc_scalars_.p + 1);
-    CheckCuda(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, d_pc_keys_[0].p, d_pc_keys_[1].p, arcs, 0, 64, s),
-              "cub sort size");
-    CheckCuda(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, d_pc_keys_[1].p, d_pc_keys_[0].p,
-                                                 d_pc_counts_.p, nruns, arcs, s), "cub rle size");
-    d_cub_tmp_.ensure(std::max(sort_bytes, rle_bytes));
-    CheckCuda(cub::DeviceRadixSort::SortKeys(d_cub_tmp_.p, sort_bytes, d_pc_keys_[0].p, d_pc_keys_[1].p, arcs, 0,
-                                             64, s), "cub sort");
-    CheckCuda(cub::DeviceRunLengthEncode::Encode(d_cub_tmp_.p, rle_bytes, d_pc_keys_[1].p, d_pc_keys_[0].p,
-                                                 d_pc_counts_.p, nruns, arcs, s), "cub rle");
+    const int bits = PairCounts();
     ++launches_;
-    PairCostKernel<<<grid, 256, 0, s>>>(d_pc_keys_[0].p, d_pc_counts_.p, nruns, d_qsize_.p, d_pc_scalars_.p,
+    PairCostKernel<<<grid, 256, 0, s>>>(d_pc_keys_[0].p, d_pc_counts_.p, nruns, bits, d_qsize_.p, d_pc_scalars_.p,
                                         d_err_.p);
   }
   unsigned long long total = 0;
