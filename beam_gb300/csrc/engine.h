@@ -341,10 +341,10 @@ class Engine {
   bool plan_on_device_ = false;
   // windows of blocks (window.cuh)
   bool windowed_ = false;
-  DevBuf<int> d_ri_of_, d_node_ri_, d_blk_end_, d_dirty_, d_win_list_;
+  DevBuf<int> d_ri_of_, d_node_ri_, d_blk_beg_, d_blk_end_, d_dirty_, d_win_list_;
   DevBuf<long long> d_win_off_;
   DevBuf<int> d_conflict_;
-  DevBuf<unsigned char> d_gs_, d_wctl_, d_units_;
+  DevBuf<unsigned char> d_gs_, d_wctl_, d_units_, d_win_big_;
   int accum_grid_ = 152 * 4;  // resident CTAs of the dynamically scheduled kernels
   int score_grid_ = 152 * 4;   // one-block iteration: Merge plans it on the device
   DevBuf<unsigned char> d_plan_tiles_;

@@ -65,6 +65,8 @@ constexpr int kWarpRowMax = 256;     // neighbour rows rewritten by one warp thr
 // Neighbour rows of more than kRowSmem entries are rewritten in two steps: the
 // renamed entries found by warps over kHugeUnit entries each, the row moved by
 // one CTA in chunks of kHugeChunk.
+// (A window's batch claims few rows: the shorter ones gain from it too.)
+constexpr int kWindowRow = 256;
 constexpr int kHugeUnit = 1024;
 constexpr int kHugeThreads = 1024;
 constexpr int kHugePer = 8;
@@ -2899,7 +2901,7 @@ __device__ __forceinline__ void ClaimRow(const CommitParams& P, int x) {
   const int len = P.Q.len[x];
   if (len <= kWarpRowMax) {
     P.rows_short[atomicAdd(&P.ctl->short_cnt, 1u)] = x;
-  } else if (len <= kRowSmem) {
+  } else if (len <= (P.windowed ? kWindowRow : kRowSmem)) {
     P.rows_long[atomicAdd(&P.ctl->long_cnt, 1u)] = x;
   } else {
     int pow2 = 1;
@@ -2929,7 +2931,7 @@ __device__ __forceinline__ void ClaimRow(const CommitParams& P, int x) {
 __device__ __forceinline__ void MarkTouched(const CommitParams& P, int x, int p, int e) {
   const int ri = P.W.node_ri[x];
   if (ri < p || ri >= e) return;
-  if (atomicExch(&P.W.dirty[ri], P.block_stamp) == P.block_stamp) return;
+  if (P.W.dirty[ri] != 0 || atomicExch(&P.W.dirty[ri], 1) != 0) return;
   P.W.list_dirty[atomicAdd(&P.W.ctl->ndirty, 1)] = ri;
 }
 
@@ -2945,6 +2947,7 @@ __device__ __forceinline__ void MarkTouched(const CommitParams& P, int x, int p,
 // and a claimed neighbour row is touched by its claimant alone, so the CTAs
 // need no ordering among themselves.
 __global__ void __launch_bounds__(kRowsThreads) CommitKernel(CommitParams P) {
+  FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RowsSmem& R = *reinterpret_cast<RowsSmem*>(smem_raw);
   __shared__ long long new_off;
@@ -3339,6 +3342,22 @@ __device__ void RewriteLongRows(const CommitParams& P, RowsSmem& R) {
   }
 }
 
+// First position of a sorted row whose neighbour is >= x, by the whole warp.
+__device__ __forceinline__ int WarpRowLowerBound(const Entry* row, int len, int x) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, hi = len;  // the answer lies in [lo, hi]
+  while (lo < hi) {
+    // 32 probes of [lo, hi), non-decreasing over the lanes
+    const int p = lo + static_cast<int>((static_cast<long long>(hi - lo) * lane) >> 5);
+    const int k = __popc(__ballot_sync(0xffffffffu, EntNb(row[p]) < x));  // lanes 0..k-1 are below
+    const int below = __shfl_sync(0xffffffffu, p, k > 0 ? k - 1 : 0);
+    const int above = __shfl_sync(0xffffffffu, p, k < 32 ? k : 31);
+    if (k < 32) hi = above;
+    if (k > 0) lo = below + 1; else hi = lo;
+  }
+  return lo;
+}
+
 // First step of the longer rows, a warp per kHugeUnit entries: marks the
 // entries of supernodes removed in this block, adds each one's count to its
 // keep's entry in the row (ids stay in place, so the row stays searchable) or
@@ -3375,10 +3394,22 @@ __device__ void ScanHugeRows(const CommitParams& P) {
         const bool renamed = st[d] == remove_stamp;
         const unsigned m = __ballot_sync(0xffffffffu, renamed);
         if (lane == 0 && i0 + 32 * d < end) mask[(i0 >> 5) + d] = m;
+        // the keep's place in the row: by the whole warp for one or two of them
+        // (three rounds of loads instead of a dozen), else each lane its own
+        int at = 0;
+        const int kp = renamed ? P.partner[EntNb(e[d])] : 0;
+        if (__popc(m) <= 2) {
+          for (unsigned rest = m; rest; rest &= rest - 1) {
+            const int src = __ffs(rest) - 1;
+            const int x = WarpRowLowerBound(row, len, __shfl_sync(0xffffffffu, kp, src));
+            if (lane == src) at = x;
+          }
+        } else if (renamed) {
+          at = RowLowerBound(row, len, kp);
+        }
         if (renamed) {
-          const int kp = P.partner[EntNb(e[d])];
           const long long c = EntCnt(e[d]);
-          const int p = RowLowerBound(row, len, kp);
+          const int p = at;
           if (p < len && EntNb(row[p]) == kp) {
             atomicAdd(&row[p], static_cast<unsigned long long>(c));
           } else {
@@ -3393,6 +3424,7 @@ __device__ void ScanHugeRows(const CommitParams& P) {
 // All claimed neighbour rows of a block: the long ones by whole CTAs, then the
 // first step of the longest, then the short ones by single warps.
 __global__ void __launch_bounds__(kRowsThreads) RewriteRowsKernel(CommitParams P) {
+  FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RowsSmem& R = *reinterpret_cast<RowsSmem*>(smem_raw);
   ScanHugeRows(P);
@@ -3460,6 +3492,7 @@ __device__ void StageMask(HugeSmem& H, const unsigned* mask, int base, int len) 
 // The last CTA clears the block control words for the next block: all their
 // readers are done by then.
 __global__ void __launch_bounds__(kHugeThreads) RewriteHugeKernel(CommitParams P) {
+  FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   HugeSmem& H = *reinterpret_cast<HugeSmem*>(smem_raw);
   __shared__ bool last;
@@ -3678,20 +3711,20 @@ __device__ __forceinline__ PlanSums PlanZero() {
 }
 
 // one group's contribution: the same rules as the host plan
-__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, int small_max) {
+__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, int windowed) {
   PlanSums f = PlanZero();
   if (g < 2) return f;
   const long long gl = g;
   f.real = 1;
   f.cand = gl * (gl - 1) / 2 < gl * k ? gl * (gl - 1) / 2 : gl * k;
   f.sel = gl / 2;
-  if (g <= small_max && e <= static_cast<unsigned>(kSmallStage)) {
+  if (windowed ? WindowSmall(g, e) : g <= kSmallGroup && e <= static_cast<unsigned>(kSmallStage)) {
     f.small[SmallClass(g)] = 1;
   } else {
     f.big = 1;
     f.moff = gl;
     f.soff = e > static_cast<unsigned>(kSmemEntries) || g > kSmemMaxGroup ? static_cast<long long>(e) : 0;
-    f.mat = (OldCostOffset(gl * gl) + 8 * gl + 255) & ~255ll;
+    f.mat = windowed ? WindowBytes(gl, e) : (OldCostOffset(gl * gl) + 8 * gl + 255) & ~255ll;
   }
   if (g <= kSelectSmallGroup) {
     f.ssmall = 1;
@@ -3708,7 +3741,7 @@ struct PlanParams {
   const unsigned* gent;
   long long G;
   long long top_k;
-  int small_max;  // members of a group that one warp handles
+  int windowed;  // 1: the sizes and limits of window.cuh
   PlanSums* tile_sums;
   PlanSums* tile_off;
   int tiles;
@@ -3736,7 +3769,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanTileKernel(PlanParams P) {
   for (int j = 0; j < kPlanItems; ++j) {
     const long long gi = base + j;
     if (gi >= P.G) break;
-    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k, P.small_max);
+    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k, P.windowed);
     acc = PlanSumOp()(acc, f);
     max_e = f.soff > max_e ? f.soff : max_e;
   }
@@ -3805,13 +3838,13 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
     const long long gi = base + j;
     g[j] = gi < P.G ? P.glen[gi] : 0;
     e[j] = gi < P.G ? P.gent[gi] : 0u;
-    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k, P.small_max));
+    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k, P.windowed));
   }
   PlanSums off;
   Scan(tmp).ExclusiveScan(acc, off, P.tile_off[blockIdx.x], PlanSumOp());
 #pragma unroll
   for (int j = 0; j < kPlanItems; ++j) {
-    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k, P.small_max);
+    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k, P.windowed);
     if (P.ri_of && base + j < P.G) P.ri_of[base + j] = f.real ? off.real : -1;
     if (f.real) {
       const int ri = off.real;
@@ -4068,7 +4101,7 @@ void Engine::PlanOnDevice() {
   P.gent = d_gent_.p;
   P.G = G;
   P.top_k = cfg_.top_k > 0 ? cfg_.top_k : 1;
-  P.small_max = windowed_ ? kEvalSmall : kSmallGroup;
+  P.windowed = windowed_ ? 1 : 0;
   P.tile_sums = reinterpret_cast<PlanSums*>(d_plan_tiles_.p);
   P.tile_off = P.tile_sums + tiles;
   P.tiles = tiles;
@@ -4147,6 +4180,24 @@ void CommitDefaults(CommitParams* C) {
 }
 }  // namespace
 
+namespace {
+// A launch whose kernel begins with FollowsOn.
+template <typename Params>
+void LaunchFollowing(void (*kernel)(Params), int grid, int threads, size_t smem, cudaStream_t stream, Params p) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  CheckCuda(cudaLaunchKernelEx(&cfg, kernel, p), "window launch");
+}
+}  // namespace
+
 void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, const void* window) {
   CommitParams C;
   CommitDefaults(&C);
@@ -4180,9 +4231,10 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, cons
   C.err = d_err_.p;
   C.rows_short = d_rows_short_.p;
   C.rows_long = d_rows_long_.p;
-  // a row of more than kRowSmem entries holds that many of the arcs
-  d_rows_huge_.ensure(sizeof(HugeRow) * (static_cast<size_t>(arcs_) / kRowSmem + 1));
-  d_huge_units_.ensure(static_cast<size_t>(arcs_) / kHugeUnit + static_cast<size_t>(arcs_) / kRowSmem + 1);
+  // a row of more than `limit` entries holds that many of the arcs
+  const size_t limit = window ? kWindowRow : kRowSmem;
+  d_rows_huge_.ensure(sizeof(HugeRow) * (static_cast<size_t>(arcs_) / limit + 1));
+  d_huge_units_.ensure(static_cast<size_t>(arcs_) / kHugeUnit + static_cast<size_t>(arcs_) / limit + 1);
   C.rows_huge = reinterpret_cast<HugeRow*>(d_rows_huge_.p);
   C.huge_units = d_huge_units_.p;
   C.ticket = d_rw_ticket_.p;
@@ -4205,11 +4257,16 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, cons
     CommitShortKernel<<<static_cast<int>(std::min<int64_t>((max_pairs + 7) / 8 + 1, 152 * 8)), 256, 0, stream_>>>(C);
     ++launches_;
   }
-  CommitKernel<<<grid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
-  ++launches_;
-  RewriteRowsKernel<<<kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
-  ++launches_;
-  RewriteHugeKernel<<<kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_>>>(C);
+  launches_ += 2;
+  if (window) {
+    LaunchFollowing(CommitKernel, grid, kRowsThreads, sizeof(RowsSmem), stream_, C);
+    LaunchFollowing(RewriteRowsKernel, kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_, C);
+    LaunchFollowing(RewriteHugeKernel, kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_, C);
+  } else {
+    CommitKernel<<<grid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
+    RewriteRowsKernel<<<kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
+    RewriteHugeKernel<<<kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_>>>(C);
+  }
   EndTimed(kTimeUpdate);
 }
 
@@ -4458,9 +4515,11 @@ void Engine::RunWindows(double threshold) {
   const size_t ur = static_cast<size_t>(R);
   d_node_ri_.ensure(static_cast<size_t>(n_));
   d_blk_end_.ensure(ur + 1);
+  d_blk_beg_.ensure(ur + 1);
   d_dirty_.ensure(ur + 1);
   d_gs_.ensure(sizeof(GroupStats) * (ur + 1));
-  d_win_list_.ensure(3 * static_cast<size_t>(kWindowList));
+  d_win_list_.ensure(2 * static_cast<size_t>(kWindowList));
+  d_win_big_.ensure(sizeof(BigGroup) * kWindowList);
   d_win_off_.ensure(2 * static_cast<size_t>(kWindowList) + 2);
   d_conflict_.ensure(ur + 1);
   d_units_.ensure(sizeof(LongUnit) * kLongUnits);
@@ -4475,6 +4534,8 @@ void Engine::RunWindows(double threshold) {
   W.real = d_real_.p;
   W.node_ri = d_node_ri_.p;
   W.blk_end = d_blk_end_.p;
+  W.blk_beg = d_blk_beg_.p;
+  W.idx_in_group = d_idx_in_group_.p;
   W.ctl = reinterpret_cast<WindowCtl*>(d_wctl_.p);
   W.gs = reinterpret_cast<GroupStats*>(d_gs_.p);
   W.conflict = d_conflict_.p;
@@ -4482,7 +4543,7 @@ void Engine::RunWindows(double threshold) {
   W.dirty = d_dirty_.p;
   W.list_dirty = d_win_list_.p;
   W.list_small = d_win_list_.p + kWindowList;
-  W.list_big = d_win_list_.p + 2 * kWindowList;
+  W.list_big = reinterpret_cast<BigGroup*>(d_win_big_.p);
   W.moff = d_win_off_.p;
   W.poff = d_win_off_.p + kWindowList + 1;
   W.mat_off = d_mat_off_.p;
@@ -4515,8 +4576,8 @@ void Engine::RunWindows(double threshold) {
   const int count = static_cast<int>(n_active_);
   ++launches_;
   WindowSetupKernel<<<(std::max(count, R) + 255) / 256, 256, 0, stream_>>>(
-      W.order, W.group_of, d_ri_of_.p, count, W.real, R, cfg_.group_batch_size, d_node_ri_.p, d_blk_end_.p, W.dirty,
-      W.ctl);
+      W.order, W.group_of, d_ri_of_.p, count, W.real, R, cfg_.group_batch_size, d_node_ri_.p, d_blk_beg_.p, d_blk_end_.p,
+      W.dirty, W.ctl);
   ++launches_;
   WindowBeginKernel<<<1, kHugeThreads, 0, stream_>>>(W, R);
   // the host keeps a few rounds queued behind the one running; a round past
@@ -4538,15 +4599,16 @@ void Engine::RunWindows(double threshold) {
     ++block_stamp_;
     W.block_stamp = block_stamp_;
     BeginTimed(kTimePrepare);
-    WindowEvalKernel<<<kEvalGrid, kEvalWarps * 32, sizeof(EvalSmem), stream_>>>(W);
-    WindowLongKernel<<<kLongGrid, kLongThreads, 0, stream_>>>(W);
+    LaunchFollowing(WindowEvalKernel, kEvalGrid, kEvalWarps * 32, sizeof(EvalSmem), stream_, W);
+    LaunchFollowing(WindowLongKernel, kLongGrid, kLongThreads, 0, stream_, W);
+    LaunchFollowing(WindowPairsKernel, kPairGrid, kPairWarps * 32, sizeof(PairTable) * kPairWarps, stream_, W);
     EndTimed(kTimePrepare);
     BeginTimed(kTimeScore);
-    WindowScoreKernel<<<kBigGrid, 256, 0, stream_>>>(W);
-    WindowSelectKernel<<<kBigGrid, kMatchThreads, 8 * kMatchSmemKeys, stream_>>>(W);
+    LaunchFollowing(WindowScoreKernel, kBigGrid, 256, 0, stream_, W);
+    LaunchFollowing(WindowSelectKernel, kBigGrid, kMatchThreads, 8 * kMatchSmemKeys, stream_, W);
     EndTimed(kTimeScore);
-    WindowMarkKernel<<<kMarkGrid, kMarkThreads, 0, stream_>>>(W);
-    launches_ += 5;
+    LaunchFollowing(WindowMarkKernel, kMarkGrid, kMarkThreads, 0, stream_, W);
+    launches_ += 6;
     LaunchCommit(0, R, kBigGrid, cfg_.verify_cuda_gain, &W);
   }
   CheckCuda(cudaMemcpyAsync(h_pin_.p + 9, &W.ctl->blocks, sizeof(long long), cudaMemcpyDeviceToHost, stream_),

@@ -17,13 +17,13 @@
 // The decisions, counters and rows are those of the blocks in order; only
 // evaluations that stood when their block's turn came are counted.
 //
-// One round is eight launches that take their work from device memory, for as
+// One round is nine launches that take their work from device memory, for as
 // many blocks as turned out independent (a block at a time took a dozen
 // launches, 75 to 120 us, latency only). Rounds follow each other without the
 // host, which watches the frontier through mapped memory and keeps a few
 // rounds queued. Measured with 64-group blocks, 20 iterations, a block at a time
-// -> windows: R-MAT 16 (edge factor 8) 621 -> 132 ms, R-MAT 12 36.7 -> 18.4 ms,
-// Chung-Lu of 20,000 nodes with twins 109 -> 69 ms.
+// -> windows: R-MAT 16 (edge factor 8) 622 -> 120 ms, R-MAT 12 37.1 -> 14.9 ms,
+// Chung-Lu of 20,000 nodes with twins 109 -> 52 ms.
 #pragma once
 
 // Blocks of at most this many groups go through windows; larger ones fill the
@@ -31,40 +31,74 @@
 constexpr int kWindowMaxBatch = 256;
 constexpr int kWindowMaxGroups = 8192;  // groups a window takes in at most (then to the block's end)
 constexpr int kWindowMinGroups = 256;
+constexpr int kWindowMinAgain = 64;
 constexpr int kWindowList = 2 * (kWindowMaxGroups + kWindowMaxBatch) + 1024;
 constexpr int kEvalWarps = 4;
-constexpr int kEvalPairs = 16;   // member pairs per work item of a big group, at most
 constexpr int kEvalCtas = 8;     // per SM
 constexpr int kEvalGrid = 152 * kEvalCtas;
 constexpr int kBigGrid = 152 * 2;
 constexpr int kMarkGrid = 16;
 constexpr int kMarkThreads = 256;
-// Rows and pairs of rows longer than this are handed on in units, so that no
-// warp holds up a round with a hub's row.
-constexpr int kLongRow = 1024;       // entries of a row (sums), of two rows to merge
-constexpr int kLongProbe = 96;       // entries to look up in a far longer row
-constexpr int kLongRowUnit = 1024;   // entries of a row per unit
-constexpr int kLongPairUnit = 128;   // entries of the shorter row per unit
+constexpr int kWindowAhead = 2;  // rounds queued by the host and not seen done
+// Rows longer than this are handed on in units, so that no warp holds up a
+// round with a hub's row.
+constexpr int kLongRow = 256;
+constexpr int kLongRowUnit = 256;   // entries per unit
 constexpr int kLongUnits = 1 << 19;  // units at most; what does not fit is done in place
 constexpr int kLongThreads = 256;
 constexpr int kLongGrid = 152 * 6;
-// Groups of at most top_k + 1 members need no ranking; a warp handles one with
-// up to this many.
-constexpr int kEvalSmall = 17;
+// A warp handles a group of this size alone. Its steps are a chain, 5 us at
+// this size and up to 75 us at 17 members with 256 entries; spread over the
+// GPU, larger groups cost three more launches' latency and little else.
+constexpr int kEvalSmall = 8;
+constexpr int kEvalEntries = 64;
 constexpr int kEvalSmallPairs = kEvalSmall * (kEvalSmall - 1) / 2;
-constexpr int kWindowAhead = 2;  // rounds queued by the host and not seen done
-// Skewed pairs (the long row at least kProbeMinLong entries and kProbeRatio
-// times the short one) look the short row up in the long one.
-constexpr int kProbeMinLong = 256;
-constexpr int kProbeRatio = 8;
+// Pair pass: rows of at most kTableRow entries go into a warp's hash table of
+// kTableSlots; a group's members are split in parts of about kPartEntries.
+constexpr int kTableRow = 512;
+constexpr int kTableSlots = 2 * kTableRow;
+constexpr int kPartEntries = 1024;
+constexpr int kMaxParts = 128;
+constexpr int kPairWarps = 4;
+constexpr int kPairDeep = 4;  // entries per lane in flight
+constexpr int kPairCtas = 6;  // per SM
+constexpr int kPairGrid = 152 * kPairCtas;
+
+__host__ __device__ __forceinline__ int WindowParts(unsigned entries) {
+  const unsigned p = (entries + kPartEntries - 1) / kPartEntries;
+  return p < 1 ? 1 : p > static_cast<unsigned>(kMaxParts) ? kMaxParts : static_cast<int>(p);
+}
+
+// A big group's memory: the pair tables and old costs, every member's place
+// among the staged entries (first, length, size), the staged entries.
+__host__ __device__ __forceinline__ long long PlaceOffset(long long g) { return (OldCostOffset(g * g) + 8 * g + 15) & ~15ll; }
+__host__ __device__ __forceinline__ long long StageOffset(long long g) { return PlaceOffset(g) + 16 * g; }
+__host__ __device__ __forceinline__ long long WindowBytes(long long g, unsigned entries) {
+  return (StageOffset(g) + 16ll * entries + 255) & ~255ll;
+}
+
+// A listed big group, for one load in the kernels.
+struct __align__(16) BigGroup {
+  int ri, gid, g, cap;  // cap: entries that the stage holds
+  int gstart, parts;
+  long long mat;
+};
+
+struct __align__(16) StagedEntry {
+  int t;       // target
+  int size;    // its size
+  unsigned c;  // edges
+  int j;       // member
+};
 
 struct WindowCtl {
   int f, e, R;     // first group not committed; end of the evaluated groups; groups of the iteration
   int p;           // end of the batch being committed
-  int take;        // groups to keep evaluated ahead
+  int stale;       // first evaluated group that is out of date and not listed (INT_MAX: none)
+  int pace;        // groups that a round commits, on average
   int nsmall, nbig, ndirty;
-  long long members, pairs;  // of the listed big groups
-  unsigned long long work;   // queue of the evaluation kernel
+  long long members, parts;  // of the listed big groups: members, and members times parts
+  unsigned long long work;  // queue of the evaluation kernel
   unsigned units;            // long units handed on
   unsigned pad;
   long long blocks;          // blocks with at least one group (per iteration)
@@ -76,17 +110,18 @@ static_assert(sizeof(WindowCtl) <= 256, "room made in Engine::Reset");
 struct GroupStats {
   unsigned long long examined, cand, uni, ovl, raw_a, raw_b, nnz, rejected, positive, selected, gain, work, entries;
   int err, err_a, err_b, pad;
+  int staged_short, staged_long;  // entries staged, of the rows with and without a table
 };
 constexpr int kGroupStatWords = 13;
+static_assert(sizeof(GroupStats) == 128, "");
 
-// Part of a long row (b < 0: its sums, `up` the approximate old cost) or of a
-// pair with a long row (the pair's two words).
+// Part of a long row.
 struct LongUnit {
-  unsigned long long* up;
-  unsigned long long* down;
-  int a, b;  // supernodes
-  int at;    // first entry (of the shorter row)
-  int ri;    // group, -1: nothing to do
+  unsigned long long* old;  // the member's approximate old cost
+  StagedEntry* stage;       // the row's place
+  int rep, i;
+  int at;  // first entry
+  int ri;  // group, -1: nothing to do
 };
 
 struct WindowParams {
@@ -99,15 +134,17 @@ struct WindowParams {
   const int* real;
   const int* node_ri;   // per active supernode: its group's position, -1 alone
   const int* blk_end;   // per group position: first position of the next block
+  const int* blk_beg;   //                     first position of its own block
+  const int* idx_in_group;
   WindowCtl* ctl;
   GroupStats* gs;
   int* conflict;        // per group position: first later group its pairs touch (INT_MAX: none)
   LongUnit* units;
-  int* dirty;           // per group position: stamp of the last commit that touched it
+  int* dirty;           // per group position: 1 touched since its evaluation (and on list_dirty)
   int* list_dirty;
   int* list_small;
-  int* list_big;
-  long long* moff;      // member / pair prefixes over list_big
+  BigGroup* list_big;
+  long long* moff;      // member / part prefixes over list_big
   long long* poff;
   const long long* mat_off;
   unsigned char* mat;
@@ -135,15 +172,25 @@ struct WindowParams {
 };
 
 __device__ __forceinline__ bool WindowSmall(int g, unsigned entries) {
-  return g <= kEvalSmall && entries <= static_cast<unsigned>(kSmallStage);
+  return g <= kEvalSmall && entries <= static_cast<unsigned>(kEvalEntries);
+}
+
+// First thing in every kernel of a round: the next kernel may be set up now,
+// and this one goes on when the one before it is complete (and its writes
+// visible). Takes the launch latency, one of the larger parts of a short
+// kernel, off the chain of a round. No effect on a kernel launched otherwise.
+__device__ __forceinline__ void FollowsOn() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
 }
 
 // ------------------------------------------------------------ lists
 
-// Per active supernode its group position, per group position the end of its
+// Per active supernode its group position, per group position the ends of its
 // block and a clean mark, and the number of blocks.
 __global__ void WindowSetupKernel(const int* order, const int* group_of, const int* ri_of, int count, const int* real,
-                                  int R, int batch, int* node_ri, int* blk_end, int* dirty, WindowCtl* ctl) {
+                                  int R, int batch, int* node_ri, int* blk_beg, int* blk_end, int* dirty,
+                                  WindowCtl* ctl) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) {
     const int rep = order[i];
@@ -157,6 +204,12 @@ __global__ void WindowSetupKernel(const int* order, const int* group_of, const i
       if (real[mid] / batch <= b) lo = mid + 1; else hi = mid;
     }
     blk_end[i] = lo;
+    lo = 0, hi = i;  // first position of this block
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (real[mid] / batch < b) lo = mid + 1; else hi = mid;
+    }
+    blk_beg[i] = lo;
     dirty[i] = 0;
     if (i == 0 || real[i - 1] / batch != b) atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->blocks), 1ull);
   }
@@ -165,12 +218,12 @@ __global__ void WindowSetupKernel(const int* order, const int* group_of, const i
 // The next evaluation's lists, by one CTA of kHugeThreads: the touched groups
 // and those that the window takes in. `done`: groups [f, p) are committed.
 struct ListSum {
-  long long members, pairs;
+  long long members, parts;
   int small, big;
 };
 struct ListSumOp {
   __device__ __forceinline__ ListSum operator()(const ListSum& a, const ListSum& b) const {
-    return ListSum{a.members + b.members, a.pairs + b.pairs, a.small + b.small, a.big + b.big};
+    return ListSum{a.members + b.members, a.parts + b.parts, a.small + b.small, a.big + b.big};
   }
 };
 
@@ -178,40 +231,57 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
   using Scan = cub::BlockScan<ListSum, kHugeThreads, cub::BLOCK_SCAN_WARP_SCANS>;
   __shared__ typename Scan::TempStorage tmp;
   __shared__ ListSum carry;
-  __shared__ int s_e0, s_e1, s_dirty;
+  __shared__ int s_e0, s_e1, s_dirty, s_again, s_kept, s_stale;
   WindowCtl* c = P.ctl;
   if (threadIdx.x == 0) {
+    // new groups are taken in for the next two rounds at the usual pace (the
+    // whole window again where all of it was committed); a touched group is
+    // evaluated again when its turn is that near, not every time it is touched
     const int committed = c->p - c->f;
-    // twice what the last rounds committed is kept evaluated: evaluations
-    // further ahead are likely to be touched before their turn
-    int take = c->p == c->e ? 2 * c->take : 2 * committed;
-    if (c->R == 0 || c->p == 0) take = c->take;  // the iteration's first lists
-    take = take < kWindowMinGroups ? kWindowMinGroups : take > kWindowMaxGroups ? kWindowMaxGroups : take;
-    c->take = take;
+    int pace = c->pace;
+    if (c->p > 0) pace = c->p == c->e ? max(committed, pace) : (3 * pace + committed) / 4;
+    pace = min(pace, kWindowMaxGroups / 2);
+    c->pace = pace;
     c->f = c->p;
+    const int take = min(max(2 * pace, kWindowMinGroups), kWindowMaxGroups);
     int e = c->f + take;
     e = e >= c->R ? c->R : e == 0 ? 0 : P.blk_end[e - 1];
     s_e0 = c->e;
     s_e1 = e > c->e ? e : c->e;
     s_dirty = c->ndirty;
+    // (the next block in any case, so that every round commits one)
+    s_again = max(c->f + max(2 * pace, kWindowMinAgain), c->f < c->R ? P.blk_end[c->f] : 0);
+    s_kept = 0;
+    s_stale = 0x7fffffff;
     carry = ListSum{0, 0, 0, 0};
   }
   __syncthreads();
   const int n = s_dirty + (s_e1 - s_e0);
   for (int base = 0; base < n; base += kHugeThreads) {
     const int i = base + threadIdx.x;
-    int ri = -1, g = 0;
+    int ri = -1, g = 0, gid = 0;
+    unsigned entries = 0;
     ListSum v{0, 0, 0, 0};
+    bool later = false;
     if (i < n) {
       ri = i < s_dirty ? P.list_dirty[i] : s_e0 + (i - s_dirty);
-      const int gid = P.real[ri];
+      later = i < s_dirty && ri >= s_again;
+    }
+    __syncthreads();  // the list's entries are read before the kept ones move down
+    if (later) {
+      P.list_dirty[atomicAdd(&s_kept, 1)] = ri;
+      atomicMin(&s_stale, ri);
+    } else if (i < n) {
+      P.dirty[ri] = 0;
+      gid = P.real[ri];
       g = P.glen[gid];
-      if (WindowSmall(g, P.gent[gid])) {
+      entries = P.gent[gid];
+      if (WindowSmall(g, entries)) {
         v.small = 1;
       } else {
         v.big = 1;
         v.members = g;
-        v.pairs = static_cast<long long>(g) * (g - 1) / 2;
+        v.parts = static_cast<long long>(g) * WindowParts(entries);
       }
       GroupStats z = {};
       P.gs[ri] = z;
@@ -222,9 +292,10 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
     const ListSum c0 = carry;
     if (v.small) P.list_small[c0.small + ex.small] = ri;
     if (v.big) {
-      P.list_big[c0.big + ex.big] = ri;
+      P.list_big[c0.big + ex.big] =
+          BigGroup{ri, gid, g, static_cast<int>(entries), P.gstart[gid], WindowParts(entries), P.mat_off[ri]};
       P.moff[c0.big + ex.big] = c0.members + ex.members;
-      P.poff[c0.big + ex.big] = c0.pairs + ex.pairs;
+      P.poff[c0.big + ex.big] = c0.parts + ex.parts;
     }
     __syncthreads();
     if (threadIdx.x == 0) carry = ListSumOp()(c0, total);
@@ -232,12 +303,13 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
   }
   if (threadIdx.x == 0) {
     P.moff[carry.big] = carry.members;
-    P.poff[carry.big] = carry.pairs;
+    P.poff[carry.big] = carry.parts;
     c->nsmall = carry.small;
     c->nbig = carry.big;
     c->members = carry.members;
-    c->pairs = carry.pairs;
-    c->ndirty = 0;
+    c->parts = carry.parts;
+    c->ndirty = s_kept;
+    c->stale = s_stale;
     c->work = 0;
     c->units = 0;
     c->e = s_e1;
@@ -446,15 +518,17 @@ struct RowPart {
   HeavyAcc heavy;
 };
 
-// Entries [k0, k1) of a row, by a warp (sums of the whole warp on return).
+// Entries [k0, k1) of member i's row staged and summed, by a warp (sums of the
+// whole warp on return).
 __device__ __forceinline__ void SumEntries(const QuotientView& Q, const Entry* row, int k0, int k1, int rep,
-                                           long long si, RowPart* out) {
+                                           long long si, int i, StagedEntry* stage, RowPart* out) {
   const int lane = threadIdx.x & 31;
 #pragma unroll 4
   for (int k = k0 + lane; k < k1; k += 32) {
     const Entry e = row[k];
     const long long c = EntCnt(e);
     const long long st = Q.size[EntNb(e)];
+    stage[k] = StagedEntry{EntNb(e), static_cast<int>(st), static_cast<unsigned>(c), i};
     out->old += EncodeCostForPair(rep, si, EntNb(e), st, c);
     if (HeavyEntry(si, st, c)) out->heavy.Add(st, c); else out->light += c;
   }
@@ -463,24 +537,53 @@ __device__ __forceinline__ void SumEntries(const QuotientView& Q, const Entry* r
   out->heavy.WarpReduce();
 }
 
-// Member i of a big group by one warp: its row sums and approximate old cost.
-__device__ void EvalMember(const WindowParams& P, int ri, int i) {
+// Member i of a big group by one warp: its row sums and approximate old cost,
+// its rows of the pair tables cleared, its entries staged beside the other
+// members' (rows that fit a table from the front, longer ones from the back).
+__device__ void EvalMember(const WindowParams& P, const BigGroup& G, int i) {
   const int lane = threadIdx.x & 31;
   const QuotientView& Q = P.Q;
-  const int gid = P.real[ri];
-  const long long g = P.glen[gid];
-  const int rep = P.order[P.gstart[gid] + i];
+  const int ri = G.ri, g = G.g, cap = G.cap;
+  const int rep = P.order[G.gstart + i];
+  unsigned char* mat = P.mat + G.mat;
+  unsigned long long* words = reinterpret_cast<unsigned long long*>(mat) + static_cast<long long>(i) * g;
+  unsigned char* flags = mat + FlagOffset(static_cast<long long>(g) * g) + static_cast<long long>(i) * g;
+  for (int k = lane; k < g; k += 32) {
+    words[k] = 0;
+    flags[k] = 0;
+  }
   const long long si = Q.size[rep];
   const int len = Q.len[rep];
+  const Entry* row = Q.ent + Q.off[rep];
   const long long internal = Q.internal[rep];
   const long long own = internal > 0 ? EncodeCostForPair(rep, si, rep, si, 2 * internal) : 0;
-  long long* old_out = reinterpret_cast<long long*>(P.mat + P.mat_off[ri] + OldCostOffset(g * g)) + i;
-  if (lane == 0) atomicAdd(&P.gs[ri].entries, static_cast<unsigned long long>(len));
-  RowPart r;
+  long long* old_out = reinterpret_cast<long long*>(mat + OldCostOffset(static_cast<long long>(g) * g)) + i;
+  GroupStats* gs = P.gs + ri;
+  int at = 0;
+  if (lane == 0) {
+    atomicAdd(&gs->entries, static_cast<unsigned long long>(len));
+    if (len <= kTableRow) {
+      at = atomicAdd(&gs->staged_short, len);
+    } else {
+      at = cap - atomicAdd(&gs->staged_long, len) - len;
+    }
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);
+  const bool fits = at >= 0 && at + len <= cap;  // rows counted at Divide time only shrink
+  if (lane == 0) {
+    reinterpret_cast<int4*>(mat + PlaceOffset(g))[i] = make_int4(at, fits ? len : 0, static_cast<int>(si), 0);
+    if (!fits) {
+      gs->err = kErrSlots;
+      gs->err_a = G.gid;
+      gs->err_b = len;
+    }
+  }
+  StagedEntry* stage = reinterpret_cast<StagedEntry*>(mat + StageOffset(g)) + at;
+  if (!fits) return;
   if (len > kLongRow) {
-    LongUnit u{reinterpret_cast<unsigned long long*>(old_out), nullptr, rep, -1, 0, ri};
+    const LongUnit u{reinterpret_cast<unsigned long long*>(old_out), stage, rep, i, 0, ri};
     if (PushUnits(P, u, len, kLongRowUnit)) {
-      // the units add their entries
+      // the units stage and add their entries
       if (lane == 0) {
         StoreRowSums(&P.rc[rep], 0, 0, HeavyAcc(), internal, static_cast<int>(si), len);
         *old_out = own;
@@ -488,146 +591,22 @@ __device__ void EvalMember(const WindowParams& P, int ri, int i) {
       return;
     }
   }
-  SumEntries(Q, Q.ent + Q.off[rep], 0, len, rep, si, &r);
+  RowPart r;
+  SumEntries(Q, row, 0, len, rep, si, i, stage, &r);
   if (lane == 0) {
     StoreRowSums(&P.rc[rep], r.old, r.light, r.heavy, internal, static_cast<int>(si), len);
     *old_out = r.old + own;
   }
 }
 
-// Members a < b of a big group by one warp: the pair's words, from a merge of
-// the two rows (32 entries of each per step, every entry up to the smaller of
-// the two tiles' last neighbours final in its step) or, where one row is far
-// longer, a search of the short one's entries in it. Returns the shared
-// targets found here.
-struct PairRows {
-  int ra, rb, sa, sb, la, lb;
-  long long offa, offb;
-};
-
-__device__ int EvalPair(const WindowParams& P, int ri, const PairRows& R, unsigned long long* up,
-                        unsigned long long* down) {
-  constexpr unsigned kFull = 0xffffffffu;
-  constexpr Entry kPadEntry = static_cast<Entry>(0x7fffffffull) << 32;
-  const int lane = threadIdx.x & 31;
-  const QuotientView& Q = P.Q;
-  const int ra = R.ra, rb = R.rb;
-  const long long sa = R.sa, sb = R.sb;
-  const Entry* pa_row = Q.ent + R.offa;
-  const Entry* pb_row = Q.ent + R.offb;
-  const int la = R.la, lb = R.lb;
-  long long delta = 0, corr = 0;
-  unsigned ea = 0, eb = 0;
-  int ovl = 0;
-  bool any_bad = false;
-  auto shared = [&](int x, long long ca, long long cb) {
-    bool bad;
-    const SharedTerm t = TermOf(sa, sb, Q.size[x], ca, cb, &bad);
-    delta += t.delta;
-    corr += t.corr;
-    any_bad |= bad;
-    ++ovl;
-  };
-  const bool a_long = la >= lb;
-  const int ll = a_long ? la : lb, ls = a_long ? lb : la;
-  const bool probe = ll >= kProbeMinLong && ll >= kProbeRatio * ls;
-  if (probe ? ls > kLongProbe : la + lb > kLongRow) {
-    if (PushUnits(P, LongUnit{up, down, ra, rb, 0, ri}, ls, kLongPairUnit)) {
-      // the units add what they find
-      if (lane == 0) {
-        *up = 0;
-        *down = 0;
-      }
-      return 0;
-    }
-  }
-  if (probe) {
-    const Entry* lr = a_long ? pa_row : pb_row;
-    const Entry* sr = a_long ? pb_row : pa_row;
-    const int long_rep = a_long ? ra : rb, short_rep = a_long ? rb : ra;
-    unsigned e_long = 0, e_short = 0;
-    for (int k = lane; k < ls + 1; k += 32) {
-      // the lane past the short row looks for it in the long one
-      const Entry e = k < ls ? sr[k] : MakeEnt(short_rep, 0);
-      const int x = EntNb(e);
-      if (x == long_rep) {
-        e_short = static_cast<unsigned>(EntCnt(e));
-        continue;
-      }
-      const int at = RowLowerBound(lr, ll, x);
-      if (at < ll && EntNb(lr[at]) == x) {
-        const long long cl = EntCnt(lr[at]);
-        if (k == ls) {
-          e_long = static_cast<unsigned>(cl);
-        } else {
-          shared(x, a_long ? cl : EntCnt(e), a_long ? EntCnt(e) : cl);
-        }
-      }
-    }
-    ea = a_long ? e_long : e_short;
-    eb = a_long ? e_short : e_long;
-  } else {
-    int pa = 0, pb = 0;
-    while (pa < la || pb < lb) {
-      const bool va = pa + lane < la, vb = pb + lane < lb;
-      const Entry xe = va ? pa_row[pa + lane] : kPadEntry;
-      const Entry ye = vb ? pb_row[pb + lane] : kPadEntry;
-      const int xa = EntNb(xe), xb = EntNb(ye);
-      const int last_a = __shfl_sync(kFull, xa, 31);
-      const int last_b = __shfl_sync(kFull, xb, 31);
-      const int lim = last_a < last_b ? last_a : last_b;
-      int pos = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int probe = __shfl_sync(kFull, xb, pos + step - 1);
-        if (probe < xa) pos += step;
-      }
-      const Entry ce = __shfl_sync(kFull, ye, pos);
-      const bool fin_a = va && xa <= lim, fin_b = vb && xb <= lim;
-      if (fin_a) {
-        if (xa == rb) {
-          ea = static_cast<unsigned>(EntCnt(xe));
-        } else if (EntNb(ce) == xa) {
-          shared(xa, EntCnt(xe), EntCnt(ce));
-        }
-      }
-      if (fin_b && xb == ra) eb = static_cast<unsigned>(EntCnt(ye));
-      pa += __popc(__ballot_sync(kFull, fin_a));
-      pb += __popc(__ballot_sync(kFull, fin_b));
-    }
-  }
-  ovl = WarpSumInt(ovl);
-  ea = __reduce_max_sync(kFull, ea);
-  eb = __reduce_max_sync(kFull, eb);
-  const bool bad = __any_sync(kFull, any_bad);
-  unsigned long long word = 0, low = 0;
-  if (ovl > 0) {  // most pairs of a group share nothing
-    delta = WarpSum(delta);
-    corr = WarpSum(corr);
-    word = static_cast<unsigned long long>(delta) + static_cast<unsigned long long>(ovl) * kOvlOne;
-    low = static_cast<unsigned long long>(bad ? kCorrBad : corr);
-  }
-  if (ea) word += ea | kRowILists;
-  if (eb) word |= kRowJLists;
-  if (lane == 0) {
-    *up = word;
-    *down = low;
-  }
-  return ovl;
-}
-
-// Work items in one queue: the members and pairs of the big groups (the longer
-// ones), then the small groups. One warp each.
+// Work items in one queue: the members of the big groups, then the small
+// groups. One warp each.
 __global__ void __launch_bounds__(kEvalWarps * 32, kEvalCtas) WindowEvalKernel(WindowParams P) {
+  FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   EvalWarpSmem& W = reinterpret_cast<EvalSmem*>(smem_raw)->w[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const long long nm = P.ctl->members;
-  // pairs per item: as few as keep every warp busy
-  const long long warps = static_cast<long long>(gridDim.x) * kEvalWarps;
-  long long per = P.ctl->pairs / (2 * warps) + 1;
-  per = per < kEvalPairs ? per : kEvalPairs;
-  const long long np = (P.ctl->pairs + per - 1) / per;
   const int ns = P.ctl->nsmall, nb = P.ctl->nbig;
   for (;;) {
     long long it = 0;
@@ -636,69 +615,17 @@ __global__ void __launch_bounds__(kEvalWarps * 32, kEvalCtas) WindowEvalKernel(W
     if (it < nm) {
       const int bl = WarpLastLE(P.moff, 0, nb, it);
       EvalMember(P, P.list_big[bl], static_cast<int>(it - P.moff[bl]));
-    } else if (it < nm + np) {
-      const long long p0 = (it - nm) * per;
-      const long long p1 = p0 + per < P.ctl->pairs ? p0 + per : P.ctl->pairs;
-      // lane d holds pair p0 + d: its group, its place and its rows' scalars,
-      // one chain of loads for all of them
-      const int bl0 = WarpLastLE(P.poff, 0, nb, p0);
-      int ri = 0, g = 0, a = 0, b = 0;
-      PairRows R = {0, 0, 0, 0, 0, 0, 0, 0};
-      unsigned long long* pmat = nullptr;
-      if (p0 + lane < p1) {
-        int bl = bl0;
-        while (P.poff[bl + 1] <= p0 + lane) ++bl;
-        ri = P.list_big[bl];
-        const int gid = P.real[ri];
-        g = P.glen[gid];
-        const int* q = P.order + P.gstart[gid];
-        pmat = reinterpret_cast<unsigned long long*>(P.mat + P.mat_off[ri]);
-        TriPair(static_cast<int>(p0 + lane - P.poff[bl]), g, &a, &b);
-        R.ra = q[a];
-        R.rb = q[b];
-        R.sa = P.Q.size[R.ra];
-        R.sb = P.Q.size[R.rb];
-        R.la = P.Q.len[R.ra];
-        R.lb = P.Q.len[R.rb];
-        R.offa = P.Q.off[R.ra];
-        R.offb = P.Q.off[R.rb];
-        unsigned char* fmat = reinterpret_cast<unsigned char*>(pmat) + FlagOffset(static_cast<long long>(g) * g);
-        fmat[static_cast<long long>(a) * g + b] = 0;
-      }
-      unsigned long long* up = pmat + static_cast<long long>(a) * g + b;
-      unsigned long long* down = pmat + static_cast<long long>(b) * g + a;
-      int examined = 0;
-      for (int d = 0; d < static_cast<int>(p1 - p0); ++d) {
-        constexpr unsigned kFull = 0xffffffffu;
-        PairRows X;
-        X.ra = __shfl_sync(kFull, R.ra, d);
-        X.rb = __shfl_sync(kFull, R.rb, d);
-        X.sa = __shfl_sync(kFull, R.sa, d);
-        X.sb = __shfl_sync(kFull, R.sb, d);
-        X.la = __shfl_sync(kFull, R.la, d);
-        X.lb = __shfl_sync(kFull, R.lb, d);
-        X.offa = __shfl_sync(kFull, R.offa, d);
-        X.offb = __shfl_sync(kFull, R.offb, d);
-        unsigned long long* xu =
-            reinterpret_cast<unsigned long long*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(up), d));
-        unsigned long long* xd =
-            reinterpret_cast<unsigned long long*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(down), d));
-        const int n = EvalPair(P, __shfl_sync(kFull, ri, d), X, xu, xd);
-        if (lane == d) examined = n;
-      }
-      if (examined) atomicAdd(&P.gs[ri].examined, static_cast<unsigned long long>(examined));
-    } else if (it < nm + np + ns) {
-      EvalSmallGroup(P, W, P.list_small[it - nm - np]);
+    } else if (it < nm + ns) {
+      EvalSmallGroup(P, W, P.list_small[it - nm]);
     } else {
       break;
     }
   }
 }
 
-// The long units, a warp each: row sums and pair words, added up.
+// The long units, a warp each: entries staged, row sums added up.
 __global__ void __launch_bounds__(kLongThreads) WindowLongKernel(WindowParams P) {
-  constexpr unsigned kFull = 0xffffffffu;
-  constexpr int kPer = kLongPairUnit / 32;
+  FollowsOn();
   const QuotientView& Q = P.Q;
   const int lane = threadIdx.x & 31;
   const unsigned total = P.ctl->units < kLongUnits ? P.ctl->units : kLongUnits;
@@ -706,98 +633,204 @@ __global__ void __launch_bounds__(kLongThreads) WindowLongKernel(WindowParams P)
   for (unsigned t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < total; t += nw) {
     const LongUnit u = P.units[t];
     if (u.ri < 0) continue;
-    if (u.b < 0) {
-      const int len = Q.len[u.a];
-      RowPart r;
-      SumEntries(Q, Q.ent + Q.off[u.a], u.at, min(u.at + kLongRowUnit, len), u.a, Q.size[u.a], &r);
-      if (lane == 0) {
-        RowSums* s = &P.rc[u.a];
-        atomicAdd(u.up, static_cast<unsigned long long>(r.old));
-        atomicAdd(reinterpret_cast<unsigned long long*>(&s->before), static_cast<unsigned long long>(r.old));
-        atomicAdd(reinterpret_cast<unsigned long long*>(&s->light), static_cast<unsigned long long>(r.light));
-        if (r.heavy.n != 0) {
-          atomicAdd(reinterpret_cast<unsigned long long*>(&s->heavy_sx), static_cast<unsigned long long>(r.heavy.sx));
-          atomicAdd(reinterpret_cast<unsigned long long*>(&s->heavy_c), static_cast<unsigned long long>(r.heavy.c));
-          atomicMin(&s->smin, r.heavy.smin);
-          atomicMax(&s->smax, r.heavy.smax);
-          atomicMax(&s->sbad, r.heavy.sbad);
-          atomicAdd(&s->nheavy, r.heavy.n);
-        }
-      }
-      continue;
-    }
-    const long long sa = Q.size[u.a], sb = Q.size[u.b];
-    const int la = Q.len[u.a], lb = Q.len[u.b];
-    const bool a_long = la >= lb;
-    const int ll = a_long ? la : lb, ls = a_long ? lb : la;
-    const Entry* lr = Q.ent + Q.off[a_long ? u.a : u.b];
-    const Entry* sr = Q.ent + Q.off[a_long ? u.b : u.a];
-    const int long_rep = a_long ? u.a : u.b, short_rep = a_long ? u.b : u.a;
-    const int end = min(u.at + kLongPairUnit, ls);
-    // the part of the long row that the unit's ids span
-    int edge = 0;
-    if (lane < 2) edge = RowLowerBound(lr, ll, EntNb(sr[lane == 0 ? u.at : end - 1]));
-    const int lo0 = __shfl_sync(kFull, edge, 0);
-    const int hi0 = min(__shfl_sync(kFull, edge, 1) + 1, ll);
-    Entry e[kPer];
-    int at[kPer], hi[kPer];
-#pragma unroll
-    for (int d = 0; d < kPer; ++d) {
-      const int k = u.at + 32 * d + lane;
-      e[d] = k < end ? sr[k] : 0;
-      at[d] = lo0;
-      hi[d] = k < end ? hi0 : lo0;
-    }
-    // the lanes' searches side by side
-    for (int span = hi0 - lo0; span > 0; span >>= 1) {
-#pragma unroll
-      for (int d = 0; d < kPer; ++d) {
-        if (at[d] < hi[d]) {
-          const int mid = (at[d] + hi[d]) >> 1;
-          if (EntNb(lr[mid]) < EntNb(e[d])) at[d] = mid + 1; else hi[d] = mid;
-        }
-      }
-    }
-    long long delta = 0, corr = 0;
-    int ovl = 0;
-    bool any_bad = false;
-    unsigned e_short = 0, e_long = 0;
-#pragma unroll
-    for (int d = 0; d < kPer; ++d) {
-      const int k = u.at + 32 * d + lane;
-      if (k >= end) continue;
-      const int x = EntNb(e[d]);
-      if (x == long_rep) {
-        e_short = static_cast<unsigned>(EntCnt(e[d]));
-      } else if (at[d] < ll && EntNb(lr[at[d]]) == x) {
-        const long long cl = EntCnt(lr[at[d]]), cs = EntCnt(e[d]);
-        bool bad;
-        const SharedTerm term = TermOf(sa, sb, Q.size[x], a_long ? cl : cs, a_long ? cs : cl, &bad);
-        delta += term.delta;
-        corr += term.corr;
-        any_bad |= bad;
-        ++ovl;
-      }
-    }
-    if (u.at == 0 && lane == 0) e_long = static_cast<unsigned>(RowLookup(lr, ll, short_rep));
-    ovl = WarpSumInt(ovl);
-    e_short = __reduce_max_sync(kFull, e_short);
-    e_long = __reduce_max_sync(kFull, e_long);
-    const bool bad = __any_sync(kFull, any_bad);
-    unsigned long long word = 0;
-    if (ovl > 0) {
-      delta = WarpSum(delta);
-      corr = WarpSum(corr);
-      word = static_cast<unsigned long long>(delta) + static_cast<unsigned long long>(ovl) * kOvlOne;
-    }
-    const unsigned ea = a_long ? e_long : e_short, eb = a_long ? e_short : e_long;
-    if (ea) word += ea | kRowILists;
-    if (eb) word |= kRowJLists;
+    const int len = Q.len[u.rep];
+    RowPart r;
+    SumEntries(Q, Q.ent + Q.off[u.rep], u.at, min(u.at + kLongRowUnit, len), u.rep, Q.size[u.rep], u.i, u.stage, &r);
     if (lane == 0) {
-      if (word) atomicAdd(u.up, word);
-      if (ovl > 0 && (bad || corr != 0)) atomicAdd(u.down, static_cast<unsigned long long>(bad ? kCorrBad : corr));
-      if (ovl > 0) atomicAdd(&P.gs[u.ri].examined, static_cast<unsigned long long>(ovl));
+      RowSums* s = &P.rc[u.rep];
+      atomicAdd(u.old, static_cast<unsigned long long>(r.old));
+      atomicAdd(reinterpret_cast<unsigned long long*>(&s->before), static_cast<unsigned long long>(r.old));
+      atomicAdd(reinterpret_cast<unsigned long long*>(&s->light), static_cast<unsigned long long>(r.light));
+      if (r.heavy.n != 0) {
+        atomicAdd(reinterpret_cast<unsigned long long*>(&s->heavy_sx), static_cast<unsigned long long>(r.heavy.sx));
+        atomicAdd(reinterpret_cast<unsigned long long*>(&s->heavy_c), static_cast<unsigned long long>(r.heavy.c));
+        atomicMin(&s->smin, r.heavy.smin);
+        atomicMax(&s->smax, r.heavy.smax);
+        atomicMax(&s->sbad, r.heavy.sbad);
+        atomicAdd(&s->nheavy, r.heavy.n);
+      }
     }
+  }
+}
+
+struct PairTable {
+  int key[kTableSlots];  // target, -1 free
+  unsigned cnt[kTableSlots];
+  int4 hit[32 + 32 * kPairDeep];  // found: member, target's size, the member's count, the table's count
+};
+
+__device__ __forceinline__ int StagedLowerBound(const StagedEntry* row, int len, int t) {
+  int lo = 0, hi = len;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (row[mid].t < t) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// The pair words of the big groups, a warp per member and part. A row of at
+// most kTableRow entries goes into a hash table in shared memory, and the
+// entries of the rows staged after it, and of all longer rows, are looked up in
+// it, four per lane in flight: two or three instructions' worth of lookups per
+// entry, where merging the rows pair by pair took 200 instructions and a chain
+// of loads per pair. What is found is queued and added up 32 at a time (a few
+// in a hundred lookups find something: handled in place, nearly every step
+// would wait for its one or two lanes). Two long rows are
+// matched by searching the shorter one's entries in the other.
+__global__ void __launch_bounds__(kPairWarps * 32, kPairCtas) WindowPairsKernel(WindowParams P) {
+  FollowsOn();
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int kDeep = kPairDeep;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  PairTable& T = reinterpret_cast<PairTable*>(smem_raw)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int nb = P.ctl->nbig;
+  const long long total = P.ctl->parts;
+  const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  for (long long it = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; it < total; it += nw) {
+    const int bl = WarpLastLE(P.poff, 0, nb, it);
+    const BigGroup G = P.list_big[bl];
+    const int ri = G.ri, gid = G.gid, g = G.g, cap = G.cap, parts = G.parts;
+    const int local = static_cast<int>(it - P.poff[bl]);
+    const int part = local / g, i = local - part * g;  // a part's members side by side
+    unsigned char* mat = P.mat + G.mat;
+    unsigned long long* pmat = reinterpret_cast<unsigned long long*>(mat);
+    const int4* place = reinterpret_cast<const int4*>(mat + PlaceOffset(g));
+    const StagedEntry* stage = reinterpret_cast<const StagedEntry*>(mat + StageOffset(g));
+    const int4 me = place[i];
+    if (me.y == 0) continue;
+    const long long si = me.z;
+    unsigned examined = 0;
+    auto direct = [&](const StagedEntry& e) {
+      if (P.group_of[e.t] == gid) AddDirect(pmat, g, i, P.idx_in_group[e.t], e.c);
+    };
+    if (me.y <= kTableRow) {
+      int mask = 32;
+      while (mask < 2 * me.y) mask <<= 1;
+      --mask;
+      __syncwarp();
+      for (int k = lane; k <= mask; k += 32) T.key[k] = -1;
+      __syncwarp();
+      for (int k = lane; k < me.y; k += 32) {
+        const StagedEntry e = stage[me.x + k];
+        int h = static_cast<int>(BucketHash(e.t, mask));
+        while (atomicCAS(&T.key[h], -1, e.t) != -1) h = (h + 1) & mask;
+        T.cnt[h] = e.c;
+        if (part == 0) direct(e);
+      }
+      __syncwarp();
+      int queued = 0;
+      auto add = [&](const int4& x) {
+        ++examined;
+        AddShared(pmat, g, i, x.x, si, place[x.x].z, x.y, static_cast<unsigned>(x.w), static_cast<unsigned>(x.z), true);
+      };
+      // the entries to look up: the shorter rows staged later, the longer rows
+      const int first = me.x + me.y, n1 = P.gs[ri].staged_short - first;
+      const int n2 = P.gs[ri].staged_long, back = cap - n2;
+      const long long n = static_cast<long long>(n1) + n2;
+      const int k0 = static_cast<int>(n * part / parts), k1 = static_cast<int>(n * (part + 1) / parts);
+      for (int b = k0; b < k1; b += 32 * kDeep) {
+        StagedEntry e[kDeep];
+#pragma unroll
+        for (int d = 0; d < kDeep; ++d) {
+          const int k = b + 32 * d + lane;
+          e[d].t = -1;
+          if (k < k1) e[d] = stage[k < n1 ? first + k : back + (k - n1)];
+        }
+#pragma unroll
+        for (int d = 0; d < kDeep; ++d) {
+          int h = static_cast<int>(BucketHash(e[d].t, mask));
+          int key = e[d].t >= 0 ? T.key[h] : -1;
+          while (key != -1 && key != e[d].t) {
+            h = (h + 1) & mask;
+            key = T.key[h];
+          }
+          const bool found = e[d].t >= 0 && key != -1;
+          const unsigned m = __ballot_sync(kFull, found);
+          if (found) {
+            T.hit[queued + __popc(m & ((1u << lane) - 1u))] =
+                make_int4(e[d].j, e[d].size, static_cast<int>(e[d].c), static_cast<int>(T.cnt[h]));
+          }
+          queued += __popc(m);
+        }
+        __syncwarp();
+        for (; queued >= 32; queued -= 32) add(T.hit[queued - 32 + lane]);
+        __syncwarp();
+      }
+      if (lane < queued) add(T.hit[lane]);
+    } else {
+      for (int k = static_cast<int>(static_cast<long long>(me.y) * part / parts) + lane;
+           k < static_cast<int>(static_cast<long long>(me.y) * (part + 1) / parts); k += 32) {
+        direct(stage[me.x + k]);
+      }
+      for (int j = i + 1; j < g; ++j) {
+        const int4 other = place[j];
+        if (other.y <= kTableRow) continue;
+        const bool mine_long = me.y >= other.y;
+        const StagedEntry* lr = stage + (mine_long ? me.x : other.x);
+        const StagedEntry* sr = stage + (mine_long ? other.x : me.x);
+        const int ll = mine_long ? me.y : other.y, ls = mine_long ? other.y : me.y;
+        const int k0 = static_cast<int>(static_cast<long long>(ls) * part / parts);
+        const int k1 = static_cast<int>(static_cast<long long>(ls) * (part + 1) / parts);
+        if (k0 >= k1) continue;
+        const long long sj = other.z;
+        // the part of the long row that these ids span
+        int edge = 0;
+        if (lane < 2) edge = StagedLowerBound(lr, ll, sr[lane == 0 ? k0 : k1 - 1].t);
+        const int lo0 = __shfl_sync(kFull, edge, 0);
+        const int hi0 = min(__shfl_sync(kFull, edge, 1) + 1, ll);
+        long long delta = 0, corr = 0;
+        unsigned ovl = 0;
+        bool any_bad = false;
+        for (int b = k0; b < k1; b += 32 * kDeep) {
+          StagedEntry e[kDeep];
+          int at[kDeep], hi[kDeep];
+#pragma unroll
+          for (int d = 0; d < kDeep; ++d) {
+            const int k = b + 32 * d + lane;
+            e[d].t = -1;
+            if (k < k1) e[d] = sr[k];
+            at[d] = lo0;
+            hi[d] = k < k1 ? hi0 : lo0;
+          }
+          // the lanes' searches side by side
+          for (int span = hi0 - lo0; span > 0; span >>= 1) {
+#pragma unroll
+            for (int d = 0; d < kDeep; ++d) {
+              if (at[d] < hi[d]) {
+                const int mid = (at[d] + hi[d]) >> 1;
+                if (lr[mid].t < e[d].t) at[d] = mid + 1; else hi[d] = mid;
+              }
+            }
+          }
+#pragma unroll
+          for (int d = 0; d < kDeep; ++d) {
+            if (e[d].t < 0 || at[d] >= ll || lr[at[d]].t != e[d].t) continue;
+            const long long cl = lr[at[d]].c, cs = e[d].c;
+            bool bad;
+            const SharedTerm x = TermOf(si, sj, e[d].size, mine_long ? cl : cs, mine_long ? cs : cl, &bad);
+            delta += x.delta;
+            corr += x.corr;
+            any_bad |= bad;
+            ++ovl;
+          }
+        }
+        ovl = __reduce_add_sync(kFull, ovl);
+        if (ovl == 0) continue;
+        delta = WarpSum(delta);
+        corr = WarpSum(corr);
+        const bool bad = __any_sync(kFull, any_bad);
+        if (lane == 0) {
+          examined += ovl;
+          atomicAdd(&pmat[static_cast<long long>(i) * g + j], static_cast<unsigned long long>(delta) + ovl * kOvlOne);
+          if (bad || corr != 0) {
+            atomicAdd(&pmat[static_cast<long long>(j) * g + i], static_cast<unsigned long long>(bad ? kCorrBad : corr));
+          }
+        }
+      }
+    }
+    examined = __reduce_add_sync(kFull, examined);
+    if (lane == 0 && examined) atomicAdd(&P.gs[ri].examined, static_cast<unsigned long long>(examined));
   }
 }
 
@@ -806,6 +839,7 @@ __global__ void __launch_bounds__(kLongThreads) WindowLongKernel(WindowParams P)
 // set a pair's flag scores it). Keys of the pairs that pass go to the group's
 // list.
 __global__ void __launch_bounds__(256, 2) WindowScoreKernel(WindowParams P) {
+  FollowsOn();
   constexpr unsigned kFull = 0xffffffffu;
   __shared__ int cand_j[8][32];
   __shared__ unsigned short kept[8][kMaxGroup];
@@ -817,12 +851,11 @@ __global__ void __launch_bounds__(256, 2) WindowScoreKernel(WindowParams P) {
   const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   for (long long w = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < total; w += nw) {
     const int bl = WarpLastLE(P.moff, 0, nb, w);
-    const int ri = P.list_big[bl];
-    const int gid = P.real[ri];
-    const int g = P.glen[gid];
+    const BigGroup G = P.list_big[bl];
+    const int ri = G.ri, g = G.g;
     const int i = static_cast<int>(w - P.moff[bl]);
-    const int* q = P.order + P.gstart[gid];
-    unsigned char* mat = P.mat + P.mat_off[ri];
+    const int* q = P.order + G.gstart;
+    unsigned char* mat = P.mat + G.mat;
     const unsigned long long* pmat = reinterpret_cast<const unsigned long long*>(mat);
     unsigned* flags = reinterpret_cast<unsigned*>(mat + FlagOffset(static_cast<long long>(g) * g));
     if (lane == 0) nkept[warp] = 0;
@@ -903,6 +936,7 @@ __global__ void __launch_bounds__(256, 2) WindowScoreKernel(WindowParams P) {
 // A big group by one CTA: matching rounds over its keys, and what the selected
 // pairs touch.
 __global__ void __launch_bounds__(kMatchThreads) WindowSelectKernel(WindowParams P) {
+  FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned long long* skeys = reinterpret_cast<unsigned long long*>(smem_raw);
   __shared__ MatchSmem M;
@@ -912,7 +946,8 @@ __global__ void __launch_bounds__(kMatchThreads) WindowSelectKernel(WindowParams
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nb = P.ctl->nbig;
   for (int bl = blockIdx.x; bl < nb; bl += gridDim.x) {
-    const int ri = P.list_big[bl];
+    const BigGroup G = P.list_big[bl];
+    const int ri = G.ri;
     GroupStats* gs = P.gs + ri;
     const int m = static_cast<int>(gs->positive);
     if (m == 0) {  // most groups
@@ -922,9 +957,8 @@ __global__ void __launch_bounds__(kMatchThreads) WindowSelectKernel(WindowParams
       }
       continue;
     }
-    const int gid = P.real[ri];
-    const int g = P.glen[gid];
-    const int* q = P.order + P.gstart[gid];
+    const int g = G.g;
+    const int* q = P.order + G.gstart;
     unsigned long long* keys = P.keys + 2 * P.cand_off[ri];
     unsigned long long* spare = keys + (P.cand_off[ri + 1] - P.cand_off[ri]);
     __syncthreads();  // the last group's shared state is read
@@ -986,6 +1020,7 @@ __global__ void __launch_bounds__(kMatchThreads) WindowSelectKernel(WindowParams
 // counters, and their pairs onto the commit list. Errors of an evaluation
 // count here too, when its block's turn has come.
 __global__ void __launch_bounds__(kMarkThreads) WindowMarkKernel(WindowParams P) {
+  FollowsOn();
   __shared__ int s_min;
   __shared__ unsigned long long acc[kGroupStatWords + 3];  // + groups, member pairs, largest group
   const int tid = threadIdx.x, lane = tid & 31;
@@ -994,7 +1029,7 @@ __global__ void __launch_bounds__(kMarkThreads) WindowMarkKernel(WindowParams P)
     if (blockIdx.x == 0 && tid == 0) P.ctl->p = f;
     return;
   }
-  if (tid == 0) s_min = e;
+  if (tid == 0) s_min = min(e, P.ctl->stale);
   if (tid < kGroupStatWords + 3) acc[tid] = 0;
   __syncthreads();
   int first = e;
@@ -1003,16 +1038,7 @@ __global__ void __launch_bounds__(kMarkThreads) WindowMarkKernel(WindowParams P)
   first = __reduce_min_sync(0xffffffffu, first);
   if (lane == 0) atomicMin(&s_min, first);
   __syncthreads();
-  int p = s_min;
-  if (p < e) {
-    // the start of its block: the first position whose block ends after it
-    int lo = f, hi = p;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (P.blk_end[mid] <= p) lo = mid + 1; else hi = mid;
-    }
-    p = lo;
-  }
+  const int p = s_min < e ? P.blk_beg[s_min] : e;
   if (blockIdx.x == 0 && tid == 0) P.ctl->p = p;
   // commit list, a thread per group
   unsigned long long raw = 0;
