@@ -151,6 +151,8 @@ struct BlockPlan {
   int rg0 = 0, rg1 = 0;                 // real-group positions
   long long slots = 0, sel_slots = 0;   // candidate / selection slots
   int s0 = 0, s1 = 0, b0 = 0, b1 = 0;   // small / big prepare list ranges
+  int m0 = 0, m1 = 0;                   // medium groups handled by one kernel
+  bool fused = false;                   // whether there may be any
   long long members = 0;                // members of the big groups
   long long slot0 = 0, nslots = 0;      // sort slots of the deferred big groups
   long long max_e = 0;                  // largest deferred group's row entries
@@ -243,6 +245,9 @@ class Engine {
   void RankerTrain();
   void RankerFinishIteration();
   void LaunchPrepare(const BlockPlan& bp);
+  void LaunchMedium(const BlockPlan& bp, double threshold);
+  bool FusedOn() const;
+  bool PlanFused() const;
   bool RowSumsOn() const;
   bool WindowsOn() const;
   void RunWindows(double threshold);
@@ -322,7 +327,9 @@ class Engine {
   std::vector<int> h_block_rg_;  // per 64-group block: first real-group position
   std::vector<int> h_small_, h_big_;              // real-group positions by prepare kernel
   std::vector<int> h_block_small_, h_block_big_;  // per block: first entry in those lists
-  DevBuf<int> d_small_, d_big_;
+  std::vector<int> h_med_, h_block_med_;
+  std::vector<unsigned char> h_block_fused_;
+  DevBuf<int> d_small_, d_med_, d_big_;
   std::vector<int> h_sel_small_, h_sel_mid_, h_sel_big_;  // real-group positions by select kernel
   std::vector<int> h_block_sel_small_, h_block_sel_mid_, h_block_sel_big_;  // per block: first entries
   DevBuf<int> d_sel_small_, d_sel_mid_, d_sel_big_;

@@ -248,6 +248,7 @@ __device__ __forceinline__ bool HeavyEntry(long long size_r, long long size_x, l
 }
 
 __device__ __forceinline__ int HeavyLimit(long long size_x, long long c) {
+  if (c < (1ll << 30)) return static_cast<int>(static_cast<unsigned>(2 * c - 2) / static_cast<unsigned>(size_x));
   const long long l = (2 * c - 2) / size_x;
   return l > 0x7fffffffll ? 0x7fffffff : static_cast<int>(l);
 }
@@ -255,6 +256,10 @@ __device__ __forceinline__ int HeavyLimit(long long size_x, long long c) {
 // Least size whose block with a target of size_x holds cnt edges. An entry
 // beyond its own block's capacity is always heavy.
 __device__ __forceinline__ int HeavyNeed(long long size_x, long long cnt) {
+  if (cnt < (1ll << 30)) {
+    const unsigned x = static_cast<unsigned>(size_x);
+    return static_cast<int>((static_cast<unsigned>(cnt) + x - 1u) / x);
+  }
   const long long n = (cnt + size_x - 1) / size_x;
   return n > 0x7fffffffll ? 0x7fffffff : static_cast<int>(n);
 }
@@ -450,6 +455,16 @@ __device__ __forceinline__ DeferredView Deferred(unsigned char* base, int g) {
 
 constexpr unsigned long long kSlotPad = ~0ull;  // key of an unused sort slot
 
+// The same in 32 bits: sizes below 2^13, counts below 2^28.
+__device__ __forceinline__ void TermOf32(int sa, int sb, int st, int ca, int cb, int* delta, int* corr, bool* bad) {
+  const int cap_a = sa * st, cap_b = sb * st, cap = cap_a + cap_b, c = ca + cb;
+  const int ga = min(ca, 1 + cap_a - ca), gb = min(cb, 1 + cap_b - cb), f = min(c, 1 + cap - c);
+  const int d = max(ga + gb - f, 0);
+  *delta = d;
+  *corr = f - min(ca, 1 + cap - ca) - min(cb, 1 + cap - cb) + d;
+  *bad = c > cap;
+}
+
 struct PrepareParams {
   QuotientView Q;
   const int* order;
@@ -513,6 +528,45 @@ __device__ __forceinline__ bool Better(const RankKey& x, const RankKey& y) {
   if (x.pg != y.pg) return x.pg > y.pg;
   if (x.lo != y.lo) return x.lo < y.lo;
   return x.hi < y.hi;
+}
+
+// The same order without a double, for proxies and denominators below
+// kExactRatio: two different quotients p / d of such numbers are more than
+// 2^-52 apart (relative), so they round to different doubles, and cross products
+// order them as the rounded quotients. One double division by a warp holds this
+// GPU's FP64 pipe for some 250 cycles; ranked that way, it was what the member
+// passes waited for. Between partners of one member, (rep_lo, rep_hi) ascending
+// is the partner's id ascending.
+constexpr long long kExactRatio = 1ll << 26;
+
+struct RankCand {
+  unsigned p, d;  // proxy gain (0: no candidate), denominator
+  int q;          // partner
+};
+
+// Ranks of a member's candidates, kPer to a lane, by the whole warp: rank[t] is
+// the number of candidates better than the lane's t-th (meaningful for a
+// candidate; p == 0 is none). Every lane's candidate in turn, four in flight.
+template <int kPer>
+__device__ __forceinline__ void ExactRanks(const RankCand (&c)[kPer], int (&rank)[kPer]) {
+#pragma unroll
+  for (int t = 0; t < kPer; ++t) rank[t] = 0;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+#pragma unroll 4
+    for (int o = 0; o < 32; ++o) {
+      const unsigned op = __shfl_sync(0xffffffffu, c[u].p, o);
+      const unsigned od = __shfl_sync(0xffffffffu, c[u].d, o);
+      const int oq = __shfl_sync(0xffffffffu, c[u].q, o);
+#pragma unroll
+      for (int t = 0; t < kPer; ++t) {
+        const unsigned long long l = static_cast<unsigned long long>(op) * c[t].d;
+        const unsigned long long r = static_cast<unsigned long long>(c[t].p) * od;
+        const bool better = l != r ? l > r : op != c[t].p ? op > c[t].p : oq < c[t].q;  // not better than itself
+        rank[t] += better ? 1 : 0;
+      }
+    }
+  }
 }
 
 // The reference's threshold test RN(gain / before) >= threshold (doubles, gain
@@ -1076,9 +1130,9 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
 
 // Top-k partners of member i of a big group whose partners fill NT slots of
 // 32 (the fp32 prescreen branch of PrepareMembersKernel).
-template <int NT, typename KeepFn>
+template <int NT, typename ProxyFn, typename KeepFn>
 __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int top_k, int cnt,
-                                            const unsigned long long* pmat, const long long* old, long long old_i, const int* q, int* cj,
+                                            ProxyFn proxy, const long long* old, long long old_i, const int* q, int* cj,
                                             KeepFn keep) {
   auto ratio_of = [&](int j, long long pg) {
     long long denom = old_i + old[j];
@@ -1090,7 +1144,7 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
   // candidates that can be in the member's top_k. The fp32 ratio of a
   // candidate is within relative 3 * 2^-24 of its double ratio, so every
   // candidate of the exact top_k has an fp32 ratio >= tau * (1 - 2^-20),
-  // where tau is the top_k-th largest fp32 ratio (found by bisection on the
+  // where tau is the top_k-th largest fp32 ratio (bounded by bisection on the
   // float bit patterns, which order like the positive values).
   float rf[NT];
 #pragma unroll
@@ -1098,7 +1152,7 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     const int j = lane + 32 * t;
     float v = 0.0f;  // not a candidate
     if (j < g && j != i) {
-      const long long pg = ProxyOf(PairWord(pmat, g, i, j));
+      const long long pg = proxy(i, j);
       if (pg > 0) {
         long long denom = old_i + old[j];
         if (denom < 1) denom = 1;
@@ -1122,13 +1176,21 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     }
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi) + 1u;
-    while (hi - lo > 1) {
+    // (any lo with a lane's worth of candidates left will do: a few steps
+    // instead of the two dozen that single out tau)
+    int left = cnt;
+    while (hi - lo > 1 && left > 30) {
       const unsigned mid = lo + ((hi - lo) >> 1);
       int c = 0;
 #pragma unroll
       for (int t = 0; t < NT; ++t) c += __float_as_uint(rf[t]) >= mid ? 1 : 0;
       c = WarpSumInt(c);
-      if (c >= top_k) lo = mid; else hi = mid;
+      if (c >= top_k) {
+        lo = mid;
+        left = c;
+      } else {
+        hi = mid;
+      }
     }
     cut = __uint_as_float(lo) * (1.0f - 9.5367431640625e-7f);
   }
@@ -1156,24 +1218,35 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     mine.lo = 0;
     mine.hi = 0;
     mine.j = -1;
+    long long denom = 1;
     if (have) {
       const int j = cj[lane];
-      const long long pg = ProxyOf(PairWord(pmat, g, i, j));
+      const long long pg = proxy(i, j);
       const int qj = q[j];
+      denom = old_i + old[j];
+      if (denom < 1) denom = 1;
       mine.j = j;
-      mine.rb = ratio_of(j, pg);
       mine.pg = pg;
       mine.lo = qi < qj ? qi : qj;
       mine.hi = qi < qj ? qj : qi;
     }
     int rank = 0;
-    for (int o = 0; o < npass; ++o) {
-      RankKey other;
-      other.rb = __shfl_sync(0xffffffffu, mine.rb, o);
-      other.pg = __shfl_sync(0xffffffffu, mine.pg, o);
-      other.lo = __shfl_sync(0xffffffffu, mine.lo, o);
-      other.hi = __shfl_sync(0xffffffffu, mine.hi, o);
-      if (have && o != lane && Better(other, mine)) ++rank;
+    if (!__any_sync(0xffffffffu, mine.pg >= kExactRatio || denom >= kExactRatio)) {
+      const RankCand c[1] = {{static_cast<unsigned>(mine.pg), static_cast<unsigned>(denom),
+                              have ? q[mine.j] : 0}};
+      int r[1];
+      ExactRanks(c, r);
+      rank = r[0];
+    } else {
+      if (have) mine.rb = ratio_of(mine.j, mine.pg);
+      for (int o = 0; o < npass; ++o) {
+        RankKey other;
+        other.rb = __shfl_sync(0xffffffffu, mine.rb, o);
+        other.pg = __shfl_sync(0xffffffffu, mine.pg, o);
+        other.lo = __shfl_sync(0xffffffffu, mine.lo, o);
+        other.hi = __shfl_sync(0xffffffffu, mine.hi, o);
+        if (have && o != lane && Better(other, mine)) ++rank;
+      }
     }
     if (have && rank < top_k) {
       const int a = i < mine.j ? i : mine.j;
@@ -1189,7 +1262,7 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
     for (int t = 0; t < NT; ++t) {
       const int j = lane + 32 * t;
       if (rf[t] <= 0.0f || rf[t] < cut) continue;
-      const long long pg = ProxyOf(PairWord(pmat, g, i, j));
+      const long long pg = proxy(i, j);
       RankKey k;
       k.j = j;
       k.rb = ratio_of(j, pg);
@@ -1238,16 +1311,12 @@ __device__ __forceinline__ void MembersTopK(int lane, int g, int i, int qi, int 
   }
 }
 
-// Member i of a big group (members q, pair tables mat) by one warp: keep(a, b)
-// is called for the pair of each of its top_k partners, by some lane. cj: 32
-// words of the warp's own.
-template <typename KeepFn>
-__device__ __forceinline__ void RankMember(int g, int i, const int* q, const unsigned char* mat, int top_k_max, int* cj,
-                                           KeepFn keep) {
+// Member i of a group (members q, old costs, proxy(i, j)) by one warp: keep(a, b) is called for the pair of each of its top_k partners, by
+// some lane. cj: 32 words of the warp's own.
+template <typename ProxyFn, typename KeepFn>
+__device__ __forceinline__ void RankMember(int g, int i, const int* q, const long long* old, int top_k_max, int* cj,
+                                           ProxyFn proxy, KeepFn keep) {
   const int lane = threadIdx.x & 31;
-  const long long gg = static_cast<long long>(g) * g;
-  const unsigned long long* pmat = reinterpret_cast<const unsigned long long*>(mat);
-  const long long* old = reinterpret_cast<const long long*>(mat + OldCostOffset(gg));
   // candidates with positive proxy, ratio, top-k (the ratio is recomputed where
   // it is needed instead of being stored)
   int top_k = top_k_max < g - 1 ? top_k_max : g - 1;
@@ -1262,13 +1331,13 @@ __device__ __forceinline__ void RankMember(int g, int i, const int* q, const uns
   int cnt = 0;
   for (int base = 0; base < g; base += 32) {
     const int j = base + lane;
-    const bool pred = j < g && j != i && ProxyOf(PairWord(pmat, g, i, j)) > 0;
+    const bool pred = j < g && j != i && proxy(i, j) > 0;
     cnt += __popc(__ballot_sync(0xffffffffu, pred));
   }
   const int qi = q[i];
   if (cnt <= top_k) {
     for (int j = lane; j < g; j += 32) {
-      if (j == i || ProxyOf(PairWord(pmat, g, i, j)) <= 0) continue;
+      if (j == i || proxy(i, j) <= 0) continue;
       const int a = i < j ? i : j;
       const int b = i < j ? j : i;
       keep(a, b);
@@ -1276,15 +1345,15 @@ __device__ __forceinline__ void RankMember(int g, int i, const int* q, const uns
   } else if (top_k <= kLaneTopK) {
     const int nt = (g + 31) >> 5;
     if (nt <= 1) {
-      MembersTopK<1>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
+      MembersTopK<1>(lane, g, i, qi, top_k, cnt, proxy, old, old_i, q, cj, keep);
     } else if (nt <= 2) {
-      MembersTopK<2>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
+      MembersTopK<2>(lane, g, i, qi, top_k, cnt, proxy, old, old_i, q, cj, keep);
     } else if (nt <= 4) {
-      MembersTopK<4>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
+      MembersTopK<4>(lane, g, i, qi, top_k, cnt, proxy, old, old_i, q, cj, keep);
     } else if (nt <= 8) {
-      MembersTopK<8>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
+      MembersTopK<8>(lane, g, i, qi, top_k, cnt, proxy, old, old_i, q, cj, keep);
     } else {
-      MembersTopK<kMaxGroup / 32>(lane, g, i, qi, top_k, cnt, pmat, old, old_i, q, cj, keep);
+      MembersTopK<kMaxGroup / 32>(lane, g, i, qi, top_k, cnt, proxy, old, old_i, q, cj, keep);
     }
   } else {
     RankKey prev;
@@ -1294,7 +1363,7 @@ __device__ __forceinline__ void RankMember(int g, int i, const int* q, const uns
       bool have = false;
       for (int j = lane; j < g; j += 32) {
         if (j == i) continue;
-        const long long pg = ProxyOf(PairWord(pmat, g, i, j));
+        const long long pg = proxy(i, j);
         if (pg <= 0) continue;
         RankKey k;
         k.j = j;
@@ -1350,8 +1419,12 @@ __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
   const int g = P.glen[gid];
   const int* q = P.order + P.gstart[gid];
   unsigned char* fmat = P.mat + P.mat_off[ri] + FlagOffset(static_cast<long long>(g) * g);
-  RankMember(g, i, q, P.mat + P.mat_off[ri], P.top_k, cand_j[threadIdx.x >> 5],
-             [&](int a, int b) { fmat[static_cast<long long>(a) * g + b] = 1; });
+  const unsigned long long* pmat = reinterpret_cast<const unsigned long long*>(P.mat + P.mat_off[ri]);
+  const long long* old =
+      reinterpret_cast<const long long*>(P.mat + P.mat_off[ri] + OldCostOffset(static_cast<long long>(g) * g));
+  RankMember(g, i, q, old, P.top_k, cand_j[threadIdx.x >> 5],
+                        [&](int x, int j) { return ProxyOf(PairWord(pmat, g, x, j)); },
+                        [&](int a, int b) { fmat[static_cast<long long>(a) * g + b] = 1; });
 }
 
 // Flag bytes (0 or 1) of table word w that lie in [beg, end), as a bit set
@@ -1560,7 +1633,8 @@ struct SmallPair {
   bool bad;
 };
 
-__device__ __forceinline__ SmallPair SmallMerge(const SmallRowsSmem& S, int a, int b) {
+template <typename Rows>
+__device__ __forceinline__ SmallPair SmallMerge(const Rows& S, int a, int b) {
   const int qb = S.q[b];
   const long long sa = S.sz[a], sb = S.sz[b];
   int ia = S.start[a], ib = S.start[b];
@@ -1591,11 +1665,13 @@ __device__ __forceinline__ SmallPair SmallMerge(const SmallRowsSmem& S, int a, i
   return r;
 }
 
-__device__ __forceinline__ long long StagedLookup(const SmallRowsSmem& S, int a, int key) {
+template <typename Rows>
+__device__ __forceinline__ long long StagedLookup(const Rows& S, int a, int key) {
   return RowLookup(S.ent + S.start[a], S.start[a + 1] - S.start[a], key);
 }
 
-__device__ __forceinline__ PairInfo SmallPairInfo(const SmallRowsSmem& S, int a, int b, const SmallPair& r) {
+template <typename Rows>
+__device__ __forceinline__ PairInfo SmallPairInfo(const Rows& S, int a, int b, const SmallPair& r) {
   const long long ea = StagedLookup(S, a, S.q[b]);
   const long long eb = StagedLookup(S, b, S.q[a]);
   PairInfo pi;
@@ -1653,6 +1729,46 @@ __device__ __forceinline__ int StageSmallRows(const QuotientView& Q, const int* 
   return E;
 }
 
+// One entry (count c, target size st) into member i's sums: below kSmallNarrow
+// in all, so the low words hold them.
+template <typename Rows>
+__device__ __forceinline__ void AddRowEntry(Rows& S, int i, long long c, long long st) {
+  const long long si = S.sz[i];
+  const long long alt = 1 + si * st - c;
+  const long long old = c < alt ? c : alt;
+  if (old >= 0) {
+    atomicAdd(reinterpret_cast<unsigned*>(&S.old[i]), static_cast<unsigned>(old));
+  } else {
+    atomicAdd(reinterpret_cast<unsigned long long*>(&S.old[i]), static_cast<unsigned long long>(old));
+  }
+  if (HeavyEntry(si, st, c)) {
+    HeavyAcc h;
+    h.Add(st, c);
+    HeavyAcc* a = &S.heavy[i];
+    atomicAdd(reinterpret_cast<unsigned long long*>(&a->sx), static_cast<unsigned long long>(h.sx));
+    atomicAdd(reinterpret_cast<unsigned long long*>(&a->c), static_cast<unsigned long long>(h.c));
+    atomicMin(&a->smin, h.smin);
+    atomicMax(&a->smax, h.smax);
+    atomicMax(&a->sbad, h.sbad);
+    atomicAdd(&a->n, 1);
+  } else {
+    atomicAdd(&S.light[i], static_cast<unsigned>(c));
+  }
+}
+
+// Old cost and heavy sums of member i, by one thread (counts too large for
+// AddRowEntry).
+template <typename Rows>
+__device__ __forceinline__ void WideRow(Rows& S, int i) {
+  long long old = 0;
+  for (int k = S.start[i]; k < S.start[i + 1]; ++k) {
+    const long long c = EntCnt(S.ent[k]), st = S.tsz[k];
+    old += EncodeCostForPair(S.q[i], S.sz[i], EntNb(S.ent[k]), st, c);
+    if (HeavyEntry(S.sz[i], st, c)) S.heavy[i].Add(st, c);
+  }
+  S.old[i] = old;
+}
+
 // The staged group's row sums and pair sums, by a warp: S.old (with the
 // internal term), S.light and S.heavy per member, and the pair sums. Returns
 // the shared targets visited; *slow: the 32-bit sums do not hold, SmallMerge
@@ -1679,27 +1795,7 @@ __device__ __forceinline__ unsigned SmallSums(const QuotientView& Q, SmallRowsSm
       const Entry e = S.ent[k];
       const int t = EntNb(e), i = S.row[k];
       const long long c = EntCnt(e), st = S.tsz[k], si = S.sz[i];
-      // row sums: below 2^28 in all, so the low words hold them
-      const long long alt = 1 + si * st - c;
-      const long long old = c < alt ? c : alt;
-      if (old >= 0) {
-        atomicAdd(reinterpret_cast<unsigned*>(&S.old[i]), static_cast<unsigned>(old));
-      } else {
-        atomicAdd(reinterpret_cast<unsigned long long*>(&S.old[i]), static_cast<unsigned long long>(old));
-      }
-      if (HeavyEntry(si, st, c)) {
-        HeavyAcc h;
-        h.Add(st, c);
-        HeavyAcc* a = &S.heavy[i];
-        atomicAdd(reinterpret_cast<unsigned long long*>(&a->sx), static_cast<unsigned long long>(h.sx));
-        atomicAdd(reinterpret_cast<unsigned long long*>(&a->c), static_cast<unsigned long long>(h.c));
-        atomicMin(&a->smin, h.smin);
-        atomicMax(&a->smax, h.smax);
-        atomicMax(&a->sbad, h.sbad);
-        atomicAdd(&a->n, 1);
-      } else {
-        atomicAdd(&S.light[i], static_cast<unsigned>(c));
-      }
+      AddRowEntry(S, i, c, st);
       for (int j = i + 1; j < g; ++j) {
         const int b = TriIndex(i, j, g);
         if (t == S.q[j]) {  // a row does not list itself: no search needed
@@ -1727,15 +1823,7 @@ __device__ __forceinline__ unsigned SmallSums(const QuotientView& Q, SmallRowsSm
   __syncwarp();
   if (wide) {
     // too large for 32 bits: a lane per member, a lane per pair
-    if (lane < g) {
-      long long old = 0;
-      for (int k = S.start[lane]; k < S.start[lane + 1]; ++k) {
-        const long long c = EntCnt(S.ent[k]), st = S.tsz[k];
-        old += EncodeCostForPair(S.q[lane], S.sz[lane], EntNb(S.ent[k]), st, c);
-        if (HeavyEntry(S.sz[lane], st, c)) S.heavy[lane].Add(st, c);
-      }
-      S.old[lane] = old;
-    }
+    if (lane < g) WideRow(S, lane);
     for (int pidx = lane; pidx < npairs; pidx += 32) {
       int a, b;
       TriPair(pidx, g, &a, &b);
@@ -1746,7 +1834,8 @@ __device__ __forceinline__ unsigned SmallSums(const QuotientView& Q, SmallRowsSm
 }
 
 // Member i's record and its old cost's internal term, by one lane.
-__device__ __forceinline__ void SmallFinishRow(const QuotientView& Q, SmallRowsSmem& S, int i, bool wide,
+template <typename Rows>
+__device__ __forceinline__ void SmallFinishRow(const QuotientView& Q, Rows& S, int i, bool wide,
                                                RowSums* out) {
   const int rep = S.q[i];
   const long long si = S.sz[i];
@@ -1778,7 +1867,8 @@ __device__ __forceinline__ SmallPair SmallPairAt(const SmallRowsSmem& S, const S
 }
 
 // Sum of f_s(c) over staged row i, by one lane.
-__device__ __forceinline__ long long StagedRowAfter(const SmallRowsSmem& S, int i, long long s) {
+template <typename Rows>
+__device__ __forceinline__ long long StagedRowAfter(const Rows& S, int i, long long s) {
   long long sum = 0;
   for (int k = S.start[i]; k < S.start[i + 1]; ++k) {
     const long long c = EntCnt(S.ent[k]);
@@ -1819,11 +1909,21 @@ __device__ __forceinline__ void SmallTopK(SmallRowsSmem& S, int g, int top_k_max
         if (valid) atomicOr(&S.fmask[i < j ? i : j], 1u << (i < j ? j : i));
         continue;
       }
+      long long denom = 1;
+      if (valid) {
+        denom = S.old[i] + S.old[j];
+        if (denom < 1) denom = 1;
+      }
+      if (!__any_sync(0xffffffffu, pg >= kExactRatio || denom >= kExactRatio)) {
+        const RankCand c[1] = {{static_cast<unsigned>(pg), static_cast<unsigned>(denom), valid ? S.q[j] : 0}};
+        int r[1];
+        ExactRanks(c, r);
+        if (valid && r[0] < top_k) atomicOr(&S.fmask[i < j ? i : j], 1u << (i < j ? j : i));
+        continue;
+      }
       long long rbits = 0;
       int lo = 0, hi = 0;
       if (valid) {
-        long long denom = S.old[i] + S.old[j];
-        if (denom < 1) denom = 1;
         rbits = __double_as_longlong(static_cast<double>(pg) / static_cast<double>(denom));
         const int qi = S.q[i];
         const int qj = S.q[j];
@@ -2371,37 +2471,39 @@ __global__ void __launch_bounds__(kThreads) SelectKernel(SelectParams P) {
 constexpr int kMatchThreads = 512;
 constexpr int kMatchSmemKeys = 8192;
 
+template <int kGroup>
 struct MatchSmem {
-  unsigned long long best[kMaxGroup];
-  unsigned long long chosen[kMaxGroup / 2];
-  unsigned char matched[kMaxGroup];
+  unsigned long long best[kGroup];
+  unsigned long long chosen[kGroup / 2];
+  unsigned char matched[kGroup];
   int nchosen, live_any;
 };
 
 // The greedy choice among m keys of a group of g members by a CTA of
-// kMatchThreads (kin, kout: two buffers of m keys, the first holds them);
+// kThreads (kin, kout: two buffers of m keys, the first holds them);
 // chosen[] gets the selected keys in ascending order, their number is
 // returned. Ends with a barrier.
-__device__ int MatchKeys(MatchSmem& M, unsigned long long* kin, unsigned long long* kout, int m, int g) {
+template <int kThreads, int kGroup>
+__device__ int MatchKeys(MatchSmem<kGroup>& M, unsigned long long* kin, unsigned long long* kout, int m, int g) {
   const int tid = threadIdx.x;
   if (tid == 0) M.nchosen = 0;
-  for (int i = tid; i < g; i += kMatchThreads) M.matched[i] = 0;
+  for (int i = tid; i < g; i += kThreads) M.matched[i] = 0;
   // rounds of locally dominant keys (each round selects at least the
   // smallest live key, so at most g/2 rounds); the keys still live after a
   // round move to the other buffer (the matching depends on the key values
   // only, not on their order)
   int nlive = m;
-  for (int round = 0; round <= kMaxGroup / 2 && nlive > 0; ++round) {
-    for (int i = tid; i < g; i += kMatchThreads) M.best[i] = ~0ull;
+  for (int round = 0; round <= kGroup / 2 && nlive > 0; ++round) {
+    for (int i = tid; i < g; i += kThreads) M.best[i] = ~0ull;
     if (tid == 0) M.live_any = 0;
     __syncthreads();
-    for (int k = tid; k < nlive; k += kMatchThreads) {
+    for (int k = tid; k < nlive; k += kThreads) {
       const unsigned long long key = kin[k];
       atomicMin(&M.best[(key >> kKeyIdxBits) & kKeyIdxMask], key);
       atomicMin(&M.best[key & kKeyIdxMask], key);
     }
     __syncthreads();
-    for (int k = tid; k < nlive; k += kMatchThreads) {
+    for (int k = tid; k < nlive; k += kThreads) {
       const unsigned long long key = kin[k];
       const int a = static_cast<int>((key >> kKeyIdxBits) & kKeyIdxMask);
       const int b = static_cast<int>(key & kKeyIdxMask);
@@ -2412,7 +2514,7 @@ __device__ int MatchKeys(MatchSmem& M, unsigned long long* kin, unsigned long lo
       }
     }
     __syncthreads();
-    for (int k = tid; k < nlive; k += kMatchThreads) {
+    for (int k = tid; k < nlive; k += kThreads) {
       const unsigned long long key = kin[k];
       if (!M.matched[(key >> kKeyIdxBits) & kKeyIdxMask] && !M.matched[key & kKeyIdxMask]) {
         kout[atomicAdd(&M.live_any, 1)] = key;
@@ -2429,7 +2531,7 @@ __device__ int MatchKeys(MatchSmem& M, unsigned long long* kin, unsigned long lo
   const int ns = M.nchosen;
   int pow2 = 1;
   while (pow2 < ns) pow2 <<= 1;
-  for (int i = ns + tid; i < pow2; i += kMatchThreads) M.chosen[i] = ~0ull;
+  for (int i = ns + tid; i < pow2; i += kThreads) M.chosen[i] = ~0ull;
   __syncthreads();
   if (ns > 1) CtaBitonicSort(M.chosen, pow2);
   return ns;
@@ -2438,7 +2540,7 @@ __device__ int MatchKeys(MatchSmem& M, unsigned long long* kin, unsigned long lo
 __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned long long* skeys = reinterpret_cast<unsigned long long*>(smem_raw);
-  __shared__ MatchSmem M;
+  __shared__ MatchSmem<kMaxGroup> M;
   __shared__ int nkeys;
   __shared__ unsigned long long* gkeys;
   __shared__ unsigned long long rej_thr;
@@ -2487,7 +2589,7 @@ __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) 
   __syncthreads();
   const int m = nkeys;
   // the selected keys in greedy (ascending key) order
-  const int ns = MatchKeys(M, keys, keys + cnt, m, g);
+  const int ns = MatchKeys<kMatchThreads>(M, keys, keys + cnt, m, g);
   const int* q = P.order + P.gstart[gid];
   const long long so = P.sel_off[ri];
   long long my_total = 0;
@@ -2667,6 +2769,7 @@ __global__ void __launch_bounds__(kSelectSmallWarps * 32) SelectSmallKernel(Sele
   }
 }
 
+#include "medium.cuh"
 #include "window.cuh"
 
 // ------------------------------------------------------------ commit
@@ -3638,6 +3741,8 @@ void Engine::ConfigureKernels() {
                                  static_cast<int>(sizeof(RowsSmem))), "rewrite smem attribute");
   CheckCuda(cudaFuncSetAttribute(RewriteHugeKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(sizeof(HugeSmem))), "long-row rewrite smem attribute");
+  CheckCuda(cudaFuncSetAttribute(MediumKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(sizeof(MediumSmem))), "medium smem attribute");
   CheckCuda(cudaFuncSetAttribute(WindowEvalKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(sizeof(EvalSmem))), "window evaluation smem attribute");
   CheckCuda(cudaFuncSetAttribute(WindowSelectKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3668,7 +3773,7 @@ constexpr int kPlanItems = 8;
 constexpr int kPlanTile = kPlanThreads * kPlanItems;
 enum PlanScalar : int {
   kPlanR = 0, kPlanCand, kPlanSel, kPlanSmall, kPlanBig, kPlanMembers, kPlanSlots, kPlanMat, kPlanMaxE,
-  kPlanSelSmall, kPlanSelMid, kPlanSelBig, kPlanSmallBase, kPlanScalars = kPlanSmallBase + 4
+  kPlanSelSmall, kPlanSelMid, kPlanSelBig, kPlanMed, kPlanSmallBase, kPlanScalars = kPlanSmallBase + 4
 };
 // The small-group list is laid out by member count, largest class first
 // (more than 24, 17..24, 9..16, at most 8 members): the longest warps start
@@ -3676,9 +3781,14 @@ enum PlanScalar : int {
 constexpr int kPlanSmallClasses = 4;
 __device__ __forceinline__ int SmallClass(int g) { return g > 24 ? 0 : g > 16 ? 1 : g > 8 ? 2 : 3; }
 
+// What the medium groups do: candidates for the later passes like the rest
+// (the ranker prunes them there), or everything in one kernel (medium.cuh);
+// windows of blocks have their own limits.
+enum PlanMode : int { kPlanLists = 0, kPlanFused = 1, kPlanWindows = 2 };
+
 struct PlanSums {
   long long cand, sel, moff, soff, mat;
-  int real, big, ssmall, smid, sbig;
+  int real, med, big, ssmall, smid, sbig;
   int small[kPlanSmallClasses];
 };
 
@@ -3693,6 +3803,7 @@ struct PlanSumOp {
     r.real = a.real + b.real;
 #pragma unroll
     for (int c = 0; c < kPlanSmallClasses; ++c) r.small[c] = a.small[c] + b.small[c];
+    r.med = a.med + b.med;
     r.big = a.big + b.big;
     r.ssmall = a.ssmall + b.ssmall;
     r.smid = a.smid + b.smid;
@@ -3704,22 +3815,26 @@ struct PlanSumOp {
 __device__ __forceinline__ PlanSums PlanZero() {
   PlanSums z;
   z.cand = z.sel = z.moff = z.soff = z.mat = 0;
-  z.real = z.big = z.ssmall = z.smid = z.sbig = 0;
+  z.real = z.med = z.big = z.ssmall = z.smid = z.sbig = 0;
 #pragma unroll
   for (int c = 0; c < kPlanSmallClasses; ++c) z.small[c] = 0;
   return z;
 }
 
 // one group's contribution: the same rules as the host plan
-__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, int windowed) {
+__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, int mode) {
   PlanSums f = PlanZero();
   if (g < 2) return f;
   const long long gl = g;
   f.real = 1;
   f.cand = gl * (gl - 1) / 2 < gl * k ? gl * (gl - 1) / 2 : gl * k;
   f.sel = gl / 2;
+  const bool windowed = mode == kPlanWindows;
   if (windowed ? WindowSmall(g, e) : g <= kSmallGroup && e <= static_cast<unsigned>(kSmallStage)) {
     f.small[SmallClass(g)] = 1;
+  } else if (mode == kPlanFused && MediumFits(g, e)) {
+    f.med = 1;  // with its selection
+    return f;
   } else {
     f.big = 1;
     f.moff = gl;
@@ -3741,7 +3856,7 @@ struct PlanParams {
   const unsigned* gent;
   long long G;
   long long top_k;
-  int windowed;  // 1: the sizes and limits of window.cuh
+  int mode;  // PlanMode
   PlanSums* tile_sums;
   PlanSums* tile_off;
   int tiles;
@@ -3751,6 +3866,7 @@ struct PlanParams {
   long long* sel_off;
   long long* mat_off;
   int* small;
+  int* med;
   int* big;
   long long* big_moff;
   long long* soff;
@@ -3769,7 +3885,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanTileKernel(PlanParams P) {
   for (int j = 0; j < kPlanItems; ++j) {
     const long long gi = base + j;
     if (gi >= P.G) break;
-    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k, P.windowed);
+    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k, P.mode);
     acc = PlanSumOp()(acc, f);
     max_e = f.soff > max_e ? f.soff : max_e;
   }
@@ -3811,6 +3927,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScanKernel(PlanParams P) {
       sb += T.small[c];
     }
     s[kPlanSmall] = sb;
+    s[kPlanMed] = T.med;
     s[kPlanBig] = T.big;
     s[kPlanMembers] = T.moff;
     s[kPlanSlots] = T.soff;
@@ -3838,13 +3955,13 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
     const long long gi = base + j;
     g[j] = gi < P.G ? P.glen[gi] : 0;
     e[j] = gi < P.G ? P.gent[gi] : 0u;
-    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k, P.windowed));
+    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k, P.mode));
   }
   PlanSums off;
   Scan(tmp).ExclusiveScan(acc, off, P.tile_off[blockIdx.x], PlanSumOp());
 #pragma unroll
   for (int j = 0; j < kPlanItems; ++j) {
-    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k, P.windowed);
+    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k, P.mode);
     if (P.ri_of && base + j < P.G) P.ri_of[base + j] = f.real ? off.real : -1;
     if (f.real) {
       const int ri = off.real;
@@ -3852,7 +3969,9 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
       P.cand_off[ri] = off.cand;
       P.sel_off[ri] = off.sel;
       P.mat_off[ri] = f.big ? off.mat : 0;
-      if (!f.big) {
+      if (f.med) {
+        P.med[off.med] = ri;
+      } else if (!f.big) {
         const int c = SmallClass(g[j]);
         P.small[P.scalars[kPlanSmallBase + c] + off.small[c]] = ri;
       } else {
@@ -3864,7 +3983,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
         P.sel_small[off.ssmall] = ri;
       } else if (f.smid) {
         P.sel_mid[off.smid] = ri;
-      } else {
+      } else if (f.sbig) {
         P.sel_big[off.sbig] = ri;
       }
     }
@@ -3873,6 +3992,13 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
 }
 
 }  // namespace
+
+// Medium groups go from rows to selected pairs in one kernel where there are
+// enough of them, unless something wants to see their candidates (the ranker)
+// or the exact gain needs the rows again.
+bool Engine::FusedOn() const { return RowSumsOn() && !cfg_.ranker; }
+
+bool Engine::PlanFused() const { return FusedOn() && n_groups_ >= kMedMinAll; }
 
 void Engine::PrepareIterationBuffers() {
   const int64_t G = n_groups_;
@@ -3905,16 +4031,30 @@ void Engine::PrepareIterationBuffers() {
   h_big_.clear();
   h_big_moff_.assign(1, 0);
   h_soff_.assign(1, 0);
+  h_med_.clear();
   h_block_small_.clear();
+  h_block_med_.clear();
   h_block_big_.clear();
   std::vector<long long> block_mat;
   auto is_small = [&](int ri) {
     const size_t gid = static_cast<size_t>(h_real_[static_cast<size_t>(ri)]);
     return h_glen_[gid] <= kSmallGroup && h_gent_[gid] <= static_cast<unsigned>(kSmallStage);
   };
+  auto is_medium = [&](int ri) {
+    const size_t gid = static_cast<size_t>(h_real_[static_cast<size_t>(ri)]);
+    return !is_small(ri) && MediumFits(h_glen_[gid], h_gent_[gid]);
+  };
+  h_block_fused_.clear();
   for (size_t b = 0; b + 1 < h_block_rg_.size(); ++b) {
     h_block_small_.push_back(static_cast<int>(h_small_.size()));
+    h_block_med_.push_back(static_cast<int>(h_med_.size()));
     h_block_big_.push_back(static_cast<int>(h_big_.size()));
+    int medium = 0;
+    if (FusedOn()) {
+      for (int ri = h_block_rg_[b]; ri < h_block_rg_[b + 1]; ++ri) medium += is_medium(ri) ? 1 : 0;
+    }
+    const bool fused = medium >= kMedMinGroups;
+    h_block_fused_.push_back(fused ? 1 : 0);
     // a small block with any big group sends all its groups to the big path
     // (one prepare path, fewer launches; the same candidates)
     bool all_big = false;
@@ -3931,6 +4071,10 @@ void Engine::PrepareIterationBuffers() {
         h_small_.push_back(ri);
         continue;
       }
+      if (fused && is_medium(ri)) {
+        h_med_.push_back(ri);
+        continue;
+      }
       h_big_.push_back(ri);
       h_big_moff_.push_back(h_big_moff_.back() + g);
       // groups beyond the shared-memory bucket table get sort slots
@@ -3943,6 +4087,7 @@ void Engine::PrepareIterationBuffers() {
     block_mat.push_back(off);
   }
   h_block_small_.push_back(static_cast<int>(h_small_.size()));
+  h_block_med_.push_back(static_cast<int>(h_med_.size()));
   h_block_big_.push_back(static_cast<int>(h_big_.size()));
   // selection: groups of at most kSelectSmallGroup members (at most 28
   // candidates) get one warp each, the others one CTA each
@@ -3958,6 +4103,7 @@ void Engine::PrepareIterationBuffers() {
     h_block_sel_big_.push_back(static_cast<int>(h_sel_big_.size()));
     for (int ri = h_block_rg_[b]; ri < h_block_rg_[b + 1]; ++ri) {
       const int g = h_glen_[static_cast<size_t>(h_real_[static_cast<size_t>(ri)])];
+      if (h_block_fused_[b] && is_medium(ri)) continue;  // selected by its own kernel
       (g <= kSelectSmallGroup ? h_sel_small_ : g <= kSelectMidGroup ? h_sel_mid_ : h_sel_big_).push_back(ri);
     }
   }
@@ -3978,6 +4124,11 @@ void Engine::PrepareIterationBuffers() {
   if (!h_sel_big_.empty()) {
     CheckCuda(cudaMemcpyAsync(d_sel_big_.p, h_sel_big_.data(), sizeof(int) * h_sel_big_.size(),
                               cudaMemcpyHostToDevice, stream_), "h2d select big list");
+  }
+  d_med_.ensure(h_med_.size() + 1);
+  if (!h_med_.empty()) {
+    CheckCuda(cudaMemcpyAsync(d_med_.p, h_med_.data(), sizeof(int) * h_med_.size(), cudaMemcpyHostToDevice, stream_),
+              "h2d medium list");
   }
   d_small_.ensure(h_small_.size() + 1);
   d_big_.ensure(h_big_.size() + 1);
@@ -4025,6 +4176,9 @@ void Engine::PrepareIterationBuffers() {
     bp.sel_slots = h_sel_off_[static_cast<size_t>(bp.rg1)] - h_sel_off_[static_cast<size_t>(bp.rg0)];
     bp.s0 = h_block_small_[b];
     bp.s1 = h_block_small_[b + 1];
+    bp.m0 = h_block_med_[b];
+    bp.m1 = h_block_med_[b + 1];
+    bp.fused = h_block_fused_[b] != 0;
     bp.b0 = h_block_big_[b];
     bp.b1 = h_block_big_[b + 1];
     bp.members = h_big_moff_[static_cast<size_t>(bp.b1)] - h_big_moff_[static_cast<size_t>(bp.b0)];
@@ -4090,7 +4244,7 @@ void Engine::SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nb
 void Engine::PlanOnDevice() {
   const long long G = n_groups_;
   const size_t cap = static_cast<size_t>(G) + 1;
-  for (DevBuf<int>* b : {&d_real_, &d_small_, &d_big_, &d_sel_small_, &d_sel_mid_, &d_sel_big_}) b->ensure(cap);
+  for (DevBuf<int>* b : {&d_real_, &d_small_, &d_med_, &d_big_, &d_sel_small_, &d_sel_mid_, &d_sel_big_}) b->ensure(cap);
   for (DevBuf<long long>* b : {&d_cand_off_, &d_sel_off_, &d_mat_off_, &d_big_moff_, &d_soff_}) b->ensure(cap);
   const int tiles = static_cast<int>((G + kPlanTile - 1) / kPlanTile);
   d_plan_tiles_.ensure(sizeof(PlanSums) * (2 * static_cast<size_t>(tiles) + 1));
@@ -4101,7 +4255,7 @@ void Engine::PlanOnDevice() {
   P.gent = d_gent_.p;
   P.G = G;
   P.top_k = cfg_.top_k > 0 ? cfg_.top_k : 1;
-  P.windowed = windowed_ ? 1 : 0;
+  P.mode = windowed_ ? kPlanWindows : PlanFused() ? kPlanFused : kPlanLists;
   P.tile_sums = reinterpret_cast<PlanSums*>(d_plan_tiles_.p);
   P.tile_off = P.tile_sums + tiles;
   P.tiles = tiles;
@@ -4111,6 +4265,7 @@ void Engine::PlanOnDevice() {
   P.sel_off = d_sel_off_.p;
   P.mat_off = d_mat_off_.p;
   P.small = d_small_.p;
+  P.med = d_med_.p;
   P.big = d_big_.p;
   P.big_moff = d_big_moff_.p;
   P.soff = d_soff_.p;
@@ -4132,6 +4287,7 @@ void Engine::PlanOnDevice() {
     ++launches_;
     PlanScatterKernel<<<tiles, kPlanThreads, 0, stream_>>>(P);
   }
+  static_assert(kPlanScalars + 1 <= 32, "room in the pinned words");
   long long* hs = h_pin_.p + 16;  // read back: totals and pool top
   CheckCuda(cudaMemcpyAsync(hs, d_plan_scalars_.p, sizeof(long long) * kPlanScalars, cudaMemcpyDeviceToHost,
                             stream_), "d2h plan");
@@ -4150,7 +4306,9 @@ void Engine::PlanOnDevice() {
   bp.slots = v[kPlanCand];
   bp.sel_slots = v[kPlanSel];
   bp.s1 = static_cast<int>(v[kPlanSmall]);
+  bp.m1 = static_cast<int>(v[kPlanMed]);
   bp.b1 = static_cast<int>(v[kPlanBig]);
+  bp.fused = PlanFused();
   bp.members = v[kPlanMembers];
   bp.nslots = v[kPlanSlots];
   bp.max_e = v[kPlanMaxE];
@@ -4367,6 +4525,42 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
   EndTimed(kTimePrepare);
 }
 
+void Engine::LaunchMedium(const BlockPlan& bp, double threshold) {
+  if (bp.m1 <= bp.m0) return;
+  MediumParams M{};
+  M.Q = View();
+  M.order = d_order_.p;
+  M.gstart = d_gstart_.p;
+  M.glen = d_glen_.p;
+  M.group_of = d_group_of_.p;
+  M.idx_in_group = d_idx_in_group_.p;
+  M.real = d_real_.p;
+  M.list = d_med_.p;
+  M.list0 = bp.m0;
+  M.top_k = cfg_.top_k;
+  M.threshold = threshold;
+  M.thr = SplitThreshold(threshold);
+  M.use_threshold = cfg_.ea_use_threshold ? 1 : 0;
+  M.strict = bp.rg1 - bp.rg0 <= kFewGroups ? 1 : 0;
+  M.sel_off = d_sel_off_.p;
+  M.sel_keep = d_sel_keep_.p;
+  M.sel_rem = d_sel_rem_.p;
+  M.sel_gain = d_sel_gain_.p;
+  M.sel_cnt = d_sel_cnt_.p;
+  M.stamp = d_stamp_.p;
+  M.partner = d_partner_.p;
+  M.seq = d_seq_.p;
+  M.sel_list = d_sel_list_.p;
+  M.ctl = d_ctl_.p;
+  M.block_stamp = block_stamp_;
+  M.stats = d_stats_.p;
+  M.err = d_err_.p;
+  BeginTimed(kTimePrepare);
+  ++launches_;
+  MediumKernel<<<bp.m1 - bp.m0, kMedThreads, sizeof(MediumSmem), stream_>>>(M);
+  EndTimed(kTimePrepare);
+}
+
 void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total_iterations) {
   ++block_stamp_;
   ++hstats_.blocks;
@@ -4376,6 +4570,7 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
   const long long sel_slots = bp.sel_slots;
   // the block control words are zero: cleared by Merge before the first
   // block and by the previous block's last kernel
+  LaunchMedium(bp, threshold);
   LaunchPrepare(bp);
   ScoreParams SP;
   SP.Q = View();
@@ -4467,7 +4662,7 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
   LP.sel_list = d_sel_list_.p;
   const int ss0 = bp.ss0, ss1 = bp.ss1;
   const int sb0 = bp.sb0, sb1 = bp.sb1;
-  if (nrg <= kFewGroups) {
+  if (nrg <= kFewGroups && !bp.fused) {
     // a small block: one launch, a CTA per group (same selection)
     LP.list = nullptr;
     LP.list0 = rg0;

@@ -860,7 +860,9 @@ __global__ void __launch_bounds__(256, 2) WindowScoreKernel(WindowParams P) {
     unsigned* flags = reinterpret_cast<unsigned*>(mat + FlagOffset(static_cast<long long>(g) * g));
     if (lane == 0) nkept[warp] = 0;
     __syncwarp();
-    RankMember(g, i, q, mat, P.top_k, cand_j[warp], [&](int a, int b) {
+    const long long* old = reinterpret_cast<const long long*>(mat + OldCostOffset(static_cast<long long>(g) * g));
+    auto proxy = [&](int x, int j) { return ProxyOf(PairWord(pmat, g, x, j)); };
+    RankMember(g, i, q, old, P.top_k, cand_j[warp], proxy, [&](int a, int b) {
       const long long at = static_cast<long long>(a) * g + b;
       const unsigned bit = 1u << (8 * (at & 3));
       if (!(atomicOr(&flags[at >> 2], bit) & bit)) {
@@ -939,7 +941,7 @@ __global__ void __launch_bounds__(kMatchThreads) WindowSelectKernel(WindowParams
   FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned long long* skeys = reinterpret_cast<unsigned long long*>(smem_raw);
-  __shared__ MatchSmem M;
+  __shared__ MatchSmem<kMaxGroup> M;
   __shared__ unsigned long long s_gain, s_work;
   __shared__ int s_conflict;
   const QuotientView& Q = P.Q;
@@ -972,7 +974,7 @@ __global__ void __launch_bounds__(kMatchThreads) WindowSelectKernel(WindowParams
       s_conflict = 0x7fffffff;
     }
     __syncthreads();
-    const int ns = MatchKeys(M, keys, spare, m, g);
+    const int ns = MatchKeys<kMatchThreads>(M, keys, spare, m, g);
     // the selected pairs in greedy order, and what they touch: a warp per
     // pair, the whole CTA where a row is long
     const long long so = P.sel_off[ri];
