@@ -14,9 +14,12 @@
 // counts toward a row's own representative drop its self-loops first
 // (src/cuda_scoring.cu:146-252, 282-357).
 //
-// GB300 form: one warp per pair. Lanes take 32 entries of row a at a time and
-// find each neighbour in row b by binary search; then 32 entries of row b at a
-// time, skipping those present in row a. Terms are summed per lane and
+// GB300 form: one warp per pair. Lanes take 32 entries of row a at a time, four
+// steps in flight, and find each neighbour in row b by binary search; then the
+// entries of row b, skipping those present in row a. Pairs of more than
+// kFlatLong entries are shared by the CTA's eight warps once each warp has done
+// its own: a hub row of 1,600 entries is two chains of loads instead of 50,
+// which were most of the kernel's time. Terms are summed per lane and
 // reduced once per pair. A call packs the host inputs into one pinned buffer,
 // copies it with one H2D, runs one kernel and copies 16 bytes per pair back.
 
@@ -44,17 +47,28 @@ struct FlatView {
   const long long* self;
 };
 
-// Count of neighbour `key` in the sorted flat row [s, e) (0 when absent), and
-// whether it is present.
-__device__ __forceinline__ long long FlatLookup(const int* nb, const long long* wt, int s, int e, int key,
-                                                bool* found) {
-  int lo = s, hi = e;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (nb[mid] < key) lo = mid + 1; else hi = mid;
+// Positions of four keys in the sorted flat row [s, e) (lower bounds), searched
+// side by side.
+constexpr int kFlatDeep = 4;
+constexpr int kFlatLong = 256;
+
+__device__ __forceinline__ void FlatLowerBounds(const int* nb, int s, int e, const int (&key)[kFlatDeep],
+                                                int (&lo)[kFlatDeep]) {
+  int hi[kFlatDeep];
+#pragma unroll
+  for (int d = 0; d < kFlatDeep; ++d) {
+    lo[d] = s;
+    hi[d] = e;
   }
-  *found = lo < e && nb[lo] == key;
-  return *found ? wt[lo] : 0;
+  for (int span = e - s; span > 0; span >>= 1) {
+#pragma unroll
+    for (int d = 0; d < kFlatDeep; ++d) {
+      if (lo[d] < hi[d]) {
+        const int mid = (lo[d] + hi[d]) >> 1;
+        if (nb[mid] < key[d]) lo[d] = mid + 1; else hi[d] = mid;
+      }
+    }
+  }
 }
 
 struct LegacyPair {
@@ -75,53 +89,109 @@ __device__ __forceinline__ void LegacyTerm(const LegacyPair& p, int x, long long
   *after += EncodeCostForPair(p.ra, p.sm, mrep, msz, ea + eb);
 }
 
+// The pair's terms over entries first, first + stride, ... of both rows.
+struct LegacySums {
+  long long before = 0, after = 0;
+  bool seen_a = false, seen_b = false;
+};
+
+__device__ __forceinline__ void LegacyRows(const FlatView& F, const LegacyPair& p, int a0, int a1, int b0, int b1,
+                                           int first, int stride, LegacySums* s) {
+  for (int k0 = a0 + first; k0 < a1; k0 += stride * kFlatDeep) {
+    int x[kFlatDeep], at[kFlatDeep];
+#pragma unroll
+    for (int d = 0; d < kFlatDeep; ++d) x[d] = k0 + d * stride < a1 ? F.nb[k0 + d * stride] : 0x7fffffff;
+    FlatLowerBounds(F.nb, b0, b1, x, at);
+#pragma unroll
+    for (int d = 0; d < kFlatDeep; ++d) {
+      const int k = k0 + d * stride;
+      if (k >= a1) continue;
+      const long long eb = at[d] < b1 && F.nb[at[d]] == x[d] ? F.wt[at[d]] : 0;
+      LegacyTerm(p, x[d], F.nsz[k], F.wt[k], eb, &s->before, &s->after);
+      s->seen_a |= x[d] == p.ra;
+      s->seen_b |= x[d] == p.rb;
+    }
+  }
+  for (int k0 = b0 + first; k0 < b1; k0 += stride * kFlatDeep) {
+    int x[kFlatDeep], at[kFlatDeep];
+#pragma unroll
+    for (int d = 0; d < kFlatDeep; ++d) x[d] = k0 + d * stride < b1 ? F.nb[k0 + d * stride] : 0x7fffffff;
+    FlatLowerBounds(F.nb, a0, a1, x, at);
+#pragma unroll
+    for (int d = 0; d < kFlatDeep; ++d) {
+      const int k = k0 + d * stride;
+      if (k >= b1 || (at[d] < a1 && F.nb[at[d]] == x[d])) continue;
+      LegacyTerm(p, x[d], F.nsz[k], 0, F.wt[k], &s->before, &s->after);
+      s->seen_a |= x[d] == p.ra;
+      s->seen_b |= x[d] == p.rb;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kLegacyThreads) LegacyFlatScoreKernel(FlatView F, const int2* pairs,
                                                                          long long count, long long* out) {
   constexpr unsigned kFull = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const long long warps = static_cast<long long>(gridDim.x) * (kLegacyThreads / 32);
-  for (long long w = (static_cast<long long>(blockIdx.x) * kLegacyThreads + threadIdx.x) >> 5; w < count;
-       w += warps) {
-    const int2 pr = pairs[w];
-    LegacyPair p;
-    p.ra = F.rep[pr.x];
-    p.rb = F.rep[pr.y];
-    p.sa = F.rsz[pr.x];
-    p.sb = F.rsz[pr.y];
-    p.sm = p.sa + p.sb;
-    p.la = F.self[pr.x];
-    p.lb = F.self[pr.y];
-    const int a0 = F.off[pr.x], a1 = F.off[pr.x + 1];
-    const int b0 = F.off[pr.y], b1 = F.off[pr.y + 1];
-    long long before = 0, after = 0;
-    bool seen_a = false, seen_b = false;
-    for (int k = a0 + lane; k < a1; k += 32) {
-      const int x = F.nb[k];
-      bool in_b = false;
-      const long long eb = FlatLookup(F.nb, F.wt, b0, b1, x, &in_b);
-      LegacyTerm(p, x, F.nsz[k], F.wt[k], eb, &before, &after);
-      seen_a |= x == p.ra;
-      seen_b |= x == p.rb;
-    }
-    for (int k = b0 + lane; k < b1; k += 32) {
-      const int x = F.nb[k];
-      bool in_a = false;
-      FlatLookup(F.nb, F.wt, a0, a1, x, &in_a);
-      if (in_a) continue;
-      LegacyTerm(p, x, F.nsz[k], 0, F.wt[k], &before, &after);
-      seen_a |= x == p.ra;
-      seen_b |= x == p.rb;
-    }
-    before = WarpSum(before);
-    after = WarpSum(after);
-    seen_a = __any_sync(kFull, seen_a);
-    seen_b = __any_sync(kFull, seen_b);
-    if (lane == 0) {
-      // a row that does not list its own representative still pays for it
-      if (!seen_a) LegacyTerm(p, p.ra, p.sa, 0, 0, &before, &after);
-      if (p.rb != p.ra && !seen_b) LegacyTerm(p, p.rb, p.sb, 0, 0, &before, &after);
-      out[2 * w] = before - after;
-      out[2 * w + 1] = before;
+  constexpr int kWarps = kLegacyThreads / 32;
+  __shared__ int is_long[kWarps];
+  __shared__ long long part[kWarps][2];
+  __shared__ int seen[kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long w0 = static_cast<long long>(blockIdx.x) * kWarps; w0 < count;
+       w0 += static_cast<long long>(gridDim.x) * kWarps) {
+    // pass 0: a warp per pair; then the long ones of the eight, all warps on each
+    for (int pass = 0; pass <= kWarps; ++pass) {
+      const int which = pass == 0 ? warp : pass - 1;
+      const long long w = w0 + which;
+      if (pass > 0 && !is_long[which]) continue;
+      LegacySums s;
+      LegacyPair p = {0, 0, 0, 0, 0, 0, 0};
+      bool mine = false;  // summed here
+      if (w < count) {
+        const int2 pr = pairs[w];
+        const int a0 = F.off[pr.x], a1 = F.off[pr.x + 1];
+        const int b0 = F.off[pr.y], b1 = F.off[pr.y + 1];
+        mine = pass > 0 || (a1 - a0) + (b1 - b0) <= kFlatLong;
+        if (mine) {
+          p.ra = F.rep[pr.x];
+          p.rb = F.rep[pr.y];
+          p.sa = F.rsz[pr.x];
+          p.sb = F.rsz[pr.y];
+          p.sm = p.sa + p.sb;
+          p.la = F.self[pr.x];
+          p.lb = F.self[pr.y];
+          LegacyRows(F, p, a0, a1, b0, b1, pass > 0 ? static_cast<int>(threadIdx.x) : lane,
+                     pass > 0 ? kLegacyThreads : 32, &s);
+        }
+      }
+      s.before = WarpSum(s.before);
+      s.after = WarpSum(s.after);
+      s.seen_a = __any_sync(kFull, s.seen_a);
+      s.seen_b = __any_sync(kFull, s.seen_b);
+      if (pass > 0) {
+        if (lane == 0) {
+          part[warp][0] = s.before;
+          part[warp][1] = s.after;
+          seen[warp] = (s.seen_a ? 1 : 0) | (s.seen_b ? 2 : 0);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          for (int k = 1; k < kWarps; ++k) {
+            s.before += part[k][0];
+            s.after += part[k][1];
+            s.seen_a |= (seen[k] & 1) != 0;
+            s.seen_b |= (seen[k] & 2) != 0;
+          }
+        }
+      }
+      if (mine && lane == 0 && (pass == 0 || warp == 0)) {
+        // a row that does not list its own representative still pays for it
+        if (!s.seen_a) LegacyTerm(p, p.ra, p.sa, 0, 0, &s.before, &s.after);
+        if (p.rb != p.ra && !s.seen_b) LegacyTerm(p, p.rb, p.sb, 0, 0, &s.before, &s.after);
+        out[2 * w] = s.before - s.after;
+        out[2 * w + 1] = s.before;
+      }
+      if (pass == 0 && lane == 0) is_long[warp] = w < count && !mine ? 1 : 0;
+      __syncthreads();
     }
   }
 }
@@ -221,15 +291,17 @@ int beam_flat_scorer_score(beam_flat_scorer* s, const int32_t* pairs, int64_t co
   if (offsets[0] != 0 || offsets[rows] != entries) return FlatFail("offsets must rise from 0 to entries");
   for (int32_t i = 0; i < rows; ++i) {
     if (offsets[i] > offsets[i + 1]) return FlatFail("offsets must rise from 0 to entries");
-    for (int32_t k = offsets[i] + 1; k < offsets[i + 1]; ++k) {
-      if (neighbors[k - 1] >= neighbors[k]) {
-        return FlatFail("row " + std::to_string(i) + " is not sorted by neighbour without repeats");
-      }
-    }
+    unsigned falls = 0;  // no branch in the loop: it vectorises
+    for (int32_t k = offsets[i] + 1; k < offsets[i + 1]; ++k) falls |= neighbors[k - 1] >= neighbors[k] ? 1u : 0u;
+    if (falls) return FlatFail("row " + std::to_string(i) + " is not sorted by neighbour without repeats");
   }
-  for (int64_t p = 0; p < count; ++p) {
-    if (pairs[2 * p] < 0 || pairs[2 * p] >= rows || pairs[2 * p + 1] < 0 || pairs[2 * p + 1] >= rows) {
-      return FlatFail("pair " + std::to_string(p) + " names a row outside [0, rows)");
+  uint32_t largest = 0;  // a negative index is a large one
+  for (int64_t p = 0; p < 2 * count; ++p) largest = std::max(largest, static_cast<uint32_t>(pairs[p]));
+  if (largest >= static_cast<uint32_t>(rows)) {
+    for (int64_t p = 0; p < count; ++p) {
+      if (pairs[2 * p] < 0 || pairs[2 * p] >= rows || pairs[2 * p + 1] < 0 || pairs[2 * p + 1] >= rows) {
+        return FlatFail("pair " + std::to_string(p) + " names a row outside [0, rows)");
+      }
     }
   }
   try {

@@ -101,28 +101,25 @@ struct GainWork {
   long long bytes;  // algorithmic bytes of the gain computations
 };
 
-// Warp-cooperative ExactMergeGainPersistentImpl as a tiled merge of the two
-// sorted rows: each step loads the next 32 entries of both rows (coalesced);
-// with lim = the smaller of the two tiles' last neighbours, every entry <= lim
-// is final in this step (an equal neighbour in the other row, if any, is in
-// the other tile), and each lane finds its entry in the other tile by a
-// 5-step shuffle search. Shared neighbours give two before-terms, one-sided
-// neighbours one; e(a,b) is read from both rows and must agree. Every term
-// is exact int64; the work is O(|R_a| + |R_b|).
-__device__ void WarpExactGain(const QuotientView& Q, int a, int b, long long* gain_out, long long* before_out,
-                              GainWork* work, DevError* err) {
+// The before and after terms of the union of two sorted row ranges (entries
+// toward a and b themselves aside), by a warp, as a tiled merge: each step
+// loads the next 32 entries of both (coalesced); with lim = the smaller of the
+// two tiles' last neighbours, every entry <= lim is final in this step (an
+// equal neighbour in the other range, if any, is in the other tile), and each
+// lane finds its entry in the other tile by a 5-step shuffle search. Shared
+// neighbours give two before-terms, one-sided neighbours one. Every term is
+// exact int64; the work is O(la + lb). Sums are the lanes' own.
+struct MergeTerms {
+  long long before = 0, after = 0, eab_a = 0, eab_b = 0;  // e(a, b) as read from either row
+  int uni = 0, ovl = 0, bad = 0;
+};
+
+__device__ __forceinline__ void WarpMergeTerms(const QuotientView& Q, int a, int b, long long sa, long long sb,
+                                               const Entry* ra, int la, const Entry* rb, int lb, MergeTerms* T) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr Entry kPadEntry = static_cast<Entry>(0x7fffffffull) << 32;  // neighbour INT_MAX, count 0
   const int lane = threadIdx.x & 31;
-  const long long sa = Q.size[a];
-  const long long sb = Q.size[b];
   const long long sw = sa + sb;
-  const Entry* ra = Q.ent + Q.off[a];
-  const Entry* rb = Q.ent + Q.off[b];
-  const int la = Q.len[a];
-  const int lb = Q.len[b];
-  long long before = 0, after = 0, eab_a = 0, eab_b = 0;
-  int uni = 0, ovl = 0, bad = 0;
   int pa = 0, pb = 0;
   while (pa < la || pb < lb) {
     const bool va = pa + lane < la;
@@ -150,35 +147,52 @@ __device__ void WarpExactGain(const QuotientView& Q, int a, int b, long long* ga
     if (fin_a) {
       const long long ca = EntCnt(ea_e);
       if (xa == b) {
-        eab_a = ca;
+        T->eab_a = ca;
       } else {
         const long long sx = Q.size[xa];
         if (EntNb(cand_b) == xa) {
           const long long cb = EntCnt(cand_b);
-          before += BlockCost(sa, sx, ca, false, bad) + BlockCost(sb, sx, cb, false, bad);
-          after += BlockCost(sw, sx, ca + cb, false, bad);
-          ++ovl;
+          T->before += BlockCost(sa, sx, ca, false, T->bad) + BlockCost(sb, sx, cb, false, T->bad);
+          T->after += BlockCost(sw, sx, ca + cb, false, T->bad);
+          ++T->ovl;
         } else {
-          before += BlockCost(sa, sx, ca, false, bad);
-          after += BlockCost(sw, sx, ca, false, bad);
+          T->before += BlockCost(sa, sx, ca, false, T->bad);
+          T->after += BlockCost(sw, sx, ca, false, T->bad);
         }
-        ++uni;
+        ++T->uni;
       }
     }
     if (fin_b) {
       const long long cb = EntCnt(eb_e);
       if (xb == a) {
-        eab_b = cb;
+        T->eab_b = cb;
       } else if (EntNb(cand_a) != xb) {
         const long long sx = Q.size[xb];
-        before += BlockCost(sb, sx, cb, false, bad);
-        after += BlockCost(sw, sx, cb, false, bad);
-        ++uni;
+        T->before += BlockCost(sb, sx, cb, false, T->bad);
+        T->after += BlockCost(sw, sx, cb, false, T->bad);
+        ++T->uni;
       }
     }
     pa += __popc(__ballot_sync(kFull, fin_a));
     pb += __popc(__ballot_sync(kFull, fin_b));
   }
+}
+
+// ExactMergeGainPersistentImpl by a warp; e(a,b) is read from both rows and
+// must agree.
+__device__ void WarpExactGain(const QuotientView& Q, int a, int b, long long* gain_out, long long* before_out,
+                              GainWork* work, DevError* err) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const long long sa = Q.size[a];
+  const long long sb = Q.size[b];
+  const long long sw = sa + sb;
+  const int la = Q.len[a];
+  const int lb = Q.len[b];
+  MergeTerms T;
+  WarpMergeTerms(Q, a, b, sa, sb, Q.ent + Q.off[a], la, Q.ent + Q.off[b], lb, &T);
+  long long before = T.before, after = T.after, eab_a = T.eab_a, eab_b = T.eab_b;
+  int uni = T.uni, ovl = T.ovl, bad = T.bad;
   before = WarpSum(before);
   after = WarpSum(after);
   // e(a,b) is read by one lane per row (counts < 2^32)
@@ -2254,10 +2268,34 @@ __global__ void __launch_bounds__(kScoreThreads, 4) ScoreKernel(ScoreParams P) {
   }
 }
 
-// Scoring service over an explicit pair list (ScoreCandidatesCuda's role).
+// Scoring service over an explicit pair list (ScoreCandidatesCuda's role), a
+// warp per pair. Pairs whose rows hold more than kPairLong entries together are
+// left to ScoreLongPairsKernel in units of kPairUnit entries of the longer row
+// and the part of the other that these ids span: a hub pair of 100,000 entries
+// is a chain of thousands of steps for one warp, and was the kernel's tail
+// (1.16 ms for 262,144 pairs at R-MAT 20, a tenth of it work).
+constexpr int kPairLong = 2048;
+constexpr int kPairUnit = 1024;
+
+struct PairUnit {
+  long long pair;
+  int at;  // first entry of the longer row
+  int pad;
+};
+
+// The terms of e(a, b) and of the two supernodes themselves.
+__device__ __forceinline__ void PairOwnTerms(const QuotientView& Q, int a, int b, long long eab, long long* before,
+                                             long long* after, int* bad) {
+  const long long sa = Q.size[a], sb = Q.size[b], ia = Q.internal[a], ib = Q.internal[b];
+  *before = BlockCost(sa, sa, ia, true, *bad) + BlockCost(sb, sb, ib, true, *bad) + BlockCost(sa, sb, eab, false, *bad);
+  *after = BlockCost(sa + sb, sa + sb, ia + ib + eab, true, *bad);
+}
+
 __global__ void __launch_bounds__(kScoreThreads) ScorePairsKernel(QuotientView Q, const int* rep_a,
                                                                   const int* rep_b, long long count,
-                                                                  longlong2* res, DevError* err) {
+                                                                  long long* gain_out, long long* before_out,
+                                                                  PairUnit* units, unsigned long long* nunits,
+                                                                  unsigned long long max_units, DevError* err) {
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -2267,13 +2305,78 @@ __global__ void __launch_bounds__(kScoreThreads) ScorePairsKernel(QuotientView Q
     if (a == b || Q.size[a] <= 0 || Q.size[b] <= 0) {
       if (lane == 0) {
         RaiseError(err, kErrInactive, a, b, 0);
-        res[p] = make_longlong2(0, 0);
+        gain_out[p] = 0;
+        before_out[p] = 0;
       }
       continue;
     }
+    const int la = Q.len[a], lb = Q.len[b];
+    if (la + lb > kPairLong) {
+      const int longer = la > lb ? la : lb;
+      const unsigned n = static_cast<unsigned>((longer + kPairUnit - 1) / kPairUnit);
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(nunits, static_cast<unsigned long long>(n));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      for (unsigned k = lane; k < n && at + k < max_units; k += 32) {
+        units[at + k] = PairUnit{at + n <= max_units ? p : -1, static_cast<int>(k) * kPairUnit, 0};
+      }
+      if (at + n <= max_units) {
+        if (lane == 0) {
+          const long long ea = RowLookup(Q.ent + Q.off[a], la, b), eb = RowLookup(Q.ent + Q.off[b], lb, a);
+          long long before, after;
+          int bad = 0;
+          PairOwnTerms(Q, a, b, ea, &before, &after, &bad);
+          if (ea != eb) RaiseError(err, kErrAsymmetric, a, b, 0);
+          if (bad) RaiseError(err, kErrBlockCost, a, b, 0);
+          gain_out[p] = before - after;  // the units add theirs
+          before_out[p] = before;
+        }
+        continue;
+      }
+    }
     long long gain = 0, before = 0;
     WarpExactGain(Q, a, b, &gain, &before, nullptr, err);
-    if (lane == 0) res[p] = make_longlong2(gain, before);
+    if (lane == 0) {
+      gain_out[p] = gain;
+      before_out[p] = before;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kScoreThreads) ScoreLongPairsKernel(QuotientView Q, const int* rep_a,
+                                                                      const int* rep_b, long long* gain_out,
+                                                                      long long* before_out, const PairUnit* units,
+                                                                      const unsigned long long* nunits,
+                                                                      unsigned long long max_units, DevError* err) {
+  const unsigned long long total = *nunits < max_units ? *nunits : max_units;
+  const unsigned long long nw = (static_cast<unsigned long long>(gridDim.x) * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  for (unsigned long long t = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < total;
+       t += nw) {
+    const PairUnit u = units[t];
+    if (u.pair < 0) continue;
+    const int a = rep_a[u.pair], b = rep_b[u.pair];
+    const bool a_long = Q.len[a] >= Q.len[b];
+    const int x = a_long ? a : b, y = a_long ? b : a;
+    const Entry* rx = Q.ent + Q.off[x];
+    const Entry* ry = Q.ent + Q.off[y];
+    const int lx = Q.len[x], ly = Q.len[y];
+    const int end = u.at + kPairUnit < lx ? u.at + kPairUnit : lx;
+    // ids from the unit's first (the first unit: from the start) up to the
+    // next unit's first (the last unit: to the end)
+    int edge = 0;
+    if (lane == 0 && u.at > 0) edge = RowLowerBound(ry, ly, EntNb(rx[u.at]));
+    if (lane == 1) edge = end < lx ? RowLowerBound(ry, ly, EntNb(rx[end])) : ly;
+    const int y0 = __shfl_sync(0xffffffffu, edge, 0), y1 = __shfl_sync(0xffffffffu, edge, 1);
+    MergeTerms T;
+    WarpMergeTerms(Q, x, y, Q.size[x], Q.size[y], rx + u.at, end - u.at, ry + y0, y1 - y0, &T);
+    const long long before = WarpSum(T.before), after = WarpSum(T.after);
+    const bool bad = __any_sync(0xffffffffu, T.bad);
+    if (lane == 0) {
+      atomicAdd(reinterpret_cast<unsigned long long*>(&gain_out[u.pair]), static_cast<unsigned long long>(before - after));
+      atomicAdd(reinterpret_cast<unsigned long long*>(&before_out[u.pair]), static_cast<unsigned long long>(before));
+      if (bad) RaiseError(err, kErrBlockCost, a, b, 0);
+    }
   }
 }
 
@@ -4853,35 +4956,35 @@ void Engine::ScorePairs(const int32_t* rep_a, const int32_t* rep_b, int64_t coun
                         int64_t* before) {
   AllocScope alloc(stream_);
   if (count <= 0) return;
+  uint32_t largest = 0;  // a negative id is a large one
   for (int64_t i = 0; i < count; ++i) {
-    if (rep_a[i] < 0 || rep_a[i] >= n_ || rep_b[i] < 0 || rep_b[i] >= n_) {
-      throw std::out_of_range("quotient supernode is out of range");
-    }
+    largest = std::max(largest, std::max(static_cast<uint32_t>(rep_a[i]), static_cast<uint32_t>(rep_b[i])));
   }
+  if (largest >= static_cast<uint32_t>(n_)) throw std::out_of_range("quotient supernode is out of range");
+  const size_t uc = static_cast<size_t>(count);
+  const unsigned long long max_units = 1ull << 20;  // longer pairs beyond these are one warp's work
   DevBuf<int> da, db;
-  DevBuf<longlong2> dr;
-  da.ensure(static_cast<size_t>(count));
-  db.ensure(static_cast<size_t>(count));
-  dr.ensure(static_cast<size_t>(count));
-  CheckCuda(cudaMemcpyAsync(da.p, rep_a, sizeof(int) * static_cast<size_t>(count), cudaMemcpyHostToDevice, stream_),
-            "h2d pairs");
-  CheckCuda(cudaMemcpyAsync(db.p, rep_b, sizeof(int) * static_cast<size_t>(count), cudaMemcpyHostToDevice, stream_),
-            "h2d pairs");
+  DevBuf<long long> dg;
+  DevBuf<unsigned char> du;
+  da.ensure(uc);
+  db.ensure(uc);
+  dg.ensure(2 * uc + 1);
+  du.ensure(sizeof(PairUnit) * max_units);
+  CheckCuda(cudaMemcpyAsync(da.p, rep_a, sizeof(int) * uc, cudaMemcpyHostToDevice, stream_), "h2d pairs");
+  CheckCuda(cudaMemcpyAsync(db.p, rep_b, sizeof(int) * uc, cudaMemcpyHostToDevice, stream_), "h2d pairs");
+  unsigned long long* nunits = reinterpret_cast<unsigned long long*>(dg.p + 2 * uc);
+  CheckCuda(cudaMemsetAsync(nunits, 0, sizeof(unsigned long long), stream_), "memset units");
   const int blocks = static_cast<int>(std::min<int64_t>((count + 7) / 8, 152 * 16));
-  ++launches_;
-  ScorePairsKernel<<<blocks, 256, 0, stream_>>>(View(), da.p, db.p, count, dr.p, d_err_.p);
-  std::vector<longlong2> h(static_cast<size_t>(count));
-  CheckCuda(cudaMemcpyAsync(h.data(), dr.p, sizeof(longlong2) * static_cast<size_t>(count), cudaMemcpyDeviceToHost,
-                            stream_), "d2h results");
+  PairUnit* units = reinterpret_cast<PairUnit*>(du.p);
+  launches_ += 2;
+  ScorePairsKernel<<<blocks, kScoreThreads, 0, stream_>>>(View(), da.p, db.p, count, dg.p, dg.p + uc, units, nunits,
+                                                          max_units, d_err_.p);
+  ScoreLongPairsKernel<<<152 * 6, kScoreThreads, 0, stream_>>>(View(), da.p, db.p, dg.p, dg.p + uc, units, nunits,
+                                                               max_units, d_err_.p);
+  CheckCuda(cudaMemcpyAsync(gain, dg.p, sizeof(int64_t) * uc, cudaMemcpyDeviceToHost, stream_), "d2h gains");
+  CheckCuda(cudaMemcpyAsync(before, dg.p + uc, sizeof(int64_t) * uc, cudaMemcpyDeviceToHost, stream_), "d2h costs");
   CheckCuda(cudaStreamSynchronize(stream_), "score sync");
-  da.release();
-  db.release();
-  dr.release();
   CheckError();
-  for (int64_t i = 0; i < count; ++i) {
-    gain[i] = h[static_cast<size_t>(i)].x;
-    before[i] = h[static_cast<size_t>(i)].y;
-  }
 }
 
 int64_t Engine::PrepareGroup(const int32_t* q, int g, int32_t* a_idx, int32_t* b_idx, int64_t cap) {

@@ -45,3 +45,31 @@ def test_hub_row_after_merges(length, kind):
         assert np.array_equal(got_nb, ids)
         assert np.array_equal(got_cnt, counts)
         e.validate_quotient()
+
+
+@pytest.mark.parametrize("longer,shorter,tied", [(1024, 1024, False), (1025, 1024, True), (2048, 1, False),
+                                                 (2049, 0, False), (3072, 3072, True), (3073, 700, True),
+                                                 (9001, 5000, True)])
+def test_scores_of_long_pairs(longer, shorter, tied):
+    """ScorePairsKernel's pairs in units (ScoreLongPairsKernel) against the
+    oracle, around the length limit and the unit; some neighbours merged."""
+    from beam_gb300 import Engine, Graph
+    from oracle import Oracle
+    rng = np.random.default_rng(longer + shorter)
+    n = 3 + longer + shorter
+    u = [np.full(longer, 0), np.full(shorter, 1), [2]]
+    v = [3 + rng.choice(n - 3, longer, replace=False), 3 + rng.choice(n - 3, shorter, replace=False), [3]]
+    if tied:
+        u.append([0])
+        v.append([1])
+    g = Graph.from_edges(np.concatenate(u).astype(np.int32), np.concatenate(v).astype(np.int32))
+    o = Oracle.from_graph(g)
+    with Engine(g) as e:
+        ends = 3 + rng.permutation(g.n - 3)[:40]
+        for k, r in zip(ends[:20].tolist(), ends[20:].tolist()):
+            o.merge_pair(k, r)
+        e.merge_pairs(ends[:20], ends[20:])
+        pairs = [(0, 1), (1, 0), (0, 2), (2, 1), (0, int(ends[0])), (int(ends[3]), 1)]
+        gain, before = e.score_pairs([a for a, _ in pairs], [b for _, b in pairs])
+        for i, (a, b) in enumerate(pairs):
+            assert (gain[i], before[i]) == o.exact_gain(a, b), (a, b)
