@@ -615,9 +615,10 @@ void Engine::Divide(int iter) {
                               cudaMemcpyDeviceToDevice, s), "copy glen");
   }
   n_groups_ = segs;
-  // one block of every group: Merge plans the iteration on the device from
-  // d_glen_ / d_gent_, so nothing is read back here
-  plan_on_device_ = static_cast<long long>(cfg_.group_batch_size) >= static_cast<long long>(segs);
+  // large blocks: Merge plans the iteration on the device from d_glen_ /
+  // d_gent_, so nothing is read back here
+  plan_on_device_ = cfg_.group_batch_size >= kDevicePlanGroups ||
+                    static_cast<long long>(cfg_.group_batch_size) >= static_cast<long long>(segs);
   windowed_ = !plan_on_device_ && WindowsOn();
   if (!plan_on_device_ && !windowed_) {
     h_glen_.resize(static_cast<size_t>(segs));

@@ -46,6 +46,8 @@ struct RankerInfo {
 // Largest group the kernels accept (bounded by the packed select keys and
 // the per-group pair tables); the reference default is 512.
 constexpr int kMaxGroup = 1024;
+// Blocks of at least this many groups are planned on the device.
+constexpr int kDevicePlanGroups = 1024;
 // Persistent grid of the row-update kernels (four CTAs per SM of a GB300).
 constexpr int kRowsGrid = 4 * 152;
 
@@ -152,11 +154,10 @@ struct BlockPlan {
   long long slots = 0, sel_slots = 0;   // candidate / selection slots
   int s0 = 0, s1 = 0, b0 = 0, b1 = 0;   // small / big prepare list ranges
   int m0 = 0, m1 = 0;                   // medium groups handled by one kernel
-  bool fused = false;                   // whether there may be any
+  bool by_lists = false;                // selection by the lists whatever the number of groups
   long long members = 0;                // members of the big groups
   long long slot0 = 0, nslots = 0;      // sort slots of the deferred big groups
-  long long max_e = 0;                  // largest deferred group's row entries
-  long long mat_bytes = 0;              // pair tables of the big groups
+  long long mat0 = 0, mat_bytes = 0;    // pair tables of the big groups
   int ss0 = 0, ss1 = 0, sm0 = 0, sm1 = 0, sb0 = 0, sb1 = 0;  // select list ranges
 };
 
@@ -354,7 +355,7 @@ class Engine {
   DevBuf<unsigned char> d_gs_, d_wctl_, d_units_, d_win_big_;
   int accum_grid_ = 152 * 4;  // resident CTAs of the dynamically scheduled kernels
   int score_grid_ = 152 * 4;   // one-block iteration: Merge plans it on the device
-  DevBuf<unsigned char> d_plan_tiles_;
+  DevBuf<unsigned char> d_plan_tiles_, d_plan_blocks_;
   DevBuf<long long> d_plan_scalars_;
   PinnedBuf<long long> h_pin_;
   int block_stamp_ = 0;

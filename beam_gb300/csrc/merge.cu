@@ -3875,7 +3875,7 @@ constexpr int kPlanThreads = 256;
 constexpr int kPlanItems = 8;
 constexpr int kPlanTile = kPlanThreads * kPlanItems;
 enum PlanScalar : int {
-  kPlanR = 0, kPlanCand, kPlanSel, kPlanSmall, kPlanBig, kPlanMembers, kPlanSlots, kPlanMat, kPlanMaxE,
+  kPlanR = 0, kPlanCand, kPlanSel, kPlanSmall, kPlanBig, kPlanMembers, kPlanSlots, kPlanMat,
   kPlanSelSmall, kPlanSelMid, kPlanSelBig, kPlanMed, kPlanSmallBase, kPlanScalars = kPlanSmallBase + 4
 };
 // The small-group list is laid out by member count, largest class first
@@ -3925,7 +3925,7 @@ __device__ __forceinline__ PlanSums PlanZero() {
 }
 
 // one group's contribution: the same rules as the host plan
-__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, int mode) {
+__device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, int mode, int one_class) {
   PlanSums f = PlanZero();
   if (g < 2) return f;
   const long long gl = g;
@@ -3934,7 +3934,7 @@ __device__ __forceinline__ PlanSums PlanOfGroup(int g, unsigned e, long long k, 
   f.sel = gl / 2;
   const bool windowed = mode == kPlanWindows;
   if (windowed ? WindowSmall(g, e) : g <= kSmallGroup && e <= static_cast<unsigned>(kSmallStage)) {
-    f.small[SmallClass(g)] = 1;
+    f.small[one_class ? 0 : SmallClass(g)] = 1;
   } else if (mode == kPlanFused && MediumFits(g, e)) {
     f.med = 1;  // with its selection
     return f;
@@ -3976,6 +3976,11 @@ struct PlanParams {
   int* sel_small;
   int* sel_mid;
   int* sel_big;
+  // several blocks: the sums before each block's first group, and the small
+  // groups in one class, so that every list is in group order
+  PlanSums* block_sums;
+  long long batch;
+  int one_class;
   int* ri_of;  // per Divide group: its position, -1 for a group of one (nullptr: not needed)
 };
 
@@ -3984,19 +3989,14 @@ __global__ void __launch_bounds__(kPlanThreads) PlanTileKernel(PlanParams P) {
   __shared__ typename Reduce::TempStorage tmp;
   const long long base = static_cast<long long>(blockIdx.x) * kPlanTile + threadIdx.x * kPlanItems;
   PlanSums acc = PlanZero();
-  long long max_e = 0;
   for (int j = 0; j < kPlanItems; ++j) {
     const long long gi = base + j;
     if (gi >= P.G) break;
-    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k, P.mode);
+    const PlanSums f = PlanOfGroup(P.glen[gi], P.gent[gi], P.top_k, P.mode, P.one_class);
     acc = PlanSumOp()(acc, f);
-    max_e = f.soff > max_e ? f.soff : max_e;
   }
   const PlanSums t = Reduce(tmp).Reduce(acc, PlanSumOp());
   if (threadIdx.x == 0) P.tile_sums[blockIdx.x] = t;
-  if (max_e > 0) {
-    atomicMax(reinterpret_cast<unsigned long long*>(P.scalars + kPlanMaxE), static_cast<unsigned long long>(max_e));
-  }
 }
 
 // one CTA: exclusive offsets of the tiles, the totals, and the closing
@@ -4058,13 +4058,14 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
     const long long gi = base + j;
     g[j] = gi < P.G ? P.glen[gi] : 0;
     e[j] = gi < P.G ? P.gent[gi] : 0u;
-    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k, P.mode));
+    acc = PlanSumOp()(acc, PlanOfGroup(g[j], e[j], P.top_k, P.mode, P.one_class));
   }
   PlanSums off;
   Scan(tmp).ExclusiveScan(acc, off, P.tile_off[blockIdx.x], PlanSumOp());
 #pragma unroll
   for (int j = 0; j < kPlanItems; ++j) {
-    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k, P.mode);
+    const PlanSums f = PlanOfGroup(g[j], e[j], P.top_k, P.mode, P.one_class);
+    if (P.block_sums && base + j < P.G && (base + j) % P.batch == 0) P.block_sums[(base + j) / P.batch] = off;
     if (P.ri_of && base + j < P.G) P.ri_of[base + j] = f.real ? off.real : -1;
     if (f.real) {
       const int ri = off.real;
@@ -4075,7 +4076,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
       if (f.med) {
         P.med[off.med] = ri;
       } else if (!f.big) {
-        const int c = SmallClass(g[j]);
+        const int c = P.one_class ? 0 : SmallClass(g[j]);
         P.small[P.scalars[kPlanSmallBase + c] + off.small[c]] = ri;
       } else {
         P.big[off.big] = ri;
@@ -4101,7 +4102,9 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
 // or the exact gain needs the rows again.
 bool Engine::FusedOn() const { return RowSumsOn() && !cfg_.ranker; }
 
-bool Engine::PlanFused() const { return FusedOn() && n_groups_ >= kMedMinAll; }
+bool Engine::PlanFused() const {
+  return FusedOn() && std::min<long long>(cfg_.group_batch_size, n_groups_) >= kMedMinAll;
+}
 
 void Engine::PrepareIterationBuffers() {
   const int64_t G = n_groups_;
@@ -4281,15 +4284,12 @@ void Engine::PrepareIterationBuffers() {
     bp.s1 = h_block_small_[b + 1];
     bp.m0 = h_block_med_[b];
     bp.m1 = h_block_med_[b + 1];
-    bp.fused = h_block_fused_[b] != 0;
+    bp.by_lists = h_block_fused_[b] != 0;
     bp.b0 = h_block_big_[b];
     bp.b1 = h_block_big_[b + 1];
     bp.members = h_big_moff_[static_cast<size_t>(bp.b1)] - h_big_moff_[static_cast<size_t>(bp.b0)];
     bp.slot0 = h_soff_[static_cast<size_t>(bp.b0)];
     bp.nslots = h_soff_[static_cast<size_t>(bp.b1)] - bp.slot0;
-    for (int i = bp.b0; i < bp.b1; ++i) {
-      bp.max_e = std::max(bp.max_e, h_soff_[static_cast<size_t>(i) + 1] - h_soff_[static_cast<size_t>(i)]);
-    }
     bp.mat_bytes = block_mat[b];
     bp.ss0 = h_block_sel_small_[b];
     bp.ss1 = h_block_sel_small_[b + 1];
@@ -4341,9 +4341,12 @@ void Engine::SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nb
   rk_iter_slots_ = static_cast<long long>(ncand);
 }
 
-// The plan of a one-block iteration, made on the device from the Divide
-// output (the same lists and offsets as PrepareIterationBuffers); one small
-// read-back brings the totals and the entry-pool top to the host.
+// The plan of an iteration of one block, or of several of at least
+// kDevicePlanGroups groups, made on the device from the Divide output (the same
+// lists and offsets as PrepareIterationBuffers); one small read-back brings the
+// totals, the sums at the blocks' borders and the entry-pool top to the host.
+// (Planned on the host, an iteration of 1.7 million groups read 13.5 MB back and
+// spent 5 ms in loops with the GPU idle.)
 void Engine::PlanOnDevice() {
   const long long G = n_groups_;
   const size_t cap = static_cast<size_t>(G) + 1;
@@ -4375,6 +4378,15 @@ void Engine::PlanOnDevice() {
   P.sel_small = d_sel_small_.p;
   P.sel_mid = d_sel_mid_.p;
   P.sel_big = d_sel_big_.p;
+  const long long batch = cfg_.group_batch_size;
+  const long long blocks = windowed_ ? 1 : (G + batch - 1) / batch;
+  P.block_sums = nullptr;
+  P.batch = batch;
+  P.one_class = blocks > 1 ? 1 : 0;
+  if (blocks > 1) {
+    d_plan_blocks_.ensure(sizeof(PlanSums) * static_cast<size_t>(blocks));
+    P.block_sums = reinterpret_cast<PlanSums*>(d_plan_blocks_.p);
+  }
   P.ri_of = nullptr;
   if (windowed_) {
     d_ri_of_.ensure(cap);
@@ -4396,30 +4408,66 @@ void Engine::PlanOnDevice() {
                             stream_), "d2h plan");
   CheckCuda(cudaMemcpyAsync(hs + kPlanScalars, d_pool_top_.p, sizeof(long long), cudaMemcpyDeviceToHost, stream_),
             "d2h pool top");
+  std::vector<PlanSums> sums(static_cast<size_t>(blocks) + 1);
+  if (blocks > 1) {
+    CheckCuda(cudaMemcpyAsync(sums.data(), d_plan_blocks_.p, sizeof(PlanSums) * static_cast<size_t>(blocks),
+                              cudaMemcpyDeviceToHost, stream_), "d2h block plan");
+  }
   CheckCuda(cudaStreamSynchronize(stream_), "plan sync");
   CheckError();
   long long v[kPlanScalars + 1];
   std::memcpy(v, hs, sizeof(v));
   EnsurePoolRoom(static_cast<unsigned long long>(v[kPlanScalars]));
   const size_t R = static_cast<size_t>(v[kPlanR]);
+  if (blocks <= 1) sums[0] = PlanSums{};
+  PlanSums& end = sums[static_cast<size_t>(std::max(blocks, 1ll))];
+  end = PlanSums{};
+  end.real = static_cast<int>(R);
+  end.cand = v[kPlanCand];
+  end.sel = v[kPlanSel];
+  end.small[0] = static_cast<int>(v[kPlanSmall]);
+  end.med = static_cast<int>(v[kPlanMed]);
+  end.big = static_cast<int>(v[kPlanBig]);
+  end.moff = v[kPlanMembers];
+  end.soff = v[kPlanSlots];
+  end.mat = v[kPlanMat];
+  end.ssmall = static_cast<int>(v[kPlanSelSmall]);
+  end.smid = static_cast<int>(v[kPlanSelMid]);
+  end.sbig = static_cast<int>(v[kPlanSelBig]);
+  plans_.clear();
+  long long max_mat = 0, max_slots = 0;
+  for (size_t i = 0; i + 1 < sums.size(); ++i) {
+    const PlanSums& p = sums[i];
+    const PlanSums& q = sums[i + 1];
+    BlockPlan bp;
+    bp.rg0 = p.real;
+    bp.rg1 = q.real;
+    bp.slots = q.cand - p.cand;
+    bp.sel_slots = q.sel - p.sel;
+    bp.s0 = p.small[0];
+    bp.s1 = q.small[0];
+    bp.m0 = p.med;
+    bp.m1 = q.med;
+    bp.b0 = p.big;
+    bp.b1 = q.big;
+    bp.by_lists = blocks > 1 || PlanFused();
+    bp.members = q.moff - p.moff;
+    bp.slot0 = p.soff;
+    bp.nslots = q.soff - p.soff;
+    bp.mat0 = p.mat;
+    bp.mat_bytes = q.mat - p.mat;
+    bp.ss0 = p.ssmall;
+    bp.ss1 = q.ssmall;
+    bp.sm0 = p.smid;
+    bp.sm1 = q.smid;
+    bp.sb0 = p.sbig;
+    bp.sb1 = q.sbig;
+    max_mat = std::max(max_mat, bp.mat_bytes);
+    max_slots = std::max(max_slots, bp.nslots);
+    plans_.push_back(bp);
+  }
   SizeIterationBuffers(R, static_cast<size_t>(v[kPlanCand]), static_cast<size_t>(v[kPlanSel]),
-                       static_cast<size_t>(v[kPlanBig]), v[kPlanMat], v[kPlanSlots], windowed_);
-  BlockPlan bp;
-  bp.rg1 = static_cast<int>(R);
-  bp.slots = v[kPlanCand];
-  bp.sel_slots = v[kPlanSel];
-  bp.s1 = static_cast<int>(v[kPlanSmall]);
-  bp.m1 = static_cast<int>(v[kPlanMed]);
-  bp.b1 = static_cast<int>(v[kPlanBig]);
-  bp.fused = PlanFused();
-  bp.members = v[kPlanMembers];
-  bp.nslots = v[kPlanSlots];
-  bp.max_e = v[kPlanMaxE];
-  bp.mat_bytes = v[kPlanMat];
-  bp.ss1 = static_cast<int>(v[kPlanSelSmall]);
-  bp.sm1 = static_cast<int>(v[kPlanSelMid]);
-  bp.sb1 = static_cast<int>(v[kPlanSelBig]);
-  plans_.assign(1, bp);
+                       static_cast<size_t>(v[kPlanBig]), max_mat, max_slots, windowed_);
 }
 
 QuotientView Engine::View() {
@@ -4552,7 +4600,8 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
   PP.cand = d_cand_.p;
   PP.cand_cnt = d_cand_cnt_.p;
   PP.mat_off = d_mat_off_.p;
-  PP.mat = d_mat_.p;
+  // the block's pair tables start at the buffer's start
+  PP.mat = reinterpret_cast<unsigned char*>(reinterpret_cast<uintptr_t>(d_mat_.p) - static_cast<uintptr_t>(bp.mat0));
   PP.mat_zeroed = 0;
   PP.rc = nullptr;
   PP.info = nullptr;
@@ -4765,7 +4814,7 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
   LP.sel_list = d_sel_list_.p;
   const int ss0 = bp.ss0, ss1 = bp.ss1;
   const int sb0 = bp.sb0, sb1 = bp.sb1;
-  if (nrg <= kFewGroups && !bp.fused) {
+  if (nrg <= kFewGroups && !bp.by_lists) {
     // a small block: one launch, a CTA per group (same selection)
     LP.list = nullptr;
     LP.list0 = rg0;
