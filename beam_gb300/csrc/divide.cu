@@ -33,6 +33,7 @@ namespace beam {
 namespace {
 
 __global__ void ActiveFlagsKernel(const int* __restrict__ qsize, int n, int* __restrict__ flags) {
+  FollowsOn();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) flags[i] = qsize[i] > 0 ? 1 : 0;
 }
@@ -40,6 +41,7 @@ __global__ void ActiveFlagsKernel(const int* __restrict__ qsize, int n, int* __r
 // order[scan[i]] = i for active reps; scan is exclusive.
 __global__ void ScatterActiveKernel(const int* __restrict__ qsize, const int* __restrict__ scan, int n,
                                     int* __restrict__ order, int* __restrict__ head_flag) {
+  FollowsOn();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && qsize[i] > 0) {
     const int p = scan[i];
@@ -52,12 +54,14 @@ __global__ void ScatterActiveKernel(const int* __restrict__ qsize, const int* __
 // position, start per segment.
 __global__ void SegStartsKernel(const int* __restrict__ head_flag, const int* __restrict__ incl, int count,
                                 int* __restrict__ seg_start) {
+  FollowsOn();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < count && head_flag[p]) seg_start[incl[p] - 1] = p;
 }
 
 __global__ void SegLenKernel(const int* __restrict__ seg_start, int segs, int count, int max_group,
                              int* __restrict__ seg_len, int* __restrict__ unf_flag, int* __restrict__ unf_len) {
+  FollowsOn();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < segs) {
     const int end = s + 1 < segs ? seg_start[s + 1] : count;
@@ -78,6 +82,7 @@ __global__ void SegLenKernel(const int* __restrict__ seg_start, int segs, int co
 __global__ void SegLenAllKernel(const int* __restrict__ seg_start, const int* __restrict__ segs_p, int count,
                                 int max_group, int* __restrict__ seg_len, int* __restrict__ unf_flag,
                                 unsigned long long* __restrict__ unf_pk) {
+  FollowsOn();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= count) return;
   const int segs = *segs_p;
@@ -102,6 +107,7 @@ __global__ void SegLenAllKernel(const int* __restrict__ seg_start, const int* __
 __global__ void DepthZeroKernel(int count, int max_group, int* __restrict__ incl, int* __restrict__ seg_start,
                                 int* __restrict__ seg_len, int* __restrict__ unf_flag,
                                 unsigned long long* __restrict__ unf_ex) {
+  FollowsOn();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= count) return;
   incl[p] = 1;
@@ -116,6 +122,7 @@ __global__ void DepthZeroKernel(int count, int max_group, int* __restrict__ incl
 
 __global__ void DepthCountsKernel(const int* __restrict__ incl_last, const unsigned long long* __restrict__ ex_last,
                                   const unsigned long long* __restrict__ pk_last, int* __restrict__ out) {
+  FollowsOn();
   const unsigned long long total = *ex_last + *pk_last;
   out[0] = *incl_last;
   out[1] = static_cast<int>(total >> 32);
@@ -129,6 +136,7 @@ __global__ void CompactItemsKernel(const int* __restrict__ incl, const int* __re
                                    const unsigned long long* __restrict__ unf_ex, int count,
                                    int* __restrict__ pos_map, int* __restrict__ item_seg,
                                    int* __restrict__ ubeg, int* __restrict__ uend) {
+  FollowsOn();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= count) return;
   const int s = incl[p] - 1;
@@ -147,6 +155,7 @@ __global__ void CompactItemsKernel(const int* __restrict__ incl, const int* __re
 
 __global__ void MarkNeedKernel(const int* __restrict__ order, const int* __restrict__ pos_map, int items,
                                int* __restrict__ need, int stamp, unsigned long long* __restrict__ hash) {
+  FollowsOn();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < items) {
     const int rep = order[pos_map[k]];
@@ -172,6 +181,7 @@ __global__ void __launch_bounds__(256) MinHashKernel(const int* __restrict__ arc
                                                      long long arcs, int n, int stamp, uint64_t base,
                                                      unsigned long long* __restrict__ hash,
                                                      unsigned long long* __restrict__ stats) {
+  FollowsOn();
   const long long total = arcs + n;
   // algorithmic bytes of one dimension: per arc its source, the source's
   // label and its need stamp (12 B), per node its label and stamp (8 B), and
@@ -228,6 +238,7 @@ __global__ void GatherKeysKernel(const int* __restrict__ order, const int* __res
                                  const unsigned long long* __restrict__ hash, int fallback, uint64_t seed,
                                  int iter, unsigned long long* __restrict__ keys, unsigned* __restrict__ keys_hi,
                                  int* __restrict__ vals) {
+  FollowsOn();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < items) {
     const int rep = order[pos_map[k]];
@@ -239,12 +250,14 @@ __global__ void GatherKeysKernel(const int* __restrict__ order, const int* __res
 }
 
 __global__ void IotaKernel(int* __restrict__ out, int items) {
+  FollowsOn();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < items) out[k] = k;
 }
 
 __global__ void SegKeyKernel(const int* __restrict__ item_seg, const int* __restrict__ perm, int items,
                              int* __restrict__ segkey) {
+  FollowsOn();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < items) segkey[j] = item_seg[perm[j]];
 }
@@ -252,6 +265,7 @@ __global__ void SegKeyKernel(const int* __restrict__ item_seg, const int* __rest
 __global__ void GatherSortedKernel(const int* __restrict__ perm, int items, const unsigned long long* __restrict__ keys,
                                    const int* __restrict__ vals, unsigned long long* __restrict__ keys_out,
                                    int* __restrict__ vals_out) {
+  FollowsOn();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < items) {
     keys_out[j] = keys[perm[j]];
@@ -269,6 +283,7 @@ __global__ void GatherSortedKernel(const int* __restrict__ perm, int items, cons
 __global__ void MixedRunsKernel(const unsigned long long* __restrict__ keys, const int* __restrict__ item_seg,
                                 const int* __restrict__ ubeg, int items, int* __restrict__ list,
                                 int* __restrict__ cnt) {
+  FollowsOn();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x + 1; j < items; j += gridDim.x * blockDim.x) {
     const unsigned long long kj = keys[j];
     const unsigned long long kp = keys[j - 1];
@@ -301,6 +316,7 @@ __global__ void __launch_bounds__(256) SortMixedRunsKernel(unsigned long long* _
                                                            const int* __restrict__ uend, const int* __restrict__ list,
                                                            const int* __restrict__ cnt,
                                                            unsigned long long* __restrict__ tk, int* __restrict__ tv) {
+  FollowsOn();
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -369,6 +385,7 @@ __global__ void ScatterSortedKernel(const int* __restrict__ pos_map, const int* 
                                     const unsigned long long* __restrict__ keys, const int* __restrict__ vals,
                                     int fallback, int max_group, int* __restrict__ order,
                                     int* __restrict__ head_flag) {
+  FollowsOn();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= items) return;
   const int p = pos_map[k];
@@ -385,6 +402,7 @@ __global__ void GroupInfoKernel(const int* __restrict__ order, const int* __rest
                                 int* __restrict__ group_of, int* __restrict__ idx_in_group,
                                 const int* __restrict__ qlen, unsigned* __restrict__ gent,
                                 unsigned long long* __restrict__ stats) {
+  FollowsOn();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= count) return;
   const int s = incl[p] - 1;
@@ -458,11 +476,11 @@ void Engine::Divide(int iter) {
 
   // Active supernodes in ascending id order.
   ++launches_;
-  ActiveFlagsKernel<<<Blocks(n, T), T, 0, s>>>(d_qsize_.p, n, flags);
+  LaunchFollowing(ActiveFlagsKernel, Blocks(n, T), T, 0, s, d_qsize_.p, n, flags);
   scan_excl(flags, scan, n);
   CheckCuda(cudaMemsetAsync(d_head_flag_.p, 0, sizeof(int) * static_cast<size_t>(n), s), "memset");
   ++launches_;
-  ScatterActiveKernel<<<Blocks(n, T), T, 0, s>>>(d_qsize_.p, scan, n, d_order_.p, d_head_flag_.p);
+  LaunchFollowing(ScatterActiveKernel, Blocks(n, T), T, 0, s, d_qsize_.p, scan, n, d_order_.p, d_head_flag_.p);
   // active supernodes: known on the host after a Merge (n - accepted
   // merges, read back with the Merge's final synchronisation), else read
   int count = 0;
@@ -492,15 +510,15 @@ void Engine::Divide(int iter) {
       const bool fallback = depth == cfg_.divide_hash_dims;
       if (depth == 0) {
         ++launches_;
-        DepthZeroKernel<<<Blocks(count, T), T, 0, s>>>(count, cfg_.divide_max_group, scan, seg_start, seg_len,
-                                                       unf_flag, unf_ex);
+        LaunchFollowing(DepthZeroKernel, Blocks(count, T), T, 0, s, count, cfg_.divide_max_group, scan, seg_start,
+                        seg_len, unf_flag, unf_ex);
       } else {
         scan_incl(d_head_flag_.p, scan, count);
         ++launches_;
-        SegStartsKernel<<<Blocks(count, T), T, 0, s>>>(d_head_flag_.p, scan, count, seg_start);
+        LaunchFollowing(SegStartsKernel, Blocks(count, T), T, 0, s, d_head_flag_.p, scan, count, seg_start);
         ++launches_;
-        SegLenAllKernel<<<Blocks(count, T), T, 0, s>>>(seg_start, scan + count - 1, count, cfg_.divide_max_group,
-                                                       seg_len, unf_flag, unf_pk);
+        LaunchFollowing(SegLenAllKernel, Blocks(count, T), T, 0, s, seg_start, scan + count - 1, count,
+                        cfg_.divide_max_group, seg_len, unf_flag, unf_pk);
         size_t pk_bytes = 0;
         CheckCuda(cub::DeviceScan::ExclusiveSum(nullptr, pk_bytes, unf_pk, unf_ex, count, s), "cub scan size");
         d_cub_tmp_.ensure(pk_bytes);
@@ -517,7 +535,7 @@ void Engine::Divide(int iter) {
       } else {
         int* dc = uend + n;
         ++launches_;
-        DepthCountsKernel<<<1, 1, 0, s>>>(scan + count - 1, unf_ex + count - 1, unf_pk + count - 1, dc);
+        LaunchFollowing(DepthCountsKernel, 1, 1, 0, s, scan + count - 1, unf_ex + count - 1, unf_pk + count - 1, dc);
         CheckCuda(cudaMemcpyAsync(h_pin_.p, dc, 3 * sizeof(int), cudaMemcpyDeviceToHost, s), "d2h depth counts");
         CheckCuda(cudaStreamSynchronize(s), "sync");
         std::memcpy(hc, h_pin_.p, sizeof(hc));
@@ -530,29 +548,29 @@ void Engine::Divide(int iter) {
       }
       const int items = hc[2];
       ++launches_;
-      CompactItemsKernel<<<Blocks(count, T), T, 0, s>>>(scan, seg_start, seg_len, unf_flag, unf_ex, count,
-                                                        d_pos_map_.p, item_seg, ubeg, uend);
+      LaunchFollowing(CompactItemsKernel, Blocks(count, T), T, 0, s, scan, seg_start, seg_len, unf_flag, unf_ex,
+                      count, d_pos_map_.p, item_seg, ubeg, uend);
       if (fallback) {
         hstats_.divide_fallback_splits += static_cast<uint64_t>(nu);
       } else {
         ++need_stamp_;
         ++launches_;
-        MarkNeedKernel<<<Blocks(items, T), T, 0, s>>>(d_order_.p, d_pos_map_.p, items, d_need_.p, need_stamp_,
-                                                      d_hash_.p);
+        LaunchFollowing(MarkNeedKernel, Blocks(items, T), T, 0, s, d_order_.p, d_pos_map_.p, items, d_need_.p,
+                        need_stamp_, d_hash_.p);
         const uint64_t base = HashRankBase(cfg_.seed, dim_order[static_cast<size_t>(depth)], iter);
         BeginTimed(kTimeDivide);
         ++launches_;
-        MinHashKernel<<<152 * 8, 256, 0, s>>>(d_arc_src_.p, d_col_.p, d_label_.p, d_need_.p, arcs_, n,
+        LaunchFollowing(MinHashKernel, 152 * 8, 256, 0, s, d_arc_src_.p, d_col_.p, d_label_.p, d_need_.p, arcs_, n,
                                               need_stamp_, base, d_hash_.p, d_stats_.p);
         EndTimed(kTimeDivide);
       }
       ++launches_;
-      GatherKeysKernel<<<Blocks(items, T), T, 0, s>>>(d_order_.p, d_pos_map_.p, items, d_hash_.p, fallback ? 1 : 0,
-                                                      cfg_.seed, iter, d_keys_.p, d_keys_hi_[0].p, d_vals_.p);
+      LaunchFollowing(GatherKeysKernel, Blocks(items, T), T, 0, s, d_order_.p, d_pos_map_.p, items, d_hash_.p,
+                      fallback ? 1 : 0, cfg_.seed, iter, d_keys_.p, d_keys_hi_[0].p, d_vals_.p);
       // (segment, key) order, stable on the rep order inside each segment:
       // a stable LSD radix sort by key, then a stable one by segment index.
       ++launches_;
-      IotaKernel<<<Blocks(items, T), T, 0, s>>>(d_perm_.p, items);
+      LaunchFollowing(IotaKernel, Blocks(items, T), T, 0, s, d_perm_.p, items);
       size_t bytes = 0;
       // by the high key words (equal-high runs are put in key order below;
       // the full keys follow the permutation in GatherSortedKernel)
@@ -566,7 +584,7 @@ void Engine::Divide(int iter) {
         int bits = 1;
         while ((1 << bits) < nu) ++bits;
         ++launches_;
-        SegKeyKernel<<<Blocks(items, T), T, 0, s>>>(item_seg, d_perm_alt_.p, items, d_segkey_.p);
+        LaunchFollowing(SegKeyKernel, Blocks(items, T), T, 0, s, item_seg, d_perm_alt_.p, items, d_segkey_.p);
         bytes = 0;
         CheckCuda(cub::DeviceRadixSort::SortPairs(nullptr, bytes, d_segkey_.p, d_segkey_alt_.p, d_perm_alt_.p,
                                                   d_perm_.p, items, 0, bits, s), "cub radix sort size");
@@ -576,39 +594,40 @@ void Engine::Divide(int iter) {
         perm = d_perm_.p;
       }
       ++launches_;
-      GatherSortedKernel<<<Blocks(items, T), T, 0, s>>>(perm, items, d_keys_.p, d_vals_.p, d_keys_alt_.p,
+      LaunchFollowing(GatherSortedKernel, Blocks(items, T), T, 0, s, perm, items, d_keys_.p, d_vals_.p, d_keys_alt_.p,
                                                         d_vals_alt_.p);
       // runs of equal high words with mixed low words into full-key order
       // (d_keys_ / d_vals_ are free once gathered)
       ++launches_;
       CheckCuda(cudaMemsetAsync(fix_cnt, 0, sizeof(int), s), "memset mixed-run counter");
-      MixedRunsKernel<<<Blocks(items, T), T, 0, s>>>(d_keys_alt_.p, item_seg, ubeg, items, d_fix_list_.p, fix_cnt);
+      LaunchFollowing(MixedRunsKernel, Blocks(items, T), T, 0, s, d_keys_alt_.p, item_seg, ubeg, items, d_fix_list_.p,
+                      fix_cnt);
       ++launches_;
-      SortMixedRunsKernel<<<152 * 2, 256, 0, s>>>(d_keys_alt_.p, d_vals_alt_.p, item_seg, uend, d_fix_list_.p,
-                                                  fix_cnt, d_keys_.p, d_vals_.p);
+      LaunchFollowing(SortMixedRunsKernel, 152 * 2, 256, 0, s, d_keys_alt_.p, d_vals_alt_.p, item_seg, uend,
+                      d_fix_list_.p, fix_cnt, d_keys_.p, d_vals_.p);
       ++launches_;
-      ScatterSortedKernel<<<Blocks(items, T), T, 0, s>>>(d_pos_map_.p, item_seg, ubeg, items, d_keys_alt_.p,
-                                                         d_vals_alt_.p, fallback ? 1 : 0, cfg_.divide_max_group,
-                                                         d_order_.p, d_head_flag_.p);
+      LaunchFollowing(ScatterSortedKernel, Blocks(items, T), T, 0, s, d_pos_map_.p, item_seg, ubeg, items,
+                      d_keys_alt_.p, d_vals_alt_.p, fallback ? 1 : 0, cfg_.divide_max_group, d_order_.p,
+                      d_head_flag_.p);
     }
     // final segments are the groups (already described when the loop
     // settled; after the fallback depth they are recounted)
     if (!settled) {
       scan_incl(d_head_flag_.p, scan, count);
       ++launches_;
-      SegStartsKernel<<<Blocks(count, T), T, 0, s>>>(d_head_flag_.p, scan, count, seg_start);
+      LaunchFollowing(SegStartsKernel, Blocks(count, T), T, 0, s, d_head_flag_.p, scan, count, seg_start);
       int seg_total = 0, dummy = 0;
       fetch2(scan + count - 1, scan + count - 1, &seg_total, &dummy);
       segs = seg_total;
       ++launches_;
-      SegLenKernel<<<Blocks(segs, T), T, 0, s>>>(seg_start, segs, count, cfg_.divide_max_group, seg_len, unf_flag,
-                                                 unf_len);
+      LaunchFollowing(SegLenKernel, Blocks(segs, T), T, 0, s, seg_start, segs, count, cfg_.divide_max_group, seg_len,
+                      unf_flag, unf_len);
     }
     d_gent_.ensure(static_cast<size_t>(segs) + 1);
     CheckCuda(cudaMemsetAsync(d_gent_.p, 0, sizeof(unsigned) * static_cast<size_t>(segs), s), "memset gent");
     ++launches_;
-    GroupInfoKernel<<<Blocks(count, T), T, 0, s>>>(d_order_.p, scan, seg_start, seg_len, count, d_group_of_.p,
-                                                   d_idx_in_group_.p, d_qlen_.p, d_gent_.p, d_stats_.p);
+    LaunchFollowing(GroupInfoKernel, Blocks(count, T), T, 0, s, d_order_.p, scan, seg_start, seg_len, count,
+                    d_group_of_.p, d_idx_in_group_.p, d_qlen_.p, d_gent_.p, d_stats_.p);
     CheckCuda(cudaMemcpyAsync(d_gstart_.p, seg_start, sizeof(int) * static_cast<size_t>(segs),
                               cudaMemcpyDeviceToDevice, s), "copy gstart");
     CheckCuda(cudaMemcpyAsync(d_glen_.p, seg_len, sizeof(int) * static_cast<size_t>(segs),

@@ -292,9 +292,19 @@ void Engine::Reset() {
   RankerReset();
 }
 
+void Engine::QueueError() {
+  CheckCuda(cudaMemcpyAsync(h_pin_.p + 60, d_err_.p, sizeof(DevError), cudaMemcpyDeviceToHost, stream_), "d2h error");
+}
+
 void Engine::CheckError() {
+  QueueError();
+  CheckCuda(cudaStreamSynchronize(stream_), "error sync");
+  ThrowError();
+}
+
+void Engine::ThrowError() {
   DevError e;
-  CheckCuda(cudaMemcpy(&e, d_err_.p, sizeof(e), cudaMemcpyDeviceToHost), "d2h error");
+  std::memcpy(&e, h_pin_.p + 60, sizeof(e));
   if (e.code == kErrNone) return;
   std::string msg;
   switch (e.code) {

@@ -53,6 +53,26 @@ constexpr int kRowsGrid = 4 * 152;
 
 void CheckCuda(cudaError_t status, const char* what);
 
+#ifdef __CUDACC__
+// A launch that may be set up while the kernel before it on the stream still
+// runs; the kernel begins with FollowsOn (common.cuh).
+template <typename... Params, typename... Args>
+void LaunchFollowing(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream,
+                     Args&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  CheckCuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...), "kernel launch");
+}
+#endif
+
 // Device memory. Inside an AllocScope (every engine call sets one for its
 // stream) buffers come from the device's stream-ordered pool, which keeps
 // freed memory for the next allocation, so creating, growing and destroying
@@ -231,6 +251,8 @@ class Engine {
 
  private:
   void CheckError();
+  void QueueError();  // the error word read back with the stream's next synchronisation,
+  void ThrowError();  // and turned into an exception
   void InitQuotient();
   void EnsurePoolRoom();
   void EnsurePoolRoom(unsigned long long top);

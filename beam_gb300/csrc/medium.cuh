@@ -549,6 +549,7 @@ __device__ void MediumGroup(const MediumParams& P, MediumSmem& S, int ri) {
 }
 
 __global__ void __launch_bounds__(kMedThreads, kMedCtas) MediumKernel(MediumParams P) {
+  FollowsOn();
   extern __shared__ __align__(64) unsigned char med_smem[];
   MediumSmem& S = *reinterpret_cast<MediumSmem*>(med_smem);
   MediumGroup(P, S, P.list[P.list0 + blockIdx.x]);

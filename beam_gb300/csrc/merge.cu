@@ -670,6 +670,7 @@ struct PrepSmem {
 };
 
 __global__ void __launch_bounds__(kPrepThreads) PrepareKernel(PrepareParams P) {
+  FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PrepSmem& S = *reinterpret_cast<PrepSmem*>(smem_raw);
   using BlockScan = cub::BlockScan<int, kPrepThreads>;
@@ -892,6 +893,7 @@ constexpr int kFillWindow = 2048;
 constexpr int kAccumThreads = 256;
 
 __global__ void __launch_bounds__(kFillThreads) PrepareFillKernel(PrepareParams P) {
+  FollowsOn();
   __shared__ int first_group;
   const int lane = threadIdx.x & 31;
   const QuotientView& Q = P.Q;
@@ -1046,6 +1048,7 @@ constexpr int kAccumSplit = 4;
 constexpr int kAccumFetch = 8;
 
 __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PrepareParams P) {
+  FollowsOn();
   const int lane = threadIdx.x & 31;
   unsigned long long examined = 0;
   const bool counted = P.rc != nullptr;
@@ -1421,6 +1424,7 @@ __device__ __forceinline__ void RankMember(int g, int i, const int* q, const lon
 // launch's big-group list (moff = prefix of the member counts), so a large
 // group's members are ranked by the whole GPU instead of one CTA.
 __global__ void __launch_bounds__(256) PrepareMembersKernel(PrepareParams P) {
+  FollowsOn();
   __shared__ int cand_j[8][32];  // per warp: the candidates that survive the prescreen
   const long long wg = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long total = P.moff[P.list0 + P.nlist] - P.moff[P.list0];
@@ -1474,6 +1478,7 @@ __device__ __forceinline__ PairInfo PairInfoOf(const QuotientView& Q, int a, int
 // Output pass of the big groups: the union of kept pairs in (a_idx, b_idx)
 // order, one CTA per group.
 __global__ void __launch_bounds__(kPrepThreads) PrepareOutputKernel(PrepareParams P) {
+  FollowsOn();
   using BlockScan = cub::BlockScan<int, kPrepThreads>;
   __shared__ typename BlockScan::TempStorage scan_tmp;
   __shared__ int carry;
@@ -1962,6 +1967,7 @@ __device__ __forceinline__ void SmallTopK(SmallRowsSmem& S, int g, int top_k_max
 }
 
 __global__ void __launch_bounds__(kSmallWarps * 32) PrepareSmallKernel(PrepareParams P) {
+  FollowsOn();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmallWarpSmem& W = reinterpret_cast<SmallSmem*>(smem_raw)->w[threadIdx.x >> 5];
   SmallRowsSmem& S = W.rows;
@@ -2149,6 +2155,7 @@ constexpr int kScoreFetch = 32;
 constexpr int kScoreFetchMerge = 8;
 
 __global__ void __launch_bounds__(kScoreThreads, 4) ScoreKernel(ScoreParams P) {
+  FollowsOn();
   constexpr unsigned kFull = 0xffffffffu;
   const long long s0 = P.cand_off[P.rg0];
   const long long s1 = P.cand_off[P.rg0 + P.nrg];
@@ -2746,6 +2753,7 @@ __device__ __forceinline__ void SelectMatchGroup(const SelectParams& P, int ri) 
 }
 
 __global__ void __launch_bounds__(kMatchThreads) SelectMatchKernel(SelectParams P) {
+  FollowsOn();
   // list == nullptr: the real groups list0, list0 + 1, ... (a whole block)
   SelectMatchGroup(P, P.list ? P.list[P.list0 + blockIdx.x] : P.list0 + static_cast<int>(blockIdx.x));
 }
@@ -2772,6 +2780,7 @@ __device__ __forceinline__ unsigned long long WarpBitonicSortAsc(unsigned long l
 }
 
 __global__ void __launch_bounds__(kSelectSmallWarps * 32) SelectSmallKernel(SelectParams P) {
+  FollowsOn();
   __shared__ unsigned long long acc[9];
   const int lane = threadIdx.x & 31;
   const int li = blockIdx.x * kSelectSmallWarps + (threadIdx.x >> 5);
@@ -3254,6 +3263,7 @@ __global__ void __launch_bounds__(kRowsThreads) CommitKernel(CommitParams P) {
 // Update_S bookkeeping), with the keep row built in registers (bitonic sort
 // across the lanes, segmented sum, compaction).
 __global__ void __launch_bounds__(256) CommitShortKernel(CommitParams P) {
+  FollowsOn();
   const QuotientView& Q = P.Q;
   const int lane = threadIdx.x & 31;
   const int remove_stamp = 2 * P.block_stamp + 1;
@@ -3823,6 +3833,7 @@ __global__ void ScatterGroupKernel(const int* __restrict__ q, const int* __restr
 }
 
 __global__ void RelabelKernel(int* __restrict__ label, const int* __restrict__ fwd, int n) {
+  FollowsOn();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v < n) label[v] = fwd[label[v]];
 }
@@ -3985,6 +3996,7 @@ struct PlanParams {
 };
 
 __global__ void __launch_bounds__(kPlanThreads) PlanTileKernel(PlanParams P) {
+  FollowsOn();
   using Reduce = cub::BlockReduce<PlanSums, kPlanThreads>;
   __shared__ typename Reduce::TempStorage tmp;
   const long long base = static_cast<long long>(blockIdx.x) * kPlanTile + threadIdx.x * kPlanItems;
@@ -4002,6 +4014,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanTileKernel(PlanParams P) {
 // one CTA: exclusive offsets of the tiles, the totals, and the closing
 // entries of the offset arrays
 __global__ void __launch_bounds__(kPlanThreads) PlanScanKernel(PlanParams P) {
+  FollowsOn();
   using Scan = cub::BlockScan<PlanSums, kPlanThreads>;
   __shared__ typename Scan::TempStorage tmp;
   __shared__ PlanSums carry;
@@ -4047,6 +4060,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScanKernel(PlanParams P) {
 }
 
 __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) {
+  FollowsOn();
   using Scan = cub::BlockScan<PlanSums, kPlanThreads>;
   __shared__ typename Scan::TempStorage tmp;
   const long long base = static_cast<long long>(blockIdx.x) * kPlanTile + threadIdx.x * kPlanItems;
@@ -4394,13 +4408,13 @@ void Engine::PlanOnDevice() {
   }
   if (tiles > 0) {
     ++launches_;
-    PlanTileKernel<<<tiles, kPlanThreads, 0, stream_>>>(P);
+    LaunchFollowing(PlanTileKernel, tiles, kPlanThreads, 0, stream_, P);
   }
   ++launches_;
-  PlanScanKernel<<<1, kPlanThreads, 0, stream_>>>(P);
+  LaunchFollowing(PlanScanKernel, 1, kPlanThreads, 0, stream_, P);
   if (tiles > 0) {
     ++launches_;
-    PlanScatterKernel<<<tiles, kPlanThreads, 0, stream_>>>(P);
+    LaunchFollowing(PlanScatterKernel, tiles, kPlanThreads, 0, stream_, P);
   }
   static_assert(kPlanScalars + 1 <= 32, "room in the pinned words");
   long long* hs = h_pin_.p + 16;  // read back: totals and pool top
@@ -4413,8 +4427,9 @@ void Engine::PlanOnDevice() {
     CheckCuda(cudaMemcpyAsync(sums.data(), d_plan_blocks_.p, sizeof(PlanSums) * static_cast<size_t>(blocks),
                               cudaMemcpyDeviceToHost, stream_), "d2h block plan");
   }
+  QueueError();
   CheckCuda(cudaStreamSynchronize(stream_), "plan sync");
-  CheckError();
+  ThrowError();
   long long v[kPlanScalars + 1];
   std::memcpy(v, hs, sizeof(v));
   EnsurePoolRoom(static_cast<unsigned long long>(v[kPlanScalars]));
@@ -4489,24 +4504,6 @@ void CommitDefaults(CommitParams* C) {
 }
 }  // namespace
 
-namespace {
-// A launch whose kernel begins with FollowsOn.
-template <typename Params>
-void LaunchFollowing(void (*kernel)(Params), int grid, int threads, size_t smem, cudaStream_t stream, Params p) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(static_cast<unsigned>(threads));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  CheckCuda(cudaLaunchKernelEx(&cfg, kernel, p), "window launch");
-}
-}  // namespace
-
 void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, const void* window) {
   CommitParams C;
   CommitDefaults(&C);
@@ -4563,19 +4560,14 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, cons
   // CommitKernel (its keep row can only be short), which skips it; a long
   // pair is untouched until CommitKernel
   if (C.warp_pairs) {
-    CommitShortKernel<<<static_cast<int>(std::min<int64_t>((max_pairs + 7) / 8 + 1, 152 * 8)), 256, 0, stream_>>>(C);
+    LaunchFollowing(CommitShortKernel, static_cast<int>(std::min<int64_t>((max_pairs + 7) / 8 + 1, 152 * 8)), 256, 0,
+                    stream_, C);
     ++launches_;
   }
   launches_ += 2;
-  if (window) {
-    LaunchFollowing(CommitKernel, grid, kRowsThreads, sizeof(RowsSmem), stream_, C);
-    LaunchFollowing(RewriteRowsKernel, kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_, C);
-    LaunchFollowing(RewriteHugeKernel, kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_, C);
-  } else {
-    CommitKernel<<<grid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
-    RewriteRowsKernel<<<kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_>>>(C);
-    RewriteHugeKernel<<<kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_>>>(C);
-  }
+  LaunchFollowing(CommitKernel, grid, kRowsThreads, sizeof(RowsSmem), stream_, C);
+  LaunchFollowing(RewriteRowsKernel, kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_, C);
+  LaunchFollowing(RewriteHugeKernel, kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_, C);
   EndTimed(kTimeUpdate);
 }
 
@@ -4624,8 +4616,8 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
     PP.list0 = s0;
     PP.nlist = s1 - s0;
     ++launches_;
-    PrepareSmallKernel<<<(s1 - s0 + kSmallWarps - 1) / kSmallWarps, kSmallWarps * 32, sizeof(SmallSmem), stream_>>>(
-        PP);
+    LaunchFollowing(PrepareSmallKernel, (s1 - s0 + kSmallWarps - 1) / kSmallWarps, kSmallWarps * 32,
+                    sizeof(SmallSmem), stream_, PP);
   }
   if (b1 > b0) {
     PP.list = d_big_.p;
@@ -4650,11 +4642,12 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
     PP.skey_sorted = d_skey_[1].p;
     PP.sval_sorted = d_sval_[1].p;
     ++launches_;
-    PrepareKernel<<<b1 - b0, kPrepThreads, sizeof(PrepSmem), stream_>>>(PP);
+    LaunchFollowing(PrepareKernel, b1 - b0, kPrepThreads, sizeof(PrepSmem), stream_, PP);
     if (PP.nslots > 0) {
       const long long windows = (PP.nslots + kFillWindow - 1) / kFillWindow;
       ++launches_;
-      PrepareFillKernel<<<static_cast<int>(std::min(windows, 152ll * 32)), kFillThreads, 0, stream_>>>(PP);
+      LaunchFollowing(PrepareFillKernel, static_cast<int>(std::min(windows, 152ll * 32)), kFillThreads, 0, stream_,
+                      PP);
       // key = launch-local group index << tbits | target; the group index
       // stays below 2^(bits - tbits) - 1, so no key has the padding's low bits
       int bits = PP.tbits;
@@ -4667,12 +4660,13 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
                                                 d_sval_[1].p, PP.nslots, 0, bits, stream_), "cub radix sort");
       const long long want = ((PP.nslots + 31) / 32 * kAccumSplit + kAccumThreads / 32 - 1) / (kAccumThreads / 32);
       ++launches_;
-      PrepareAccumKernel<<<static_cast<int>(std::min<long long>(want, accum_grid_)), kAccumThreads, 0, stream_>>>(PP);
+      LaunchFollowing(PrepareAccumKernel, static_cast<int>(std::min<long long>(want, accum_grid_)), kAccumThreads, 0,
+                      stream_, PP);
     }
     ++launches_;
-    PrepareMembersKernel<<<static_cast<int>((members + 7) / 8), 256, 0, stream_>>>(PP);
+    LaunchFollowing(PrepareMembersKernel, static_cast<int>((members + 7) / 8), 256, 0, stream_, PP);
     ++launches_;
-    PrepareOutputKernel<<<b1 - b0, kPrepThreads, 0, stream_>>>(PP);
+    LaunchFollowing(PrepareOutputKernel, b1 - b0, kPrepThreads, 0, stream_, PP);
   }
   EndTimed(kTimePrepare);
 }
@@ -4709,7 +4703,7 @@ void Engine::LaunchMedium(const BlockPlan& bp, double threshold) {
   M.err = d_err_.p;
   BeginTimed(kTimePrepare);
   ++launches_;
-  MediumKernel<<<bp.m1 - bp.m0, kMedThreads, sizeof(MediumSmem), stream_>>>(M);
+  LaunchFollowing(MediumKernel, bp.m1 - bp.m0, kMedThreads, sizeof(MediumSmem), stream_, M);
   EndTimed(kTimePrepare);
 }
 
@@ -4771,14 +4765,14 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
     SP.zcap = static_cast<unsigned>(RankerExploreCap(slots));
     BeginTimed(kTimeScore);
     ++launches_;
-    ScoreKernel<<<sgrid, kScoreThreads, 0, stream_>>>(SP);
+    LaunchFollowing(ScoreKernel, sgrid, kScoreThreads, 0, stream_, SP);
     EndTimed(kTimeScore);
     RankerCutoff(slots);
     SP.phase = 2;
   }
   BeginTimed(kTimeScore);
   ++launches_;
-  ScoreKernel<<<sgrid, kScoreThreads, 0, stream_>>>(SP);
+  LaunchFollowing(ScoreKernel, sgrid, kScoreThreads, 0, stream_, SP);
   EndTimed(kTimeScore);
   if (cfg_.ranker && !rk_trained_ && iter <= cfg_.ranker_train_iters) {
     RankerLog(rg0, nrg, slots, iter, threshold, total_iterations);
@@ -4820,7 +4814,7 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
     LP.list0 = rg0;
     LP.nlist = nrg;
     ++launches_;
-    SelectMatchKernel<<<nrg, kMatchThreads, 8 * kMatchSmemKeys, stream_>>>(LP);
+    LaunchFollowing(SelectMatchKernel, nrg, kMatchThreads, 8 * kMatchSmemKeys, stream_, LP);
     LaunchCommit(rg0, nrg, sel_slots, cfg_.verify_cuda_gain, nullptr);
     return;
   }
@@ -4829,8 +4823,8 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
     LP.list0 = ss0;
     LP.nlist = ss1 - ss0;
     ++launches_;
-    SelectSmallKernel<<<(ss1 - ss0 + kSelectSmallWarps - 1) / kSelectSmallWarps, kSelectSmallWarps * 32, 0,
-                        stream_>>>(LP);
+    LaunchFollowing(SelectSmallKernel, (ss1 - ss0 + kSelectSmallWarps - 1) / kSelectSmallWarps,
+                    kSelectSmallWarps * 32, 0, stream_, LP);
   }
   const int sm0 = bp.sm0, sm1 = bp.sm1;
   if (sm1 > sm0) {
@@ -4845,7 +4839,7 @@ void Engine::RunBlock(const BlockPlan& bp, double threshold, int iter, int total
     LP.list0 = sb0;
     LP.nlist = sb1 - sb0;
     ++launches_;
-    SelectMatchKernel<<<sb1 - sb0, kMatchThreads, 8 * kMatchSmemKeys, stream_>>>(LP);
+    LaunchFollowing(SelectMatchKernel, sb1 - sb0, kMatchThreads, 8 * kMatchSmemKeys, stream_, LP);
   }
   LaunchCommit(rg0, nrg, sel_slots, cfg_.verify_cuda_gain, nullptr);
 }
@@ -4922,11 +4916,11 @@ void Engine::RunWindows(double threshold) {
   CheckCuda(cudaMemsetAsync(&W.ctl->blocks, 0, sizeof(long long), stream_), "memset blocks");
   const int count = static_cast<int>(n_active_);
   ++launches_;
-  WindowSetupKernel<<<(std::max(count, R) + 255) / 256, 256, 0, stream_>>>(
-      W.order, W.group_of, d_ri_of_.p, count, W.real, R, cfg_.group_batch_size, d_node_ri_.p, d_blk_beg_.p, d_blk_end_.p,
-      W.dirty, W.ctl);
+  LaunchFollowing(WindowSetupKernel, (std::max(count, R) + 255) / 256, 256, 0, stream_, W.order, W.group_of,
+                  d_ri_of_.p, count, W.real, R, cfg_.group_batch_size, d_node_ri_.p, d_blk_beg_.p, d_blk_end_.p,
+                  W.dirty, W.ctl);
   ++launches_;
-  WindowBeginKernel<<<1, kHugeThreads, 0, stream_>>>(W, R);
+  LaunchFollowing(WindowBeginKernel, 1, kHugeThreads, 0, stream_, W, R);
   // the host keeps a few rounds queued behind the one running; a round past
   // the end finds nothing to do
   long long queued = 0;
@@ -4984,14 +4978,15 @@ void Engine::Merge(int iter, int total_iterations) {
     }
   }
   ++launches_;
-  RelabelKernel<<<(n_ + 255) / 256, 256, 0, stream_>>>(d_label_.p, d_fwd_.p, n_);
+  LaunchFollowing(RelabelKernel, (n_ + 255) / 256, 256, 0, stream_, d_label_.p, d_fwd_.p, n_);
   n_groups_ = -1;  // the groups are consumed
   // accepted merges so far, read back with this synchronisation: the next
   // Divide knows the active count without a round trip of its own
   CheckCuda(cudaMemcpyAsync(h_pin_.p + 8, d_stats_.p + kStAccepted, sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, stream_), "d2h accepted");
+  QueueError();
   CheckCuda(cudaStreamSynchronize(stream_), "merge sync");
-  CheckError();
+  ThrowError();
   {
     unsigned long long accepted = 0;
     std::memcpy(&accepted, h_pin_.p + 8, sizeof(accepted));
@@ -5144,7 +5139,7 @@ void Engine::MergePairs(const int32_t* keep, const int32_t* remove, int64_t coun
                                                     d_seq_.p, block_stamp_, d_sel_list_.p, d_ctl_.p);
   LaunchCommit(0, 1, count, false, nullptr);
   ++launches_;
-  RelabelKernel<<<(n_ + 255) / 256, 256, 0, stream_>>>(d_label_.p, d_fwd_.p, n_);
+  LaunchFollowing(RelabelKernel, (n_ + 255) / 256, 256, 0, stream_, d_label_.p, d_fwd_.p, n_);
   n_groups_ = -1;
   CheckCuda(cudaStreamSynchronize(stream_), "merge pairs sync");
   CheckError();

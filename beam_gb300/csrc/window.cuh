@@ -175,15 +175,6 @@ __device__ __forceinline__ bool WindowSmall(int g, unsigned entries) {
   return g <= kEvalSmall && entries <= static_cast<unsigned>(kEvalEntries);
 }
 
-// First thing in every kernel of a round: the next kernel may be set up now,
-// and this one goes on when the one before it is complete (and its writes
-// visible). Takes the launch latency, one of the larger parts of a short
-// kernel, off the chain of a round. No effect on a kernel launched otherwise.
-__device__ __forceinline__ void FollowsOn() {
-  cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();
-}
-
 // ------------------------------------------------------------ lists
 
 // Per active supernode its group position, per group position the ends of its
@@ -191,6 +182,7 @@ __device__ __forceinline__ void FollowsOn() {
 __global__ void WindowSetupKernel(const int* order, const int* group_of, const int* ri_of, int count, const int* real,
                                   int R, int batch, int* node_ri, int* blk_beg, int* blk_end, int* dirty,
                                   WindowCtl* ctl) {
+  FollowsOn();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) {
     const int rep = order[i];
@@ -320,6 +312,7 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
 }
 
 __global__ void __launch_bounds__(kHugeThreads) WindowBeginKernel(WindowParams P, int R) {
+  FollowsOn();
   if (threadIdx.x == 0) {
     P.ctl->f = P.ctl->e = P.ctl->p = 0;
     P.ctl->R = R;
