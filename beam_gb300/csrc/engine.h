@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <stdexcept>
 #include <string>
@@ -48,20 +49,27 @@ struct RankerInfo {
 constexpr int kMaxGroup = 1024;
 // Blocks of at least this many groups are planned on the device.
 constexpr int kDevicePlanGroups = 1024;
+// The kernels whose grid is made for the chip (Commit, RewriteRows, RewriteHuge,
+// PrepareFill) are set up ahead of their turn only where a block stands for at
+// most this many arcs. CTAs placed while others still run crowd the SMs that are
+// free first, and stay there: RMAT-23's updates took 114 ms for 94 and its fills
+// 14 ms more, while 2 us a launch are nothing at that size. Blocks of 16384
+// groups of the union graph (40 thousand arcs) take 191 ms for 218 with it.
+constexpr long long kAheadArcs = 1 << 22;
 // Persistent grid of the row-update kernels (four CTAs per SM of a GB300).
 constexpr int kRowsGrid = 4 * 152;
 
 void CheckCuda(cudaError_t status, const char* what);
 
 #ifdef __CUDACC__
-// A launch that may be set up while the kernel before it on the stream still
-// runs; the kernel begins with FollowsOn (common.cuh).
+// A launch that, if `ahead`, may be set up while the kernel before it on the
+// stream still runs; the kernel begins with FollowsOn (common.cuh).
 template <typename... Params, typename... Args>
-void LaunchFollowing(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream,
-                     Args&&... args) {
+void LaunchAhead(bool ahead, void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream,
+                 Args&&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  attr.val.programmaticStreamSerializationAllowed = ahead ? 1 : 0;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(static_cast<unsigned>(threads));
@@ -70,6 +78,12 @@ void LaunchFollowing(void (*kernel)(Params...), int grid, int threads, size_t sm
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   CheckCuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...), "kernel launch");
+}
+
+template <typename... Params, typename... Args>
+void LaunchFollowing(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream,
+                     Args&&... args) {
+  LaunchAhead(true, kernel, grid, threads, smem, stream, static_cast<Args&&>(args)...);
 }
 #endif
 
@@ -272,6 +286,7 @@ class Engine {
   bool FusedOn() const;
   bool PlanFused() const;
   bool RowSumsOn() const;
+  bool SmallBlocks() const { return arcs_ / std::max<long long>(1, static_cast<long long>(plans_.size())) <= kAheadArcs; }
   bool WindowsOn() const;
   void RunWindows(double threshold);
   void PlanOnDevice();

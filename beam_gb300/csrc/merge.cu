@@ -4564,10 +4564,11 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, cons
                     stream_, C);
     ++launches_;
   }
-  launches_ += 2;
-  LaunchFollowing(CommitKernel, grid, kRowsThreads, sizeof(RowsSmem), stream_, C);
-  LaunchFollowing(RewriteRowsKernel, kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_, C);
-  LaunchFollowing(RewriteHugeKernel, kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_, C);
+  launches_ += 3;
+  const bool ahead = window || SmallBlocks();
+  LaunchAhead(ahead, CommitKernel, grid, kRowsThreads, sizeof(RowsSmem), stream_, C);
+  LaunchAhead(ahead, RewriteRowsKernel, kRowsGrid, kRowsThreads, sizeof(RowsSmem), stream_, C);
+  LaunchAhead(ahead, RewriteHugeKernel, kHugeGrid, kHugeThreads, sizeof(HugeSmem), stream_, C);
   EndTimed(kTimeUpdate);
 }
 
@@ -4646,8 +4647,8 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
     if (PP.nslots > 0) {
       const long long windows = (PP.nslots + kFillWindow - 1) / kFillWindow;
       ++launches_;
-      LaunchFollowing(PrepareFillKernel, static_cast<int>(std::min(windows, 152ll * 32)), kFillThreads, 0, stream_,
-                      PP);
+      LaunchAhead(SmallBlocks(), PrepareFillKernel, static_cast<int>(std::min(windows, 152ll * 32)), kFillThreads, 0,
+                  stream_, PP);
       // key = launch-local group index << tbits | target; the group index
       // stays below 2^(bits - tbits) - 1, so no key has the padding's low bits
       int bits = PP.tbits;
