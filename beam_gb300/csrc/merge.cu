@@ -467,7 +467,56 @@ __device__ __forceinline__ DeferredView Deferred(unsigned char* base, int g) {
   return V;
 }
 
-constexpr unsigned long long kSlotPad = ~0ull;  // key of an unused sort slot
+// Sort key of a deferred group's entry, from the top: low bits of the
+// launch-local group index, its other bits, the target. Fill writes the slots
+// in the order of the groups and the sort is stable, so it needs the lower two
+// fields only: entries of one (group, target) come out side by side, the
+// targets of 2^low neighbouring groups interleaved. Low bits are left out where
+// that saves a digit of the sort, a pass bound by its ranking and not by bytes
+// (keys and values in one word were no faster), up to kSlotGroupBits of them:
+// the pair tables of 32 groups of 512 members are 64 MB, half the L2. RMAT-23,
+// 23 + 14 bits in 4 passes for 5: sorts 152 -> 117 ms of a run, the adding up
+// 136.5 -> 137.7; RMAT-20 with the ranker 135.7 -> 130 ms in all.
+constexpr unsigned long long kSlotPad = ~0ull;  // an unused sort slot
+constexpr int kSlotGroupBits = 5;
+constexpr int kSortDigit = 8;
+
+struct SlotBits {
+  int target;  // bits of a target
+  int group;   // bits of a group index that are sorted
+  int low;     // bits of a group index that are not
+  __host__ __device__ int sorted() const { return target + group; }
+  __device__ unsigned long long Key(int k, int t) const {
+    const unsigned long long high = static_cast<unsigned long long>(k >> low) << target | static_cast<unsigned>(t);
+    return static_cast<unsigned long long>(k & ((1 << low) - 1)) << sorted() | high;
+  }
+  __device__ int Target(unsigned long long key) const { return static_cast<int>(key & ((1ull << target) - 1ull)); }
+  __device__ int Group(unsigned long long key) const {
+    return static_cast<int>(key >> target & ((1ull << group) - 1ull)) << low | static_cast<int>(key >> sorted());
+  }
+};
+
+// No sorted field of a key has the padding's bits: the group index's upper
+// part stays below all ones.
+SlotBits SlotLayout(int n, int groups) {
+  SlotBits b{1, 1, 0};
+  while ((1ll << b.target) < n) ++b.target;
+  auto sorted_bits = [&](int low) {
+    int bits = 1;
+    while ((groups - 1) >> low >= (1 << bits) - 1) ++bits;
+    return bits;
+  };
+  b.group = sorted_bits(0);
+  // the fewest low bits that save a digit
+  const int digits = (b.sorted() + kSortDigit - 1) / kSortDigit;
+  for (int low = 1; low <= kSlotGroupBits && b.low == 0; ++low) {
+    if (b.target + sorted_bits(low) <= (digits - 1) * kSortDigit) {
+      b.group = sorted_bits(low);
+      b.low = low;
+    }
+  }
+  return b;
+}
 
 // The same in 32 bits: sizes below 2^13, counts below 2^28.
 __device__ __forceinline__ void TermOf32(int sa, int sb, int st, int ca, int cb, int* delta, int* corr, bool* bad) {
@@ -496,7 +545,7 @@ struct PrepareParams {
   int2* cand_rep;         // per candidate slot: the pair's supernode ids (unused slots stay -1)
   const long long* soff;  // sort-slot prefix over the big-group list (0 slots: not deferred)
   long long slot0;        // soff of the launch's first entry
-  int tbits;                 // bits of a target supernode id in a sort key
+  SlotBits bits;             // fields of a sort key
   unsigned long long* skey;  // unsorted keys / values of the launch's slots
   unsigned long long* sval;
   const unsigned long long* skey_sorted;
@@ -947,7 +996,7 @@ __global__ void __launch_bounds__(kFillThreads) PrepareFillKernel(PrepareParams 
             if (HeavyEntry(V.msz[i], st, c)) heavy.Add(st, c); else light = c;
           }
           const long long slot = P.soff[P.list0 + k] - P.slot0 + idx;
-          P.skey[slot] = (static_cast<unsigned long long>(k) << P.tbits) | static_cast<unsigned>(t);
+          P.skey[slot] = P.bits.Key(k, t);
           P.sval[slot] = static_cast<unsigned long long>(i) << 32 | static_cast<unsigned long long>(c);
           if (P.group_of[t] == gid) {
             AddDirect(reinterpret_cast<unsigned long long*>(P.mat + P.mat_off[ri]), g, i, P.idx_in_group[t], c);
@@ -1081,13 +1130,13 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
     me.key = p < P.nslots ? P.skey_sorted[p] : kSlotPad;
     me.c = 0;
     me.s = me.i = 0;
-    const bool valid = me.key != kSlotPad && static_cast<int>(me.key >> P.tbits) < P.nlist;
+    const bool valid = me.key != kSlotPad;
     int g = 0;
     long long st = 0;
     unsigned long long* pmat = nullptr;
     if (valid) {
-      const int bl = static_cast<int>(me.key >> P.tbits);
-      const int t = static_cast<int>(me.key & ((1ull << P.tbits) - 1ull));
+      const int bl = P.bits.Group(me.key);
+      const int t = P.bits.Target(me.key);
       const int ri = P.list[P.list0 + bl];
       g = P.glen[P.real[ri]];
       pmat = reinterpret_cast<unsigned long long*>(P.mat + P.mat_off[ri]);
@@ -1117,8 +1166,7 @@ __global__ void __launch_bounds__(kAccumThreads, 6) PrepareAccumKernel(PreparePa
     // the run holding the chunk's first slot may start in earlier chunks
     const unsigned long long first = __shfl_sync(0xffffffffu, me.key, 0);
     if (first == kSlotPad || p0 == 0 || P.skey_sorted[p0 - 1] != first) continue;
-    const int fbl = static_cast<int>(first >> P.tbits);
-    if (fbl >= P.nlist) continue;
+    const int fbl = P.bits.Group(first);
     const int fg = P.glen[P.real[P.list[P.list0 + fbl]]];
     const DeferredView FV = Deferred(P.desc[P.list0 + fbl].base, fg);
     const bool mine = valid && me.key == first;
@@ -4636,8 +4684,7 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
       CheckCuda(cudaMemsetAsync(d_mat_.p, 0, static_cast<size_t>(bp.mat_bytes), stream_), "memset pair tables");
       PP.mat_zeroed = 1;
     }
-    PP.tbits = 1;
-    while ((1ll << PP.tbits) < n_) ++PP.tbits;
+    PP.bits = SlotLayout(n_, b1 - b0);
     PP.skey = d_skey_[0].p;
     PP.sval = d_sval_[0].p;
     PP.skey_sorted = d_skey_[1].p;
@@ -4649,10 +4696,7 @@ void Engine::LaunchPrepare(const BlockPlan& bp) {
       ++launches_;
       LaunchAhead(SmallBlocks(), PrepareFillKernel, static_cast<int>(std::min(windows, 152ll * 32)), kFillThreads, 0,
                   stream_, PP);
-      // key = launch-local group index << tbits | target; the group index
-      // stays below 2^(bits - tbits) - 1, so no key has the padding's low bits
-      int bits = PP.tbits;
-      while ((1ll << (bits - PP.tbits)) <= b1 - b0) ++bits;
+      const int bits = PP.bits.sorted();
       size_t bytes = 0;
       CheckCuda(cub::DeviceRadixSort::SortPairs(nullptr, bytes, d_skey_[0].p, d_skey_[1].p, d_sval_[0].p,
                                                 d_sval_[1].p, PP.nslots, 0, bits, stream_), "cub radix sort size");

@@ -99,3 +99,22 @@ def test_first_rows_of_long_adjacency_lists():
             nbrs, cnts, _, _ = e.row(i)
             ids, counts = np.unique(v[i], return_counts=True)
             assert np.array_equal(nbrs, ids) and np.array_equal(cnts, counts)
+
+
+@pytest.mark.parametrize("scale", [9, 10, 11, 12, 13, 14, 15])
+@pytest.mark.parametrize("limit", [48, 512])
+def test_sort_slots_of_large_groups(scale, limit):
+    """Groups whose shared targets are found by a sort: target widths and numbers
+    of groups that leave out from none to several bits of the group index."""
+    from beam_gb300 import Engine, Graph, partition_hash
+    from oracle import Oracle
+    g = Graph.generate(f"rmat:scale={scale},ef=24,a=0.57,b=0.19,c=0.19,seed={scale}")
+    kw = {"ea_use_threshold": True, "group_batch_size": 1 << 30, "divide_max_group": limit}
+    o = Oracle.from_graph(g, **kw)
+    o.run(3)
+    with Engine(g, **kw) as e:
+        e.run(3)
+        assert partition_hash(e.partition()[0]) == o.partition_hash()
+        st, ost = e.stats(), o.stats()
+        for k in ("candidate_proxy_pairs_examined", "exact_gain_input_nnz", "merge_total_local_gain"):
+            assert st[k] == ost[k], k
