@@ -118,3 +118,24 @@ def test_sort_slots_of_large_groups(scale, limit):
         st, ost = e.stats(), o.stats()
         for k in ("candidate_proxy_pairs_examined", "exact_gain_input_nnz", "merge_total_local_gain"):
             assert st[k] == ost[k], k
+
+
+@pytest.mark.parametrize("length", [1, 127, 128, 129, 383, 1000])
+def test_divide_over_rows_of_whole_steps(length):
+    """MinHashKernel's steps that lie in one row: hubs whose rows begin and end
+    on, before and behind a step, the last row of the graph among them."""
+    from beam_gb300 import Engine, Graph
+    from oracle import Oracle
+    rng = np.random.default_rng(length)
+    hubs, leaves = 40, 3000
+    u = np.repeat(np.arange(hubs), length)
+    v = np.concatenate([hubs + rng.choice(leaves, length, replace=False) for _ in range(hubs)])
+    last = np.full(1024, hubs + leaves)
+    g = Graph.from_edges(np.concatenate([u, last]), np.concatenate([v, hubs + np.arange(1024)]))
+    o = Oracle.from_graph(g, divide_max_group=16)
+    with Engine(g, divide_max_group=16) as e:
+        for it in (1, 2, 3):
+            e.divide(it), o.divide(it)
+            for a, b in zip(e.groups(), o.groups()):
+                assert np.array_equal(a, b)
+            e.merge(it), o.merge(it)
