@@ -47,8 +47,13 @@ struct RankerInfo {
 // Largest group the kernels accept (bounded by the packed select keys and
 // the per-group pair tables); the reference default is 512.
 constexpr int kMaxGroup = 1024;
-// Blocks of at least this many groups are planned on the device.
-constexpr int kDevicePlanGroups = 1024;
+// Blocks of at least this many groups are planned on the device. The host's
+// plan sends a block with few groups of two members or more down one path with
+// fewer launches, which pays below. 20 iterations planned on the host -> the
+// device: grid + Chung-Lu union of 0.5 M nodes 409 -> 389 ms in blocks of 2048
+// groups, 281 -> 259 of 4096, 191 -> 168 of 8192; R-MAT 18 (edge factor 8) 240
+// -> 261, 164 -> 164, 110 -> 105 ms.
+constexpr int kDevicePlanGroups = 4096;
 // The kernels whose grid is made for the chip (Commit, RewriteRows, RewriteHuge,
 // PrepareFill) are set up ahead of their turn only where a block stands for at
 // most this many arcs. CTAs placed while others still run crowd the SMs that are

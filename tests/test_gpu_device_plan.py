@@ -1,4 +1,4 @@
-"""Iterations of several blocks planned on the device (blocks of 1024 groups
+"""Iterations of several blocks planned on the device (blocks of 4096 groups
 and more) against the oracle: a border at the first size planned there, one
 that no tile of the plan ends on, blocks of more than one tile and a last block
 of a few groups; groups of every preparation class; the ranker, which has no
@@ -21,7 +21,10 @@ COUNTERS = ["merge_group_count", "merge_raw_pair_count", "candidate_proxy_pairs_
     ("rmat:scale=14,ef=6,a=0.57,b=0.19,c=0.19,seed=9", 1025, {"top_k": 2}),
     ("chunglu:n=20000,gamma=2.3,deg=8,twins=1000,seed=2", 1500, {}),
     ("chunglu:n=20000,gamma=2.3,deg=8,twins=1000,seed=2", 2048, {"ranker": True}),
-    ("grid:side=120,del=0.1,diag=0.02,seed=4", 1111, {"divide_max_group": 40})])
+    ("grid:side=120,del=0.1,diag=0.02,seed=4", 1111, {"divide_max_group": 40}),
+    ("grid:side=300,del=0.1,diag=0.02,seed=4", 4095, {}), ("grid:side=300,del=0.1,diag=0.02,seed=4", 4096, {}),
+    ("chunglu:n=150000,gamma=2.3,deg=8,twins=7500,seed=2", 4097, {}),
+    ("chunglu:n=150000,gamma=2.3,deg=8,twins=7500,seed=2", 5000, {"ranker": True})])
 def test_blocks_planned_on_the_device(spec, batch, kw):
     from beam_gb300 import Engine, Graph, partition_hash
     from oracle import Oracle
