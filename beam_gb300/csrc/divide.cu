@@ -187,13 +187,13 @@ __global__ void __launch_bounds__(256) MinHashKernel(const int* __restrict__ arc
                                                      unsigned long long* __restrict__ stats) {
   FollowsOn();
   const long long total = arcs + n;
-  // algorithmic bytes of one dimension: per arc its source, the source's
-  // label and its need stamp (12 B), per node its label and stamp (8 B), and
-  // the target of every arc that is hashed (4 B, counted per warp below)
+  // algorithmic bytes of one dimension: per arc its source (4 B), the labels and
+  // stamps of the steps that look them up per arc or node and once for those in
+  // one row (8 B each), the target of every arc that is hashed (4 B)
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    atomicAdd(&stats[kStDivideBytes], 12ull * static_cast<unsigned long long>(arcs) +
-                                          8ull * static_cast<unsigned long long>(n));
+    atomicAdd(&stats[kStDivideBytes], 4ull * static_cast<unsigned long long>(arcs));
   }
+  unsigned looked_up = 0;
   unsigned hashed_arcs = 0;  // warp-uniform; a warp's share of one launch stays far below 2^32
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(256) MinHashKernel(const int* __restrict__ arc
     const int row = __shfl_sync(0xffffffffu, node[0], 0);
     if (__shfl_sync(0xffffffffu, node[kHashUnroll - 1], 31) == row && t0 + kTile <= arcs) {
       const int one = label[row];
+      ++looked_up;
       if (need[one] != stamp) continue;
       hashed_arcs += static_cast<unsigned>(kTile);
       uint64_t h = ~0ull;
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(256) MinHashKernel(const int* __restrict__ arc
     }
 #pragma unroll
     for (int u = 0; u < kHashUnroll; ++u) rep[u] = node[u] >= 0 ? label[node[u]] : -1;
+    looked_up += static_cast<unsigned>(total - t0 < kTile ? total - t0 : kTile);
 #pragma unroll
     for (int u = 0; u < kHashUnroll; ++u) {
       if (rep[u] >= 0 && need[rep[u]] != stamp) rep[u] = -1;
@@ -255,7 +257,10 @@ __global__ void __launch_bounds__(256) MinHashKernel(const int* __restrict__ arc
       if (rep[u] >= 0 && lane == leader) atomicMin(&hash[rep[u]], g);
     }
   }
-  if (lane == 0 && hashed_arcs) atomicAdd(&stats[kStDivideBytes], 4ull * static_cast<unsigned long long>(hashed_arcs));
+  if (lane == 0 && looked_up) {
+    atomicAdd(&stats[kStDivideBytes],
+              8ull * static_cast<unsigned long long>(looked_up) + 4ull * static_cast<unsigned long long>(hashed_arcs));
+  }
 }
 
 __global__ void GatherKeysKernel(const int* __restrict__ order, const int* __restrict__ pos_map, int items,

@@ -3,8 +3,8 @@
 // (64 in the reference's recommended mode; one block of all groups in the
 // batched form).
 //
-//   Plan*Kernel        the block bookkeeping of a one-block iteration on the
-//                      device (lists and offsets of the groups)
+//   Plan*Kernel        the bookkeeping of large blocks on the device (lists and
+//                      offsets of the groups, sums at the blocks' borders)
 //   Prepare*Kernel     EA-proxy candidates per group (src/sweg.cpp:1598-1727,
 //                      1800-1999): a warp per small group; big groups by CTA
 //                      or by a GPU-wide sort of their row entries
@@ -2197,7 +2197,7 @@ __device__ __forceinline__ void FlushScoreStats(unsigned long long* stats, const
 // by one by the whole warp. Before, every pair merged its two rows here
 // (8-byte entries, 32 of each per step), although the prepare kernels had
 // already visited every shared target: at R-MAT scale 23 that was 330 ms of a
-// 1,291 ms run; now the run takes 973 ms. Without row sums (graphs beyond kFusedMaxArcs) a warp merges
+// 1,291 ms run, and is 30 ms here. Without row sums (graphs beyond kFusedMaxArcs) a warp merges
 // one pair's rows at a time, and fetches fewer of them.
 constexpr int kScoreFetch = 32;
 constexpr int kScoreFetchMerge = 8;

@@ -22,8 +22,8 @@
 // launches, 75 to 120 us, latency only). Rounds follow each other without the
 // host, which watches the frontier through mapped memory and keeps a few
 // rounds queued. Measured with 64-group blocks, 20 iterations, a block at a time
-// -> windows: R-MAT 16 (edge factor 8) 622 -> 120 ms, R-MAT 12 37.1 -> 14.9 ms,
-// Chung-Lu of 20,000 nodes with twins 109 -> 52 ms.
+// -> windows: R-MAT 16 (edge factor 8) 609 -> 119 ms, R-MAT 12 36.7 -> 13.9 ms,
+// Chung-Lu of 20,000 nodes with twins 108 -> 50 ms.
 #pragma once
 
 // Blocks of at most this many groups go through windows; larger ones fill the
