@@ -27,8 +27,12 @@
 #pragma once
 
 // Blocks of at most this many groups go through windows; larger ones fill the
-// GPU by themselves and touch too much of each other.
-constexpr int kWindowMaxBatch = 256;
+// GPU by themselves and touch too much of each other. 20 iterations a block at a
+// time -> windows, blocks of 512, 1024 and 2048 groups: grid + Chung-Lu union of
+// 0.5 M nodes 836 -> 295, 590 -> 257, 410 -> 215 ms; Chung-Lu of 100,000 nodes
+// 169 -> 107, 118 -> 83, 79 -> 65; R-MAT 15 (edge factor 16) 71 -> 54, 50 -> 46,
+// 37 -> 41; a uniform graph of 20,000 nodes 15.9 -> 12.2, 11.6 -> 10.9, 9.1 -> 10.0.
+constexpr int kWindowMaxBatch = 1024;
 constexpr int kWindowMaxGroups = 8192;  // groups a window takes in at most (then to the block's end)
 constexpr int kWindowMinGroups = 256;
 constexpr int kWindowMinAgain = 64;

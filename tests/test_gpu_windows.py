@@ -40,7 +40,9 @@ GRAPHS = {"hubs": None, "rmat": "rmat:scale=13,ef=6,a=0.57,b=0.19,c=0.19,seed=9"
     ("hubs", 64, {}), ("hubs", 7, {}), ("hubs", 256, {}), ("rmat", 33, {}), ("rmat", 256, {}), ("rmat", 257, {}),
     ("rmat", 64, {"top_k": 1}), ("rmat", 64, {"top_k": 33}), ("rmat", 64, {"ea_use_threshold": False}),
     ("rmat", 64, {"divide_max_group": 1024}), ("rmat", 64, {"verify_cuda_gain": True}), ("twins", 64, {}),
-    ("twins", 1, {}), ("twins", 100, {"top_k": 4}), ("grid", 64, {}), ("grid", 10, {"seed": 7})])
+    ("twins", 1, {}), ("twins", 100, {"top_k": 4}), ("grid", 64, {}), ("grid", 10, {"seed": 7}),
+    ("rmat", 1024, {}), ("rmat", 1025, {}), ("hubs", 700, {}), ("twins", 1024, {}), ("grid", 1024, {}),
+    ("grid", 1025, {})])
 def test_windows_match_the_blocks_in_order(graph, batch, kw):
     from beam_gb300 import Engine, Graph, partition_hash
     from oracle import Oracle
