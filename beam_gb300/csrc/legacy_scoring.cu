@@ -193,6 +193,9 @@ __global__ void __launch_bounds__(kLegacyThreads) LegacyFlatScoreKernel(FlatView
       if (pass == 0 && lane == 0) is_long[warp] = w < count && !mine ? 1 : 0;
       __syncthreads();
     }
+    // A pass that is skipped has no barrier: without this one a warp could write
+    // the next eight pairs' flags while another still reads these.
+    __syncthreads();
   }
 }
 
