@@ -34,6 +34,15 @@ __host__ __device__ __forceinline__ bool MediumFits(int g, unsigned entries) {
   return g <= kMedGroup && entries <= static_cast<unsigned>(kMedStage);
 }
 
+// Pair sums, upper triangle by TriIndex(a, b): proxy << 32 | corr, and the
+// number of shared targets, two to a word (16 bits each).
+struct MediumPairsSmem {
+  unsigned long long pc[kMedPairs];
+  unsigned ovl[(kMedPairs + 1) / 2];
+};
+static_assert(2 * (sizeof(MediumPairsSmem::ovl) / sizeof(unsigned)) >= kMedPairs, "a half word per pair");
+static_assert(kMedStage / 2 < 1 << 16, "two rows share at most half of the staged entries");
+
 struct MediumSmem {
   // the members' rows (the names the staged-row helpers use)
   Entry ent[kMedStage];  // afterwards: the selection keys
@@ -54,7 +63,7 @@ struct MediumSmem {
       int key[kMedSlots];
       unsigned cnt[kMedSlots / 2];  // two to a word: entries of the slot, then its run's start
     } hash;
-    SmallPairsSmem<kMedPairs> pairs;
+    MediumPairsSmem pairs;
   } u;
   unsigned keep[kMedGroup][2];  // kept partners b > a of member a
   int cj[kMedThreads / 32][32];

@@ -1661,6 +1661,7 @@ struct SmallPairsSmem {
   unsigned long long pc[kPairs];
   unsigned ovl[(kPairs + 3) / 4];
 };
+static_assert(kSmallStage / 2 < 1 << 8, "two rows share at most half of the staged entries");
 
 struct SmallWarpSmem {
   SmallRowsSmem rows;
