@@ -94,6 +94,7 @@ class FlatScorerStats(C.Structure):
         return {name: getattr(self, name) for name, _ in self._fields_}
 
 
+LIMIT_WINDOW_TABLES = 1
 TIME_NONE, TIME_SCORE, TIME_PREPARE, TIME_UPDATE, TIME_DIVIDE = 0, 1, 2, 3, 4
 
 # name -> (restype, argtypes); every symbol declared in include/beam_gb300.h
@@ -135,6 +136,7 @@ SIGNATURES = {
     "beam_engine_ranker_info": (C.c_int, [vp, C.POINTER(RankerInfo)]),
     "beam_ranker_grad": (C.c_int, [i32, vp, vp, vp, i64, vp, vp, P_f64, vp]),
     "beam_ranker_last_error": (C.c_char_p, []),
+    "beam_engine_set_limit": (C.c_int, [vp, i32, i64]),
     "beam_engine_set_timed_kernel": (C.c_int, [vp, i32]),
     "beam_engine_timed_kernel": (C.c_int, [vp, P_f64, P_i64]),
     "beam_engine_synchronize": (C.c_int, [vp]),

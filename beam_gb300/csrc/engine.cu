@@ -859,6 +859,10 @@ int beam_engine_quotient_nnz(beam_engine* e, int64_t* nnz) {
   return Guard([&] { *nnz = e->impl->QuotientNnz(); });
 }
 
+int beam_engine_set_limit(beam_engine* e, int32_t which, int64_t value) {
+  return Guard([&] { e->impl->SetLimit(which, value); });
+}
+
 int beam_engine_set_timed_kernel(beam_engine* e, int32_t which) {
   return Guard([&] { e->impl->SetTimedKernel(which); });
 }

@@ -208,6 +208,9 @@ struct HostStats {
   uint64_t divide_fallback_splits = 0;
 };
 
+// Settable limits (BEAM_LIMIT_* of include/beam_gb300.h).
+enum Limit : int { kLimitWindowTables = 1 };
+
 // Timing of one kernel class with CUDA events on the engine stream.
 enum TimedKernel : int { kTimeNone = 0, kTimeScore = 1, kTimePrepare = 2, kTimeUpdate = 3, kTimeDivide = 4 };
 
@@ -255,6 +258,9 @@ class Engine {
   const EngineConfig& config() const { return cfg_; }
   cudaStream_t stream() const { return stream_; }
 
+  // Limits of internal choices (Limit).
+  void SetLimit(int which, int64_t value);
+
   // Kernel timing for the roofline: events around every launch of one kernel class.
   void SetTimedKernel(int which);
   double TimedKernelMs();
@@ -294,6 +300,7 @@ class Engine {
   bool SmallBlocks() const { return arcs_ / std::max<long long>(1, static_cast<long long>(plans_.size())) <= kAheadArcs; }
   bool WindowsOn() const;
   void RunWindows(double threshold);
+  int WindowTables(int R);
   void PlanOnDevice();
   void SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nbig, long long max_mat, long long max_slots,
                             bool windows);
@@ -391,6 +398,7 @@ class Engine {
   bool plan_on_device_ = false;
   // windows of blocks (window.cuh)
   bool windowed_ = false;
+  long long window_tables_ = 0;  // bytes of a round's tables (SetLimit)
   DevBuf<int> d_ri_of_, d_node_ri_, d_blk_beg_, d_blk_end_, d_dirty_, d_win_list_;
   DevBuf<long long> d_win_off_;
   DevBuf<int> d_conflict_;

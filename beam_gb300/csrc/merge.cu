@@ -3892,6 +3892,7 @@ __global__ void RelabelKernel(int* __restrict__ label, const int* __restrict__ f
 // --------------------------------------------------------------- host side
 
 void Engine::ConfigureKernels() {
+  window_tables_ = kWindowTables;
   CheckCuda(cudaFuncSetAttribute(PrepareKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(sizeof(PrepSmem))), "prepare smem attribute");
   CheckCuda(cudaFuncSetAttribute(PrepareSmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3918,6 +3919,11 @@ void Engine::ConfigureKernels() {
   accum_grid_ = std::max(1, sms * per_sm);
   CheckCuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ScoreKernel, kScoreThreads, 0), "score occupancy");
   score_grid_ = std::max(1, sms * per_sm);
+}
+
+void Engine::SetLimit(int which, int64_t value) {
+  if (which != kLimitWindowTables || value < 1) throw std::invalid_argument("unknown limit or value out of range");
+  window_tables_ = value;
 }
 
 // Per-iteration layout: the groups with >= 2 members in Divide order, their
@@ -4102,7 +4108,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScanKernel(PlanParams P) {
     s[kPlanSelBig] = T.sbig;
     P.cand_off[T.real] = T.cand;
     P.sel_off[T.real] = T.sel;
-    P.mat_off[T.real] = 0;
+    P.mat_off[T.real] = T.mat;
     P.big_moff[T.big] = T.moff;
     P.soff[T.big] = T.soff;
   }
@@ -4135,7 +4141,7 @@ __global__ void __launch_bounds__(kPlanThreads) PlanScatterKernel(PlanParams P) 
       P.real[ri] = static_cast<int>(base + j);
       P.cand_off[ri] = off.cand;
       P.sel_off[ri] = off.sel;
-      P.mat_off[ri] = f.big ? off.mat : 0;
+      P.mat_off[ri] = off.mat;
       if (f.med) {
         P.med[off.med] = ri;
       } else if (!f.big) {
@@ -4372,8 +4378,8 @@ void Engine::SizeIterationBuffers(size_t R, size_t ncand, size_t nsel, size_t nb
   d_sel_keep_.ensure(nsel + 1);
   d_sel_rem_.ensure(nsel + 1);
   d_sel_gain_.ensure(nsel + 1);
+  if (windows) return;  // neither candidate lists nor sort slots, and tables by the window (WindowTables)
   d_mat_.ensure(static_cast<size_t>(max_mat) + 256);
-  if (windows) return;  // neither candidate lists nor sort slots
   d_bigdesc_.ensure(sizeof(BigDesc) * (nbig + 1));
   max_slots = std::max(max_slots, 1ll);
   for (int k = 0; k < 2; ++k) {
@@ -4895,6 +4901,37 @@ bool Engine::WindowsOn() const {
   return cfg_.group_batch_size <= kWindowMaxBatch && !cfg_.ranker && RowSumsOn();
 }
 
+// Makes room for the tables of a round's big groups (group positions and block
+// ends are set up); returns the groups that a window may take in: all it likes
+// where the whole iteration's tables are few, else as many as stay within the
+// limit, one block at the least. Where the device has no such room left, fewer.
+int Engine::WindowTables(int R) {
+  auto fits = [&](long long bytes) {
+    try {
+      d_mat_.ensure(static_cast<size_t>(bytes) + 256);
+      return true;
+    } catch (const std::runtime_error&) {
+      cudaGetLastError();  // a failed allocation is no later call's error
+      return false;
+    }
+  };
+  const long long total = plans_[0].mat_bytes;
+  if (total <= window_tables_ && fits(total)) return kWindowMaxGroups;
+  static_assert(kWindowLengths <= kPlanScalars, "room in the plan's words");
+  unsigned long long* most = reinterpret_cast<unsigned long long*>(d_plan_scalars_.p);
+  CheckCuda(cudaMemsetAsync(most, 0, sizeof(long long) * kWindowLengths, stream_), "memset window spans");
+  ++launches_;
+  LaunchFollowing(WindowSpanKernel, (R + 255) / 256, 256, 0, stream_, d_mat_off_.p, d_blk_beg_.p, d_blk_end_.p, R, most);
+  CheckCuda(cudaMemcpyAsync(h_pin_.p + 16, most, sizeof(long long) * kWindowLengths, cudaMemcpyDeviceToHost, stream_),
+            "d2h window spans");
+  CheckCuda(cudaStreamSynchronize(stream_), "sync");
+  for (int k = 0; k + 1 < kWindowLengths; ++k) {
+    if (h_pin_.p[16 + k] <= window_tables_ && fits(h_pin_.p[16 + k])) return kWindowMaxGroups >> k;
+  }
+  d_mat_.ensure(static_cast<size_t>(h_pin_.p[16 + kWindowLengths - 1]) + 256);
+  return 1;
+}
+
 // An iteration's blocks through windows (window.cuh).
 void Engine::RunWindows(double threshold) {
   const int R = plans_[0].rg1;
@@ -4933,8 +4970,6 @@ void Engine::RunWindows(double threshold) {
   W.list_big = reinterpret_cast<BigGroup*>(d_win_big_.p);
   W.moff = d_win_off_.p;
   W.poff = d_win_off_.p + kWindowList + 1;
-  W.mat_off = d_mat_off_.p;
-  W.mat = d_mat_.p;
   W.cand_off = d_cand_off_.p;
   W.keys = reinterpret_cast<unsigned long long*>(d_res_.p);
   W.rc = reinterpret_cast<RowSums*>(d_rc_.p);
@@ -4965,6 +5000,8 @@ void Engine::RunWindows(double threshold) {
   LaunchFollowing(WindowSetupKernel, (std::max(count, R) + 255) / 256, 256, 0, stream_, W.order, W.group_of,
                   d_ri_of_.p, count, W.real, R, cfg_.group_batch_size, d_node_ri_.p, d_blk_beg_.p, d_blk_end_.p,
                   W.dirty, W.ctl);
+  W.max_groups = WindowTables(R);
+  W.mat = d_mat_.p;
   ++launches_;
   LaunchFollowing(WindowBeginKernel, 1, kHugeThreads, 0, stream_, W, R);
   // the host keeps a few rounds queued behind the one running; a round past

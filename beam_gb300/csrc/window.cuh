@@ -36,6 +36,13 @@ constexpr int kWindowMaxBatch = 1024;
 constexpr int kWindowMaxGroups = 8192;  // groups a window takes in at most (then to the block's end)
 constexpr int kWindowMinGroups = 256;
 constexpr int kWindowMinAgain = 64;
+// Tables of a round's big groups take at most this much memory, unless one block
+// needs more by itself: an iteration whose tables are beyond it in all goes
+// through windows of fewer groups (WindowSpanKernel). 4.5 KB a node in groups of
+// 500 members, 9 KB at 1,024, else limit the graphs that fit.
+constexpr long long kWindowTables = 4ll << 30;
+constexpr int kWindowLengths = 14;  // kWindowMaxGroups, halved down to 1 (then to the block's end)
+static_assert(kWindowMaxGroups >> (kWindowLengths - 1) == 1, "the last length is one block");
 constexpr int kWindowList = 2 * (kWindowMaxGroups + kWindowMaxBatch) + 1024;
 constexpr int kEvalWarps = 4;
 constexpr int kEvalCtas = 8;     // per SM
@@ -150,8 +157,8 @@ struct WindowParams {
   BigGroup* list_big;
   long long* moff;      // member / part prefixes over list_big
   long long* poff;
-  const long long* mat_off;
-  unsigned char* mat;
+  unsigned char* mat;   // tables of the listed big groups
+  int max_groups;       // groups that a window takes in at most, by the room for their tables
   const long long* cand_off;
   unsigned long long* keys;  // two per candidate slot
   RowSums* rc;
@@ -211,15 +218,32 @@ __global__ void WindowSetupKernel(const int* order, const int* group_of, const i
   }
 }
 
+// Bytes of the tables of a window of at most kWindowMaxGroups >> k groups, the
+// most over all blocks that it may start with. A round's groups lie between the
+// first block not committed and the end of the blocks taken in (no further than
+// the window's length from that block, or from an earlier one).
+__global__ void WindowSpanKernel(const long long* mat_off, const int* blk_beg, const int* blk_end, int R,
+                                 unsigned long long* most) {
+  FollowsOn();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool starts = i < R && blk_beg[i] == i;
+  for (int k = 0; k < kWindowLengths; ++k) {
+    long long bytes = 0;
+    if (starts) bytes = mat_off[blk_end[min(i + (kWindowMaxGroups >> k), R) - 1]] - mat_off[i];
+    bytes = WarpMax(bytes);
+    if ((threadIdx.x & 31) == 0 && bytes > 0) atomicMax(&most[k], static_cast<unsigned long long>(bytes));
+  }
+}
+
 // The next evaluation's lists, by one CTA of kHugeThreads: the touched groups
 // and those that the window takes in. `done`: groups [f, p) are committed.
 struct ListSum {
-  long long members, parts;
+  long long members, parts, mat;
   int small, big;
 };
 struct ListSumOp {
   __device__ __forceinline__ ListSum operator()(const ListSum& a, const ListSum& b) const {
-    return ListSum{a.members + b.members, a.parts + b.parts, a.small + b.small, a.big + b.big};
+    return ListSum{a.members + b.members, a.parts + b.parts, a.mat + b.mat, a.small + b.small, a.big + b.big};
   }
 };
 
@@ -239,7 +263,7 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
     pace = min(pace, kWindowMaxGroups / 2);
     c->pace = pace;
     c->f = c->p;
-    const int take = min(max(2 * pace, kWindowMinGroups), kWindowMaxGroups);
+    const int take = min(max(2 * pace, kWindowMinGroups), P.max_groups);
     int e = c->f + take;
     e = e >= c->R ? c->R : e == 0 ? 0 : P.blk_end[e - 1];
     s_e0 = c->e;
@@ -249,7 +273,7 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
     s_again = max(c->f + max(2 * pace, kWindowMinAgain), c->f < c->R ? P.blk_end[c->f] : 0);
     s_kept = 0;
     s_stale = 0x7fffffff;
-    carry = ListSum{0, 0, 0, 0};
+    carry = ListSum{0, 0, 0, 0, 0};
   }
   __syncthreads();
   const int n = s_dirty + (s_e1 - s_e0);
@@ -257,7 +281,7 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
     const int i = base + threadIdx.x;
     int ri = -1, g = 0, gid = 0;
     unsigned entries = 0;
-    ListSum v{0, 0, 0, 0};
+    ListSum v{0, 0, 0, 0, 0};
     bool later = false;
     if (i < n) {
       ri = i < s_dirty ? P.list_dirty[i] : s_e0 + (i - s_dirty);
@@ -278,18 +302,19 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
         v.big = 1;
         v.members = g;
         v.parts = static_cast<long long>(g) * WindowParts(entries);
+        v.mat = WindowBytes(g, entries);
       }
       GroupStats z = {};
       P.gs[ri] = z;
       P.conflict[ri] = 0x7fffffff;
     }
     ListSum ex, total;
-    Scan(tmp).ExclusiveScan(v, ex, ListSum{0, 0, 0, 0}, ListSumOp(), total);
+    Scan(tmp).ExclusiveScan(v, ex, ListSum{0, 0, 0, 0, 0}, ListSumOp(), total);
     const ListSum c0 = carry;
     if (v.small) P.list_small[c0.small + ex.small] = ri;
     if (v.big) {
       P.list_big[c0.big + ex.big] =
-          BigGroup{ri, gid, g, static_cast<int>(entries), P.gstart[gid], WindowParts(entries), P.mat_off[ri]};
+          BigGroup{ri, gid, g, static_cast<int>(entries), P.gstart[gid], WindowParts(entries), c0.mat + ex.mat};
       P.moff[c0.big + ex.big] = c0.members + ex.members;
       P.poff[c0.big + ex.big] = c0.parts + ex.parts;
     }

@@ -255,6 +255,10 @@ class Engine:
         N.check(N.lib().beam_engine_quotient_nnz(self._h, C.byref(out)))
         return int(out.value)
 
+    def set_limit(self, which: int, value: int) -> None:
+        """One of the engine's limits (LIMIT_* of _native); results do not depend on it."""
+        N.check(N.lib().beam_engine_set_limit(self._h, which, value))
+
     def set_timed_kernel(self, which: int) -> None:
         N.check(N.lib().beam_engine_set_timed_kernel(self._h, which))
 

@@ -194,6 +194,13 @@ int beam_engine_validate_quotient(beam_engine* e);
 int beam_engine_exact_partition_cost(beam_engine* e, int64_t* cost);
 /* QuotientGraph::Nnz (src/quotient_graph.cpp:259-270). */
 int beam_engine_quotient_nnz(beam_engine* e, int64_t* nnz);
+/* Limits of the engine's internal choices, for hosts that share the GPU and for
+ * tests of what lies beyond a limit. Results do not depend on them.
+ *   BEAM_LIMIT_WINDOW_TABLES  device bytes for the pair tables of the groups
+ *     that the plain form evaluates at once [4 GiB]; a block that needs more
+ *     by itself gets it */
+enum { BEAM_LIMIT_WINDOW_TABLES = 1 };
+int beam_engine_set_limit(beam_engine* e, int32_t which, int64_t value);
 /* CUDA-event timing of every launch of one kernel class (BEAM_TIME_*). */
 int beam_engine_set_timed_kernel(beam_engine* e, int32_t which);
 int beam_engine_timed_kernel(beam_engine* e, double* ms, int64_t* launches);
