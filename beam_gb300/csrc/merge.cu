@@ -5108,10 +5108,10 @@ void Engine::ScorePairs(const int32_t* rep_a, const int32_t* rep_b, int64_t coun
                                                           max_units, d_err_.p);
   ScoreLongPairsKernel<<<152 * 6, kScoreThreads, 0, stream_>>>(View(), da.p, db.p, dg.p, dg.p + uc, units, nunits,
                                                                max_units, d_err_.p);
+  CheckError();  // a call that fails leaves the caller's arrays alone
   CheckCuda(cudaMemcpyAsync(gain, dg.p, sizeof(int64_t) * uc, cudaMemcpyDeviceToHost, stream_), "d2h gains");
   CheckCuda(cudaMemcpyAsync(before, dg.p + uc, sizeof(int64_t) * uc, cudaMemcpyDeviceToHost, stream_), "d2h costs");
   CheckCuda(cudaStreamSynchronize(stream_), "score sync");
-  CheckError();
 }
 
 int64_t Engine::PrepareGroup(const int32_t* q, int g, int32_t* a_idx, int32_t* b_idx, int64_t cap) {
