@@ -301,6 +301,7 @@ Engine::Engine(int n, int64_t arcs, const int64_t* row_ptr, const int32_t* col_i
 
 Engine::~Engine() {
   for (cudaEvent_t e : ev_pool_) cudaEventDestroy(e);
+  for (cudaEvent_t e : round_ev_) cudaEventDestroy(e);
   for (cudaEvent_t e : step_ev_) {
     if (e) cudaEventDestroy(e);
   }

@@ -398,6 +398,7 @@ class Engine {
   bool plan_on_device_ = false;
   // windows of blocks (window.cuh)
   bool windowed_ = false;
+  std::vector<cudaEvent_t> round_ev_;  // ends of the rounds queued, where the host sleeps for them
   long long window_tables_ = 0;  // bytes of a round's tables (SetLimit)
   DevBuf<int> d_ri_of_, d_node_ri_, d_blk_beg_, d_blk_end_, d_dirty_, d_win_list_;
   DevBuf<long long> d_win_off_;

@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <thread>
 
 #include "engine.h"
 
@@ -5005,12 +5006,29 @@ void Engine::RunWindows(double threshold) {
   ++launches_;
   LaunchFollowing(WindowBeginKernel, 1, kHugeThreads, 0, stream_, W, R);
   // the host keeps a few rounds queued behind the one running; a round past
-  // the end finds nothing to do
+  // the end finds nothing to do. It waits as the process has asked the driver to
+  // wait: asleep on the round's event, giving its core away, or (the driver's
+  // default too) watching the mapped words, which reach it some microseconds
+  // before an event would.
+  unsigned flags = 0;
+  CheckCuda(cudaGetDeviceFlags(&flags), "device flags");
+  const bool asleep = (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
+  const bool yielding = (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleYield;
+  while (asleep && round_ev_.size() < kWindowAhead) {
+    cudaEvent_t e;
+    CheckCuda(cudaEventCreateWithFlags(&e, cudaEventBlockingSync | cudaEventDisableTiming), "cudaEventCreate");
+    round_ev_.push_back(e);
+  }
   long long queued = 0;
   for (long long idle = 0;;) {
     const int done = __atomic_load_n(&seen[1], __ATOMIC_ACQUIRE) - 1;  // the first lists count as one
     if (__atomic_load_n(&seen[0], __ATOMIC_ACQUIRE) >= R) break;
     if (queued - done >= kWindowAhead) {
+      if (asleep) {  // until the oldest round not seen done is
+        CheckCuda(cudaEventSynchronize(round_ev_[static_cast<size_t>((done + 1) % kWindowAhead)]), "window rounds");
+        continue;
+      }
+      if (yielding) std::this_thread::yield();
       if (++idle % 4096 == 0) {
         const cudaError_t st = cudaStreamQuery(stream_);
         if (st != cudaErrorNotReady) CheckCuda(st, "window rounds");
@@ -5034,6 +5052,9 @@ void Engine::RunWindows(double threshold) {
     LaunchFollowing(WindowMarkKernel, kMarkGrid, kMarkThreads, 0, stream_, W);
     launches_ += 6;
     LaunchCommit(0, R, kBigGrid, cfg_.verify_cuda_gain, &W);
+    if (asleep) {
+      CheckCuda(cudaEventRecord(round_ev_[static_cast<size_t>(queued % kWindowAhead)], stream_), "event record");
+    }
   }
   CheckCuda(cudaMemcpyAsync(h_pin_.p + 9, &W.ctl->blocks, sizeof(long long), cudaMemcpyDeviceToHost, stream_),
             "d2h blocks");
