@@ -94,7 +94,7 @@ class FlatScorerStats(C.Structure):
         return {name: getattr(self, name) for name, _ in self._fields_}
 
 
-LIMIT_WINDOW_TABLES = 1
+LIMIT_WINDOW_TABLES, LIMIT_ROW_SUM_ARCS = 1, 2
 TIME_NONE, TIME_SCORE, TIME_PREPARE, TIME_UPDATE, TIME_DIVIDE = 0, 1, 2, 3, 4
 
 # name -> (restype, argtypes); every symbol declared in include/beam_gb300.h

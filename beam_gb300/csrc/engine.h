@@ -209,7 +209,7 @@ struct HostStats {
 };
 
 // Settable limits (BEAM_LIMIT_* of include/beam_gb300.h).
-enum Limit : int { kLimitWindowTables = 1 };
+enum Limit : int { kLimitWindowTables = 1, kLimitRowSumArcs = 2 };
 
 // Timing of one kernel class with CUDA events on the engine stream.
 enum TimedKernel : int { kTimeNone = 0, kTimeScore = 1, kTimePrepare = 2, kTimeUpdate = 3, kTimeDivide = 4 };
@@ -399,7 +399,9 @@ class Engine {
   // windows of blocks (window.cuh)
   bool windowed_ = false;
   std::vector<cudaEvent_t> round_ev_;  // ends of the rounds queued, where the host sleeps for them
-  long long window_tables_ = 0;  // bytes of a round's tables (SetLimit)
+  // limits (SetLimit): bytes of a round's tables; arcs below which scoring reads sums
+  long long window_tables_ = 0;
+  long long row_sum_arcs_ = 0;
   DevBuf<int> d_ri_of_, d_node_ri_, d_blk_beg_, d_blk_end_, d_dirty_, d_win_list_;
   DevBuf<long long> d_win_off_;
   DevBuf<int> d_conflict_;

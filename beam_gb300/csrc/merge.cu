@@ -3894,6 +3894,7 @@ __global__ void RelabelKernel(int* __restrict__ label, const int* __restrict__ f
 
 void Engine::ConfigureKernels() {
   window_tables_ = kWindowTables;
+  row_sum_arcs_ = kFusedMaxArcs;
   CheckCuda(cudaFuncSetAttribute(PrepareKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(sizeof(PrepSmem))), "prepare smem attribute");
   CheckCuda(cudaFuncSetAttribute(PrepareSmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3923,8 +3924,9 @@ void Engine::ConfigureKernels() {
 }
 
 void Engine::SetLimit(int which, int64_t value) {
-  if (which != kLimitWindowTables || value < 1) throw std::invalid_argument("unknown limit or value out of range");
-  window_tables_ = value;
+  const int64_t most = which == kLimitWindowTables ? INT64_MAX : which == kLimitRowSumArcs ? kFusedMaxArcs : 0;
+  if (value < 1 || value > most) throw std::invalid_argument("unknown limit or value out of range");
+  (which == kLimitWindowTables ? window_tables_ : row_sum_arcs_) = value;
 }
 
 // Per-iteration layout: the groups with >= 2 members in Divide order, their
@@ -4633,7 +4635,7 @@ void Engine::LaunchCommit(int rg0, int nrg, int64_t max_pairs, bool verify, cons
 // Row sums and pair sums are written by the block's own prepare kernels from
 // its block-start state and read by its scoring pass only, so every block uses
 // them, on graphs whose shared targets fit their field of the pair words.
-bool Engine::RowSumsOn() const { return arcs_ < kFusedMaxArcs; }
+bool Engine::RowSumsOn() const { return arcs_ < row_sum_arcs_; }
 
 void Engine::LaunchPrepare(const BlockPlan& bp) {
   const int s0 = bp.s0, s1 = bp.s1, b0 = bp.b0, b1 = bp.b1;

@@ -198,8 +198,11 @@ int beam_engine_quotient_nnz(beam_engine* e, int64_t* nnz);
  * tests of what lies beyond a limit. Results do not depend on them.
  *   BEAM_LIMIT_WINDOW_TABLES  device bytes for the pair tables of the groups
  *     that the plain form evaluates at once [4 GiB]; a block that needs more
- *     by itself gets it */
-enum { BEAM_LIMIT_WINDOW_TABLES = 1 };
+ *     by itself gets it
+ *   BEAM_LIMIT_ROW_SUM_ARCS   graphs of this many arcs and more are scored by
+ *     merging rows, in blocks planned one at a time [2^30, which is also the
+ *     most: the sums' fields hold no more]; takes effect with the next Divide */
+enum { BEAM_LIMIT_WINDOW_TABLES = 1, BEAM_LIMIT_ROW_SUM_ARCS = 2 };
 int beam_engine_set_limit(beam_engine* e, int32_t which, int64_t value);
 /* CUDA-event timing of every launch of one kernel class (BEAM_TIME_*). */
 int beam_engine_set_timed_kernel(beam_engine* e, int32_t which);
