@@ -1798,18 +1798,14 @@ __device__ __forceinline__ int StageSmallRows(const QuotientView& Q, const int* 
   return E;
 }
 
-// One entry (count c, target size st) into member i's sums: below kSmallNarrow
-// in all, so the low words hold them.
+// One entry (count c, target size st) into member i's sums, in the low words: the
+// counts sum to less than kSmallNarrow. Old costs are signed there (a count
+// beyond its block's capacity has a negative one, above -c) until SmallFinishRow.
 template <typename Rows>
 __device__ __forceinline__ void AddRowEntry(Rows& S, int i, long long c, long long st) {
   const long long si = S.sz[i];
   const long long alt = 1 + si * st - c;
-  const long long old = c < alt ? c : alt;
-  if (old >= 0) {
-    atomicAdd(reinterpret_cast<unsigned*>(&S.old[i]), static_cast<unsigned>(old));
-  } else {
-    atomicAdd(reinterpret_cast<unsigned long long*>(&S.old[i]), static_cast<unsigned long long>(old));
-  }
+  atomicAdd(reinterpret_cast<unsigned*>(&S.old[i]), static_cast<unsigned>(c < alt ? c : alt));
   if (HeavyEntry(si, st, c)) {
     HeavyAcc h;
     h.Add(st, c);
@@ -1909,6 +1905,7 @@ __device__ __forceinline__ void SmallFinishRow(const QuotientView& Q, Rows& S, i
   const int rep = S.q[i];
   const long long si = S.sz[i];
   const long long internal = Q.internal[rep];
+  if (!wide) S.old[i] = static_cast<int>(static_cast<unsigned>(S.old[i]));
   if (out) {
     long long light = S.light[i];
     if (wide) {
