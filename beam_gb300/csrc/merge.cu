@@ -5001,6 +5001,7 @@ void Engine::RunWindows(double threshold) {
                   d_ri_of_.p, count, W.real, R, cfg_.group_batch_size, d_node_ri_.p, d_blk_beg_.p, d_blk_end_.p,
                   W.dirty, W.ctl);
   W.max_groups = WindowTables(R);
+  W.mat_off = d_mat_off_.p;
   W.mat = d_mat_.p;
   ++launches_;
   LaunchFollowing(WindowBeginKernel, 1, kHugeThreads, 0, stream_, W, R);

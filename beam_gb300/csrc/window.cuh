@@ -157,8 +157,9 @@ struct WindowParams {
   BigGroup* list_big;
   long long* moff;      // member / part prefixes over list_big
   long long* poff;
-  unsigned char* mat;   // tables of the listed big groups
-  int max_groups;       // groups that a window takes in at most, by the room for their tables
+  const long long* mat_off;  // per group position: bytes of the tables before its own
+  unsigned char* mat;        // tables of the window's groups, from the first not committed
+  int max_groups;            // groups that a window takes in at most, by the room for their tables
   const long long* cand_off;
   unsigned long long* keys;  // two per candidate slot
   RowSums* rc;
@@ -238,12 +239,12 @@ __global__ void WindowSpanKernel(const long long* mat_off, const int* blk_beg, c
 // The next evaluation's lists, by one CTA of kHugeThreads: the touched groups
 // and those that the window takes in. `done`: groups [f, p) are committed.
 struct ListSum {
-  long long members, parts, mat;
+  long long members, parts;
   int small, big;
 };
 struct ListSumOp {
   __device__ __forceinline__ ListSum operator()(const ListSum& a, const ListSum& b) const {
-    return ListSum{a.members + b.members, a.parts + b.parts, a.mat + b.mat, a.small + b.small, a.big + b.big};
+    return ListSum{a.members + b.members, a.parts + b.parts, a.small + b.small, a.big + b.big};
   }
 };
 
@@ -252,6 +253,7 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
   __shared__ typename Scan::TempStorage tmp;
   __shared__ ListSum carry;
   __shared__ int s_e0, s_e1, s_dirty, s_again, s_kept, s_stale;
+  __shared__ long long s_mat0;  // the window's first table
   WindowCtl* c = P.ctl;
   if (threadIdx.x == 0) {
     // new groups are taken in for the next two rounds at the usual pace (the
@@ -271,9 +273,10 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
     s_dirty = c->ndirty;
     // (the next block in any case, so that every round commits one)
     s_again = max(c->f + max(2 * pace, kWindowMinAgain), c->f < c->R ? P.blk_end[c->f] : 0);
+    s_mat0 = P.mat_off[c->f];
     s_kept = 0;
     s_stale = 0x7fffffff;
-    carry = ListSum{0, 0, 0, 0, 0};
+    carry = ListSum{0, 0, 0, 0};
   }
   __syncthreads();
   const int n = s_dirty + (s_e1 - s_e0);
@@ -281,7 +284,7 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
     const int i = base + threadIdx.x;
     int ri = -1, g = 0, gid = 0;
     unsigned entries = 0;
-    ListSum v{0, 0, 0, 0, 0};
+    ListSum v{0, 0, 0, 0};
     bool later = false;
     if (i < n) {
       ri = i < s_dirty ? P.list_dirty[i] : s_e0 + (i - s_dirty);
@@ -302,19 +305,18 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
         v.big = 1;
         v.members = g;
         v.parts = static_cast<long long>(g) * WindowParts(entries);
-        v.mat = WindowBytes(g, entries);
       }
       GroupStats z = {};
       P.gs[ri] = z;
       P.conflict[ri] = 0x7fffffff;
     }
     ListSum ex, total;
-    Scan(tmp).ExclusiveScan(v, ex, ListSum{0, 0, 0, 0, 0}, ListSumOp(), total);
+    Scan(tmp).ExclusiveScan(v, ex, ListSum{0, 0, 0, 0}, ListSumOp(), total);
     const ListSum c0 = carry;
     if (v.small) P.list_small[c0.small + ex.small] = ri;
     if (v.big) {
       P.list_big[c0.big + ex.big] =
-          BigGroup{ri, gid, g, static_cast<int>(entries), P.gstart[gid], WindowParts(entries), c0.mat + ex.mat};
+          BigGroup{ri, gid, g, static_cast<int>(entries), P.gstart[gid], WindowParts(entries), P.mat_off[ri] - s_mat0};
       P.moff[c0.big + ex.big] = c0.members + ex.members;
       P.poff[c0.big + ex.big] = c0.parts + ex.parts;
     }
