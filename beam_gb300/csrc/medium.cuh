@@ -72,6 +72,7 @@ struct MediumSmem {
   unsigned long long acc[10];
   int nkeys, err[3], bad;
 };
+static_assert(kMedCtas * (sizeof(MediumSmem) + kSmemReserved) <= kSmemPerSm, "kMedCtas of them fit an SM");
 
 struct MediumParams {
   QuotientView Q;

@@ -41,6 +41,9 @@
 namespace beam {
 namespace {
 
+// Shared memory of an SM, and what every resident CTA takes of it beside its own.
+constexpr size_t kSmemPerSm = 228 << 10;
+constexpr size_t kSmemReserved = 1 << 10;
 constexpr int kPrepThreads = 512;
 constexpr int kLaneTopK = 32;        // per-lane candidate lists for top_k up to this
 constexpr int kSmemEntries = 2048;   // bucket entries held in shared memory

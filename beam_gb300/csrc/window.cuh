@@ -72,7 +72,7 @@ constexpr int kPartEntries = 1024;
 constexpr int kMaxParts = 128;
 constexpr int kPairWarps = 4;
 constexpr int kPairDeep = 4;  // entries per lane in flight
-constexpr int kPairCtas = 6;  // per SM
+constexpr int kPairCtas = 5;  // per SM: what shared memory holds (42 KB of tables each)
 constexpr int kPairGrid = 152 * kPairCtas;
 
 __host__ __device__ __forceinline__ int WindowParts(unsigned entries) {
@@ -376,6 +376,7 @@ struct EvalWarpSmem {
 struct EvalSmem {
   EvalWarpSmem w[kEvalWarps];
 };
+static_assert(kEvalCtas * (sizeof(EvalSmem) + kSmemReserved) <= kSmemPerSm, "the grid is one wave");
 
 // A small group by one warp: candidates, gains and selection.
 __device__ void EvalSmallGroup(const WindowParams& P, EvalWarpSmem& W, int ri) {
@@ -682,6 +683,7 @@ struct PairTable {
   unsigned cnt[kTableSlots];
   int4 hit[32 + 32 * kPairDeep];  // found: member, target's size, the member's count, the table's count
 };
+static_assert(kPairCtas * (kPairWarps * sizeof(PairTable) + kSmemReserved) <= kSmemPerSm, "the grid is one wave");
 
 __device__ __forceinline__ int StagedLowerBound(const StagedEntry* row, int len, int t) {
   int lo = 0, hi = len;
