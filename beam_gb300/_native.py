@@ -94,6 +94,7 @@ class FlatScorerStats(C.Structure):
         return {name: getattr(self, name) for name, _ in self._fields_}
 
 
+ROUTE_MEDIUM_GROUPS, ROUTE_WINDOW_ROUNDS, ROUTE_DEVICE_PLANS, ROUTE_HOST_PLANS = range(4)
 LIMIT_WINDOW_TABLES, LIMIT_ROW_SUM_ARCS = 1, 2
 TIME_NONE, TIME_SCORE, TIME_PREPARE, TIME_UPDATE, TIME_DIVIDE = 0, 1, 2, 3, 4
 
@@ -137,6 +138,7 @@ SIGNATURES = {
     "beam_ranker_grad": (C.c_int, [i32, vp, vp, vp, i64, vp, vp, P_f64, vp]),
     "beam_ranker_last_error": (C.c_char_p, []),
     "beam_engine_set_limit": (C.c_int, [vp, i32, i64]),
+    "beam_engine_route_count": (C.c_int, [vp, i32, P_i64]),
     "beam_engine_set_timed_kernel": (C.c_int, [vp, i32]),
     "beam_engine_timed_kernel": (C.c_int, [vp, P_f64, P_i64]),
     "beam_engine_synchronize": (C.c_int, [vp]),

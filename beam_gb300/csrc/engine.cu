@@ -864,6 +864,10 @@ int beam_engine_set_limit(beam_engine* e, int32_t which, int64_t value) {
   return Guard([&] { e->impl->SetLimit(which, value); });
 }
 
+int beam_engine_route_count(beam_engine* e, int32_t which, int64_t* count) {
+  return Guard([&] { *count = e->impl->RouteCount(which); });
+}
+
 int beam_engine_set_timed_kernel(beam_engine* e, int32_t which) {
   return Guard([&] { e->impl->SetTimedKernel(which); });
 }

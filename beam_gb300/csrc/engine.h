@@ -208,6 +208,9 @@ struct HostStats {
   uint64_t divide_fallback_splits = 0;
 };
 
+// Ways that an iteration's groups can go (BEAM_ROUTE_* of include/beam_gb300.h).
+enum Route : int { kRouteMediumGroups = 0, kRouteWindowRounds, kRouteDevicePlans, kRouteHostPlans, kRoutes };
+
 // Settable limits (BEAM_LIMIT_* of include/beam_gb300.h).
 enum Limit : int { kLimitWindowTables = 1, kLimitRowSumArcs = 2 };
 
@@ -260,6 +263,11 @@ class Engine {
 
   // Limits of internal choices (Limit).
   void SetLimit(int which, int64_t value);
+  // How often a Route was taken since creation.
+  int64_t RouteCount(int which) const {
+    if (which < 0 || which >= kRoutes) throw std::invalid_argument("unknown route");
+    return routes_[which];
+  }
 
   // Kernel timing for the roofline: events around every launch of one kernel class.
   void SetTimedKernel(int which);
@@ -440,6 +448,7 @@ class Engine {
 
   // launch accounting and step timing
   int64_t launches_ = 0;
+  int64_t routes_[kRoutes] = {};
   cudaEvent_t step_ev_[2] = {nullptr, nullptr};
   DevBuf<unsigned char> d_flush_;
 

@@ -4756,6 +4756,7 @@ void Engine::LaunchMedium(const BlockPlan& bp, double threshold) {
   M.block_stamp = block_stamp_;
   M.stats = d_stats_.p;
   M.err = d_err_.p;
+  routes_[kRouteMediumGroups] += bp.m1 - bp.m0;
   BeginTimed(kTimePrepare);
   ++launches_;
   LaunchFollowing(MediumKernel, bp.m1 - bp.m0, kMedThreads, sizeof(MediumSmem), stream_, M);
@@ -5041,6 +5042,7 @@ void Engine::RunWindows(double threshold) {
     // every round commits at least one block
     if (queued > R + kWindowAhead) throw std::runtime_error("merge windows made no progress");
     ++queued;
+    ++routes_[kRouteWindowRounds];
     ++block_stamp_;
     W.block_stamp = block_stamp_;
     BeginTimed(kTimePrepare);
@@ -5071,8 +5073,10 @@ void Engine::Merge(int iter, int total_iterations) {
   // ComputeMergeThreshold, reciprocal policy (src/sweg.cpp:400-406)
   const double threshold = 1.0 / static_cast<double>(iter + 1);
   if (plan_on_device_ || windowed_) {
+    if (!windowed_) ++routes_[kRouteDevicePlans];
     PlanOnDevice();
   } else {
+    ++routes_[kRouteHostPlans];
     EnsurePoolRoom();
     PrepareIterationBuffers();
   }

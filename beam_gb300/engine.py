@@ -259,6 +259,12 @@ class Engine:
         """One of the engine's limits (LIMIT_* of _native); results do not depend on it."""
         N.check(N.lib().beam_engine_set_limit(self._h, which, value))
 
+    def route_count(self, which: int) -> int:
+        """How often a ROUTE_* of _native was taken since creation."""
+        out = C.c_int64()
+        N.check(N.lib().beam_engine_route_count(self._h, which, C.byref(out)))
+        return int(out.value)
+
     def set_timed_kernel(self, which: int) -> None:
         N.check(N.lib().beam_engine_set_timed_kernel(self._h, which))
 

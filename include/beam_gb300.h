@@ -204,6 +204,21 @@ int beam_engine_quotient_nnz(beam_engine* e, int64_t* nnz);
  *     most: the sums' fields hold no more]; takes effect with the next Divide */
 enum { BEAM_LIMIT_WINDOW_TABLES = 1, BEAM_LIMIT_ROW_SUM_ARCS = 2 };
 int beam_engine_set_limit(beam_engine* e, int32_t which, int64_t value);
+/* How often the engine took one of its ways since creation, so that a test or a
+ * measurement that aims at one can tell. Which way is taken does not change a
+ * result.
+ *   BEAM_ROUTE_MEDIUM_GROUPS  groups that one kernel took from rows to pairs
+ *   BEAM_ROUTE_WINDOW_ROUNDS  rounds of the plain form's windows, queued ahead
+ *     and found empty included
+ *   BEAM_ROUTE_DEVICE_PLANS   iterations of blocks planned on the device
+ *   BEAM_ROUTE_HOST_PLANS     iterations of blocks planned on the host */
+enum {
+  BEAM_ROUTE_MEDIUM_GROUPS = 0,
+  BEAM_ROUTE_WINDOW_ROUNDS = 1,
+  BEAM_ROUTE_DEVICE_PLANS = 2,
+  BEAM_ROUTE_HOST_PLANS = 3
+};
+int beam_engine_route_count(beam_engine* e, int32_t which, int64_t* count);
 /* CUDA-event timing of every launch of one kernel class (BEAM_TIME_*). */
 int beam_engine_set_timed_kernel(beam_engine* e, int32_t which);
 int beam_engine_timed_kernel(beam_engine* e, double* ms, int64_t* launches);
