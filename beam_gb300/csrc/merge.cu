@@ -4991,6 +4991,7 @@ void Engine::RunWindows(double threshold) {
   W.threshold = threshold;
   W.thr = SplitThreshold(threshold);
   W.use_threshold = cfg_.ea_use_threshold ? 1 : 0;
+  W.all_strict = cfg_.group_batch_size <= kFewGroups ? 1 : 0;
   W.stats = d_stats_.p;
   W.err = d_err_.p;
   // the frontier and the rounds done, written by the device after each round

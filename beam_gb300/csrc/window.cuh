@@ -178,6 +178,7 @@ struct WindowParams {
   double threshold;
   ThresholdBits thr;
   int use_threshold;
+  int all_strict;  // no block has more than kFewGroups groups
   unsigned long long* stats;
   DevError* err;
   volatile int* host_f;  // mapped: the frontier, and the lists made so far
@@ -356,6 +357,12 @@ __global__ void __launch_bounds__(kHugeThreads) WindowBeginKernel(WindowParams P
 
 // ------------------------------------------------------------ evaluation
 
+// Whether a pair of this group is checked against its rows' own capacities too,
+// as for a block committed by itself (ScoreParams::strict).
+__device__ __forceinline__ int WindowStrict(const WindowParams& P, int ri) {
+  return P.all_strict || P.blk_end[ri] - P.blk_beg[ri] <= kFewGroups ? 1 : 0;
+}
+
 // First later group (another block) that merging a and b touches: by a warp,
 // over one row given by its entries.
 __device__ __forceinline__ int FirstTouched(const WindowParams& P, const Entry* row, int len, int end, int first,
@@ -407,6 +414,7 @@ __device__ void EvalSmallGroup(const WindowParams& P, EvalWarpSmem& W, int ri) {
     return slow ? SmallMerge(S, a, b).proxy : static_cast<long long>(W.pairs.pc[TriIndex(a, b, g)] >> 32);
   });
   // gains of the kept pairs, one lane each; the keys of those that pass
+  const int strict = WindowStrict(P, ri);
   long long uni = 0, ovl = 0, raw_a = 0, raw_b = 0, nnz = 0;
   int cand = 0, passed = 0, err = 0, err_a = 0, err_b = 0;
   for (int pidx = lane; pidx < npairs; pidx += 32) {
@@ -417,7 +425,7 @@ __device__ void EvalSmallGroup(const WindowParams& P, EvalWarpSmem& W, int ri) {
       const PairInfo pi = SmallPairInfo(S, a, b, SmallPairAt(S, W.pairs, pidx, a, b, slow));
       const RowSums &A = W.rs[a], &B = W.rs[b];
       GainParts gp;
-      if (!GainFromSums(A, B, pi, 1, &gp)) {
+      if (!GainFromSums(A, B, pi, strict, &gp)) {
         const long long s = static_cast<long long>(A.size) + B.size;
         long long part;
         if (!RowAfter(A, s, &part)) gp.gain += part - StagedRowAfter(S, a, s);
@@ -900,6 +908,7 @@ __global__ void __launch_bounds__(256, 2) WindowScoreKernel(WindowParams P) {
     if (n == 0) continue;
     GroupStats* gs = P.gs + ri;
     unsigned long long* keys = P.keys + 2 * P.cand_off[ri];
+    const int strict = WindowStrict(P, ri);
     long long uni = 0, ovl = 0, raw_a = 0, raw_b = 0, nnz = 0;
     for (int k0 = 0; k0 < n; k0 += 32) {
       const bool have = k0 + lane < n;
@@ -917,7 +926,7 @@ __global__ void __launch_bounds__(256, 2) WindowScoreKernel(WindowParams P) {
         B = P.rc[qb];
         const PairInfo pi = PairInfoOf(Q, qa, qb, pmat[static_cast<long long>(a) * g + b],
                                        static_cast<long long>(pmat[static_cast<long long>(b) * g + a]));
-        sums = GainFromSums(A, B, pi, 1, &gp);
+        sums = GainFromSums(A, B, pi, strict, &gp);
       }
       for (unsigned rest = __ballot_sync(kFull, !sums); rest; rest &= rest - 1) {
         const int src = __ffs(rest) - 1;

@@ -38,3 +38,47 @@ def test_small_groups_match_the_oracle(copies, targets, q):
     o = Oracle.from_graph(g, top_k=1)
     with Engine(g, top_k=1) as e:
         assert np.array_equal(e.prepare_group(q), o.prepare_group(q))
+
+
+def twins_with_leaves(clusters):
+    """Pairs of twins with six targets of their own; the first twin has a leaf too.
+    Edges and the leaf edges, one of each a cluster."""
+    c = 9 * np.arange(clusters)
+    e = [(c + m, c + 2 + t) for m in (0, 1) for t in range(6)]
+    u, v = (np.concatenate(x) for x in zip(*e))
+    return u, v, np.stack([c, c + 8], 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", [700, 1024, 1025, 4096, 1 << 30])
+def test_large_blocks_check_counts_at_the_merged_size(batch):
+    """A leaf edge given twice is beyond the capacity of two single nodes, but
+    not beyond that of the merged twins and the leaf. Blocks of more than 256
+    groups of two members or more accept the merge (smaller ones report the
+    state, as the reference does). The leaf, alone in its group, takes part in
+    no pair, and the twins' gain of 5 for 6 decides nothing: the partition is the
+    one of the graph without repeated edges."""
+    from beam_gb300 import Engine, Graph
+    from oracle import Oracle
+    u, v, leaf = twins_with_leaves(2000)
+    once = Graph.from_edges(np.concatenate([u, leaf[:, 0]]).astype(np.int32),
+                            np.concatenate([v, leaf[:, 1]]).astype(np.int32))
+    kw = {"ea_use_threshold": True, "group_batch_size": batch}
+    o = Oracle.from_graph(once, **kw)
+    o.divide(4)
+    order, starts, lengths = o.groups()
+    real = np.array([(lengths[i:i + batch] >= 2).sum() for i in range(0, len(lengths), batch)])
+    group = np.zeros(once.n, int)
+    group[order] = np.repeat(np.arange(len(starts)), lengths)
+    first, alone = group[leaf[:, 0]], lengths[group[leaf[:, 1]]] == 1
+    twice = leaf[(first == group[leaf[:, 0] + 1]) & alone & (real[first // batch] > 256)]
+    assert len(twice) > 100
+    g = Graph.from_edges(np.concatenate([u, leaf[:, 0], twice[:, 0]]).astype(np.int32),
+                         np.concatenate([v, leaf[:, 1], twice[:, 1]]).astype(np.int32))
+    o.merge(4)
+    assert (o.labels()[twice[:, 0] + 1] == twice[:, 0]).sum() > 100
+    with Engine(g, **kw) as e:
+        e.divide(4)
+        e.merge(4)
+        assert np.array_equal(e.partition()[0], o.labels())
+        e.validate_quotient()
