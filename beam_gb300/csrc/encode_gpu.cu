@@ -12,7 +12,8 @@
 //   Cm                 per dense block with missing pairs, every member pair is
 //                      looked up among the block's sorted edges
 // The lengths of the lists alone (EncodeCounts) need no list: the quotient
-// rows hold every block's edge count.
+// rows hold every block's edge count, which is its number of joined member pairs
+// where no edge is repeated.
 // P comes out sorted; Cp and Cm are radix-sorted by (u, v). The host writes
 // G.txt / P.txt / Cp.txt / Cm.txt with the same formatting as beam_encode.
 #include <cub/device/device_radix_sort.cuh>
@@ -75,9 +76,24 @@ __global__ void ArcKeyKernel(const int* __restrict__ arc_src, const int* __restr
   }
 }
 
-// per block: Cp count, Cm count, superedge flag
+// Edges that a block lists again, for inputs with repeated edges: equal arcs are
+// neighbours in the order of the sort. A thread per sorted edge position.
+__global__ void RepeatedEdgesKernel(const unsigned long long* __restrict__ key, const int* __restrict__ arc,
+                                    const int* __restrict__ arc_src, const int* __restrict__ col,
+                                    const long long* __restrict__ run_off, int nruns, long long positions,
+                                    int* __restrict__ again) {
+  for (long long p = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x + 1; p < positions;
+       p += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int k = arc[p], before = arc[p - 1];
+    if (key[p] == kNone || key[p] != key[p - 1] || arc_src[k] != arc_src[before] || col[k] != col[before]) continue;
+    atomicAdd(&again[OwnerOfSlot(run_off, 0, nruns, p)], 1);
+  }
+}
+
+// per block: Cp count, Cm count, superedge flag (again: edges listed again, nullptr: none)
 __global__ void BlockDecideKernel(const unsigned long long* __restrict__ uniq, const int* __restrict__ cnt,
-                                  const int* __restrict__ nruns_p, const int* __restrict__ ssize,
+                                  const int* __restrict__ again, const int* __restrict__ nruns_p,
+                                  const int* __restrict__ ssize,
                                   long long* __restrict__ cp_n, long long* __restrict__ cm_n,
                                   long long* __restrict__ p_n, int max_runs) {
   const int nruns = *nruns_p;
@@ -93,7 +109,7 @@ __global__ void BlockDecideKernel(const unsigned long long* __restrict__ uniq, c
         cp = real;
       } else {
         p = 1;
-        cm = cap - real;
+        cm = cap - (again ? real - again[r] : real);
       }
     }
     cp_n[r] = cp;
@@ -167,8 +183,10 @@ __global__ void DenseUnitsKernel(EmitParams E, DenseUnit* units, unsigned long l
   }
 }
 
-// A warp per unit: the pairs without an edge.
-__global__ void EmitMissingKernel(EmitParams E, const DenseUnit* units, const unsigned long long* nunits) {
+// A warp per unit: the pairs without an edge. (More of them than the block's
+// room are those of a row out of order.)
+__global__ void EmitMissingKernel(EmitParams E, const DenseUnit* units, const unsigned long long* nunits,
+                                  DevError* err) {
   const int lane = threadIdx.x & 31;
   const long long total = static_cast<long long>(*nunits);
   const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -181,7 +199,7 @@ __global__ void EmitMissingKernel(EmitParams E, const DenseUnit* units, const un
     const int* mb = E.members + E.moff[B];
     const long long lo0 = E.run_off[r];
     const long long hi0 = lo0 + E.cnt[r];
-    const long long cm_base = E.cm_off[r];
+    const long long cm_base = E.cm_off[r], room = E.cm_off[r + 1] - cm_base;
     const long long t1 = units[w].t0 + kDenseUnit < sa * sb ? units[w].t0 + kDenseUnit : sa * sb;
     for (long long t = units[w].t0 + lane; t < t1; t += 32) {
       const int u = ma[t / sb];
@@ -202,6 +220,10 @@ __global__ void EmitMissingKernel(EmitParams E, const DenseUnit* units, const un
       }
       if (!present) {
         const unsigned at = atomicAdd(&E.cm_fill[r], 1u);
+        if (at >= room) {
+          RaiseError(err, kErrGraph, u, v, 0);
+          continue;
+        }
         E.Cm[cm_base + at] = static_cast<unsigned long long>(u) << 32 | static_cast<unsigned>(v);
       }
     }
@@ -274,6 +296,7 @@ __global__ void __launch_bounds__(1024) EncodeLongRowsKernel(QuotientView Q, uns
 }  // namespace
 
 void Engine::EncodeCounts(EncodeOutput* out) {
+  if (repeats_) return Encode(out);  // a row's counts do not tell how many member pairs they cover
   AllocScope alloc(stream_);
   d_pc_scalars_.ensure(8);
   CheckCuda(cudaMemsetAsync(d_pc_scalars_.p, 0, 8 * sizeof(unsigned long long), stream_), "memset counts");
@@ -410,8 +433,16 @@ void Engine::Encode(EncodeOutput* out) {
     WidenKernel<<<(nruns + T) / T, T, 0, s>>>(cnt.p, nruns, cnt64.p);
     scan_ll(cnt64.p, run_off.p, nruns + 1);
   }
+  DevBuf<int> again;
+  if (repeats_) {
+    again.ensure(ur);
+    CheckCuda(cudaMemsetAsync(again.p, 0, sizeof(int) * ur, s), "memset");
+    ++launches_;
+    RepeatedEdgesKernel<<<blocks(arcs), T, 0, s>>>(akey2.p, arc_sorted.p, d_arc_src_.p, d_col_.p, run_off.p, nruns, arcs,
+                                                   again.p);
+  }
   ++launches_;
-  BlockDecideKernel<<<blocks(nruns + 1), T, 0, s>>>(uniq.p, cnt.p, nruns_d, ssize.p, cp_n.p, cm_n.p, p_n.p,
+  BlockDecideKernel<<<blocks(nruns + 1), T, 0, s>>>(uniq.p, cnt.p, again.p, nruns_d, ssize.p, cp_n.p, cm_n.p, p_n.p,
                                                     nruns + 1);
   scan_ll(cp_n.p, cp_off.p, nruns + 1);
   scan_ll(cm_n.p, cm_off.p, nruns + 1);
@@ -455,7 +486,7 @@ void Engine::Encode(EncodeOutput* out) {
   CheckCuda(cudaMemsetAsync(nunits.p, 0, sizeof(unsigned long long), s), "memset");
   DenseUnitsKernel<<<blocks(nruns), T, 0, s>>>(E, units.p, nunits.p);
   ++launches_;
-  EmitMissingKernel<<<152 * 8, T, 0, s>>>(E, units.p, nunits.p);
+  EmitMissingKernel<<<152 * 8, T, 0, s>>>(E, units.p, nunits.p, d_err_.p);
   if (ncp > 0) sort_keys(Cp.p, Cp2.p, ncp);
   if (ncm > 0) sort_keys(Cm.p, Cm2.p, ncm);
   out->supernodes = S;

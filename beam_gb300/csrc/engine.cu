@@ -104,7 +104,7 @@ constexpr int kInitWarpRow = 512;
 __global__ void InitRowsKernel(const long long* __restrict__ rowptr, const int* __restrict__ col, int n,
                                Entry* __restrict__ pool, long long* __restrict__ qoff, int* __restrict__ qlen,
                                int* __restrict__ qcap, int* __restrict__ arc_src, int* __restrict__ long_rows,
-                               unsigned* __restrict__ nlong, DevError* err) {
+                               unsigned* __restrict__ nlong, unsigned* __restrict__ repeats, DevError* err) {
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long nw = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -138,6 +138,7 @@ __global__ void InitRowsKernel(const long long* __restrict__ rowptr, const int* 
       qoff[u] = s;
       qlen[u] = rank;
       qcap[u] = static_cast<int>(e - s);
+      if (rank != e - s) *repeats = 1;
     }
   }
 }
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(kInitThreads)
     InitLongRowsKernel(const long long* __restrict__ rowptr, const int* __restrict__ col, int n,
                        Entry* __restrict__ pool, long long* __restrict__ qoff, int* __restrict__ qlen,
                        int* __restrict__ qcap, int* __restrict__ arc_src, const int* __restrict__ long_rows,
-                       const unsigned* __restrict__ nlong, DevError* err) {
+                       const unsigned* __restrict__ nlong, unsigned* __restrict__ repeats, DevError* err) {
   __shared__ int totals[2][kInitThreads / 32];
   const int lane = threadIdx.x & 31;
   const int wid = threadIdx.x >> 5;
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(kInitThreads)
       qoff[u] = s;
       qlen[u] = rank;
       qcap[u] = static_cast<int>(e - s);
+      if (rank != e - s) *repeats = 1;
     }
   }
 }
@@ -359,16 +361,21 @@ void Engine::Reset() {
   CheckCuda(cudaMemsetAsync(d_wctl_.p, 0, 256, stream_), "memset window control");
   launches_ += 2;
   InitRowsKernel<<<152 * 16, 256, 0, stream_>>>(d_rowptr_.p, d_col_.p, n_, d_pool_[0].p, d_qoff_.p, d_qlen_.p,
-                                                d_qcap_.p, d_arc_src_.p, d_rows_long_.p, d_rw_ticket_.p, d_err_.p);
+                                                d_qcap_.p, d_arc_src_.p, d_rows_long_.p, d_rw_ticket_.p, &d_ctl_.p->repeats,
+                                                d_err_.p);
   InitLongRowsKernel<<<152 * 4, kInitThreads, 0, stream_>>>(d_rowptr_.p, d_col_.p, n_, d_pool_[0].p, d_qoff_.p,
                                                             d_qlen_.p, d_qcap_.p, d_arc_src_.p, d_rows_long_.p,
-                                                            d_rw_ticket_.p, d_err_.p);
+                                                            d_rw_ticket_.p, &d_ctl_.p->repeats, d_err_.p);
+  CheckCuda(cudaMemcpyAsync(h_pin_.p + 58, &d_ctl_.p->repeats, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_),
+            "d2h repeated edges");
   CheckCuda(cudaMemsetAsync(d_rw_ticket_.p, 0, sizeof(unsigned), stream_), "memset ticket");
   const unsigned long long top = static_cast<unsigned long long>(arcs_);
   CheckCuda(cudaMemcpyAsync(d_pool_top_.p, &top, sizeof(top), cudaMemcpyHostToDevice, stream_), "h2d pool top");
   CheckCuda(cudaMemsetAsync(d_stats_.p, 0, sizeof(unsigned long long) * kStCount, stream_), "memset stats");
-  CheckCuda(cudaStreamSynchronize(stream_), "reset sync");
   CheckError();
+  unsigned repeats = 0;
+  std::memcpy(&repeats, h_pin_.p + 58, sizeof(repeats));
+  repeats_ = repeats != 0;
   block_stamp_ = 0;
   need_stamp_ = 0;
   n_groups_ = -1;

@@ -180,7 +180,7 @@ struct BlockCtl {
   unsigned int sel_total;   // selected pairs of the block (entries of the selection list)
   unsigned int huge_cnt;    // claimed neighbour rows rewritten in two steps
   unsigned int huge_units;  // their scan units
-  unsigned int pad;
+  unsigned int repeats;     // written by Reset: the input lists some edge more than once
   // work queues of the dynamically scheduled kernels: the accumulate pass and
   // the two scoring passes (exploration / the rest, or the only one)
   unsigned long long work_next[3];
@@ -447,6 +447,7 @@ class Engine {
   RankerInfo rk_info_;
 
   // launch accounting and step timing
+  bool repeats_ = false;  // the input lists some edge more than once
   int64_t launches_ = 0;
   int64_t routes_[kRoutes] = {};
   cudaEvent_t step_ev_[2] = {nullptr, nullptr};
