@@ -327,7 +327,10 @@ void Engine::Encode(EncodeOutput* out) {
   const long long arcs = arcs_;
   cudaStream_t s = stream_;
   const int T = 256;
-  auto blocks = [&](long long items) { return static_cast<int>(std::min<long long>((items + T - 1) / T, 152 * 16)); };
+  // (one block at least: the kernels find nothing to do in a graph without edges)
+  auto blocks = [&](long long items) {
+    return static_cast<int>(std::clamp<long long>((items + T - 1) / T, 1, 152 * 16));
+  };
   auto sort_pairs = [&](const unsigned long long* kin, unsigned long long* kout, const int* vin, int* vout,
                         long long items) {
     size_t bytes = 0;
@@ -406,6 +409,7 @@ void Engine::Encode(EncodeOutput* out) {
   ArcKeyKernel<<<blocks(arcs), T, 0, s>>>(d_arc_src_.p, d_col_.p, nts.p, arcs, akey.p, arc_val.p);
   sort_pairs(akey.p, akey2.p, arc_val.p, arc_sorted.p, arcs);
   int* nruns_d = reinterpret_cast<int*>(ll.p);
+  CheckCuda(cudaMemsetAsync(nruns_d, 0, sizeof(int), s), "memset");
   {
     size_t bytes = 0;
     CheckCuda(cub::DeviceRunLengthEncode::Encode(nullptr, bytes, akey2.p, uniq.p, cnt.p, nruns_d, arcs, s),

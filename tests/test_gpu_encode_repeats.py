@@ -83,3 +83,29 @@ def test_repeats_of_one_graph_are_not_the_next_ones(tmp_path):
             for _ in range(2):
                 compare(e, g, o, tmp_path)
                 e.reset()
+
+
+@pytest.mark.parametrize("n", [1, 4, 300])
+def test_graph_without_edges(n, tmp_path):
+    from beam_gb300 import Engine
+    from oracle import Oracle
+
+    class Edgeless:
+        def __init__(self):
+            self.n, self.arcs = n, 0
+            self.row_ptr, self.col_idx = np.zeros(n + 1, np.int64), np.zeros(0, np.int32)
+
+    o = Oracle(np.zeros(n + 1, np.int64), np.zeros(0, np.int32))
+    (tmp_path / "a").mkdir()
+    (tmp_path / "c").mkdir()
+    with Engine(Edgeless()) as e:
+        for merged in (False, True):
+            files, ref = e.encode(tmp_path / "a"), o.encode(tmp_path / "c")
+            assert files == e.encode() and files["supernodes"] == ref["n_supernodes"]
+            assert files["encoding_cost_mags_x2"] == ref["encoding_cost_mags_x2"] == 0
+            for f in FILES:
+                assert (tmp_path / "a" / f).read_bytes() == (tmp_path / "c" / f).read_bytes(), f
+            if n > 2 and not merged:
+                e.merge_pairs([0], [2])
+                o.merge_pair(0, 2)
+        e.run(2)
