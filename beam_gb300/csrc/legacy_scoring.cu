@@ -64,7 +64,7 @@ __device__ __forceinline__ void FlatLowerBounds(const int* nb, int s, int e, con
 #pragma unroll
     for (int d = 0; d < kFlatDeep; ++d) {
       if (lo[d] < hi[d]) {
-        const int mid = (lo[d] + hi[d]) >> 1;
+        const int mid = lo[d] + ((hi[d] - lo[d]) >> 1);  // up to 2^31 - 1 entries in a call
         if (nb[mid] < key[d]) lo[d] = mid + 1; else hi[d] = mid;
       }
     }
@@ -89,38 +89,40 @@ __device__ __forceinline__ void LegacyTerm(const LegacyPair& p, int x, long long
   *after += EncodeCostForPair(p.ra, p.sm, mrep, msz, ea + eb);
 }
 
-// The pair's terms over entries first, first + stride, ... of both rows.
+// The pair's terms over entries first, first + stride, ... of both rows (unsigned
+// positions: the steps may pass 2^31 beyond a last entry near it).
 struct LegacySums {
   long long before = 0, after = 0;
   bool seen_a = false, seen_b = false;
 };
 
 __device__ __forceinline__ void LegacyRows(const FlatView& F, const LegacyPair& p, int a0, int a1, int b0, int b1,
-                                           int first, int stride, LegacySums* s) {
-  for (int k0 = a0 + first; k0 < a1; k0 += stride * kFlatDeep) {
+                                           unsigned first, unsigned stride, LegacySums* s) {
+  const unsigned end_a = static_cast<unsigned>(a1), end_b = static_cast<unsigned>(b1);
+  for (unsigned k0 = static_cast<unsigned>(a0) + first; k0 < end_a; k0 += stride * kFlatDeep) {
     int x[kFlatDeep], at[kFlatDeep];
 #pragma unroll
-    for (int d = 0; d < kFlatDeep; ++d) x[d] = k0 + d * stride < a1 ? F.nb[k0 + d * stride] : 0x7fffffff;
+    for (int d = 0; d < kFlatDeep; ++d) x[d] = k0 + d * stride < end_a ? F.nb[k0 + d * stride] : 0x7fffffff;
     FlatLowerBounds(F.nb, b0, b1, x, at);
 #pragma unroll
     for (int d = 0; d < kFlatDeep; ++d) {
-      const int k = k0 + d * stride;
-      if (k >= a1) continue;
+      const unsigned k = k0 + d * stride;
+      if (k >= end_a) continue;
       const long long eb = at[d] < b1 && F.nb[at[d]] == x[d] ? F.wt[at[d]] : 0;
       LegacyTerm(p, x[d], F.nsz[k], F.wt[k], eb, &s->before, &s->after);
       s->seen_a |= x[d] == p.ra;
       s->seen_b |= x[d] == p.rb;
     }
   }
-  for (int k0 = b0 + first; k0 < b1; k0 += stride * kFlatDeep) {
+  for (unsigned k0 = static_cast<unsigned>(b0) + first; k0 < end_b; k0 += stride * kFlatDeep) {
     int x[kFlatDeep], at[kFlatDeep];
 #pragma unroll
-    for (int d = 0; d < kFlatDeep; ++d) x[d] = k0 + d * stride < b1 ? F.nb[k0 + d * stride] : 0x7fffffff;
+    for (int d = 0; d < kFlatDeep; ++d) x[d] = k0 + d * stride < end_b ? F.nb[k0 + d * stride] : 0x7fffffff;
     FlatLowerBounds(F.nb, a0, a1, x, at);
 #pragma unroll
     for (int d = 0; d < kFlatDeep; ++d) {
-      const int k = k0 + d * stride;
-      if (k >= b1 || (at[d] < a1 && F.nb[at[d]] == x[d])) continue;
+      const unsigned k = k0 + d * stride;
+      if (k >= end_b || (at[d] < a1 && F.nb[at[d]] == x[d])) continue;
       LegacyTerm(p, x[d], F.nsz[k], 0, F.wt[k], &s->before, &s->after);
       s->seen_a |= x[d] == p.ra;
       s->seen_b |= x[d] == p.rb;
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(kLegacyThreads) LegacyFlatScoreKernel(FlatView
         const int2 pr = pairs[w];
         const int a0 = F.off[pr.x], a1 = F.off[pr.x + 1];
         const int b0 = F.off[pr.y], b1 = F.off[pr.y + 1];
-        mine = pass > 0 || (a1 - a0) + (b1 - b0) <= kFlatLong;
+        mine = pass > 0 || static_cast<long long>(a1 - a0) + (b1 - b0) <= kFlatLong;
         if (mine) {
           p.ra = F.rep[pr.x];
           p.rb = F.rep[pr.y];

@@ -124,3 +124,60 @@ def test_gpu_matches_oracle_over_several_trips(count):
             gain, before = scorer.score(flat, pairs)
             assert np.array_equal(gain, want_gain)
             assert np.array_equal(before, want_before)
+
+
+def steps(first, end, lane, stride, deep, wrap):
+    """Positions that one lane visits of the row entries [first, end): four steps
+    of `stride` in flight, in 32-bit arithmetic of the given kind."""
+    k0, seen, turns = wrap(first + lane), [], 0
+    while k0 < end and turns < 40:  # (a position that wraps never ends)
+        for d in range(deep):
+            k = wrap(k0 + d * stride)
+            if k < end:
+                seen.append(k)
+        k0 = wrap(k0 + stride * deep)
+        turns += 1
+    return seen
+
+
+def lower_bound_mids(lo, hi, at, wrap, mid):
+    out = []
+    span = hi - lo
+    while span > 0:
+        if lo < hi:
+            m = mid(lo, hi, wrap)
+            out.append(m)
+            if m < at:
+                lo = m + 1
+            else:
+                hi = m
+        span >>= 1
+    return out, lo
+
+
+def test_positions_near_the_largest_entry_count():
+    """LegacyRows and FlatLowerBounds on rows that end at 2^31 - 1, the most
+    entries a call takes: every position once and none outside the row."""
+    def unsigned(x):
+        return x % (1 << 32)
+
+    def signed(x):
+        return (x + (1 << 31)) % (1 << 32) - (1 << 31)
+
+    top = (1 << 31) - 1
+    for length, stride in ((1, 32), (33, 32), (700, 32), (5000, 256), (4096, 256)):
+        for end in (top, top - 1, top - 1023, 5000):
+            first = end - length
+            seen = sorted(k for lane in range(stride) for k in steps(first, end, lane, stride, 4, unsigned))
+            assert seen == list(range(first, end))
+    wrapped = [k for lane in range(32) for k in steps(top - 33, top, lane, 32, 4, signed)]
+    assert min(wrapped) < 0  # what signed positions did there
+    rng = random.Random(2)
+    for _ in range(2000):
+        lo = rng.choice((0, 1 << 30, top - 5000))
+        hi = min(top, lo + rng.choice((1, 2, 31, 4999, 1 << 29)))
+        at = rng.randint(lo, hi)
+        mids, found = lower_bound_mids(lo, hi, at, signed, lambda l, h, w: w(l + ((h - l) >> 1)))
+        assert found == at and all(lo <= m < hi for m in mids)
+    mids, _ = lower_bound_mids(1 << 30, (1 << 30) + 9, 1 << 30, signed, lambda l, h, w: w(l + h) >> 1)
+    assert min(mids) < 0  # what the sum of both ends did there
