@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kLegacyThreads) LegacyFlatScoreKernel(FlatView
     }
     // A pass that is skipped has no barrier: without this one a warp could write
     // the next eight pairs' flags while another still reads these.
-    __syncthreads();
+    if (w0 + static_cast<long long>(gridDim.x) * kWarps < count) __syncthreads();
   }
 }
 

@@ -3,7 +3,7 @@
 
 On the CPU: the kernel's passes and barriers restated warp by warp under random
 schedules. The flags of the long pairs are read by passes that may be skipped,
-and a skipped pass has no barrier, so the trip has to end with one.
+and a skipped pass has no barrier, so a trip that is not the last has to end with one.
 
 On the GPU: more than four trips of pairs, long and short ones changing places
 from trip to trip, against the oracle. Integer work: every value must be equal."""
@@ -27,7 +27,7 @@ class Stuck(Exception):
 
 def run_cta(pairs, closing, rng):
     """One CTA over `pairs` ((long?, value) each, WARPS a trip), one step of one
-    warp at a time; returns the results. closing: the trip ends with a barrier."""
+    warp at a time; returns the results. closing: a barrier between two trips."""
     is_long, part, out = [False] * WARPS, [0] * WARPS, [None] * len(pairs)
 
     def warp(me):
@@ -53,7 +53,7 @@ def run_cta(pairs, closing, rng):
                 if p == 0:
                     is_long[me] = w < len(pairs) and not mine
                 yield "barrier"
-            if closing:
+            if closing and w0 + WARPS < len(pairs):
                 yield "barrier"
 
     warps = {i: warp(i) for i in range(WARPS)}
