@@ -70,6 +70,7 @@ void DeviceFree(void* p, cudaStream_t s) {
 
 void CheckCuda(cudaError_t status, const char* what) {
   if (status != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by a later call that asks for the last error
     throw std::runtime_error(std::string(what) + " failed: " + cudaGetErrorString(status));
   }
 }

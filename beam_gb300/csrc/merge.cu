@@ -4915,7 +4915,6 @@ int Engine::WindowTables(int R) {
       d_mat_.ensure(static_cast<size_t>(bytes) + 256);
       return true;
     } catch (const std::runtime_error&) {
-      cudaGetLastError();  // a failed allocation is no later call's error
       return false;
     }
   };
