@@ -257,27 +257,31 @@ __device__ __noinline__ void BuildLists(const WindowParams& P) {
   __shared__ long long s_mat0;  // the window's first table
   WindowCtl* c = P.ctl;
   if (threadIdx.x == 0) {
+    // (what does not wait for the pace is loaded first: one memory latency)
+    const int f = c->p, e0 = c->e, R = c->R;
+    const int next = f < R ? P.blk_end[f] : 0;
+    const long long mat0 = P.mat_off[f];
     // new groups are taken in for the next two rounds at the usual pace (the
     // whole window again where all of it was committed); a touched group is
     // evaluated again when its turn is that near, not every time it is touched
-    const int committed = c->p - c->f;
+    const int committed = f - c->f;
     int pace = c->pace;
-    if (c->p > 0) pace = c->p == c->e ? max(committed, pace) : (3 * pace + committed) / 4;
+    if (f > 0) pace = f == e0 ? max(committed, pace) : (3 * pace + committed) / 4;
     pace = min(pace, kWindowMaxGroups / 2);
-    c->pace = pace;
-    c->f = c->p;
     const int take = min(max(2 * pace, kWindowMinGroups), P.max_groups);
-    int e = c->f + take;
-    e = e >= c->R ? c->R : e == 0 ? 0 : P.blk_end[e - 1];
-    s_e0 = c->e;
-    s_e1 = e > c->e ? e : c->e;
+    int e = f + take;
+    e = e >= R ? R : e == 0 ? 0 : P.blk_end[e - 1];
+    s_e0 = e0;
+    s_e1 = e > e0 ? e : e0;
     s_dirty = c->ndirty;
     // (the next block in any case, so that every round commits one)
-    s_again = max(c->f + max(2 * pace, kWindowMinAgain), c->f < c->R ? P.blk_end[c->f] : 0);
-    s_mat0 = P.mat_off[c->f];
+    s_again = max(f + max(2 * pace, kWindowMinAgain), next);
+    s_mat0 = mat0;
     s_kept = 0;
     s_stale = 0x7fffffff;
     carry = ListSum{0, 0, 0, 0};
+    c->pace = pace;
+    c->f = f;
   }
   __syncthreads();
   const int n = s_dirty + (s_e1 - s_e0);
