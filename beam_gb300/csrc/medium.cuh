@@ -27,7 +27,15 @@ constexpr int kMedCtas = 3;  // per SM
 // iteration, is even; Chung-Lu 1M, 14,000 to 25,000, 138 -> 116 ms a run; the
 // 16,384-group blocks of the grid + Chung-Lu union, a handful, 335 -> 354 ms.)
 constexpr int kMedMinGroups = 2 * 152;
-// An iteration planned on the device counts its groups of all sizes instead.
+// An iteration planned on the device goes by its groups of all sizes instead,
+// which the host knows before the plan; the medium ones among them would tell
+// better. 20 iterations without the kernel -> with it, groups of iteration 1 and
+// medium groups an iteration: Chung-Lu (degree 17) 3,493 / 370 15.8 -> 16.0 ms,
+// 10,409 / 1,090 22.2 -> 21.4, 35,682 / 3,560 38.9 -> 34.9, 92,925 / 8,830 73.1
+// -> 61.0; R-MAT 15 and 17 (edge factor 8) 19,549 / 170 17.0 -> 17.8 and 82,247 /
+// 620 27.1 -> 27.6; R-MAT 18 and 19 (edge factor 2) 205,762 / 450 21.65 -> 21.97
+// and 418,211 / 890 27.8 -> 27.5; the union of 0.26 M nodes in blocks of 16,384
+// groups, 190 medium an iteration, 51.8 -> 55.5.
 constexpr long long kMedMinAll = 1 << 16;
 
 __host__ __device__ __forceinline__ bool MediumFits(int g, unsigned entries) {

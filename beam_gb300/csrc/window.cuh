@@ -22,8 +22,8 @@
 // launches, 75 to 120 us, latency only). Rounds follow each other without the
 // host, which watches the frontier through mapped memory and keeps a few
 // rounds queued. Measured with 64-group blocks, 20 iterations, a block at a time
-// -> windows: R-MAT 16 (edge factor 8) 609 -> 119 ms, R-MAT 12 36.7 -> 13.9 ms,
-// Chung-Lu of 20,000 nodes with twins 108 -> 50 ms.
+// -> windows: R-MAT 16 (edge factor 8) 609 -> 116 ms, R-MAT 12 36.7 -> 13.8 ms,
+// Chung-Lu of 20,000 nodes with twins 108 -> 49 ms.
 #pragma once
 
 // Blocks of at most this many groups go through windows; larger ones fill the
@@ -39,7 +39,11 @@ constexpr int kWindowMinAgain = 64;
 // Tables of a round's big groups take at most this much memory, unless one block
 // needs more by itself: an iteration whose tables are beyond it in all goes
 // through windows of fewer groups (WindowSpanKernel). 4.5 KB a node in groups of
-// 500 members, 9 KB at 1,024, else limit the graphs that fit.
+// 500 members, 9 KB at 1,024, else limit the graphs that fit. Runs with the limit
+// at one block / 64 MB / 256 MB / 1 GB / 4 GB / none: 2 M nodes in groups of 500,
+// two iterations, 1070 / 228 / 146 / 121 / 133 / 138 ms; R-MAT 20 (edge factor
+// 16), two iterations, 1153 / 267 / 112 / 111 / 110 / 111; R-MAT 22 with groups of
+// up to 1,024, one iteration, 2434 / 861 / 476 / 390 / 387 / 384.
 constexpr long long kWindowTables = 4ll << 30;
 constexpr int kWindowLengths = 14;  // kWindowMaxGroups, halved down to 1 (then to the block's end)
 static_assert(kWindowMaxGroups >> (kWindowLengths - 1) == 1, "the last length is one block");
@@ -72,7 +76,9 @@ constexpr int kPartEntries = 1024;
 constexpr int kMaxParts = 128;
 constexpr int kPairWarps = 4;
 constexpr int kPairDeep = 4;  // entries per lane in flight
-constexpr int kPairCtas = 5;  // per SM: what shared memory holds (42 KB of tables each)
+// Per SM: what shared memory holds (42 KB of tables each). With a grid of six,
+// a sixth of the work is a second wave: R-MAT 16 118.7 ms, 116.0 with five.
+constexpr int kPairCtas = 5;
 constexpr int kPairGrid = 152 * kPairCtas;
 
 __host__ __device__ __forceinline__ int WindowParts(unsigned entries) {
