@@ -399,6 +399,7 @@ class Engine {
   DevBuf<long long> d_big_moff_;
   DevBuf<int> d_real_;
   std::vector<long long> h_cand_off_, h_sel_off_, h_mat_off_;
+  bool members_repeat_ = false;  // the planned group lists a supernode twice (PrepareGroup)
   std::vector<BlockPlan> plans_;  // this iteration's blocks
   // sums of a block's start state that the exact gains are made from: per row,
   // and per candidate slot

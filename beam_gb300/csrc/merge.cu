@@ -4199,7 +4199,8 @@ void Engine::PrepareIterationBuffers() {
   long long max_mat = 0;
   for (size_t ri = 0; ri < R; ++ri) {
     const long long g = h_glen_[static_cast<size_t>(h_real_[ri])];
-    h_cand_off_[ri + 1] = h_cand_off_[ri] + std::min(g * (g - 1) / 2, g * k);
+    // (a member listed twice ties with itself, and more than k partners are kept)
+    h_cand_off_[ri + 1] = h_cand_off_[ri] + (members_repeat_ ? g * (g - 1) / 2 : std::min(g * (g - 1) / 2, g * k));
     h_sel_off_[ri + 1] = h_sel_off_[ri] + g / 2;
   }
   // groups of at most kSmallGroup members whose rows fit the staging buffer
@@ -5161,9 +5162,10 @@ int64_t Engine::PrepareGroup(const int32_t* q, int g, int32_t* a_idx, int32_t* b
     CheckCuda(cudaMemcpyAsync(lens.data(), d_qlen_.p, sizeof(int) * static_cast<size_t>(n_), cudaMemcpyDeviceToHost,
                               stream_), "d2h row lengths");
     CheckCuda(cudaStreamSynchronize(stream_), "sync");
-    unsigned e = 0;
-    for (int i = 0; i < g; ++i) e += static_cast<unsigned>(lens[static_cast<size_t>(hq[static_cast<size_t>(i)])]);
-    h_gent_.assign(1, e);
+    int64_t e = 0;
+    for (int i = 0; i < g; ++i) e += lens[static_cast<size_t>(hq[static_cast<size_t>(i)])];
+    if (e > INT32_MAX) throw std::invalid_argument("group row entries exceed the supported maximum");
+    h_gent_.assign(1, static_cast<unsigned>(e));
   }
   const int zero = 0;
   CheckCuda(cudaMemcpyAsync(d_order_.p, hq.data(), sizeof(int) * static_cast<size_t>(g), cudaMemcpyHostToDevice,
@@ -5184,7 +5186,11 @@ int64_t Engine::PrepareGroup(const int32_t* q, int g, int32_t* a_idx, int32_t* b
             "h2d");
   ++launches_;
   ScatterGroupKernel<<<(g + 255) / 256, 256, 0, stream_>>>(dq.p, di.p, g, d_group_of_.p, d_idx_in_group_.p);
+  std::vector<int> sorted(hq);
+  std::sort(sorted.begin(), sorted.end());
+  members_repeat_ = std::adjacent_find(sorted.begin(), sorted.end()) != sorted.end();
   PrepareIterationBuffers();
+  members_repeat_ = false;
   CheckCuda(cudaMemsetAsync(d_ctl_.p, 0, sizeof(BlockCtl), stream_), "memset ctl");
   LaunchPrepare(plans_.at(0));
   int cnt = 0;
